@@ -19,6 +19,7 @@
 
 #include "memd_internal.h"
 #include "memd_kernels.cuh"
+#include "memd_mean_fix.cuh"
 #include "memd_tc.cuh"
 
 namespace memd {
@@ -63,7 +64,7 @@ struct memd_plan {
     int GS, ngroups;
     int evalG, evalSPT, evalT;  // FP64 evaluation tile
     int ewG, ewSPL;             // FP32 / mixed evaluation tile
-    int cum, cumG;              // mixed fixed mode: impulse-accumulation mean, channels per lane group
+    int cum, cumG;              // impulse-accumulation mean (FP64 and mixed forms, fixed mode), channels per lane group
     int bpass;                  // (sift, chunk) passes enqueued so far in the decomposition being built
     size_t proj_smem;
     void* X;
@@ -78,8 +79,10 @@ struct memd_plan {
     void* dbuf;  // forward-eliminated right-hand sides [2][Kc][cap][C]
     void* fac;
     void* rtab;
-    void* rtab3;  // impulse-accumulation mean: 1/(3h) as double-float
-    unsigned* bnd;  // impulse-accumulation mean: [2 passes][2 parts][C] per-channel bounds (float bits)
+    void* rtab3;  // impulse-accumulation mean: 1/(3h) as double-float / in FP64
+    unsigned* xexp;            // impulse-accumulation mean, FP64: largest exponent [records][C] of the run's input
+    unsigned long long* tot;   // the same, several passes: knots per record over all directions
+    unsigned* bnd;  // impulse-accumulation mean, mixed form: [2 passes][2 parts][C] per-channel bounds (float bits)
     int* cumcfg;    // impulse-accumulation mean: anchor span (words) and CTAs per span, set by the factor kernel
     // batched runs (cfg.max_epochs > 0): epochs concatenated at multiples of
     // kEpochAlign samples; ep describes the current call's layout (n = 0: one record)
@@ -270,6 +273,19 @@ static void launch_eval(memd_plan* p, cudaStream_t s, int k0, int kc, int first,
     using XT = typename Prec<P>::X;
     const Geom& g = p->g;
     if constexpr (P == MEMD_PREC_F64) {
+        if (p->cum) {
+            const dim3 grid((unsigned)g.W, (unsigned)((g.C + p->cumG - 1) / p->cumG));
+#define MEMD_CASE(G_)                                                                                              \
+    if (p->cumG == G_) {                                                                                           \
+        k_mean_fix<G_><<<grid, 256, fix_smem_bytes(G_), s>>>(                                                      \
+            (const double*)p->X, (double*)p->Xb, (ulonglong2*)p->acc, p->bits, p->wpref, p->knots, p->cnt,         \
+            (const double*)p->rtab, (const double*)p->rtab3, (const double*)p->sv, (const double*)p->yend,         \
+            p->xexp, p->nchunks > 1 ? p->tot : nullptr, g, k0, kc, first, last, p->st, p->ep);                      \
+        return;                                                                                                    \
+    }
+            MEMD_CASE(32) MEMD_CASE(16) MEMD_CASE(8)
+#undef MEMD_CASE
+        }
 #define MEMD_CASE(G_, S_)                                                                                  \
     if (p->evalG == G_ && p->evalSPT == S_) {                                                              \
         using Sh = EvalShape<R, G_, S_>;                                                                   \
@@ -337,6 +353,8 @@ static cudaError_t set_attrs(memd_plan* p)
                                  (int)EvalShape<R, G_, S_>::smem_bytes(p->Kc, p->g.mirror));
         MEMD_EVAL_CASES(MEMD_CASE)
 #undef MEMD_CASE
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(k_mean_fix<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fix_smem_bytes(32));
     } else {
 #define MEMD_CASE(G_, S_)                                                                                     \
     if (p->ewG == G_ && p->ewSPL == S_) {                                                                     \
@@ -382,6 +400,25 @@ static void enqueue_sift(memd_plan* p, cudaStream_t s, memd_trace_entry* trace, 
     const Geom& g = p->g;
     const bool stop = p->cfg.stop_mode == MEMD_STOP_CRITERION;
     const int trace_rows = stop && trace ? (int)(p->cfg.num_imfs * (p->cfg.max_iter + 1)) : 0;
+    if constexpr (P == MEMD_PREC_F64) {
+        if (p->cum && p->nchunks > 1) {
+            // several passes: the knots of all directions first, which set the
+            // mean's anchor spacing, so that it does not depend on the passes
+            cudaMemsetAsync(p->tot, 0, sizeof(unsigned long long) * (size_t)std::max(1, p->ep.n), s);
+            for (int ch = 0; ch < p->nchunks; ++ch) {
+                const int k0 = ch * p->Kc, kc = std::min(p->Kc, g.K - k0);
+                lc.begin(MEMD_STAGE_PROJECT);
+                k_project_extrema<R, XT><<<dim3((unsigned)((g.L + kProjTN - 1) / kProjTN),
+                                                (unsigned)((kc + kProjTK - 1) / kProjTK)), 256, p->proj_smem, s>>>(
+                    (const XT*)p->X, (const R*)p->dir, p->bits, g, k0, kc, p->ep);
+                lc.end(MEMD_STAGE_PROJECT);
+                lc.begin(MEMD_STAGE_COMPACT);
+                k_count_knots<<<dim3((unsigned)((g.W + 4095) / 4096), (unsigned)(2 * kc)), 256, 0, s>>>(p->bits, p->tot,
+                                                                                                       g, p->ep);
+                lc.end(MEMD_STAGE_COMPACT);
+            }
+        }
+    }
     for (int ch = 0; ch < p->nchunks; ++ch) {
         const int k0 = ch * p->Kc;
         const int kc = std::min(p->Kc, g.K - k0);
@@ -438,16 +475,16 @@ static void enqueue_sift(memd_plan* p, cudaStream_t s, memd_trace_entry* trace, 
         if (g.nak)
             k_factor<R, true><<<(unsigned)((nf + 127) / 128), 128, 0, s>>>(p->knots, p->cnt, (const R*)p->rtab,
                                                                        (Fac<R>*)p->fac, g, k0, kc, p->Sf, p->Hf,
-                                                                       p->cum ? p->cumcfg : nullptr, p->ep, p->cum_ctas);
+                                                                       p->cumcfg, p->ep, p->cum_ctas);
         else
             k_factor<R, false><<<(unsigned)((nf + 127) / 128), 128, 0, s>>>(p->knots, p->cnt, (const R*)p->rtab,
                                                                         (Fac<R>*)p->fac, g, k0, kc, p->Sf, p->Hf,
-                                                                        p->cum ? p->cumcfg : nullptr, p->ep, p->cum_ctas);
+                                                                        p->cumcfg, p->ep, p->cum_ctas);
         lc.end(MEMD_STAGE_FACTOR);
         const long nseg = solve_segments_max(g.cap, p->S, p->Ss, p->H);
         const long ns = 2L * kc * nseg * p->ngroups * 32;
         const unsigned nb = (unsigned)((ns + kSolveThreads - 1) / kSolveThreads);
-        unsigned* bcur = p->cum ? p->bnd + (size_t)(p->bpass & 1) * 2 * g.C : nullptr;
+        unsigned* bcur = p->bnd ? p->bnd + (size_t)(p->bpass & 1) * 2 * g.C : nullptr;
         SolveQueue q{};  // null prefix: the static mapping
         if (p->squeue) {
             q = p->sq;
@@ -464,7 +501,7 @@ static void enqueue_sift(memd_plan* p, cudaStream_t s, memd_trace_entry* trace, 
         (const R*)p->yv, p->cnt, (const Fac<R>*)p->fac, (R*)p->dbuf, g, k0, kc, p->S, p->Ss, p->H, p->ngroups, \
         bcur, XM_ ? (const XT*)p->X : nullptr, p->knots, XM_ ? (const R*)p->yend : nullptr, p->ep,               \
         p->inplace ? (R*)p->hz : nullptr, p->hsegs, q)
-        if constexpr (P == MEMD_PREC_MIXED) {
+        if constexpr (P != MEMD_PREC_F32) {
             if (p->cum) {  // knot values from the working signal (the impulse-accumulation path)
                 xm = true;
                 if (p->ep.n > 0) {  // batched runs: record ends found by position
@@ -564,7 +601,7 @@ static void enqueue_decomposition(memd_plan* p, cudaStream_t s, Launches& lc)
     dim3 tb(32, 8), tg((unsigned)((g.L + 31) / 32), (unsigned)((g.C + 31) / 32));
     p->bpass = 0;
     void* const x0 = p->X;
-    if (p->cum) cudaMemsetAsync(p->bnd, 0, sizeof(unsigned) * 4 * (size_t)g.C, s);
+    if (p->bnd) cudaMemsetAsync(p->bnd, 0, sizeof(unsigned) * 4 * (size_t)g.C, s);
     for (int i = 0; i + 1 < nimf; ++i) {
         nvtxRangePushA("imf");
         cudaMemcpyAsync(p->X, p->run, CL * sizeof(XT), cudaMemcpyDeviceToDevice, s);
@@ -749,8 +786,9 @@ static void enqueue_inputs(memd_plan* p, const typename Prec<P>::T* d_y, const t
     using T = typename Prec<P>::T;
     const Geom& g = p->g;
     dim3 tb(32, 8), tg((unsigned)((g.L + 31) / 32), (unsigned)((g.C + 31) / 32));
+    if (p->xexp) cudaMemsetAsync(p->xexp, 0, sizeof(unsigned) * (size_t)g.C, s);
     lc.begin(MEMD_STAGE_OTHER);
-    k_to_sample_major<XT, T><<<tg, tb, 0, s>>>(d_y, (XT*)p->run, g.C, g.L);
+    k_to_sample_major<XT, T><<<tg, tb, 0, s>>>(d_y, (XT*)p->run, g.C, g.L, p->xexp);
     lc.end(MEMD_STAGE_OTHER);
     cudaMemcpyAsync(p->dir, d_dir, sizeof(T) * (size_t)g.K * g.C, cudaMemcpyDeviceToDevice, s);
     if constexpr (P == MEMD_PREC_MIXED) {  // float directions: the low words are zero
@@ -905,8 +943,9 @@ static memd_status batched_inputs(memd_plan* p, int n, const int64_t* lengths, c
     cudaMemsetAsync(p->run, 0, CL * sizeof(XT), s);
     cudaMemsetAsync(p->X, 0, CL * sizeof(XT), s);
     if (p->Xb) cudaMemsetAsync(p->Xb, 0, CL * sizeof(XT), s);
-    k_batched_in<XT, T><<<dim3((unsigned)g.W, (unsigned)((C + 31) / 32)), dim3(32, 8), 0, s>>>(d_y, p->ep_yoff, (XT*)p->run,
-                                                                                              C, p->ep);
+    if (p->xexp) cudaMemsetAsync(p->xexp, 0, sizeof(unsigned) * (size_t)n * C, s);
+    k_batched_in<XT, T><<<dim3((unsigned)g.W, (unsigned)((C + 31) / 32)), dim3(32, 8), 0, s>>>(
+        d_y, p->ep_yoff, (XT*)p->run, C, p->ep, p->xexp);
     cudaMemcpyAsync(p->dir, d_dir, sizeof(T) * (size_t)g.K * C, cudaMemcpyDeviceToDevice, s);
     if constexpr (P == MEMD_PREC_MIXED) {
         cudaMemsetAsync((float*)p->dir + (size_t)g.K * C, 0, sizeof(float) * (size_t)g.K * C, s);
@@ -1249,7 +1288,7 @@ static memd_status create_plan(const memd_config* cfg, const memd_tuning* tun, m
         // automatic: as many directions per pass as the free memory allows,
         // with separate right-hand-side and solution arrays while all of them
         // fit (the faster layout), solving in place when that fits more
-        const bool cum_cfg = c.precision == MEMD_PREC_MIXED && c.stop_mode == MEMD_STOP_FIXED &&
+        const bool cum_cfg = c.precision != MEMD_PREC_F32 && c.stop_mode == MEMD_STOP_FIXED &&
                              c.boundary == MEMD_BOUNDARY_REFERENCE && c.mean_eval != 1;
         const int want = std::min(K, kc_limit);
         const int fit_sep = directions_that_fit(c, p->g, p->real_bytes, p->xbytes, p->tbytes, cum_cfg, false);
@@ -1261,7 +1300,7 @@ static memd_status create_plan(const memd_config* cfg, const memd_tuning* tun, m
             want_inplace = fit_inp > fit_sep;
         }
     } else if (c.dir_chunk <= 0) {  // layout fixed by the tuning: the directions that fit with it
-        const bool cum_cfg = c.precision == MEMD_PREC_MIXED && c.stop_mode == MEMD_STOP_FIXED &&
+        const bool cum_cfg = c.precision != MEMD_PREC_F32 && c.stop_mode == MEMD_STOP_FIXED &&
                              c.boundary == MEMD_BOUNDARY_REFERENCE && c.mean_eval != 1;
         const int fit = directions_that_fit(c, p->g, p->real_bytes, p->xbytes, p->tbytes, cum_cfg, want_inplace);
         p->Kc = std::max(1, std::min({K, fit, kc_limit}));
@@ -1308,8 +1347,9 @@ static memd_status create_plan(const memd_config* cfg, const memd_tuning* tun, m
         p->ewSPL = 32;
     }
     p->egroups = (C + (f64 ? p->evalG : p->ewG) - 1) / (f64 ? p->evalG : p->ewG);
-    // mean envelope: impulse accumulation for the mixed form in fixed mode
-    // (mean_eval 0 = automatic, 1 = direct evaluation, 2 = impulse accumulation)
+    // mean envelope: impulse accumulation for the FP64 and mixed forms in fixed
+    // mode (mean_eval 0 = automatic, 1 = direct evaluation, 2 = impulse
+    // accumulation, mixed form only)
     if (c.mean_eval < 0 || c.mean_eval > 2) {
         delete p;
         return set_error(MEMD_ERR_INVALID, "plan: mean_eval must be 0, 1 or 2");
@@ -1321,7 +1361,8 @@ static memd_status create_plan(const memd_config* cfg, const memd_tuning* tun, m
         return set_error(MEMD_ERR_UNSUPPORTED,
                          "plan: impulse-accumulation mean needs the mixed form in fixed mode with the reference boundary");
     }
-    p->cum = cum_ok && c.mean_eval != 1;
+    p->cum = (cum_ok || (f64 && c.stop_mode == MEMD_STOP_FIXED && c.boundary == MEMD_BOUNDARY_REFERENCE)) &&
+             c.mean_eval != 1;
     p->cumG = C >= 32 ? 32 : (C > 8 ? 16 : 8);
     const size_t rb = (size_t)p->real_bytes;
     if (c.precision == MEMD_PREC_MIXED)
@@ -1339,7 +1380,7 @@ static memd_status create_plan(const memd_config* cfg, const memd_tuning* tun, m
     if (p->cum) ALLOC(p->Xb, (size_t)p->xbytes * CL);
     ALLOC(p->run, (size_t)p->xbytes * CL);
     ALLOC(p->dir, 8 * (size_t)K * C);
-    if (p->nchunks > 1) ALLOC(p->acc, rb * CL);
+    if (p->nchunks > 1) ALLOC(p->acc, (p->cum && f64 ? 16 : rb) * CL);  // FP64: the exact 128-bit sum
     ALLOC(p->imf, (size_t)p->tbytes * CL * (size_t)c.num_imfs);
     ALLOC(p->bits, sizeof(uint32_t) * 2 * Kc * p->g.W);
     ALLOC(p->wpref, sizeof(int) * 2 * Kc * (p->g.W + 1));
@@ -1365,8 +1406,11 @@ static memd_status create_plan(const memd_config* cfg, const memd_tuning* tun, m
     // longest knot gap: a record (epoch) length; mirrored knots reach 2L - 2
     const int Lh = p->batched ? std::max(p->Lrec, kEpochAlign) : (p->g.mirror ? 2 * L : L);
     ALLOC(p->rtab, rb * (size_t)(Lh + 1));
-    if (p->cum) {
-        ALLOC(p->rtab3, sizeof(dd) * (size_t)(Lh + 1));
+    if (p->cum) ALLOC(p->rtab3, 8 * (size_t)(Lh + 1));
+    if (p->cum && f64) {
+        ALLOC(p->xexp, sizeof(unsigned) * (size_t)std::max<int64_t>(1, c.max_epochs) * C);
+        if (p->nchunks > 1) ALLOC(p->tot, sizeof(unsigned long long) * (size_t)std::max<int64_t>(1, c.max_epochs));
+    } else if (p->cum) {
         ALLOC(p->bnd, sizeof(unsigned) * 4 * (size_t)C);
         ALLOC(p->cumcfg, sizeof(int) * 4);
         ALLOC(p->cumsh.kq, sizeof(unsigned long long) * 35 * (size_t)p->g.W * C);
@@ -1446,7 +1490,8 @@ static memd_status create_plan(const memd_config* cfg, const memd_tuning* tun, m
         if (e == cudaSuccess) e = cudaMalloc((void**)&r32, sizeof(float) * (size_t)(Lh + 1));
         if (e == cudaSuccess) e = cudaMalloc((void**)&rdd, sizeof(dd) * (size_t)(Lh + 1));
         if (e == cudaSuccess) {
-            k_fill_reciprocals<<<256, 256>>>(r64, r32, rdd, (dd*)p->rtab3, Lh + 1);
+            k_fill_reciprocals<<<256, 256>>>(r64, r32, rdd, f64 ? nullptr : (dd*)p->rtab3, f64 ? (double*)p->rtab3 : nullptr,
+                                             Lh + 1);
             const void* src = f64 ? (void*)r64 : (c.precision == MEMD_PREC_MIXED ? (void*)rdd : (void*)r32);
             e = cudaMemcpy(p->rtab, src, rb * (size_t)(Lh + 1), cudaMemcpyDeviceToDevice);
         }
@@ -1456,7 +1501,7 @@ static memd_status create_plan(const memd_config* cfg, const memd_tuning* tun, m
     }
     if (e == cudaSuccess) e = cudaMemset(p->csh.hacc, 0, sizeof(unsigned long long) * 2 * (size_t)p->Kc);
     if (e == cudaSuccess) e = cudaMemset(p->csh.arrive, 0, sizeof(int) * 2 * (size_t)p->Kc);
-    if (e == cudaSuccess && p->cum) {
+    if (e == cudaSuccess && p->cum && !f64) {
         e = cudaMemset(p->cumsh.kq, 0, sizeof(unsigned long long) * 35 * (size_t)p->g.W * C);
         if (e == cudaSuccess) e = cudaMemset(p->cumsh.anc, 0, sizeof(unsigned long long) * 4 * (size_t)p->g.W * C);
         if (e == cudaSuccess) e = cudaMemset(p->cumsh.arrive, 0, sizeof(int) * (size_t)p->g.W * ((C + 7) / 8));

@@ -17,6 +17,8 @@
 //                      in windows of S knots with an H-knot halo (REF:1227-1241)
 //   k_mean_cum         mixed form, fixed mode: the mean envelope rebuilt from
 //                      per-knot impulses and per-word anchors (REF:775-864)
+//   k_mean_fix         the same for the FP64 form, in wide fixed point
+//                      (memd_mean_fix.cuh)
 //   k_eval             spline coefficients per interval, envelope evaluation
 //                      fused with the mean over directions and the update of
 //                      the working signal (REF:775-864)
@@ -2723,15 +2725,32 @@ __global__ void k_zero_unused_b(real* __restrict__ imf, const RecStop* __restric
 // Layout transforms and IMF bookkeeping (REF:1174, 1178, 1328-1338).
 // 32 x 32 tiles through shared memory; block (32, 8).
 // ---------------------------------------------------------------------------
-// run[n][c] = (real) y[c][n]
+// Raises *xexp (nullptr: none) to the largest biased exponent of the warp's
+// finite values v; 0 only if all are zero (subnormals count as 1).
+__device__ __forceinline__ void raise_exponent(unsigned* xexp, double v)
+{
+    if (!xexp) return;  // uniform
+    unsigned e = (unsigned)((unsigned long long)__double_as_longlong(v) >> 52) & 0x7ffu;
+    if (e == 0x7ffu) e = 0u;
+    else if (e == 0u && v != 0.0) e = 1u;
+    e = __reduce_max_sync(kFull, e);
+    if ((threadIdx.x & 31) == 0 && e > *(volatile unsigned*)xexp) atomicMax(xexp, e);
+}
+
+// run[n][c] = (real) y[c][n]; xexp (optional, zero before): the largest biased
+// FP64 exponent of each channel
 template <typename XT, typename tin>
-__global__ void k_to_sample_major(const tin* __restrict__ y, XT* __restrict__ run, int C, int L)
+__global__ void k_to_sample_major(const tin* __restrict__ y, XT* __restrict__ run, int C, int L,
+                                  unsigned* __restrict__ xexp)
 {
     __shared__ XT tile[32][33];
     const int n_base = blockIdx.x * 32, c_base = blockIdx.y * 32;
     for (int r = threadIdx.y; r < 32; r += 8) {
         const int c = c_base + r, n = n_base + threadIdx.x;
-        if (c < C && n < L) tile[r][threadIdx.x] = xfrom<XT>(y[(size_t)c * L + n]);
+        const bool in = c < C && n < L;
+        if (in) tile[r][threadIdx.x] = xfrom<XT>(y[(size_t)c * L + n]);
+        if constexpr (std::is_same<XT, double>::value)
+            raise_exponent(xexp && c < C ? xexp + c : nullptr, in ? tile[r][threadIdx.x] : 0.0);
     }
     __syncthreads();
     for (int r = threadIdx.y; r < 32; r += 8) {
@@ -2746,7 +2765,7 @@ __global__ void k_to_sample_major(const tin* __restrict__ y, XT* __restrict__ ru
 // are (zeroed by the caller).
 template <typename XT, typename tin>
 __global__ void k_batched_in(const tin* __restrict__ y, const long long* __restrict__ yoff, XT* __restrict__ run,
-                             int C, Epochs ep)
+                             int C, Epochs ep, unsigned* __restrict__ xexp)
 {
     __shared__ XT tile[32][33];
     const int w = blockIdx.x;
@@ -2757,7 +2776,10 @@ __global__ void k_batched_in(const tin* __restrict__ y, const long long* __restr
     const tin* ye = y + yoff[e];
     for (int r = threadIdx.y; r < 32; r += 8) {
         const int c = c_base + r, t = t_base + threadIdx.x;
-        if (c < C && t < Le) tile[r][threadIdx.x] = xfrom<XT>(ye[(size_t)c * Le + t]);
+        const bool in = c < C && t < Le;
+        if (in) tile[r][threadIdx.x] = xfrom<XT>(ye[(size_t)c * Le + t]);
+        if constexpr (std::is_same<XT, double>::value)  // [epoch][channel]
+            raise_exponent(xexp && c < C ? xexp + (size_t)e * C + c : nullptr, in ? tile[r][threadIdx.x] : 0.0);
     }
     __syncthreads();
     for (int r = threadIdx.y; r < 32; r += 8) {
@@ -2815,15 +2837,16 @@ __global__ void k_check_coords(const int32_t* __restrict__ x, int L, int* __rest
 }
 
 __global__ void k_fill_reciprocals(double* __restrict__ r64, float* __restrict__ r32, dd* __restrict__ rdd,
-                                   dd* __restrict__ r3dd, int n)
+                                   dd* __restrict__ r3dd, double* __restrict__ r3_64, int n)
 {
-    // r3dd (optional): 1/(3h) as a double-float
+    // r3dd, r3_64 (optional): 1/(3h) as a double-float / in FP64
     for (int h = blockIdx.x * blockDim.x + threadIdx.x; h < n; h += gridDim.x * blockDim.x) {
         const double r = h > 0 ? __ddiv_rn(1.0, (double)h) : 0.0;
         r64[h] = r;
         r32[h] = h > 0 ? __fdiv_rn(1.0f, (float)h) : 0.0f;
         rdd[h] = dd(r);
         if (r3dd) r3dd[h] = h > 0 ? dd(__ddiv_rn(1.0, 3.0 * (double)h)) : dd(0.0f, 0.0f);
+        if (r3_64) r3_64[h] = h > 0 ? __ddiv_rn(1.0, 3.0 * (double)h) : 0.0;
     }
 }
 

@@ -1,0 +1,437 @@
+// memd_mean_fix.cuh -- mean envelope of the FP64 form by impulse accumulation
+// in wide fixed point (fixed number of sifts, reference boundary).
+#pragma once
+
+#include "memd_kernels.cuh"
+
+namespace memd {
+
+// The reference evaluates every envelope at every sample (REF:795-864): four
+// FP64 operations per direction, envelope, channel and sample, on a pipe that
+// issues two lanes per clock and SM (1.25 TFLOP/s, 1/63 of the FP32 rate).
+// Here, as in the mixed form's mean (k_mean_cum), the mean is rebuilt from
+// what happens at the knots: between an anchor sample and its neighbours the
+// sum of all envelopes is one cubic, whose third-order coefficient jumps by
+// d_j - d_{j-1} at every knot x_j.  FP64 operations are left at the knots
+// (two) and at the anchors (thirteen) only; every sum is an integer sum.
+//
+// Fixed point: values are integers in units of 2^-sh, 2^-sh = 2^(ex - 85) with
+// 2^ex > max|x| over the record's channel (k_to_sample_major, k_batched_in),
+// held as two words, v = hi 2^52 + lo with 0 <= lo < 2^52.  An FP64 value keeps all its
+// bits down to 2^-33 of the channel's largest sample and 2^-85 of it below
+// that; sums over at most 2048 (direction, envelope) pairs stay inside both
+// words, and the exact sums make the result independent of the order, of the
+// direction chunks and of the batch a record is in.
+//
+// Anchors: every T samples, T the power of two in [8, 64] with T <= 2 h (h:
+// the record's mean knot spacing over all directions; 8 at the densest
+// knots).  Rounding in a piece's coefficients grows with the distance from
+// the anchor, at most T/2, about one knot spacing.  Error of the mean against
+// a long double evaluation, relative to the signal (3 channels, 32
+// directions, EEG-shaped; direct FP64 evaluation 1.5e-16 in an IMF's first
+// sift, 2.3e-17 .. 4.2e-17 in its last; the update's own rounding ~4e-17):
+// T = 8 at h = 3.7 / 2.8: 3.8e-17 / 6.2e-17; T = 8 at h = 7.0 / 5.2: 3.4e-17 /
+// 3.5e-17; T = 16 at h = 13 / 10: 2.9e-17 / 5.0e-17; twice the span, 2x .. 3x
+// the error.
+//
+// Measured (FP64 form, all sifts of a decomposition, against the direct
+// evaluation k_eval, which is 82% busy on the FP64 pipe): 32 x 30,504, 64
+// directions, 80 sifts: 117.6 -> 29.6 ms of the mean, 163.4 -> 70.2 ms in all;
+// 12 epochs x 32 channels: 279 -> 53.5 ms, 363 -> 127 ms; error of the IMFs
+// against a separate FP64 evaluation 8.2e-16 -> 3.9e-16.
+//
+// A span whose values leave the fixed-point range (non-finite values, or
+// splines that overshoot the signal thousands of times), and a channel so
+// small that its third-order coefficients would be subnormal, is evaluated
+// directly, pair by pair in direction order, with k_eval's arithmetic.
+struct FixSum {
+    unsigned long long hi, lo;
+};
+constexpr unsigned long long kFixLo = (1ull << 52) - 1ull;
+constexpr int kFixBits = 85;   // units per 2^ex: 2^85
+constexpr unsigned kFixMinExp = 128;  // smallest biased exponent of a channel's maximum (0: an all-zero channel)
+constexpr int kFixRows = 64;   // longest span
+constexpr int kFixAnchors = 4; // anchors of a span: 32 / 8
+
+// v 2^sh rounded to nearest; false when |v 2^sh| could reach 2^lim (or v is
+// not finite).  Integer instructions only: FP64 <-> integer conversions run on
+// the FP64 pipe.
+__device__ __forceinline__ bool to_fix(double v, int sh, int lim, FixSum& r)
+{
+    const long long b = __double_as_longlong(v);
+    const int be = (int)((unsigned long long)b >> 52) & 0x7ff;
+    long long m = (b & (long long)kFixLo) | (be ? (1ll << 52) : 0ll);
+    if (b < 0) m = -m;
+    const int s = max(be, 1) - 1075 + sh;  // value = m 2^s units
+    if (s >= 0) {
+        r.hi = (unsigned long long)(s < 52 ? m >> (52 - s) : m << min(s - 52, 63));
+        r.lo = s < 52 ? ((unsigned long long)m << s) & kFixLo : 0ull;
+    } else {
+        const int q = min(-s, 62);
+        const long long n = (m + (1ll << (q - 1))) >> q;
+        r.hi = (unsigned long long)(n >> 52);
+        r.lo = (unsigned long long)n & kFixLo;
+    }
+    return be != 0x7ff && (s <= lim - 53 || m == 0);
+}
+
+// the 128-bit two's-complement integer n times 2^-sh, rounded to nearest even
+__device__ __forceinline__ double from_fix(__int128 n, int sh)
+{
+    if (n == 0) return 0.0;
+    const bool neg = n < 0;
+    const unsigned __int128 a = neg ? -(unsigned __int128)n : (unsigned __int128)n;
+    const unsigned long long ah = (unsigned long long)(a >> 64), al = (unsigned long long)a;
+    const int lz = ah ? __clzll((long long)ah) : 64 + __clzll((long long)al);
+    const unsigned __int128 t = a << lz;  // leading bit at 127
+    unsigned long long top = (unsigned long long)(t >> 75);  // 53 bits
+    const unsigned long long rest = (unsigned long long)(t >> 11);  // the 64 bits below, sticky from the last 11
+    const bool sticky = ((unsigned long long)t & 0x7ffull) != 0ull;
+    const unsigned long long half = 1ull << 63;
+    if (rest > half || (rest == half && (sticky || (top & 1ull)))) ++top;  // 2^53: the exponent absorbs the carry
+    const int be = 127 - lz - sh + 1023;
+    double v;
+    if (be >= 1 && be <= 2045) v = __longlong_as_double((long long)(((unsigned long long)be << 52) + (top - (1ull << 52))));
+    else v = ldexp((double)top, 127 - lz - sh - 52);
+    return neg ? -v : v;
+}
+
+// accumulator of several direction passes: the exact sum, or (kFixTag in the
+// top bits, which a sum below 2^116 cannot have) the FP64 sum of a span that
+// was evaluated directly
+constexpr unsigned long long kFixTag = 0x5a5ull << 52;
+__device__ __forceinline__ bool fix_tagged(ulonglong2 v) { return (v.y & (0xfffull << 52)) == kFixTag; }
+
+// 2^ex > max|x|: ex from the largest biased exponent of the channel's samples
+__device__ __forceinline__ int fix_shift(unsigned be) { return kFixBits - ((int)be - 1022); }
+
+// CTA: one span (32 samples, 64 where T = 64) x G channels, 8 warps; lane =
+// (subgroup, channel); the (direction, envelope) pairs are dealt round-robin
+// to the 8 * 32/G subgroups, which walk the span's pieces in order.
+// Bound by the FP64 pipe at dense knots, by load latency at sparse ones.
+template <int G>
+__global__ void __launch_bounds__(256, 3)
+k_mean_fix(const double* __restrict__ X, double* __restrict__ Xout, ulonglong2* __restrict__ acc_buf,
+           const uint32_t* __restrict__ bits, const int* __restrict__ wpref, const int* __restrict__ knots,
+           const int* __restrict__ cnt, const double* __restrict__ rtab, const double* __restrict__ rtab3,
+           const double* __restrict__ sv, const double* __restrict__ yend, const unsigned* __restrict__ xexp,
+           const unsigned long long* __restrict__ tot, Geom g, int k0, int Kc, int first_chunk, int last_chunk,
+           RunState* st, Epochs ep)
+{
+    constexpr int SUB = 32 / G;
+    constexpr int NWS = 8 * SUB;
+    constexpr int NE = 256;  // pairs described per round
+    extern __shared__ __align__(16) unsigned long long kq_hi[];  // [kFixRows][G] jumps at row x - p0, high words
+    unsigned long long* kq_lo = kq_hi + kFixRows * G;            // low words
+    unsigned long long* an_hi = kq_lo + kFixRows * G;            // [kFixAnchors][4][G] Taylor coefficients at the anchors
+    unsigned long long* an_lo = an_hi + kFixAnchors * 4 * G;
+    __shared__ int eJ[NE], eE[NE];  // first piece of the span (-1: the pair does not count); last piece of the record
+    __shared__ int sQ, sT;
+    __shared__ unsigned sBad;  // channels of the span to evaluate directly
+    __shared__ unsigned long long sEt;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int cc = lane % G, sub = lane / G;
+    const int C = g.C;
+    const int w = blockIdx.x;
+    const int rec = ep.n > 0 ? ep.wep[w] : 0;
+    const int roff = ep.n > 0 ? ep.off[rec] : 0;
+    const int rend = ep.n > 0 ? roff + ep.len[rec] : g.L;
+    const int p0 = w * 32;
+    if (p0 >= rend) return;  // gap between epochs; uniform over the CTA
+    if (threadIdx.x == 0) {
+        sQ = 0;
+        sBad = 0u;
+        sEt = 0ull;
+    }
+    __syncthreads();
+    {
+        // qualified directions, and the knots of all of them (spans of several
+        // passes: counted beforehand, so that T does not depend on the passes)
+        int q = 0;
+        unsigned long long et = 0ull;
+        for (int k = threadIdx.x; k < g.K; k += blockDim.x) {
+            const int a = ep.n > 0 ? ep.cnt[(size_t)k * ep.n + rec] : cnt[k];
+            const int b = ep.n > 0 ? ep.cnt[((size_t)g.K + k) * ep.n + rec] : cnt[g.K + k];
+            q += (a > 3 && b > 3) ? 1 : 0;
+            et += (unsigned long long)(a + b);
+        }
+        q = warp_sum(q);
+        et = warp_sum(et);
+        if (lane == 0) {
+            if (q) atomicAdd(&sQ, q);
+            if (et) atomicAdd(&sEt, et);
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const unsigned long long et = tot ? tot[rec] : sEt;
+        const unsigned long long lk = (unsigned long long)(rend - roff) * 2ull * (unsigned long long)g.K;
+        int t = 8;  // T <= 2 h, h = lk / et
+        while (t < kFixRows && (unsigned long long)(2 * t) * et <= 2ull * lk) t *= 2;
+        sT = t;
+    }
+    __syncthreads();
+    const int T = sT;
+    const int mw = T > 32 ? 2 : 1;
+    if (mw == 2 && (((p0 - roff) >> 5) & 1)) return;  // covered by the word before; uniform over the CTA
+    const int nl = min(32 * mw, rend - p0);
+    const int nA = (nl + T - 1) / T;
+    const int c = blockIdx.y * G + cc;
+    const bool cok = c < C;
+    const int cl = min(c, C - 1);  // loads of lanes past the last channel stay in bounds
+    for (int i = threadIdx.x; i < nl * G; i += blockDim.x) {
+        kq_hi[i] = 0ull;
+        kq_lo[i] = 0ull;
+    }
+    for (int i = threadIdx.x; i < nA * 4 * G; i += blockDim.x) {
+        an_hi[i] = 0ull;
+        an_lo[i] = 0ull;
+    }
+    const unsigned xe = xexp[(size_t)rec * C + cl];
+    const int sh = fix_shift(xe);
+    // the sum of the 2K envelopes stays below 2^115: A, B T/2, C (T/2)^2 and
+    // d (T/2)^3 of each below 2^lim
+    const int lim = 108 - (32 - __clz(2 * g.K - 1));
+    const int lt = 30 - __clz(T);  // log2(T / 2)
+    bool ok = xe == 0u || xe >= kFixMinExp;
+    const int rlast = rend - 1;
+
+    for (int base = 0; base < 2 * Kc; base += NE) {
+        __syncthreads();
+        {
+            // (1) per pair: the piece holding sample p0 and the record's last piece
+            const int ei = base + (int)threadIdx.x;
+            int j = -1, je = 0;
+            if (ei < 2 * Kc) {
+                const int kk = ei >> 1, env = ei & 1, k = k0 + kk;
+                const int Ex = cnt[k], En = cnt[g.K + k];
+                if (Ex <= g.cap && En <= g.cap && dir_qualifies(g, ep, cnt, k, rec)) {
+                    const size_t slot = (size_t)env * Kc + kk;
+                    const int* wp = wpref + slot * (g.W + 1);
+                    const int kb = ep.n > 0 ? wp[ep.w0[rec]] : 0;
+                    je = (ep.n > 0 ? wp[ep.w0[rec + 1]] : (env ? En : Ex)) - 2;
+                    const int at = wp[w] + (int)(bits[slot * g.W + w] & 1u);  // knots at or before p0
+                    j = min(max(at - 1, kb), je);
+                }
+            }
+            if (threadIdx.x < NE) {
+                eJ[threadIdx.x] = j;
+                eE[threadIdx.x] = je;
+            }
+        }
+        __syncthreads();
+        const int nround = min(NE, 2 * Kc - base);
+        for (int le = warp * SUB + sub; le < nround; le += NWS) {
+            int j = eJ[le];
+            if (j < 0) continue;
+            const int je = eE[le];
+            const int kk = (base + le) >> 1, env = (base + le) & 1;
+            const size_t slot = (size_t)env * Kc + kk;
+            const int* kn = knots + slot * g.cap;
+            const double* sp = sv + slot * (size_t)g.cap * C + cl;
+            const double* ye = yend + (slot * (ep.n > 0 ? ep.n : 1) + rec) * 2 * (size_t)C + cl;
+            // (2) the pieces of the span in order: the jump of d at each interior
+            //     knot past p0, the Taylor coefficients at each anchor
+            int xj = kn[j], xn = kn[j + 1];
+            double s0 = sp[(size_t)j * C], s1 = sp[(size_t)(j + 1) * C];
+            FixSum qp{0ull, 0ull};
+            int a = 0, na = p0 + min(T >> 1, nl - 1);
+            bool jump = false;  // x_j is past p0 (the first piece's knot is not)
+            for (;;) {
+                const bool more = j < je && xn < p0 + nl;  // another piece begins in the span
+                int x2 = 0;
+                double s2 = 0.0;
+                if (more) {
+                    x2 = kn[j + 2];
+                    s2 = sp[(size_t)(j + 2) * C];
+                }
+                const int h = xn - xj;
+                const double d = __dmul_rn(__dsub_rn(s1, s0), rtab3[h]);
+                FixSum qc;
+                ok &= to_fix(d, sh, lim - 3 * lt, qc);
+                if (jump && MEMD_CHECK(xj - p0 > 0 && xj - p0 < nl)) {
+                    atomicAdd(&kq_hi[(xj - p0) * G + cc], qc.hi - qp.hi);
+                    atomicAdd(&kq_lo[(xj - p0) * G + cc], qc.lo - qp.lo);
+                }
+                qp = qc;
+                while (a < nA && (na < xn || j == je)) {
+                    // S(na + t) = A + B t + C t^2 + d t^3 on this piece
+                    const double y0 = (xj == roff) ? ye[0] : X[(size_t)xj * C + cl];
+                    const double y1 = (xn == rlast) ? ye[C] : X[(size_t)xn * C + cl];
+                    const double u = (double)(na - xj), u3 = (double)(3 * (na - xj));
+                    const double h3 = __dmul_rn((double)h, 1.0 / 3.0);
+                    const double b = __fma_rn(-h3, __fma_rn(2.0, s0, s1), __dmul_rn(__dsub_rn(y1, y0), rtab[h]));
+                    const double e = __fma_rn(d, u, s0);
+                    const double cB = __fma_rn(__fma_rn(d, u3, __dadd_rn(s0, s0)), u, b);
+                    FixSum f;
+                    unsigned long long* ah = an_hi + (size_t)(a * 4) * G + cc;
+                    unsigned long long* al = an_lo + (size_t)(a * 4) * G + cc;
+                    ok &= to_fix(__fma_rn(__fma_rn(e, u, b), u, y0), sh, lim, f);
+                    atomicAdd(ah, f.hi);
+                    atomicAdd(al, f.lo);
+                    ok &= to_fix(cB, sh, lim - lt, f);
+                    atomicAdd(ah + G, f.hi);
+                    atomicAdd(al + G, f.lo);
+                    ok &= to_fix(__fma_rn(d, u3, s0), sh, lim - 2 * lt, f);
+                    atomicAdd(ah + 2 * G, f.hi);
+                    atomicAdd(al + 2 * G, f.lo);
+                    atomicAdd(ah + 3 * G, qc.hi);
+                    atomicAdd(al + 3 * G, qc.lo);
+                    ++a;
+                    na = p0 + a * T + min(T >> 1, nl - 1 - a * T);
+                }
+                if (!more) break;
+                ++j;
+                xj = xn;
+                xn = x2;
+                s0 = s1;
+                s1 = s2;
+                jump = true;
+            }
+        }
+    }
+    if (!ok) atomicOr(&sBad, 1u << cc);
+    __syncthreads();
+    const int Q = sQ;
+    if (last_chunk && Q == 0 && blockIdx.y == 0 && threadIdx.x == 0) atomicOr(&st->flags, 1);
+    if (!cok) return;
+    const double qd = (double)Q, rq = Q > 0 ? __ddiv_rn(1.0, qd) : __longlong_as_double(0x7ff8000000000000ll);
+    const bool bad = (sBad >> cc) & 1u;
+    // M's sum at row r is done: X -= M / 2 / Q, or on to the next pass
+    auto emit = [&](int r, __int128 v, double vd) {
+        const size_t off = (size_t)(p0 + r) * C + c;
+        bool isd = bad;
+        if (!first_chunk) {
+            const ulonglong2 o = acc_buf[off];
+            if (fix_tagged(o) || isd) {
+                const double od = fix_tagged(o) ? __longlong_as_double((long long)o.x)
+                                                : from_fix((__int128)(((unsigned __int128)o.y << 64) | o.x), sh);
+                vd = __dadd_rn(od, isd ? vd : from_fix(v, sh));
+                isd = true;
+            } else {
+                v += (__int128)(((unsigned __int128)o.y << 64) | o.x);
+            }
+        }
+        if (last_chunk) {
+            // (sum / 2) / Q rounded as a division: quotient by the reciprocal,
+            // one correction by the remainder
+            const double val = __dmul_rn(isd ? vd : from_fix(v, sh), 0.5);
+            double m;
+            if (isd) {
+                m = __ddiv_rn(val, qd);
+            } else {
+                const double q0 = __dmul_rn(val, rq);
+                m = __fma_rn(__fma_rn(-q0, qd, val), rq, q0);
+            }
+            Xout[off] = __dsub_rn(X[off], m);
+        } else {
+            ulonglong2 o;
+            if (isd) {
+                o.x = (unsigned long long)__double_as_longlong(vd);
+                o.y = kFixTag;
+            } else {
+                o.x = (unsigned long long)v;
+                o.y = (unsigned long long)((unsigned __int128)v >> 64);
+            }
+            acc_buf[off] = o;
+        }
+    };
+    auto wide = [](unsigned long long hi, unsigned long long lo) -> __int128 {
+        return ((__int128)(long long)hi << 52) + (__int128)(long long)lo;
+    };
+    // (3) every half of an anchor's T samples is one item: forwards from the
+    //     anchor, or backwards, the cubic's coefficients carried from sample
+    //     to sample and d changed at every knot
+    for (int it = warp * SUB + sub; it < 2 * nA; it += NWS) {
+        const int a = it >> 1, q0 = a * T;
+        const int q1 = min(nl, q0 + T);
+        const int ra = q0 + min(T >> 1, nl - 1 - q0);
+        const int rb = (it & 1) ? q0 : ra, re = (it & 1) ? ra : q1;  // rows [rb, re)
+        if (!bad) {
+            const unsigned long long* ah = an_hi + (size_t)(a * 4) * G + cc;
+            const unsigned long long* al = an_lo + (size_t)(a * 4) * G + cc;
+            __int128 vA = wide(ah[0], al[0]), vB = wide(ah[G], al[G]), vC = wide(ah[2 * G], al[2 * G]),
+                     vD = wide(ah[3 * G], al[3 * G]);
+            if (!(it & 1)) {
+                for (int r = rb;;) {
+                    emit(r, vA, 0.0);
+                    if (++r >= re) break;
+                    vA += vB + vC + vD;
+                    vB += 2 * vC + 3 * vD;
+                    vC += 3 * vD;
+                    vD += wide(kq_hi[r * G + cc], kq_lo[r * G + cc]);
+                }
+            } else {
+                for (int r = re; r > rb; --r) {
+                    vD -= wide(kq_hi[r * G + cc], kq_lo[r * G + cc]);
+                    vA += vC - vB - vD;
+                    vB += 3 * vD - 2 * vC;
+                    vC -= 3 * vD;
+                    emit(r - 1, vA, 0.0);
+                }
+            }
+        } else {
+            for (int r = rb; r < re; ++r) {
+                const int n = p0 + r;
+                double sum = 0.0;
+                for (int kk = 0; kk < Kc; ++kk) {
+                    const int k = k0 + kk;
+                    if (cnt[k] > g.cap || cnt[g.K + k] > g.cap || !dir_qualifies(g, ep, cnt, k, rec)) continue;
+                    double v[2];
+                    for (int env = 0; env < 2; ++env) {
+                        const size_t slot = (size_t)env * Kc + kk;
+                        const int* wp = wpref + slot * (g.W + 1);
+                        const int kb = ep.n > 0 ? wp[ep.w0[rec]] : 0;
+                        const int wn = n >> 5;
+                        const int before = wp[wn] + __popc(bits[slot * g.W + wn] & ((1u << (n & 31)) - 1u));
+                        const int i = max(before - 1, kb);
+                        const int* kn = knots + slot * g.cap;
+                        const double* sp = sv + slot * (size_t)g.cap * C + c;
+                        const double* ye = yend + (slot * (ep.n > 0 ? ep.n : 1) + rec) * 2 * (size_t)C + c;
+                        const int xi = kn[i], xn = kn[i + 1];
+                        const double y0 = (xi == roff) ? ye[0] : X[(size_t)xi * C + c];
+                        const double y1 = (xn == rlast) ? ye[C] : X[(size_t)xn * C + c];
+                        const double s0 = sp[(size_t)i * C], s1 = sp[(size_t)(i + 1) * C];
+                        const double t = (double)(n - xi);
+                        const double h3 = __dmul_rn((double)(xn - xi), 1.0 / 3.0);
+                        const double b = __fma_rn(-h3, __fma_rn(2.0, s0, s1), __dmul_rn(__dsub_rn(y1, y0), rtab[xn - xi]));
+                        const double d = __dmul_rn(__dsub_rn(s1, s0), __dmul_rn(rtab[xn - xi], 1.0 / 3.0));
+                        v[env] = __fma_rn(__fma_rn(__fma_rn(d, t, s0), t, b), t, y0);
+                    }
+                    sum = __dadd_rn(sum, __dadd_rn(v[0], v[1]));
+                }
+                emit(r, 0, sum);
+            }
+        }
+    }
+}
+
+// Knots per record over all directions of a pass, added to tot[record] (runs
+// of several direction passes, before the passes): one CTA per (slot, 4096
+// words).
+__global__ void __launch_bounds__(256)
+k_count_knots(const uint32_t* __restrict__ bits, unsigned long long* __restrict__ tot, Geom g, Epochs ep)
+{
+    const uint32_t* b = bits + (size_t)blockIdx.y * g.W;
+    const int w0 = blockIdx.x * 4096, w1 = min(g.W, w0 + 4096);
+    unsigned long long n = 0ull;
+    for (int w = w0 + (int)threadIdx.x; w < w1; w += blockDim.x) {
+        const int p = __popc(b[w]);
+        if (ep.n > 0) {
+            if (p) atomicAdd(&tot[ep.wep[w]], (unsigned long long)p);
+        } else {
+            n += (unsigned long long)p;
+        }
+    }
+    if (ep.n == 0) {
+        n = warp_sum(n);
+        if ((threadIdx.x & 31) == 0 && n) atomicAdd(&tot[0], n);
+    }
+}
+
+inline size_t fix_smem_bytes(int G)
+{
+    return sizeof(unsigned long long) * 2 * (size_t)G * (kFixRows + 4 * kFixAnchors);
+}
+
+}  // namespace memd
