@@ -1264,15 +1264,21 @@ static memd_status create_plan(const memd_config* cfg, const memd_tuning* tun, m
         // halo lengths: the truncation error decays by <= 1/2 (solve) and
         // <= 1/12 (pivots: u l / (2 (l + u) - l cp)^2 with cp <= 1/2) per
         // knot; FP64 and double-float need ~1e-15 (double-float pivots: 16
-        // rows, 12^-16 = 5e-18)
+        // rows, 12^-16 = 5e-18).  FP64 pivots: 24 rows, eight past the point
+        // where the start error is below half an ulp, so that the rounded
+        // pivots are the exact recurrence's as well (bit for bit in the
+        // windowed-solve test).  Segments of 16 rows: the recurrence is
+        // latency-bound, ~600 ns a row in FP64, once the knots are sparse
+        // (k_factor<double>, 32 x 30,504, 64 directions, segments of 64 + 40
+        // rows, divisions and integer conversions on the FP64 pipe -> 16 + 24
+        // rows, without them: 98.7 -> 51.9 us at IMF 1, 70.1 -> 25.5 us at IMF 8)
         const bool wide = f64 || c.precision == MEMD_PREC_MIXED;
         p->S = tu.solve_segment ? tu.solve_segment : 256;
         p->Ss = tu.solve_min_segment ? tu.solve_min_segment : std::min(64, p->S);
         p->H = c.solve_window > 0 ? (int)c.solve_window : (f64 ? 48 : (wide ? 32 : 24));
-        // short factorisation segments (the pivot recurrence is latency-bound),
-        // except for FP64, whose longer halo would dominate
-        p->Sf = tu.factor_segment ? tu.factor_segment : (f64 ? 64 : 16);
-        p->Hf = f64 ? 40 : (wide ? 16 : 20);
+        // short factorisation segments (the pivot recurrence is latency-bound)
+        p->Sf = tu.factor_segment ? tu.factor_segment : 16;
+        p->Hf = f64 ? 24 : (wide ? 16 : 20);
     }
     // in place (when memory limits the directions per pass): the solution
     // overwrites the eliminated right-hand side row by row (same warp, read

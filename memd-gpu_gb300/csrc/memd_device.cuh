@@ -336,17 +336,44 @@ __device__ __forceinline__ dd sqrt_(dd a) { return dd_sqrt(a); }
 __device__ __forceinline__ double fmat_(double a, float t, double c) { return __fma_rn(a, (double)t, c); }
 __device__ __forceinline__ float fmat_(float a, float t, float c) { return __fmaf_rn(a, t, c); }
 __device__ __forceinline__ dd fmat_(dd a, float t, dd c) { return dd_mulf(a, t) + c; }
-// 1/a: IEEE division for double and float (the FP64 and FP32 forms keep the
-// reference's arithmetic); for a double-float, the correctly rounded float
+// 1/a: IEEE division for float (the FP32 form keeps the reference's
+// arithmetic); for double within 0.501 ulp; for a double-float, the correctly rounded float
 // reciprocal refined by one Newton step with an fma residual (~47 bits, a
 // quarter of the instructions of the double-float division)
-__device__ __forceinline__ double recip_(double a) { return __ddiv_rn(1.0, a); }
+__device__ __forceinline__ double recip_(double a)
+{
+    // a in float's normal range (pivots of integer spacings): the float
+    // reciprocal x of a's leading 24 bits, moved between the formats by integer
+    // instructions, and one third-order step x + x (e + e^2), e = 1 - a x
+    // (|e| < 2^-21: e^3 is below the last place by 2^-10).  Three FP64
+    // operations on the pivots' serial chain, on a pipe that takes 64 cycles a
+    // warp instruction.
+    const unsigned h = (unsigned)__double2hiint(a), l = (unsigned)__double2loint(a);
+    const float x0 = __frcp_rn(__uint_as_float((h & 0x80000000u) | ((((h & 0x7fffffffu) - ((1023u - 127u) << 20)) << 3) | (l >> 29))));
+    const unsigned b = __float_as_uint(x0);
+    const double x = __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + ((1023u - 127u) << 20))), (int)(b << 29));
+    const double e = __fma_rn(-a, x, 1.0);
+    return __fma_rn(x, __fma_rn(e, e, e), x);
+}
 __device__ __forceinline__ float recip_(float a) { return __fdiv_rn(1.0f, a); }
 __device__ __forceinline__ dd recip_(dd a)
 {
     const float x0 = __frcp_rn(a.hi);
     const float e = __fmaf_rn(-a.lo, x0, __fmaf_rn(-a.hi, x0, 1.0f));  // 1 - a x0
     return dd_renorm(x0, __fmul_rn(x0, e));
+}
+// an integer in the arithmetic type; for double by integer instructions (the
+// conversion instruction runs on the FP64 pipe, like an FP64 operation)
+template <typename real>
+__device__ __forceinline__ real from_int(int n) { return real(n); }
+template <>
+__device__ __forceinline__ double from_int<double>(int n)
+{
+    const unsigned a = (unsigned)(n < 0 ? -n : n);
+    const int z = __clz((int)a);  // 32 for 0
+    const unsigned m = a << (z & 31);
+    const unsigned hi = (unsigned)(1023 + 31 - z) * (1u << 20) + ((m & 0x7fffffffu) >> 11);
+    return __hiloint2double((int)(a ? hi | ((unsigned)n & 0x80000000u) : 0u), (int)(a ? m << 21 : 0u));
 }
 // identity rows of the factorisation (natural end conditions, record ends)
 // carry m = 1 exactly; every other row has m <= 1/3 (pivot >= 3)

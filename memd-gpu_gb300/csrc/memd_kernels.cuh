@@ -509,15 +509,15 @@ k_factor(const int* __restrict__ knots, const int* __restrict__ cnt, const real*
         for (int k = 0; k < FB; ++k) {
             const int i = base + k;
             if (FULL || i < i1) {
-                const real l = real(li[k]);
-                const real gp = fmad_(-l, cp, real(di[k]));
+                const real l = from_int<real>(li[k]);
+                const real gp = fmad_(-l, cp, from_int<real>(di[k]));
                 const real m = recip_(gp);
-                cp = mul_(real(ui[k]), m);
+                cp = mul_(from_int<real>(ui[k]), m);
                 if (FULL || i >= i0) {
                     Fac<real> o;
                     o.m = m;
                     if constexpr (NAK) {
-                        if (wd[k] > 0) o.m = mul_(m, div_(real(wn[k]), real(wd[k])));
+                        if (wd[k] > 0) o.m = mul_(m, div_(from_int<real>(wn[k]), from_int<real>(wd[k])));
                     }
                     o.lm = mul_(l, m);
                     o.cp = cp;
