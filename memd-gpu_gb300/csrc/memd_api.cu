@@ -291,7 +291,7 @@ static void launch_eval(memd_plan* p, cudaStream_t s, int k0, int kc, int first,
         using Sh = EvalShape<R, G_, S_>;                                                                   \
         dim3 grid((unsigned)((g.L + Sh::T - 1) / Sh::T), (unsigned)((g.C + G_ - 1) / G_));                 \
         k_eval<R, G_, S_><<<grid, 256, Sh::smem_bytes(p->Kc, g.mirror), s>>>(                             \
-            (R*)p->X, (R*)p->acc, p->bits, p->wpref, p->knots, p->cnt, (const Fac<R>*)p->fac,            \
+            (R*)p->X, (R*)p->acc, p->bits, p->wpref, p->knots, p->cnt, (const R*)p->rtab,                 \
             (const R*)p->sv, (const R*)p->yv, g, k0, kc, first, last, p->st, (R*)p->M, (R*)p->part, p->ep, \
             p->mir);                                                                                       \
         return;                                                                                            \

@@ -140,9 +140,17 @@ template <> __device__ __forceinline__ float2 xfrom<float2>(float2 v) { return v
 //   ih = 1 / (x_{i+1} - x_i)  (0 for the last row); for the double-float
 //   form 3 / (x_{i+1} - x_i), the factor 3 of the right-hand side
 //   3 (slope_i - slope_{i-1}) folded in.
+// FP64: the right-hand side's factors folded into the row instead,
+//   m 3 (slope_i - slope_{i-1}) = a (y_{i+1} - y_i) - b (y_i - y_{i-1}),
+// so that a row of the forward sweep is four FP64 operations (a = b = 0 in
+// the identity rows of record ends).
 template <typename real>
 struct alignas(4 * sizeof(real)) Fac {
     real m, lm, cp, ih;
+};
+template <>
+struct alignas(32) Fac<double> {
+    double a, b, lm, cp;
 };
 template <typename real>
 constexpr bool kFacIh3 = false;

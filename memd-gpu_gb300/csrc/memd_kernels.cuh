@@ -440,6 +440,8 @@ k_factor(const int* __restrict__ knots, const int* __restrict__ cnt, const real*
     real cp = real(0);
     int xl = js > 0 ? x[js - 1] : 0;
     int xi = x[js];
+    [[maybe_unused]] real rl = real(0);  // FP64: 1 / (spacing to the left) of the next row
+    if constexpr (std::is_same<real, double>::value) rl = js > 0 ? rtab[xi - xl] : real(0);
     constexpr int FB = 8;  // knot positions loaded per batch (independent loads)
     // FULL (compile-time): all FB rows are owned (>= i0, < i1) and have a right
     // neighbour, so no row needs a guard
@@ -513,7 +515,21 @@ k_factor(const int* __restrict__ knots, const int* __restrict__ cnt, const real*
                 const real gp = fmad_(-l, cp, from_int<real>(di[k]));
                 const real m = recip_(gp);
                 cp = mul_(from_int<real>(ui[k]), m);
-                if (FULL || i >= i0) {
+                if constexpr (std::is_same<real, double>::value) {
+                    if (FULL || i >= i0) {
+                        Fac<double> o;
+                        double m3 = di[k] == 1 ? 0.0 : __dmul_rn(3.0, m);  // 1: an identity row
+                        if constexpr (NAK) {
+                            if (wd[k] > 0) m3 = __dmul_rn(m3, __ddiv_rn(from_int<double>(wn[k]), from_int<double>(wd[k])));
+                        }
+                        o.a = __dmul_rn(m3, rt[k]);
+                        o.b = __dmul_rn(m3, rl);
+                        o.lm = __dmul_rn(l, m);
+                        o.cp = cp;
+                        f[i] = o;
+                    }
+                    rl = rt[k];
+                } else if (FULL || i >= i0) {
                     Fac<real> o;
                     o.m = m;
                     if constexpr (NAK) {
@@ -790,8 +806,13 @@ k_solve_fwd(const real* __restrict__ yv, const int* __restrict__ cnt, const Fac<
     real* o = dbuf + slot * (size_t)g.cap * C + cl;
     const int is = (H < 0) ? 0 : max(0, i0 - H);
     real yi = yrow(is);
+    // FP64: the knot values' difference to the left instead of its slope
+    constexpr bool F64 = std::is_same<real, double>::value;
     real slope_prev = real(0);
-    if (is > 0) slope_prev = mul_(sub_(yi, yrow(is - 1)), f[is - 1].ih);
+    if (is > 0) {
+        slope_prev = sub_(yi, yrow(is - 1));
+        if constexpr (!F64) slope_prev = mul_(slope_prev, f[is - 1].ih);
+    }
     real dprev = real(0);
     float ymax = 0.0f;
     // one batch of B rows; FULL (a compile-time flag): all B rows are owned
@@ -806,9 +827,14 @@ k_solve_fwd(const real* __restrict__ yv, const int* __restrict__ cnt, const Fac<
         int fx = 0, ffl = 0, fe = 0;
         if (lane < nb) {
             const Fac<real> fr = MEMD_CHECK(base + lane < g.cap) ? f[base + lane] : Fac<real>{};
-            fm = fr.m;
+            if constexpr (F64) {
+                fm = fr.a;
+                fih = fr.b;
+            } else {
+                fm = fr.m;
+                fih = fr.ih;
+            }
             flm = fr.lm;
-            fih = fr.ih;
             if (XM && base + 1 + lane < E) {
                 fx = kn[base + 1 + lane];
                 if (EPB) ffl = endfl(base + 1 + lane, fx, fe);
@@ -850,6 +876,20 @@ k_solve_fwd(const real* __restrict__ yv, const int* __restrict__ cnt, const Fac<
             if (FULL || k < nb) {
                 const int i = base + k;
                 const real ynext = yb[k];
+                if constexpr (F64) {
+                    // d_i = (a dy_i - b dy_{i-1}) - lm d_{i-1}: one operation on the
+                    // serial chain; identity rows (a = 0) are 0
+                    const real dy = (FULL || i < E - 1) ? sub_(ynext, yi) : real(0);
+                    const real rhs = is_zero(m) ? real(0) : fmad_(m, dy, -mul_(ih, slope_prev));
+                    const real dcur = fmad_(-lm, dprev, rhs);
+                    if (FULL || i >= i0) {
+                        if (cok && MEMD_CHECK(i >= 0 && i < g.cap)) o[(size_t)i * C] = dcur;
+                    }
+                    slope_prev = dy;
+                    yi = ynext;
+                    dprev = dcur;
+                    continue;
+                }
                 real slope = real(0), r = real(0);
                 if (FULL || i < E - 1) slope = mul_(sub_(ynext, yi), ih);
                 // identity rows (record ends) have lm = 0 and m = 1; a not-a-knot
@@ -881,7 +921,7 @@ k_solve_fwd(const real* __restrict__ yv, const int* __restrict__ cnt, const Fac<
             else batch(std::false_type{}, std::false_type{}, base);
         }
     }
-    if (bnd && cok) {
+    if (!F64 && bnd && cok) {
         if (i1 < E) ymax = fmaxf(ymax, magf(yi));  // right end of the last piece
         atomicMax(&bnd[it.c], __float_as_uint(ymax * 1.01f));
     }
@@ -911,6 +951,7 @@ k_solve_bwd(const int* __restrict__ cnt, const Fac<real>* __restrict__ fac, cons
     // warp that owns row E-3 (its window always reaches row E-1, and row E-2
     // does not depend on s_{E-1}), which also writes row E-1.
     constexpr int B = kSolveBatch;
+    constexpr bool F64 = std::is_same<real, double>::value;  // no bounds (bnd is null)
     SolveItem it;
     bool first = true;
     while (solve_next(it, first, 1, q, cnt, g, k0, Kc, S, Ss, H, ngroups)) {
@@ -941,7 +982,7 @@ k_solve_bwd(const int* __restrict__ cnt, const Fac<real>* __restrict__ fac, cons
         if (lane < nb) {
             const Fac<real> fr = MEMD_CHECK(top - lane >= 0 && top - lane < g.cap) ? f[top - lane] : Fac<real>{};
             fcp = fr.cp;
-            fih = fr.ih;
+            if constexpr (!F64) fih = fr.ih;
         }
         real db[B];
 #pragma unroll
@@ -951,7 +992,8 @@ k_solve_bwd(const int* __restrict__ cnt, const Fac<real>* __restrict__ fac, cons
                         : real(0);
 #pragma unroll
         for (int k = 0; k < B; ++k) {
-            const real cp = shfl_idx_(fcp, k), ihr = shfl_idx_(fih, k);
+            const real cp = shfl_idx_(fcp, k);
+            [[maybe_unused]] const real ihr = F64 ? real(0) : shfl_idx_(fih, k);
             if (FULL || k < nb) {
                 const int i = top - k;
                 real sol = fmad_(-cp, snext, db[k]);
@@ -961,7 +1003,7 @@ k_solve_bwd(const int* __restrict__ cnt, const Fac<real>* __restrict__ fac, cons
                 }
                 if (FULL || i < i1) {
                     if (cok && !(NAK && nak && i == E - 1) && MEMD_CHECK(i >= 0 && i < g.cap)) o[(size_t)i * C] = sol;
-                    if (bnd && (FULL || i < E - 1)) {
+                    if (!F64 && bnd && (FULL || i < E - 1)) {
                         // h^2 = 1 / ih^2 (9 / ih^2 when ih holds 3/h); the approximate
                         // division's error is inside the 1.01 margin applied at the end
                         const float ih = magf(ihr);
@@ -973,7 +1015,7 @@ k_solve_bwd(const int* __restrict__ cnt, const Fac<real>* __restrict__ fac, cons
                             const real sl =
                                 add_(snext, div_(mul_(sub_(snext, sol), real(hb)), real(kn[E - 2] - kn[E - 3])));
                             if (cok) o[(size_t)(E - 1) * C] = sl;
-                            if (bnd) spart = fmaxf(spart, 0.25f * (magf(snext) + magf(sl)) * (float)hb * (float)hb);
+                            if (!F64 && bnd) spart = fmaxf(spart, 0.25f * (magf(snext) + magf(sl)) * (float)hb * (float)hb);
                         }
                     }
                 }
@@ -986,7 +1028,7 @@ k_solve_bwd(const int* __restrict__ cnt, const Fac<real>* __restrict__ fac, cons
         if (!NAK && top - B + 1 >= i0 && top < i1 && top < E - 1) batch(std::true_type{}, top);
         else batch(std::false_type{}, top);
     }
-    if (bnd && cok) atomicMax(&bnd[C + it.c], __float_as_uint(spart * 1.01f));
+    if (!F64 && bnd && cok) atomicMax(&bnd[C + it.c], __float_as_uint(spart * 1.01f));
     }  // items
 }
 
@@ -1022,7 +1064,7 @@ k_nak_ends(const int* __restrict__ knots, const int* __restrict__ cnt, const int
     if (en - b < 4) return;
     const int* kn = knots + (size_t)slot * g.cap;
     real* s = sv + (size_t)slot * g.cap * C + c;
-    const Fac<real>* f = fac + (size_t)slot * g.cap;
+    [[maybe_unused]] const Fac<real>* f = fac + (size_t)slot * g.cap;
     const real s1 = s[(size_t)(b + 1) * C], s2 = s[(size_t)(b + 2) * C];
     const real s0 = add_(s1, div_(mul_(sub_(s1, s2), real(kn[b + 1] - kn[b])), real(kn[b + 2] - kn[b + 1])));
     const real sa = s[(size_t)(en - 3) * C], sb = s[(size_t)(en - 2) * C];
@@ -1030,11 +1072,13 @@ k_nak_ends(const int* __restrict__ knots, const int* __restrict__ cnt, const int
     const real sl = add_(sb, div_(mul_(sub_(sb, sa), real(hb)), real(kn[en - 2] - kn[en - 3])));
     s[(size_t)b * C] = s0;
     s[(size_t)(en - 1) * C] = sl;
-    if (bnd) {
-        const float ih = magf(f[b].ih);
-        float v = __fdividef((kFacIh3<real> ? 2.25f : 0.25f) * (magf(s0) + magf(s1)), ih * ih);
-        v = fmaxf(v, 0.25f * (magf(sb) + magf(sl)) * (float)hb * (float)hb);
-        atomicMax(&bnd[C + c], __float_as_uint(v * 1.01f));
+    if constexpr (!std::is_same<real, double>::value) {
+        if (bnd) {
+            const float ih = magf(f[b].ih);
+            float v = __fdividef((kFacIh3<real> ? 2.25f : 0.25f) * (magf(s0) + magf(s1)), ih * ih);
+            v = fmaxf(v, 0.25f * (magf(sb) + magf(sl)) * (float)hb * (float)hb);
+            atomicMax(&bnd[C + c], __float_as_uint(v * 1.01f));
+        }
     }
 }
 
@@ -1085,7 +1129,7 @@ template <typename real, int G, int SPT>
 __global__ void __launch_bounds__(256)
 k_eval(real* __restrict__ X, real* __restrict__ acc_buf, const uint32_t* __restrict__ bits,
        const int* __restrict__ wpref, const int* __restrict__ knots, const int* __restrict__ cnt,
-       const Fac<real>* __restrict__ fac, const real* __restrict__ sv, const real* __restrict__ yv, Geom g,
+       const real* __restrict__ rtab, const real* __restrict__ sv, const real* __restrict__ yv, Geom g,
        int k0, int Kc, int first_chunk, int last_chunk, RunState* st, real* __restrict__ M,
        real* __restrict__ part, Epochs ep, const int* __restrict__ mir)
 {
@@ -1187,13 +1231,12 @@ k_eval(real* __restrict__ X, real* __restrict__ acc_buf, const uint32_t* __restr
                 m = MI - 1;
             }
             const int* kn = knots + slot * g.cap;
-            const Fac<real>* fc = fac + slot * g.cap;
             const real* svs = sv + slot * (size_t)g.cap * C;
             const real* yvs = yv + slot * (size_t)g.cap * C;
             const uint32_t* b = bits + slot * g.W;
             __syncthreads();
             for (int j = threadIdx.x; j <= m; j += blockDim.x) kx[j] = kn[ia + j];
-            for (int j = threadIdx.x; j < m; j += blockDim.x) ihs[j] = fc[ia + j].ih;
+            for (int j = threadIdx.x; j < m; j += blockDim.x) ihs[j] = rtab[kn[ia + j + 1] - kn[ia + j]];
             if (threadIdx.x < T / 32) {
                 const int w = (n0 >> 5) + threadIdx.x;
                 wds[threadIdx.x] = (w < g.W) ? b[w] : 0u;
