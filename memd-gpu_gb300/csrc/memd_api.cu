@@ -62,8 +62,7 @@ struct memd_plan {
     int Kc, nchunks;
     int S, H, Sf, Hf, Ss;  // solve segments (long / short systems) and halo; factor segments and halo
     int GS, ngroups;
-    int evalG, evalSPT, evalT;  // FP64 evaluation tile
-    int ewG, ewSPL;             // FP32 / mixed evaluation tile
+    int ewG, ewSPL, ewW, ewZ;   // evaluation tile: channel lanes, samples per lane, warps, CTAs per tile
     int cum, cumG;              // impulse-accumulation mean (FP64 and mixed forms, fixed mode), channels per lane group
     int bpass;                  // (sift, chunk) passes enqueued so far in the decomposition being built
     size_t proj_smem;
@@ -261,10 +260,25 @@ struct Launches {
 };
 
 // ----- evaluation kernels ---------------------------------------------------
-#define MEMD_EVAL_CASES(X_)                                                                \
-    X_(4, 2) X_(4, 4) X_(4, 8) X_(8, 2) X_(8, 4) X_(8, 8) X_(16, 2) X_(16, 4) X_(16, 8) \
-    X_(32, 4) X_(32, 8)
-#define MEMD_EVALW_CASES(X_) X_(4, 32) X_(8, 32) X_(16, 32) X_(32, 32) X_(4, 16) X_(8, 16) X_(16, 16)
+// (channel lanes, samples per lane, warps) of k_eval_w, per form
+template <int P, typename F>
+static bool eval_dispatch(int G, int SPL, int W, F f)
+{
+#define MEMD_CASE(G_, S_, W_)                                                                              \
+    if (G == G_ && SPL == S_ && W == W_) {                                                                 \
+        f(std::integral_constant<int, G_>{}, std::integral_constant<int, S_>{}, std::integral_constant<int, W_>{}); \
+        return true;                                                                                       \
+    }
+    if constexpr (P == MEMD_PREC_F32) {
+        MEMD_CASE(4, 32, 8) MEMD_CASE(8, 32, 8) MEMD_CASE(16, 32, 8) MEMD_CASE(32, 32, 8)
+        MEMD_CASE(4, 4, 8) MEMD_CASE(8, 8, 8) MEMD_CASE(16, 16, 8)
+    } else {
+        MEMD_CASE(4, 16, 8) MEMD_CASE(8, 16, 8) MEMD_CASE(16, 16, 8)
+        MEMD_CASE(4, 4, 8) MEMD_CASE(8, 8, 8) MEMD_CASE(4, 4, 16) MEMD_CASE(8, 8, 16) MEMD_CASE(16, 16, 16)
+    }
+#undef MEMD_CASE
+    return false;
+}
 
 template <int P>
 static void launch_eval(memd_plan* p, cudaStream_t s, int k0, int kc, int first, int last)
@@ -286,20 +300,8 @@ static void launch_eval(memd_plan* p, cudaStream_t s, int k0, int kc, int first,
             MEMD_CASE(32) MEMD_CASE(16) MEMD_CASE(8)
 #undef MEMD_CASE
         }
-#define MEMD_CASE(G_, S_)                                                                                  \
-    if (p->evalG == G_ && p->evalSPT == S_) {                                                              \
-        using Sh = EvalShape<R, G_, S_>;                                                                   \
-        dim3 grid((unsigned)((g.L + Sh::T - 1) / Sh::T), (unsigned)((g.C + G_ - 1) / G_));                 \
-        k_eval<R, G_, S_><<<grid, 256, Sh::smem_bytes(p->Kc, g.mirror), s>>>(                             \
-            (R*)p->X, (R*)p->acc, p->bits, p->wpref, p->knots, p->cnt, (const R*)p->rtab,                 \
-            (const R*)p->sv, (const R*)p->yv, g, k0, kc, first, last, p->st, (R*)p->M, (R*)p->part, p->ep, \
-            p->mir);                                                                                       \
-        return;                                                                                            \
     }
-        MEMD_EVAL_CASES(MEMD_CASE)
-#undef MEMD_CASE
-    } else {
-        if constexpr (P == MEMD_PREC_MIXED) {
+    if constexpr (P == MEMD_PREC_MIXED) {
             if (p->cum) {
                 const unsigned* cur = p->bnd + (size_t)(p->bpass & 1) * 2 * g.C;
                 unsigned* other = p->bnd + (size_t)((p->bpass + 1) & 1) * 2 * g.C;
@@ -317,27 +319,33 @@ static void launch_eval(memd_plan* p, cudaStream_t s, int k0, int kc, int first,
                 MEMD_CASE(32) MEMD_CASE(16) MEMD_CASE(8)
 #undef MEMD_CASE
             }
-        }
-        const bool stopm = p->cfg.stop_mode == MEMD_STOP_CRITERION;
-#define MEMD_CASE(G_, S_)                                                                                  \
-    if (p->ewG == G_ && p->ewSPL == S_) {                                                                  \
-        using Sh = EvalWShape<G_, S_, R>;                                                                  \
-        dim3 grid((unsigned)((g.L + Sh::T - 1) / Sh::T), (unsigned)((g.C + G_ - 1) / G_));                 \
-        if (stopm)                                                                                         \
-            k_eval_w<G_, S_, XT, R, true><<<grid, 256, Sh::smem_bytes(true), s>>>(                         \
-                (XT*)p->X, (R*)p->acc, p->bits, p->wpref, p->knots, p->cnt, (const R*)p->rtab,             \
-                (const R*)p->sv, (const R*)p->yv, g, k0, kc, first, last, p->st, (R*)p->M, (R*)p->part,   \
-                p->mir, p->ep);                                                                            \
-        else                                                                                               \
-            k_eval_w<G_, S_, XT, R, false><<<grid, 256, Sh::smem_bytes(false), s>>>(                       \
-                (XT*)p->X, (R*)p->acc, p->bits, p->wpref, p->knots, p->cnt, (const R*)p->rtab,             \
-                (const R*)p->sv, (const R*)p->yv, g, k0, kc, first, last, p->st, nullptr, nullptr, p->mir,  \
-                p->ep);                                                                                    \
-        return;                                                                                            \
     }
-        MEMD_EVALW_CASES(MEMD_CASE)
-#undef MEMD_CASE
-    }
+    const bool stopm = p->cfg.stop_mode == MEMD_STOP_CRITERION;
+    eval_dispatch<P>(p->ewG, p->ewSPL, p->ewW, [&](auto G_, auto S_, auto W_) {
+        constexpr int G = decltype(G_)::value, SPL = decltype(S_)::value, W = decltype(W_)::value;
+        using Sh = EvalWShape<G, SPL, R, W>;
+        const dim3 grid((unsigned)((g.L + Sh::T - 1) / Sh::T), (unsigned)((g.C + G - 1) / G));
+        auto go = [&](auto kern) {
+            cudaLaunchConfig_t lc{};
+            lc.gridDim = dim3(grid.x, grid.y, (unsigned)p->ewZ);
+            lc.blockDim = dim3(32 * W);
+            lc.dynamicSmemBytes = Sh::smem_bytes(stopm);
+            lc.stream = s;
+            cudaLaunchAttribute at[1];
+            at[0].id = cudaLaunchAttributeClusterDimension;
+            at[0].val.clusterDim.x = 1;
+            at[0].val.clusterDim.y = 1;
+            at[0].val.clusterDim.z = (unsigned)p->ewZ;
+            lc.attrs = at;
+            lc.numAttrs = p->ewZ > 1 ? 1 : 0;
+            cudaLaunchKernelEx(&lc, kern, (XT*)p->X, (R*)p->acc, (const uint32_t*)p->bits, (const int*)p->wpref,
+                               (const int*)p->knots, (const int*)p->cnt, (const R*)p->rtab, (const R*)p->sv,
+                               (const R*)p->yv, g, k0, kc, first, last, p->st, stopm ? (R*)p->M : (R*)nullptr,
+                               stopm ? (R*)p->part : (R*)nullptr, (const int*)p->mir, p->ep);
+        };
+        if (stopm) go(k_eval_w<G, SPL, XT, R, true, W>);
+        else go(k_eval_w<G, SPL, XT, R, false, W>);
+    });
 }
 
 template <int P>
@@ -346,28 +354,18 @@ static cudaError_t set_attrs(memd_plan* p)
     using R = typename Prec<P>::R;
     using XT = typename Prec<P>::X;
     cudaError_t e = cudaSuccess;
-    if constexpr (P == MEMD_PREC_F64) {
-#define MEMD_CASE(G_, S_)                                                                              \
-    if (p->evalG == G_ && p->evalSPT == S_)                                                            \
-        e = cudaFuncSetAttribute(k_eval<R, G_, S_>, cudaFuncAttributeMaxDynamicSharedMemorySize,       \
-                                 (int)EvalShape<R, G_, S_>::smem_bytes(p->Kc, p->g.mirror));
-        MEMD_EVAL_CASES(MEMD_CASE)
-#undef MEMD_CASE
+    if constexpr (P == MEMD_PREC_F64)
+        e = cudaFuncSetAttribute(k_mean_fix<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fix_smem_bytes(32));
+    eval_dispatch<P>(p->ewG, p->ewSPL, p->ewW, [&](auto G_, auto S_, auto W_) {
+        constexpr int G = decltype(G_)::value, SPL = decltype(S_)::value, W = decltype(W_)::value;
+        using Sh = EvalWShape<G, SPL, R, W>;
         if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(k_mean_fix<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fix_smem_bytes(32));
-    } else {
-#define MEMD_CASE(G_, S_)                                                                                     \
-    if (p->ewG == G_ && p->ewSPL == S_) {                                                                     \
-        e = cudaFuncSetAttribute(k_eval_w<G_, S_, XT, R, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,  \
-                                 (int)EvalWShape<G_, S_, R>::smem_bytes(true));                               \
-        if (e == cudaSuccess)                                                                                 \
-            e = cudaFuncSetAttribute(k_eval_w<G_, S_, XT, R, false>,                                          \
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize,                             \
-                                     (int)EvalWShape<G_, S_, R>::smem_bytes(false));                          \
-    }
-        MEMD_EVALW_CASES(MEMD_CASE)
-#undef MEMD_CASE
-    }
+            e = cudaFuncSetAttribute(k_eval_w<G, SPL, XT, R, true, W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)Sh::smem_bytes(true));
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(k_eval_w<G, SPL, XT, R, false, W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)Sh::smem_bytes(false));
+    });
     if (e != cudaSuccess) return e;
     if constexpr (P == MEMD_PREC_MIXED) {
         const int cb[3] = {32, 16, 8};
@@ -551,21 +549,22 @@ static void enqueue_sift(memd_plan* p, cudaStream_t s, memd_trace_entry* trace, 
         ++p->bpass;
         if (p->cum && ch == p->nchunks - 1) std::swap(p->X, p->Xb);  // the next pass reads the updated signal
         if (stop) {
+            const bool last = ch == p->nchunks - 1;
+            RecStop* rs = p->batched ? (RecStop*)p->recstop : nullptr;
+            if (rs && last) {  // every record decides for itself
+                lc.begin(MEMD_STAGE_OTHER);
+                k_rec_q<<<(unsigned)p->ep.n, 32, 0, s>>>(rs, g, p->ep);
+                lc.end(MEMD_STAGE_OTHER);
+            }
             lc.begin(MEMD_STAGE_OTHER);
-            k_amp<R><<<(unsigned)((g.L + 255) / 256), 256, 0, s>>>((const R*)p->part, (R*)p->amp, p->cnt, g, k0, kc,
-                                                                 p->egroups, ch == 0, p->ep);
+            k_stop_stats<R><<<(unsigned)g.W, 256, 0, s>>>(
+                (const R*)p->part, (R*)p->amp, (const R*)p->M, p->cnt, g, k0, kc, p->egroups, ch == 0, last,
+                p->cfg.stop_sd, p->cfg.stop_sd2, p->cfg.stop_tol, (int)p->cfg.max_iter, p->st, rs, p->ep, h_sift, p->mir);
             lc.end(MEMD_STAGE_OTHER);
         }
     }
-    if (stop && p->batched) {  // every record decides for itself
+    if (stop && p->batched) {
         RecStop* rs = (RecStop*)p->recstop;
-        lc.begin(MEMD_STAGE_OTHER);
-        k_rec_q<<<(unsigned)p->ep.n, 32, 0, s>>>(rs, g, p->ep);
-        lc.end(MEMD_STAGE_OTHER);
-        lc.begin(MEMD_STAGE_OTHER);
-        k_stop_stats_b<R><<<(unsigned)std::min<long>((g.L + 255) / 256, 1024), 256, 0, s>>>(
-            (const R*)p->M, (const R*)p->amp, rs, g, p->ep, p->cfg.stop_sd, p->cfg.stop_sd2);
-        lc.end(MEMD_STAGE_OTHER);
         lc.begin(MEMD_STAGE_OTHER);
         k_decide_b<<<1, 1024, 0, s>>>(p->st, rs, p->ep, p->cfg.stop_tol, (int)p->cfg.max_iter, h_sift);
         lc.end(MEMD_STAGE_OTHER);
@@ -575,13 +574,6 @@ static void enqueue_sift(memd_plan* p, cudaStream_t s, memd_trace_entry* trace, 
         lc.end(MEMD_STAGE_OTHER);
     } else if (stop) {
         const size_t CL = (size_t)g.C * g.L;
-        lc.begin(MEMD_STAGE_OTHER);
-        k_stop_stats<R><<<(unsigned)std::min<long>((g.L + 255) / 256, 1024), 256, 0, s>>>(
-            (const R*)p->M, (const R*)p->amp, p->cnt, g, p->cfg.stop_sd, p->cfg.stop_sd2, p->st);
-        lc.end(MEMD_STAGE_OTHER);
-        lc.begin(MEMD_STAGE_OTHER);
-        k_decide<<<1, 32, 0, s>>>(p->st, p->cnt, g, p->cfg.stop_tol, (int)p->cfg.max_iter, h_sift, p->mir);
-        lc.end(MEMD_STAGE_OTHER);
         lc.begin(MEMD_STAGE_OTHER);
         k_apply<R, XT><<<(unsigned)std::min<size_t>((CL + 255) / 256, 4096), 256, 0, s>>>((XT*)p->X, (const R*)p->M,
                                                                                          p->st, CL);
@@ -644,7 +636,7 @@ static memd_status build_graph(memd_plan* p)
 }
 
 // Stop mode: the IMF loop and the sift loop are conditional WHILE nodes
-// (the sift loop nested in the IMF loop's body); k_decide and k_imf_commit set
+// (the sift loop nested in the IMF loop's body); k_stop_stats and k_imf_commit set
 // their conditions on the device, so a run needs no host round trip.
 template <int P>
 static memd_status build_graph_stop(memd_plan* p)
@@ -1326,33 +1318,28 @@ static memd_status create_plan(const memd_config* cfg, const memd_tuning* tun, m
                                                    "threads (fewer directions per chunk or longer segments)");
         }
     }
-    // FP64 evaluation tile: G channels x T samples, enough CTAs to fill the GPU
-    p->evalG = std::min(32, std::max(4, next_pow2(C)));
+    // evaluation tile: G channel lanes x SPL samples per lane, in 8 warps; while
+    // tiles of that size leave the GPU idle, 32-sample tiles (SPL = G) and, but
+    // for FP32 (whose sum over the directions keeps its order), a tile's
+    // directions dealt to several CTAs
     {
-        const int NR = 256 / p->evalG;
-        const int groups = (C + p->evalG - 1) / p->evalG;
-        int best = -1, bestT = 0;
-        const int spts[3] = {2, 4, 8};
-        for (int i = 0; i < 3; ++i) {
-            const int T = NR * spts[i];
-            if (T % 32 != 0 || T > 512) continue;
-            const long ctas = (long)((L + T - 1) / T) * groups;
-            if (best < 0) { best = spts[i]; bestT = T; }
-            if (ctas >= 608) { best = spts[i]; bestT = T; }
+        const bool f32 = c.precision == MEMD_PREC_F32;
+        const int gmax = f32 ? 32 : 16, spl = f32 ? 32 : 16;
+        p->ewG = std::min(gmax, std::max(4, next_pow2(C)));
+        const long groups = (C + p->ewG - 1) / p->ewG;
+        p->ewSPL = spl;
+        p->ewW = 8;
+        p->ewZ = 1;
+        if ((L + 32 / p->ewG * spl - 1) / (32 / p->ewG * spl) * groups < 600) {  // about four CTAs of 8 warps per SM
+            p->ewSPL = p->ewG;
+            if (!f32) {
+                const long tiles = (L + 31) / 32 * groups;
+                p->ewZ = tiles < 152 ? 4 : (tiles < 304 ? 2 : 1);
+                p->ewW = p->ewZ == 4 ? 8 : 16;
+            }
         }
-        p->evalSPT = best;
-        p->evalT = bestT;
     }
-    // FP32 evaluation tile: G channel lanes x 32 samples per lane; the
-    // double-float (mixed) tile keeps half the samples per lane in registers
-    if (c.precision == MEMD_PREC_MIXED) {
-        p->ewG = std::min(16, std::max(4, next_pow2(C)));
-        p->ewSPL = 16;
-    } else {
-        p->ewG = p->evalG;
-        p->ewSPL = 32;
-    }
-    p->egroups = (C + (f64 ? p->evalG : p->ewG) - 1) / (f64 ? p->evalG : p->ewG);
+    p->egroups = (C + p->ewG - 1) / p->ewG;
     // mean envelope: impulse accumulation for the FP64 and mixed forms in fixed
     // mode (mean_eval 0 = automatic, 1 = direct evaluation, 2 = impulse
     // accumulation, mixed form only)

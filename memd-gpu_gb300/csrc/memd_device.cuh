@@ -270,6 +270,7 @@ struct RunState {
     unsigned long long over2;  // stop mode: samples with sigma > sd2 in the last pass
     int q;                     // qualified directions of the last pass
     int trace_row;             // stop mode: trace row of the current pass (-1: none)
+    int arrive;                // stop mode: CTAs of the statistics done (zero between launches)
     int pad[4];                // [0] passes over the run, [1] sift loop continues,
                                // [2] IMF loop continues (mirrors of the graph conditions),
                                // [3] extremum tests re-decided in double-float

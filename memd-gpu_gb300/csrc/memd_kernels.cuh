@@ -19,7 +19,7 @@
 //                      per-knot impulses and per-word anchors (REF:775-864)
 //   k_mean_fix         the same for the FP64 form, in wide fixed point
 //                      (memd_mean_fix.cuh)
-//   k_eval             spline coefficients per interval, envelope evaluation
+//   k_eval_w           spline coefficients per interval, envelope evaluation
 //                      fused with the mean over directions and the update of
 //                      the working signal (REF:775-864)
 //
@@ -35,6 +35,8 @@
 // env 0 = maxima (upper envelope), 1 = minima (lower envelope); kk indexes the
 // directions of the current chunk, counts cnt[env][k] use the global k.
 #pragma once
+
+#include <cooperative_groups.h>
 
 #include "memd_device.cuh"
 
@@ -1082,31 +1084,6 @@ k_nak_ends(const int* __restrict__ knots, const int* __restrict__ cnt, const int
     }
 }
 
-// ---------------------------------------------------------------------------
-// Envelope evaluation fused with the mean over directions and the update.
-// CTA: T = (256/G)*SPT samples x G channels; thread (row, ch) owns SPT
-// consecutive samples of one channel and keeps their running sum over the
-// directions in registers.  Per (direction, envelope):
-//   (a) the tile's knots, 1/h and bit words into shared memory,
-//   (b) interval index and offset t per sample; coefficients
-//       a = y_i, b = (y_{i+1}-y_i)/h - h(2 s_i + s_{i+1})/3, c = s_i,
-//       d = (s_{i+1} - s_i)/(3h) per (interval, channel),
-//   (c) S = fma(fma(fma(d, t, c), t, b), t, a) per (sample, channel).
-// The sum over qualified directions (E_max > 3 && E_min > 3) runs in
-// direction order; the last chunk applies X -= (sum/2)/Q (REF:832-864).
-// ---------------------------------------------------------------------------
-template <typename real, int G, int SPT>
-struct EvalShape {
-    static constexpr int NR = 256 / G;
-    static constexpr int T = NR * SPT;
-    static constexpr int MI = T / 2 + 4;
-    static size_t smem_bytes(int Kc, bool mirror)
-    {
-        return sizeof(real) * ((size_t)MI * 4 * G + T + MI) +
-               sizeof(int) * ((size_t)(MI + 1) + T + T / 32 + 8 * Kc + 4 + (mirror ? 10 * Kc : 0));
-    }
-};
-
 // Mirror boundary: knots before sample n among the mirrored ones (positions
 // lp0 <= lp1 left, rp0 <= rp1 right; INT_MAX where absent).  The interval of
 // sample n is (this + interior knots before n) - 1, clamped to [0, E - 2].
@@ -1125,238 +1102,46 @@ __device__ __forceinline__ void mirror_positions(const int* __restrict__ mi, con
     rp1 = nr > 1 ? kn[E - 1] : INT_MAX;
 }
 
-template <typename real, int G, int SPT>
-__global__ void __launch_bounds__(256)
-k_eval(real* __restrict__ X, real* __restrict__ acc_buf, const uint32_t* __restrict__ bits,
-       const int* __restrict__ wpref, const int* __restrict__ knots, const int* __restrict__ cnt,
-       const real* __restrict__ rtab, const real* __restrict__ sv, const real* __restrict__ yv, Geom g,
-       int k0, int Kc, int first_chunk, int last_chunk, RunState* st, real* __restrict__ M,
-       real* __restrict__ part, Epochs ep, const int* __restrict__ mir)
-{
-    // M == nullptr: fixed mode, the last chunk updates X in place.
-    // g.mirror: intervals count the mirrored knots too (mirror_before).
-    // M != nullptr: stop mode, the last chunk writes the mean envelope to M and
-    // every chunk writes part[cg][kk][n] = sum over this CTA's channels of
-    // (U - L)^2 for the amplitude statistic.
-    using Sh = EvalShape<real, G, SPT>;
-    constexpr int T = Sh::T;
-    constexpr int MI = Sh::MI;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    real* coef = reinterpret_cast<real*>(smem_raw);  // [MI][4][G]
-    real* tts = coef + MI * 4 * G;                    // [T]
-    real* ihs = tts + T;                              // [MI]
-    int* kx = reinterpret_cast<int*>(ihs + MI);       // [MI + 1]
-    int* lis = kx + MI + 1;                           // [T]
-    uint32_t* wds = reinterpret_cast<uint32_t*>(lis + T);  // [T/32]
-    int* tab = reinterpret_cast<int*>(wds + T / 32);  // [2*Kc][3]; batched: + [1] + [2*Kc] record knot bases
-    int* sQ = tab + 6 * Kc;
-    int* mtab = tab + 8 * Kc + 4;                      // mirror: [2*Kc][5] lp0, lp1, rp0, rp1, E
-
-    const int n0 = blockIdx.x * T;
-    const int cg = blockIdx.y;
-    const int cc = threadIdx.x % G;
-    const int row = threadIdx.x / G;
-    const int c = cg * G + cc;
-    const bool cok = c < g.C;
-    // the tile's record (epoch): tiles (T | 512) never straddle two
-    const int rec = ep.n > 0 ? ep.wep[n0 >> 5] : 0;
-    const int rend = ep.n > 0 ? ep.off[rec] + ep.len[rec] : g.L;
-    if (n0 >= rend) return;  // gap between epochs; uniform over the CTA
-    const int nl = min(T, rend - n0);
-    const int C = g.C;
-    const real third = real(1.0 / 3.0);
-
-    for (int idx = threadIdx.x; idx < 2 * Kc; idx += blockDim.x) {
-        const int env = idx / Kc, kk = idx - env * Kc;
-        const size_t slot = (size_t)env * Kc + kk;
-        const int* wp = wpref + slot * (g.W + 1);
-        const uint32_t* b = bits + slot * g.W;
-        // pieces of the record only: kb .. ke - 2 (n at the record's first sample uses its first piece)
-        const int kb = ep.n > 0 ? wp[ep.w0[rec]] : 0;
-        const int cl0 = wp[n0 >> 5];
-        const int nlast = n0 + nl - 1;
-        const int wl = nlast >> 5, jl = nlast & 31;
-        const int cll = wp[wl] + __popc(b[wl] & ((1u << jl) - 1u));
-        tab[idx * 3 + 0] = max(cl0 - 1, kb);
-        tab[idx * 3 + 1] = max(cll - 1, kb);
-        tab[idx * 3 + 2] = cl0;
-        if (ep.n > 0) tab[6 * Kc + 1 + idx] = kb;
-        if (g.mirror) {
-            const int E = cnt[env * g.K + k0 + kk];
-            int lp0 = INT_MAX, lp1 = INT_MAX, rp0 = INT_MAX, rp1 = INT_MAX;
-            if (E >= 2 && E <= g.cap) {
-                mirror_positions(mir + (size_t)(k0 + kk) * kMirWords, knots + slot * g.cap, env, E, lp0, lp1, rp0, rp1);
-                tab[idx * 3 + 0] = min(max(mirror_before(n0, lp0, lp1, rp0, rp1) + cl0 - 1, 0), E - 2);
-                tab[idx * 3 + 1] = min(max(mirror_before(nlast, lp0, lp1, rp0, rp1) + cll - 1, 0), E - 2);
-            }
-            int* mt = mtab + idx * 5;
-            mt[0] = lp0;
-            mt[1] = lp1;
-            mt[2] = rp0;
-            mt[3] = rp1;
-            mt[4] = E;
-        }
-    }
-    if (threadIdx.x < 32) {
-        int q = 0;
-        for (int k = threadIdx.x; k < g.K; k += 32) q += dir_qualifies(g, ep, cnt, k, rec) ? 1 : 0;
-        q = warp_sum(q);
-        if (threadIdx.x == 0) sQ[0] = q;
-    }
-    real acc[SPT];
-    real u[SPT];
-#pragma unroll
-    for (int j = 0; j < SPT; ++j) {
-        const int t = row * SPT + j;
-        acc[j] = real(0);
-        u[j] = real(0);
-        if (!first_chunk && cok && t < nl) acc[j] = acc_buf[(size_t)(n0 + t) * C + c];
-    }
-    __syncthreads();
-
-    for (int kk = 0; kk < Kc; ++kk) {
-        const int k = k0 + kk;
-        const int Emax = cnt[k], Emin = cnt[g.K + k];
-        if (!dir_qualifies(g, ep, cnt, k, rec)) continue;
-        if (Emax > g.cap || Emin > g.cap) continue;
-#pragma unroll
-        for (int env = 0; env < 2; ++env) {
-            const size_t slot = (size_t)env * Kc + kk;
-            const int ia = tab[(env * Kc + kk) * 3 + 0];
-            const int ib = tab[(env * Kc + kk) * 3 + 1];
-            const int cl0 = tab[(env * Kc + kk) * 3 + 2];
-            int m = ib - ia + 1;
-            if (m > MI - 1) {
-                if (threadIdx.x == 0) atomicOr(&st->flags, 2);
-                m = MI - 1;
-            }
-            const int* kn = knots + slot * g.cap;
-            const real* svs = sv + slot * (size_t)g.cap * C;
-            const real* yvs = yv + slot * (size_t)g.cap * C;
-            const uint32_t* b = bits + slot * g.W;
-            __syncthreads();
-            for (int j = threadIdx.x; j <= m; j += blockDim.x) kx[j] = kn[ia + j];
-            for (int j = threadIdx.x; j < m; j += blockDim.x) ihs[j] = rtab[kn[ia + j + 1] - kn[ia + j]];
-            if (threadIdx.x < T / 32) {
-                const int w = (n0 >> 5) + threadIdx.x;
-                wds[threadIdx.x] = (w < g.W) ? b[w] : 0u;
-            }
-            __syncthreads();
-            for (int t = threadIdx.x; t < nl; t += blockDim.x) {
-                const int w = t >> 5, jb = t & 31;
-                int cntl = 0;
-                for (int q = 0; q < w; ++q) cntl += __popc(wds[q]);
-                cntl += __popc(wds[w] & ((1u << jb) - 1u));
-                int iv = max(cl0 + cntl - 1, ep.n > 0 ? tab[6 * Kc + 1 + env * Kc + kk] : 0);
-                if (g.mirror) {
-                    const int* mt = mtab + (env * Kc + kk) * 5;
-                    iv = min(max(mirror_before(n0 + t, mt[0], mt[1], mt[2], mt[3]) + cl0 + cntl - 1, 0), mt[4] - 2);
-                }
-                int li = iv - ia;
-                li = min(li, m - 1);
-                lis[t] = li;
-                tts[t] = real(n0 + t - kx[li]);
-            }
-            for (int it = threadIdx.x; it < m * G; it += blockDim.x) {
-                const int li = it / G, ch = it - li * G;
-                const int cch = cg * G + ch;
-                if (cch < C) {
-                    const int i = ia + li;
-                    const real s0 = svs[(size_t)i * C + cch], s1 = svs[(size_t)(i + 1) * C + cch];
-                    const real y0 = yvs[(size_t)i * C + cch], y1 = yvs[(size_t)(i + 1) * C + cch];
-                    const real h = real(kx[li + 1] - kx[li]);
-                    const real ih = ihs[li];
-                    const real slope = mul_(sub_(y1, y0), ih);
-                    const real bq = fmad_(-mul_(h, third), fmad_(real(2), s0, s1), slope);
-                    const real dq = mul_(sub_(s1, s0), mul_(ih, third));
-                    real* cf = coef + (size_t)li * 4 * G + ch;
-                    cf[0] = y0;
-                    cf[G] = bq;
-                    cf[2 * G] = s0;
-                    cf[3 * G] = dq;
-                }
-            }
-            __syncthreads();
-            if (cok) {
-#pragma unroll
-                for (int j = 0; j < SPT; ++j) {
-                    const int t = row * SPT + j;
-                    if (t < nl) {
-                        const int li = lis[t];
-                        const real tt = tts[t];
-                        const real* cf = coef + (size_t)li * 4 * G + cc;
-                        const real v = fmad_(fmad_(fmad_(cf[3 * G], tt, cf[2 * G]), tt, cf[G]), tt, cf[0]);
-                        if (env == 0) {
-                            u[j] = v;
-                        } else {
-                            acc[j] = add_(acc[j], add_(u[j], v));
-                            if (M) u[j] = sub_(u[j], v);  // spread U - L for the amplitude
-                        }
-                    }
-                }
-            }
-            if (M && env == 1) {
-                // sum of squared spreads over the G channels of each sample row
-#pragma unroll
-                for (int j = 0; j < SPT; ++j) {
-                    const int t = row * SPT + j;
-                    real d2 = (cok && t < nl) ? mul_(u[j], u[j]) : real(0);
-#pragma unroll
-                    for (int o = 1; o < G; o <<= 1) d2 = add_(d2, shfl_xor_(d2, o));
-                    if (cc == 0 && t < nl) part[((size_t)cg * Kc + kk) * g.L + n0 + t] = d2;
-                }
-            }
-        }
-    }
-    const int Q = sQ[0];
-    if (!M && last_chunk && Q == 0 && (blockIdx.x == 0 || ep.n > 0) && blockIdx.y == 0 && threadIdx.x == 0)
-        atomicOr(&st->flags, 1);
-    if (!cok) return;
-#pragma unroll
-    for (int j = 0; j < SPT; ++j) {
-        const int t = row * SPT + j;
-        if (t < nl) {
-            const size_t idx = (size_t)(n0 + t) * C + c;
-            if (last_chunk) {
-                const real val = mul_(acc[j], real(0.5));
-                if (M) M[idx] = div_(val, real(Q));
-                else X[idx] = sub_(X[idx], div_(val, real(Q)));
-            } else {
-                acc_buf[idx] = acc[j];
-            }
-        }
-    }
-}
-
 // ---------------------------------------------------------------------------
-// Envelope evaluation, FP32 arithmetic, one warp per direction.
-// CTA: T = (32/G)*SPL samples x G channels, 8 warps; warp w handles the
-// directions w, w+8, ... of the chunk on its own (no block barrier inside the
-// direction loop), so the load latency of one direction is covered by the
+// Envelope evaluation at every sample, fused with the mean over directions and
+// the update (FP32 form; stop mode, mirror boundary or mean_eval = 1 in the
+// others), one warp per direction.
+// CTA: T = (32/G)*SPL samples x G channels, WARPS warps; warp w handles the
+// directions w, w + WARPS, ... of the chunk on its own (no block barrier inside
+// the direction loop), so the load latency of one direction is covered by the
 // other warps' work.  Per (direction, envelope) a warp stages the tile's
-// knots, knot values and solutions in its shared-memory slice, then every
-// lane walks its SPL consecutive samples of one channel, recomputing the
-// cubic's coefficients when the interval changes.  The warps' partial sums
-// are added in warp order at the end (a pairwise sum over the directions).
-// X is float (FP32 path) or float2 (double-float, mixed path).
+// knots in its shared-memory slice, then every lane walks its SPL consecutive
+// samples of one channel, recomputing the cubic's coefficients
+//   a = y_i, b = (y_{i+1}-y_i)/h - h(2 s_i + s_{i+1})/3, c = s_i,
+//   d = (s_{i+1} - s_i)/(3h)
+// when the interval changes.  The sum over qualified directions (E_max > 3 &&
+// E_min > 3): each warp's directions in order, then the warps' partial sums in
+// warp order; the last chunk applies X -= (sum/2)/Q (REF:832-864).
+// X is float (FP32 path), float2 (double-float, mixed path) or double.
+// The tile is 32 samples (SPL = G) until the launch fills the GPU, and the
+// FP64 and double-float forms deal a tile's directions to a cluster of two or
+// four CTAs then: a small record is bound by one warp's walk over its
+// directions, and in FP64 by the FP64 pipe of the few SMs that have a tile.
+// (8 channels x 2,000 samples, 64 directions, stop mode: 64-sample tiles of 8
+// warps took 104 us a pass in double-float, 20 .. 31 us so; FP64 343 us with a
+// block per tile that took one direction at a time, 53 .. 75 us so.)
 // ---------------------------------------------------------------------------
-template <int G, int SPL, typename R>
+template <int G, int SPL, typename R, int WARPS>
 struct EvalWShape {
     static constexpr int NS = 32 / G;
     static constexpr int T = NS * SPL;
     static constexpr int MI = T / 2 + 4;
-    static constexpr int WARPS = 8;
     static constexpr int NW = T / 32;
     // per warp: accumulator tile, (stop mode) spread tile, knots, bit words
     __host__ __device__ static constexpr size_t per_warp(bool stopm)
     {
         return (size_t)(stopm ? 2 : 1) * sizeof(R) * T * G + sizeof(int) * (MI + 1) + sizeof(uint32_t) * (NW + 1);
     }
-    static size_t smem_bytes(bool stopm) { return WARPS * ((per_warp(stopm) + 15) / 16 * 16); }
+    static constexpr size_t smem_bytes(bool stopm) { return WARPS * ((per_warp(stopm) + 15) / 16 * 16); }
 };
 
-template <int G, int SPL, typename XT, typename R, bool STOPM>
-__global__ void __launch_bounds__(256)
+template <int G, int SPL, typename XT, typename R, bool STOPM, int WARPS>
+__global__ void __launch_bounds__(32 * WARPS)
 k_eval_w(XT* __restrict__ X, R* __restrict__ acc_buf, const uint32_t* __restrict__ bits,
          const int* __restrict__ wpref, const int* __restrict__ knots, const int* __restrict__ cnt,
          const R* __restrict__ rtab, const R* __restrict__ sv, const R* __restrict__ yv, Geom g,
@@ -1366,7 +1151,7 @@ k_eval_w(XT* __restrict__ X, R* __restrict__ acc_buf, const uint32_t* __restrict
     // g.mirror: intervals count the mirrored knots too (mirror_before).
     // ep.n > 0 (batched): a tile (T | 512) lies in one record; pieces, the
     // qualified directions and Q are the record's own.
-    using Sh = EvalWShape<G, SPL, R>;
+    using Sh = EvalWShape<G, SPL, R, WARPS>;
     constexpr int T = Sh::T;
     constexpr int MI = Sh::MI;
     constexpr int NW = Sh::NW;
@@ -1402,7 +1187,10 @@ k_eval_w(XT* __restrict__ X, R* __restrict__ acc_buf, const uint32_t* __restrict
     const R* sc = sv + c;
     bool overflow = false;
 
-    for (int kk = warp; kk < Kc; kk += Sh::WARPS) {
+    // CTAs per tile (FP32: one, its sum over the directions keeps its order)
+    constexpr bool ONE = std::is_same<R, float>::value;
+    const int Z = ONE ? 1 : (int)gridDim.z, zr = ONE ? 0 : (int)blockIdx.z;
+    for (int kk = zr * WARPS + warp; kk < Kc; kk += WARPS * Z) {
         const int k = k0 + kk;
         if (!dir_qualifies(g, ep, cnt, k, rec)) continue;
         if (cnt[k] > g.cap || cnt[g.K + k] > g.cap) continue;
@@ -1476,12 +1264,18 @@ k_eval_w(XT* __restrict__ X, R* __restrict__ acc_buf, const uint32_t* __restrict
                         const R ih = rtab[h];
                         const R slope = mul_(sub_(ynx, y0), ih);
                         ca = y0;
-                        cb = fmad_(-mul_(R(h), third), fmad_(R(2), s0, snx), slope);
+                        cb = fmad_(-mul_(from_int<R>(h), third), fmad_(R(2), s0, snx), slope);
                         c2 = s0;
                         cd = mul_(sub_(snx, s0), mul_(ih, third));
                     }
-                    const float tt = (float)(n0 + t - x0);
-                    const R v = fmat_(fmat_(fmat_(cd, tt, c2), tt, cb), tt, ca);
+                    R v;
+                    if constexpr (std::is_same<R, double>::value) {
+                        const double tt = from_int<double>(n0 + t - x0);
+                        v = fmad_(fmad_(fmad_(cd, tt, c2), tt, cb), tt, ca);
+                    } else {
+                        const float tt = (float)(n0 + t - x0);
+                        v = fmat_(fmat_(fmat_(cd, tt, c2), tt, cb), tt, ca);
+                    }
                     const int idx = t * G + cc;
                     if constexpr (STOPM) {
                         if (env == 0) {
@@ -1516,19 +1310,29 @@ k_eval_w(XT* __restrict__ X, R* __restrict__ acc_buf, const uint32_t* __restrict
         }
     }
     if (overflow) atomicOr(&st->flags, 2);
-    __syncthreads();
+    // the tile's CTAs (a cluster along z) have their partial sums ready; each
+    // adds them up, in the order of the warps over all of them, for a share of
+    // the tile
+    namespace cg_ = cooperative_groups;
+    if (!ONE && Z > 1) cg_::this_cluster().sync();
+    else __syncthreads();
     const int Q = sQ;
     if (!M && last_chunk && Q == 0 && (blockIdx.x == 0 || ep.n > 0) && blockIdx.y == 0 && threadIdx.x == 0)
         atomicOr(&st->flags, 1);
-    for (int idx = threadIdx.x; idx < T * G; idx += blockDim.x) {
+    for (int idx = threadIdx.x + zr * (int)blockDim.x; idx < T * G; idx += (int)blockDim.x * Z) {
         const int t = idx / G, ch = idx - t * G;
         const int cch = cg * G + ch;
         if (t >= nl || cch >= C) continue;
         const size_t off = (size_t)(n0 + t) * C + cch;
         R tot = first_chunk ? R(0.0f) : acc_buf[off];
+        if constexpr (ONE) {
 #pragma unroll
-        for (int w = 0; w < Sh::WARPS; ++w)
-            tot = add_(tot, reinterpret_cast<const R*>(smem_raw + (size_t)w * PW)[idx]);
+            for (int w = 0; w < WARPS; ++w) tot = add_(tot, reinterpret_cast<const R*>(smem_raw + (size_t)w * PW)[idx]);
+        } else for (int z = 0; z < Z; ++z) {
+            const unsigned char* base = Z > 1 ? cg_::this_cluster().map_shared_rank(smem_raw, z) : smem_raw;
+#pragma unroll
+            for (int w = 0; w < WARPS; ++w) tot = add_(tot, reinterpret_cast<const R*>(base + (size_t)w * PW)[idx]);
+        }
         if (last_chunk) {
             const R mval = div_(mul_(tot, R(0.5f)), R(Q));
             if (M) M[off] = mval;
@@ -1537,6 +1341,7 @@ k_eval_w(XT* __restrict__ X, R* __restrict__ acc_buf, const uint32_t* __restrict
             acc_buf[off] = tot;
         }
     }
+    if (!ONE && Z > 1) cg_::this_cluster().sync();  // the others may still be reading this CTA's sums
 }
 
 // ---------------------------------------------------------------------------
@@ -2146,8 +1951,6 @@ k_project_mx(const float2* __restrict__ X, const float* __restrict__ dh_all, con
 // Stop mode (the sifting criterion of Rilling et al. 2003 used by Rehman &
 // Mandic 2010; no counterpart in the reference, which runs max_iter sifts).
 // ---------------------------------------------------------------------------
-// amp[n] (+)= sum over qualified directions of the chunk of
-//             sqrt(sum over channel groups of part[g][kk][n]) / 2
 // ---------------------------------------------------------------------------
 // Mirrored end knots (boundary mode MEMD_BOUNDARY_MIRROR; no reference
 // counterpart: the mirror extension of Rilling, Flandrin & Goncalves 2003,
@@ -2373,82 +2176,18 @@ k_mirror(const uint32_t* __restrict__ bits, const XT* __restrict__ X, const real
     out[15] = 0;
 }
 
-template <typename real>
-__global__ void k_amp(const real* __restrict__ part, real* __restrict__ amp, const int* __restrict__ cnt,
-                      Geom g, int k0, int Kc, int groups, int first_chunk, Epochs ep)
+// The stop rule of one record: stop, or subtract the mean and sift again.
+// Before the first subtraction of an IMF, a residual whose every direction has
+// fewer than 3 interior extrema ends the decomposition.  Drives the sift
+// loop's conditional WHILE node.  One warp.
+__device__ __forceinline__ void decide_record(RunState* st, const int* __restrict__ cnt, const Geom& g, double tol,
+                                              int max_iter, cudaGraphConditionalHandle h_sift,
+                                              const int* __restrict__ mir)
 {
-    for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < g.L; n += gridDim.x * blockDim.x) {
-        real a = first_chunk ? real(0) : amp[n];
-        const int rec = ep.n > 0 ? ep.wep[n >> 5] : 0;  // qualification of the sample's record
-        for (int kk = 0; kk < Kc; ++kk) {
-            const int k = k0 + kk;
-            if (!dir_qualifies(g, ep, cnt, k, rec)) continue;
-            real s2 = real(0);
-            for (int q = 0; q < groups; ++q) s2 = add_(s2, part[((size_t)q * Kc + kk) * g.L + n]);
-            a = fmad_(sqrt_(s2), real(0.5), a);
-        }
-        amp[n] = a;
-    }
-}
-
-// sigma(n) = ||m(n)||_2 / (amp(n) / Q); counts samples above sd and sd2.
-template <typename real>
-__global__ void __launch_bounds__(256)
-k_stop_stats(const real* __restrict__ M, const real* __restrict__ amp, const int* __restrict__ cnt, Geom g,
-             double sd, double sd2, RunState* st)
-{
-    __shared__ int sq;
-    __shared__ unsigned long long s1, s2;
-    if (threadIdx.x < 32) {
-        int q = 0;
-        for (int k = threadIdx.x; k < g.K; k += 32) q += (cnt[k] > 3 && cnt[g.K + k] > 3) ? 1 : 0;
-        q = warp_sum(q);
-        if (threadIdx.x == 0) {
-            sq = q;
-            s1 = 0;
-            s2 = 0;
-        }
-    }
-    __syncthreads();
-    const int Q = sq;
-    unsigned long long c1 = 0, c2 = 0;
-    for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < g.L; n += gridDim.x * blockDim.x) {
-        real m2 = real(0);
-        for (int c = 0; c < g.C; ++c) {
-            const real v = M[(size_t)n * g.C + c];
-            m2 = fmad_(v, v, m2);
-        }
-        const real a = div_(amp[n], real(Q));
-        real sig;
-        if (a > real(0.0f)) sig = div_(sqrt_(m2), a);
-        else sig = m2 > real(0.0f) ? real(INFINITY) : real(0.0f);
-        c1 += (static_cast<double>(sig) > sd) ? 1 : 0;
-        c2 += (static_cast<double>(sig) > sd2) ? 1 : 0;
-    }
-    c1 = warp_sum<unsigned long long>(c1);
-    c2 = warp_sum<unsigned long long>(c2);
-    if ((threadIdx.x & 31) == 0) {
-        atomicAdd(&s1, c1);
-        atomicAdd(&s2, c2);
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        atomicAdd(&st->over1, s1);
-        atomicAdd(&st->over2, s2);
-    }
-}
-
-// After each pass: stop, or subtract the mean and sift again.  Before the
-// first subtraction of an IMF, a residual whose every direction has fewer
-// than 3 interior extrema ends the decomposition.  Drives the sift loop's
-// conditional WHILE node.
-__global__ void k_decide(RunState* st, const int* __restrict__ cnt, Geom g, double tol, int max_iter,
-                         cudaGraphConditionalHandle h_sift, const int* __restrict__ mir)
-{
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+    const int lane = threadIdx.x & 31;
     int q = 0;
     bool few = true;
-    for (int k = 0; k < g.K; ++k) {
+    for (int k = lane; k < g.K; k += 32) {
         const int a = cnt[k], b = cnt[g.K + k];
         if (a > 3 && b > 3) ++q;
         // interior extrema: the knots less the two end samples (reference
@@ -2461,13 +2200,17 @@ __global__ void k_decide(RunState* st, const int* __restrict__ cnt, Geom g, doub
         }
         if (ia + ib >= 3) few = false;
     }
+    q = warp_sum(q);
+    few = __all_sync(kFull, few);
+    if (lane != 0) return;
     st->q = q;
     unsigned cont = 0;
     st->apply = 0;
+    const unsigned long long over1 = __ldcg(&st->over1), over2 = __ldcg(&st->over2);
     if (st->pass == 0 && few) {
         st->imf_done = 1;
     } else {
-        const bool stop = (q == 0) || !(((double)st->over1 / (double)g.L > tol) || st->over2 > 0);
+        const bool stop = (q == 0) || !(((double)over1 / (double)g.L > tol) || over2 > 0);
         if (!stop) {
             st->apply = 1;
             st->nbit += 1;
@@ -2481,6 +2224,108 @@ __global__ void k_decide(RunState* st, const int* __restrict__ cnt, Geom g, doub
     st->pad[0] += 1;  // passes over the whole run
     st->pad[1] = (int)cont;
     if (h_sift) cudaGraphSetConditional(h_sift, cont);
+}
+
+// amp(n) = sum over qualified directions of ||U(n) - L(n)||_2 / 2, from
+// part[group][kk][n] (the sums of squares over a group's channels), and, after
+// the last pass over the directions, sigma(n) = ||m(n)||_2 / (amp(n) / Q) and
+// the counts of samples above sd and sd2.  CTA: 32 samples (one bitmask word,
+// in one record); the 8 warps take the directions' square roots, warp 0 adds
+// them in direction order, warp 1 sums the mean's squares, lane = sample.  (With
+// a thread per sample that walked through all of it, a kernel for the sums, one
+// for the counts and one for the rule took 86 us a pass in FP64 for 2,000
+// samples and 64 directions; 17 us so.)
+// One record: the last CTA to finish (a counter, no waiting) applies the stop
+// rule.  A batch (rs): the counts go to the sample's record, k_decide_b follows.
+template <typename real>
+__global__ void __launch_bounds__(256)
+k_stop_stats(const real* __restrict__ part, real* __restrict__ amp, const real* __restrict__ M,
+             const int* __restrict__ cnt, Geom g, int k0, int Kc, int groups, int first_chunk, int last_chunk,
+             double sd, double sd2, double tol, int max_iter, RunState* st, RecStop* __restrict__ rs, Epochs ep,
+             cudaGraphConditionalHandle h_sift, const int* __restrict__ mir)
+{
+    constexpr int KB = 64;  // directions per round
+    __shared__ real root[KB][32];
+    __shared__ unsigned char qual[KB];
+    __shared__ real m2s[32];
+    __shared__ int sq, slast;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int w = blockIdx.x, n = w * 32 + lane;
+    const int rec = ep.n > 0 ? ep.wep[w] : 0;
+    const bool in = n < g.L && (ep.n == 0 || n - ep.off[rec] < ep.len[rec]);
+    if (warp == 1 && last_chunk) {
+        real m2 = real(0);
+        if (in)
+            for (int c = 0; c < g.C; ++c) {
+                const real v = M[(size_t)n * g.C + c];
+                m2 = fmad_(v, v, m2);
+            }
+        m2s[lane] = m2;
+    } else if (warp == 2 && last_chunk) {
+        int q = 0;
+        for (int k = lane; k < g.K; k += 32) q += dir_qualifies(g, ep, cnt, k, rec) ? 1 : 0;
+        q = warp_sum(q);
+        if (lane == 0) sq = q;
+    }
+    real a = real(0);
+    if (warp == 0 && in && !first_chunk) a = amp[n];
+    for (int base = 0; base < Kc; base += KB) {
+        const int nk = min(KB, Kc - base);
+        if (threadIdx.x < KB)
+            qual[threadIdx.x] = (int)threadIdx.x < nk && dir_qualifies(g, ep, cnt, k0 + base + threadIdx.x, rec);
+        real s2[KB / 8];
+#pragma unroll
+        for (int j = 0; j < KB / 8; ++j) s2[j] = real(0);
+        for (int q = 0; q < groups; ++q) {
+            const real* p = part + ((size_t)q * Kc + base) * g.L + n;
+#pragma unroll
+            for (int j = 0; j < KB / 8; ++j)
+                if (in && warp + 8 * j < nk) s2[j] = add_(s2[j], p[(size_t)(warp + 8 * j) * g.L]);
+        }
+#pragma unroll
+        for (int j = 0; j < KB / 8; ++j) root[warp + 8 * j][lane] = sqrt_(s2[j]);
+        __syncthreads();
+        if (warp == 0) {
+#pragma unroll 4
+            for (int kk = 0; kk < nk; ++kk)
+                if (qual[kk]) a = fmad_(root[kk][lane], real(0.5), a);
+        }
+        __syncthreads();
+    }
+    if (warp != 0) return;
+    if (!last_chunk) {
+        if (in) amp[n] = a;
+        return;
+    }
+    bool o1 = false, o2 = false;
+    if (in) {
+        const real m2 = m2s[lane];
+        const real av = div_(a, real(sq));
+        real sig;
+        if (av > real(0.0f)) sig = div_(sqrt_(m2), av);
+        else sig = m2 > real(0.0f) ? real(INFINITY) : real(0.0f);
+        o1 = static_cast<double>(sig) > sd;
+        o2 = static_cast<double>(sig) > sd2;
+    }
+    const unsigned b1 = __ballot_sync(kFull, o1), b2 = __ballot_sync(kFull, o2);
+    if (rs) {
+        if (lane == 0 && rs[rec].sifting) {
+            if (b1) atomicAdd(&rs[rec].over1, (unsigned long long)__popc(b1));
+            if (b2) atomicAdd(&rs[rec].over2, (unsigned long long)__popc(b2));
+        }
+        return;
+    }
+    if (lane == 0) {
+        if (b1) atomicAdd(&st->over1, (unsigned long long)__popc(b1));
+        if (b2) atomicAdd(&st->over2, (unsigned long long)__popc(b2));
+        __threadfence();
+        slast = atomicAdd(&st->arrive, 1) == (int)gridDim.x - 1;
+    }
+    __syncwarp();
+    if (!slast) return;
+    __threadfence();
+    decide_record(st, cnt, g, tol, max_iter, h_sift, mir);
+    if (lane == 0) st->arrive = 0;
 }
 
 template <typename real, typename XT>
@@ -2557,7 +2402,7 @@ __global__ void k_zero_unused(real* __restrict__ imf, const RunState* __restrict
 
 // ---------------------------------------------------------------------------
 // Stop mode, batched runs: every record (epoch) takes its own decisions, with
-// the single-record rules (k_decide, k_imf_commit) applied to its own counts,
+// the single-record rules (decide_record, k_imf_commit) applied to its own counts,
 // length and statistics; the graph's sift and IMF loops run while any record
 // goes on, and a record that has stopped is neither updated nor written
 // again.  Gap samples between records are never read or written.
@@ -2580,42 +2425,6 @@ __global__ void k_rec_q(RecStop* __restrict__ rs, Geom g, Epochs ep)
     if (lane == 0) {
         rs[e].q = q;
         rs[e].few = few ? 1 : 0;
-    }
-}
-
-// sigma statistics per record: a warp's 32 consecutive samples are one
-// bitmask word, which lies in one record.
-template <typename real>
-__global__ void __launch_bounds__(256)
-k_stop_stats_b(const real* __restrict__ M, const real* __restrict__ amp, RecStop* __restrict__ rs, Geom g, Epochs ep,
-               double sd, double sd2)
-{
-    const int lane = threadIdx.x & 31;
-    const long stride = (long)gridDim.x * blockDim.x;
-    for (long nw = (long)blockIdx.x * blockDim.x + (threadIdx.x & ~31); nw < g.L; nw += stride) {
-        const int n = (int)nw + lane;
-        const int e = ep.wep[nw >> 5];  // the word's record (uniform over the warp)
-        if (!rs[e].sifting) continue;
-        const bool in = n < g.L && n - ep.off[e] < ep.len[e];
-        bool o1 = false, o2 = false;
-        if (in) {
-            real m2 = real(0);
-            for (int c = 0; c < g.C; ++c) {
-                const real v = M[(size_t)n * g.C + c];
-                m2 = fmad_(v, v, m2);
-            }
-            const real a = div_(amp[n], real(rs[e].q));
-            real sig;
-            if (a > real(0.0f)) sig = div_(sqrt_(m2), a);
-            else sig = m2 > real(0.0f) ? real(INFINITY) : real(0.0f);
-            o1 = static_cast<double>(sig) > sd;
-            o2 = static_cast<double>(sig) > sd2;
-        }
-        const unsigned b1 = __ballot_sync(kFull, o1), b2 = __ballot_sync(kFull, o2);
-        if (lane == 0) {
-            if (b1) atomicAdd(&rs[e].over1, (unsigned long long)__popc(b1));
-            if (b2) atomicAdd(&rs[e].over2, (unsigned long long)__popc(b2));
-        }
     }
 }
 

@@ -35,7 +35,7 @@ namespace memd {
 // the error.
 //
 // Measured (FP64 form, all sifts of a decomposition, against the direct
-// evaluation k_eval, which is 82% busy on the FP64 pipe): 32 x 30,504, 64
+// evaluation of every envelope at every sample, 82% busy on the FP64 pipe): 32 x 30,504, 64
 // directions, 80 sifts: 117.6 -> 29.6 ms of the mean, 163.4 -> 70.2 ms in all;
 // 12 epochs x 32 channels: 279 -> 53.5 ms, 363 -> 127 ms; error of the IMFs
 // against a separate FP64 evaluation 8.2e-16 -> 3.9e-16.
@@ -43,7 +43,7 @@ namespace memd {
 // A span whose values leave the fixed-point range (non-finite values, or
 // splines that overshoot the signal thousands of times), and a channel so
 // small that its third-order coefficients would be subnormal, is evaluated
-// directly, pair by pair in direction order, with k_eval's arithmetic.
+// directly, pair by pair in direction order, with k_eval_w's arithmetic.
 struct FixSum {
     unsigned long long hi, lo;
 };
