@@ -288,13 +288,26 @@ static void launch_eval(memd_plan* p, cudaStream_t s, int k0, int kc, int first,
     const Geom& g = p->g;
     if constexpr (P == MEMD_PREC_F64) {
         if (p->cum) {
-            const dim3 grid((unsigned)g.W, (unsigned)((g.C + p->cumG - 1) / p->cumG));
+            cudaLaunchConfig_t lc{};
+            lc.gridDim = dim3((unsigned)(g.W + 1) / 2 * 2, (unsigned)((g.C + p->cumG - 1) / p->cumG));
+            lc.blockDim = dim3(256);
+            lc.stream = s;
+            cudaLaunchAttribute at[1];
+            at[0].id = cudaLaunchAttributeClusterDimension;
+            at[0].val.clusterDim.x = 2;
+            at[0].val.clusterDim.y = 1;
+            at[0].val.clusterDim.z = 1;
+            lc.attrs = at;
+            lc.numAttrs = 1;
 #define MEMD_CASE(G_)                                                                                              \
     if (p->cumG == G_) {                                                                                           \
-        k_mean_fix<G_><<<grid, 256, fix_smem_bytes(G_), s>>>(                                                      \
-            (const double*)p->X, (double*)p->Xb, (ulonglong2*)p->acc, p->bits, p->wpref, p->knots, p->cnt,         \
-            (const double*)p->rtab, (const double*)p->rtab3, (const double*)p->sv, (const double*)p->yend,         \
-            p->xexp, p->nchunks > 1 ? p->tot : nullptr, g, k0, kc, first, last, p->st, p->ep);                      \
+        lc.dynamicSmemBytes = fix_smem_bytes(G_);                                                                  \
+        cudaLaunchKernelEx(&lc, k_mean_fix<G_>, (const double*)p->X, (double*)p->Xb, (ulonglong2*)p->acc,          \
+                           (const uint32_t*)p->bits, (const int*)p->wpref, (const int*)p->knots,                   \
+                           (const int*)p->cnt, (const double*)p->rtab, (const double2*)p->rtab3,                   \
+                           (const double*)p->sv, (const double*)p->yend, (const unsigned*)p->xexp,                 \
+                           (const unsigned long long*)(p->nchunks > 1 ? p->tot : nullptr), g, k0, kc, first, last, \
+                           p->st, p->ep);                                                                          \
         return;                                                                                                    \
     }
             MEMD_CASE(32) MEMD_CASE(16) MEMD_CASE(8)
@@ -1399,7 +1412,7 @@ static memd_status create_plan(const memd_config* cfg, const memd_tuning* tun, m
     // longest knot gap: a record (epoch) length; mirrored knots reach 2L - 2
     const int Lh = p->batched ? std::max(p->Lrec, kEpochAlign) : (p->g.mirror ? 2 * L : L);
     ALLOC(p->rtab, rb * (size_t)(Lh + 1));
-    if (p->cum) ALLOC(p->rtab3, 8 * (size_t)(Lh + 1));
+    if (p->cum) ALLOC(p->rtab3, (f64 ? 16 : 8) * (size_t)(Lh + 1));
     if (p->cum && f64) {
         ALLOC(p->xexp, sizeof(unsigned) * (size_t)std::max<int64_t>(1, c.max_epochs) * C);
         if (p->nchunks > 1) ALLOC(p->tot, sizeof(unsigned long long) * (size_t)std::max<int64_t>(1, c.max_epochs));
@@ -1483,7 +1496,7 @@ static memd_status create_plan(const memd_config* cfg, const memd_tuning* tun, m
         if (e == cudaSuccess) e = cudaMalloc((void**)&r32, sizeof(float) * (size_t)(Lh + 1));
         if (e == cudaSuccess) e = cudaMalloc((void**)&rdd, sizeof(dd) * (size_t)(Lh + 1));
         if (e == cudaSuccess) {
-            k_fill_reciprocals<<<256, 256>>>(r64, r32, rdd, f64 ? nullptr : (dd*)p->rtab3, f64 ? (double*)p->rtab3 : nullptr,
+            k_fill_reciprocals<<<256, 256>>>(r64, r32, rdd, f64 ? nullptr : (dd*)p->rtab3, f64 ? (double2*)p->rtab3 : nullptr,
                                              Lh + 1);
             const void* src = f64 ? (void*)r64 : (c.precision == MEMD_PREC_MIXED ? (void*)rdd : (void*)r32);
             e = cudaMemcpy(p->rtab, src, rb * (size_t)(Lh + 1), cudaMemcpyDeviceToDevice);

@@ -2689,16 +2689,16 @@ __global__ void k_check_coords(const int32_t* __restrict__ x, int L, int* __rest
 }
 
 __global__ void k_fill_reciprocals(double* __restrict__ r64, float* __restrict__ r32, dd* __restrict__ rdd,
-                                   dd* __restrict__ r3dd, double* __restrict__ r3_64, int n)
+                                   dd* __restrict__ r3dd, double2* __restrict__ r3_64, int n)
 {
-    // r3dd, r3_64 (optional): 1/(3h) as a double-float / in FP64
+    // r3dd (optional): 1/(3h) as a double-float; r3_64 (optional): 1/(3h) and h/3 in FP64
     for (int h = blockIdx.x * blockDim.x + threadIdx.x; h < n; h += gridDim.x * blockDim.x) {
         const double r = h > 0 ? __ddiv_rn(1.0, (double)h) : 0.0;
         r64[h] = r;
         r32[h] = h > 0 ? __fdiv_rn(1.0f, (float)h) : 0.0f;
         rdd[h] = dd(r);
         if (r3dd) r3dd[h] = h > 0 ? dd(__ddiv_rn(1.0, 3.0 * (double)h)) : dd(0.0f, 0.0f);
-        if (r3_64) r3_64[h] = h > 0 ? __ddiv_rn(1.0, 3.0 * (double)h) : 0.0;
+        if (r3_64) r3_64[h] = make_double2(h > 0 ? __ddiv_rn(1.0, 3.0 * (double)h) : 0.0, __dmul_rn((double)h, 1.0 / 3.0));
     }
 }
 

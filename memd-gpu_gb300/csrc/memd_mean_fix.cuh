@@ -23,22 +23,21 @@ namespace memd {
 // words, and the exact sums make the result independent of the order, of the
 // direction chunks and of the batch a record is in.
 //
-// Anchors: every T samples, T the power of two in [8, 64] with T <= 2 h (h:
+// Anchors: every T samples, T the power of two in [8, 64] with T <= 3 h (h:
 // the record's mean knot spacing over all directions; 8 at the densest
 // knots).  Rounding in a piece's coefficients grows with the distance from
-// the anchor, at most T/2, about one knot spacing.  Error of the mean against
-// a long double evaluation, relative to the signal (3 channels, 32
-// directions, EEG-shaped; direct FP64 evaluation 1.5e-16 in an IMF's first
-// sift, 2.3e-17 .. 4.2e-17 in its last; the update's own rounding ~4e-17):
-// T = 8 at h = 3.7 / 2.8: 3.8e-17 / 6.2e-17; T = 8 at h = 7.0 / 5.2: 3.4e-17 /
-// 3.5e-17; T = 16 at h = 13 / 10: 2.9e-17 / 5.0e-17; twice the span, 2x .. 3x
-// the error.
-//
+// the anchor, at most T/2.  Error of the mean against a long double
+// evaluation, relative to the signal (3 channels, 32 directions, EEG-shaped;
+// direct FP64 evaluation 1.5e-16 in an IMF's first sift, 2.3e-17 .. 4.2e-17 in
+// its last; the update's own rounding ~4e-17): T = 8 at h = 3.7 / 2.8: 3.8e-17
+// / 6.2e-17; T = 16 at h = 7.0 / 5.2: 4.9e-17 / 7.5e-17; T = 32 at h = 13 / 10:
+// 4.7e-17 / 7.4e-17; twice the span, 2x .. 4x the error.
 // Measured (FP64 form, all sifts of a decomposition, against the direct
-// evaluation of every envelope at every sample, 82% busy on the FP64 pipe): 32 x 30,504, 64
-// directions, 80 sifts: 117.6 -> 29.6 ms of the mean, 163.4 -> 70.2 ms in all;
-// 12 epochs x 32 channels: 279 -> 53.5 ms, 363 -> 127 ms; error of the IMFs
-// against a separate FP64 evaluation 8.2e-16 -> 3.9e-16.
+// evaluation of every envelope at every sample, 82% busy on the FP64 pipe): 32
+// x 30,504, 64 directions, 80 sifts: 117.6 -> 21.9 ms of the mean (29.6 with T
+// <= 2 h, integer conversions on the FP64 pipe, one CTA per 64 samples and the
+// samples behind an anchor all by one warp); error of the IMFs against a
+// separate FP64 evaluation 8.2e-16 -> 4.0e-16.
 //
 // A span whose values leave the fixed-point range (non-finite values, or
 // splines that overshoot the signal thousands of times), and a channel so
@@ -105,15 +104,25 @@ __device__ __forceinline__ bool fix_tagged(ulonglong2 v) { return (v.y & (0xfffu
 // 2^ex > max|x|: ex from the largest biased exponent of the channel's samples
 __device__ __forceinline__ int fix_shift(unsigned be) { return kFixBits - ((int)be - 1022); }
 
-// CTA: one span (32 samples, 64 where T = 64) x G channels, 8 warps; lane =
-// (subgroup, channel); the (direction, envelope) pairs are dealt round-robin
-// to the 8 * 32/G subgroups, which walk the span's pieces in order.
+// 2 v (exact); by an integer addition to the exponent for a normal value
+__device__ __forceinline__ double twice(double v)
+{
+    const int hi = __double2hiint(v);
+    if ((unsigned)(hi & 0x7ff00000) - 0x00100000u < 0x7fd00000u) return __hiloint2double(hi + 0x00100000, __double2loint(v));
+    return __dadd_rn(v, v);
+}
+
+// CTA: one 32-sample word x G channels, 8 warps; lane = (subgroup, channel); the
+// (direction, envelope) pairs are dealt round-robin to the 8 * 32/G subgroups,
+// which walk the word's pieces in order.  Where T = 64 the two CTAs of a
+// cluster share a 64-sample span: each takes half the pairs, then, with the
+// other's sums from distributed shared memory, half the rows.
 // Bound by the FP64 pipe at dense knots, by load latency at sparse ones.
 template <int G>
 __global__ void __launch_bounds__(256, 3)
 k_mean_fix(const double* __restrict__ X, double* __restrict__ Xout, ulonglong2* __restrict__ acc_buf,
            const uint32_t* __restrict__ bits, const int* __restrict__ wpref, const int* __restrict__ knots,
-           const int* __restrict__ cnt, const double* __restrict__ rtab, const double* __restrict__ rtab3,
+           const int* __restrict__ cnt, const double* __restrict__ rtab, const double2* __restrict__ rtab3,
            const double* __restrict__ sv, const double* __restrict__ yend, const unsigned* __restrict__ xexp,
            const unsigned long long* __restrict__ tot, Geom g, int k0, int Kc, int first_chunk, int last_chunk,
            RunState* st, Epochs ep)
@@ -132,12 +141,11 @@ k_mean_fix(const double* __restrict__ X, double* __restrict__ Xout, ulonglong2* 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int cc = lane % G, sub = lane / G;
     const int C = g.C;
-    const int w = blockIdx.x;
-    const int rec = ep.n > 0 ? ep.wep[w] : 0;
+    const int weven = (int)blockIdx.x & ~1;  // the cluster's first word (records start at even words)
+    const int rec = ep.n > 0 ? ep.wep[weven] : 0;
     const int roff = ep.n > 0 ? ep.off[rec] : 0;
     const int rend = ep.n > 0 ? roff + ep.len[rec] : g.L;
-    const int p0 = w * 32;
-    if (p0 >= rend) return;  // gap between epochs; uniform over the CTA
+    if (weven * 32 >= rend) return;  // gap between epochs; uniform over the cluster
     if (threadIdx.x == 0) {
         sQ = 0;
         sBad = 0u;
@@ -166,15 +174,20 @@ k_mean_fix(const double* __restrict__ X, double* __restrict__ Xout, ulonglong2* 
     if (threadIdx.x == 0) {
         const unsigned long long et = tot ? tot[rec] : sEt;
         const unsigned long long lk = (unsigned long long)(rend - roff) * 2ull * (unsigned long long)g.K;
-        int t = 8;  // T <= 2 h, h = lk / et
-        while (t < kFixRows && (unsigned long long)(2 * t) * et <= 2ull * lk) t *= 2;
+        int t = 8;  // T <= 3 h, h = lk / et
+        while (t < kFixRows && (unsigned long long)(2 * t) * et <= 3ull * lk) t *= 2;
         sT = t;
     }
     __syncthreads();
     const int T = sT;
-    const int mw = T > 32 ? 2 : 1;
-    if (mw == 2 && (((p0 - roff) >> 5) & 1)) return;  // covered by the word before; uniform over the CTA
-    const int nl = min(32 * mw, rend - p0);
+    const bool pair = T > 32;  // uniform over the cluster, and the returns below over the CTA
+    const int half = (int)blockIdx.x & 1;
+    const int w = pair ? weven : (int)blockIdx.x;
+    const int p0 = w * 32;
+    if (p0 >= rend) return;
+    const int nl = min(pair ? 64 : 32, rend - p0);
+    // this CTA's pairs
+    const int e_lo = pair && half ? Kc : 0, e_hi = pair && !half ? Kc : 2 * Kc;
     const int nA = (nl + T - 1) / T;
     const int c = blockIdx.y * G + cc;
     const bool cok = c < C;
@@ -196,13 +209,13 @@ k_mean_fix(const double* __restrict__ X, double* __restrict__ Xout, ulonglong2* 
     bool ok = xe == 0u || xe >= kFixMinExp;
     const int rlast = rend - 1;
 
-    for (int base = 0; base < 2 * Kc; base += NE) {
+    for (int base = e_lo; base < e_hi; base += NE) {
         __syncthreads();
         {
             // (1) per pair: the piece holding sample p0 and the record's last piece
             const int ei = base + (int)threadIdx.x;
             int j = -1, je = 0;
-            if (ei < 2 * Kc) {
+            if (ei < e_hi) {
                 const int kk = ei >> 1, env = ei & 1, k = k0 + kk;
                 const int Ex = cnt[k], En = cnt[g.K + k];
                 if (Ex <= g.cap && En <= g.cap && dir_qualifies(g, ep, cnt, k, rec)) {
@@ -220,7 +233,7 @@ k_mean_fix(const double* __restrict__ X, double* __restrict__ Xout, ulonglong2* 
             }
         }
         __syncthreads();
-        const int nround = min(NE, 2 * Kc - base);
+        const int nround = min(NE, e_hi - base);
         for (int le = warp * SUB + sub; le < nround; le += NWS) {
             int j = eJ[le];
             if (j < 0) continue;
@@ -246,7 +259,8 @@ k_mean_fix(const double* __restrict__ X, double* __restrict__ Xout, ulonglong2* 
                     s2 = sp[(size_t)(j + 2) * C];
                 }
                 const int h = xn - xj;
-                const double d = __dmul_rn(__dsub_rn(s1, s0), rtab3[h]);
+                const double2 r3 = rtab3[h];  // 1 / (3 h), h / 3
+                const double d = __dmul_rn(__dsub_rn(s1, s0), r3.x);
                 FixSum qc;
                 ok &= to_fix(d, sh, lim - 3 * lt, qc);
                 if (jump && MEMD_CHECK(xj - p0 > 0 && xj - p0 < nl)) {
@@ -258,11 +272,10 @@ k_mean_fix(const double* __restrict__ X, double* __restrict__ Xout, ulonglong2* 
                     // S(na + t) = A + B t + C t^2 + d t^3 on this piece
                     const double y0 = (xj == roff) ? ye[0] : X[(size_t)xj * C + cl];
                     const double y1 = (xn == rlast) ? ye[C] : X[(size_t)xn * C + cl];
-                    const double u = (double)(na - xj), u3 = (double)(3 * (na - xj));
-                    const double h3 = __dmul_rn((double)h, 1.0 / 3.0);
-                    const double b = __fma_rn(-h3, __fma_rn(2.0, s0, s1), __dmul_rn(__dsub_rn(y1, y0), rtab[h]));
+                    const double u = from_int<double>(na - xj), u3 = from_int<double>(3 * (na - xj));
+                    const double b = __fma_rn(-r3.y, __fma_rn(2.0, s0, s1), __dmul_rn(__dsub_rn(y1, y0), rtab[h]));
                     const double e = __fma_rn(d, u, s0);
-                    const double cB = __fma_rn(__fma_rn(d, u3, __dadd_rn(s0, s0)), u, b);
+                    const double cB = __fma_rn(__fma_rn(d, u3, twice(s0)), u, b);
                     FixSum f;
                     unsigned long long* ah = an_hi + (size_t)(a * 4) * G + cc;
                     unsigned long long* al = an_lo + (size_t)(a * 4) * G + cc;
@@ -292,13 +305,44 @@ k_mean_fix(const double* __restrict__ X, double* __restrict__ Xout, ulonglong2* 
     }
     if (!ok) atomicOr(&sBad, 1u << cc);
     __syncthreads();
+    if (pair) {
+        // the other half's sums: read them all, and only then change this CTA's
+        namespace cg_ = cooperative_groups;
+        const auto cl_ = cg_::this_cluster();
+        cl_.sync();
+        constexpr int NV = (kFixRows + 4) * G / 256 + 1;
+        const unsigned long long* oh = cl_.map_shared_rank(kq_hi, 1 - half);
+        const unsigned long long* ol = oh + (kq_lo - kq_hi);
+        const unsigned obad = *cl_.map_shared_rank(&sBad, 1 - half);
+        unsigned long long vh[NV], vl[NV];
+        const int nk = nl * G, nv = nk + 4 * G;  // rows, then the anchor (nA = 1)
+#pragma unroll
+        for (int j = 0; j < NV; ++j) {
+            const int i = (int)threadIdx.x + 256 * j;
+            const int at = i < nk ? i : (int)(an_hi - kq_hi) + i - nk, al = i < nk ? i : (int)(an_lo - kq_lo) + i - nk;
+            vh[j] = i < nv ? oh[at] : 0ull;
+            vl[j] = i < nv ? ol[al] : 0ull;
+        }
+        cl_.sync();
+#pragma unroll
+        for (int j = 0; j < NV; ++j) {
+            const int i = (int)threadIdx.x + 256 * j;
+            const int at = i < nk ? i : (int)(an_hi - kq_hi) + i - nk, al = i < nk ? i : (int)(an_lo - kq_lo) + i - nk;
+            if (i < nv) {
+                kq_hi[at] += vh[j];
+                kq_lo[al] += vl[j];
+            }
+        }
+        if (threadIdx.x == 0) sBad |= obad;
+        __syncthreads();
+    }
     const int Q = sQ;
     if (last_chunk && Q == 0 && blockIdx.y == 0 && threadIdx.x == 0) atomicOr(&st->flags, 1);
     if (!cok) return;
     const double qd = (double)Q, rq = Q > 0 ? __ddiv_rn(1.0, qd) : __longlong_as_double(0x7ff8000000000000ll);
     const bool bad = (sBad >> cc) & 1u;
-    // M's sum at row r is done: X -= M / 2 / Q, or on to the next pass
-    auto emit = [&](int r, __int128 v, double vd) {
+    // M's sum at row r is done: X -= M / 2 / Q, or on to the next pass; x: X there
+    auto emit = [&](int r, __int128 v, double vd, double x) {
         const size_t off = (size_t)(p0 + r) * C + c;
         bool isd = bad;
         if (!first_chunk) {
@@ -323,7 +367,7 @@ k_mean_fix(const double* __restrict__ X, double* __restrict__ Xout, ulonglong2* 
                 const double q0 = __dmul_rn(val, rq);
                 m = __fma_rn(__fma_rn(-q0, qd, val), rq, q0);
             }
-            Xout[off] = __dsub_rn(X[off], m);
+            Xout[off] = __dsub_rn(x, m);
         } else {
             ulonglong2 o;
             if (isd) {
@@ -339,39 +383,63 @@ k_mean_fix(const double* __restrict__ X, double* __restrict__ Xout, ulonglong2* 
     auto wide = [](unsigned long long hi, unsigned long long lo) -> __int128 {
         return ((__int128)(long long)hi << 52) + (__int128)(long long)lo;
     };
-    // (3) every half of an anchor's T samples is one item: forwards from the
-    //     anchor, or backwards, the cubic's coefficients carried from sample
-    //     to sample and d changed at every knot
-    for (int it = warp * SUB + sub; it < 2 * nA; it += NWS) {
-        const int a = it >> 1, q0 = a * T;
+    // (3) the samples on either side of an anchor, in blocks of at most RB rows
+    //     (one block per subgroup): forwards from the anchor, or backwards, the
+    //     cubic's coefficients carried from sample to sample (at first without
+    //     output, up to the block) and d changed at every knot
+    constexpr int RB = 4;
+    const int nside = pair ? 1 : 2 * ((32 + T - 1) / T);   // sides this CTA covers
+    const int per = max(1, NWS / nside);                   // blocks per side
+    const int rows = (T / 2 + per - 1) / per;              // rows per block, at most RB
+    for (int it = warp * SUB + sub; it < nside * per; it += NWS) {
+        const int sd = it / per, blk = it - sd * per;
+        const int a = pair ? 0 : sd >> 1, back = pair ? half : sd & 1;
+        const int q0 = a * T;
+        if (q0 >= nl) continue;
         const int q1 = min(nl, q0 + T);
         const int ra = q0 + min(T >> 1, nl - 1 - q0);
-        const int rb = (it & 1) ? q0 : ra, re = (it & 1) ? ra : q1;  // rows [rb, re)
+        const int lo = back ? max(q0, ra - (blk + 1) * rows) : ra + blk * rows;  // rows [lo, hi)
+        const int hi = back ? ra - blk * rows : min(q1, lo + rows);
+        if (lo >= hi) continue;
+        double xs[RB];
+#pragma unroll
+        for (int k = 0; k < RB; ++k) xs[k] = last_chunk && lo + k < hi ? X[(size_t)(p0 + lo + k) * C + c] : 0.0;
         if (!bad) {
             const unsigned long long* ah = an_hi + (size_t)(a * 4) * G + cc;
             const unsigned long long* al = an_lo + (size_t)(a * 4) * G + cc;
             __int128 vA = wide(ah[0], al[0]), vB = wide(ah[G], al[G]), vC = wide(ah[2 * G], al[2 * G]),
                      vD = wide(ah[3 * G], al[3 * G]);
-            if (!(it & 1)) {
-                for (int r = rb;;) {
-                    emit(r, vA, 0.0);
-                    if (++r >= re) break;
-                    vA += vB + vC + vD;
-                    vB += 2 * vC + 3 * vD;
-                    vC += 3 * vD;
-                    vD += wide(kq_hi[r * G + cc], kq_lo[r * G + cc]);
+            auto forth = [&](int r) {  // from row r - 1 to row r
+                vA += vB + vC + vD;
+                vB += 2 * vC + 3 * vD;
+                vC += 3 * vD;
+                vD += wide(kq_hi[r * G + cc], kq_lo[r * G + cc]);
+            };
+            auto aback = [&](int r) {  // from row r to row r - 1
+                vD -= wide(kq_hi[r * G + cc], kq_lo[r * G + cc]);
+                vA += vC - vB - vD;
+                vB += 3 * vD - 2 * vC;
+                vC -= 3 * vD;
+            };
+            if (!back) {
+                for (int r = ra + 1; r <= lo; ++r) forth(r);
+#pragma unroll
+                for (int k = 0; k < RB; ++k) {
+                    if (lo + k >= hi) break;
+                    if (k) forth(lo + k);
+                    emit(lo + k, vA, 0.0, xs[k]);
                 }
             } else {
-                for (int r = re; r > rb; --r) {
-                    vD -= wide(kq_hi[r * G + cc], kq_lo[r * G + cc]);
-                    vA += vC - vB - vD;
-                    vB += 3 * vD - 2 * vC;
-                    vC -= 3 * vD;
-                    emit(r - 1, vA, 0.0);
+                for (int r = ra; r > hi; --r) aback(r);
+#pragma unroll
+                for (int k = RB - 1; k >= 0; --k) {
+                    if (lo + k >= hi) continue;
+                    aback(lo + k + 1);
+                    emit(lo + k, vA, 0.0, xs[k]);
                 }
             }
         } else {
-            for (int r = rb; r < re; ++r) {
+            for (int r = lo; r < hi; ++r) {
                 const int n = p0 + r;
                 double sum = 0.0;
                 for (int kk = 0; kk < Kc; ++kk) {
@@ -400,7 +468,7 @@ k_mean_fix(const double* __restrict__ X, double* __restrict__ Xout, ulonglong2* 
                     }
                     sum = __dadd_rn(sum, __dadd_rn(v[0], v[1]));
                 }
-                emit(r, 0, sum);
+                emit(r, 0, sum, last_chunk ? X[(size_t)n * C + c] : 0.0);
             }
         }
     }
