@@ -126,7 +126,10 @@ typedef struct {
     int32_t projection;    /* mixed form: 0 = automatic (tensor cores: 3xTF32
                               tcgen05.mma with TMA-staged tiles), 1 = CUDA
                               cores (FP32 fma); both certify every extremum
-                              test against the FP64 projection */
+                              test against the FP64 projection.  FP64 form: 0 =
+                              automatic (the tensor cores for all but small
+                              records, with the FP64 projection's extrema bit
+                              for bit), 1 = FP64 fma */
     int64_t reserved[2];
 } memd_config;
 
@@ -138,7 +141,8 @@ typedef struct {
     int32_t sifts[64];     /* sifts per IMF (first 64 IMFs) */
     int32_t refined;       /* mixed precision: extremum tests re-decided in
                               double-float because the FP32 margin was within
-                              the projection's error bound */
+                              the projection's error bound (FP64 form on the
+                              tensor cores: re-decided in FP64) */
     int32_t reserved;
 } memd_stats;
 

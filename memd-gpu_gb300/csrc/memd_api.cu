@@ -79,7 +79,7 @@ struct memd_plan {
     void* fac;
     void* rtab;
     void* rtab3;  // impulse-accumulation mean: 1/(3h) as double-float / in FP64
-    unsigned* xexp;            // impulse-accumulation mean, FP64: largest exponent [records][C] of the run's input
+    unsigned* xexp;            // FP64: largest exponent [records][C] of the run's input
     unsigned long long* tot;   // the same, several passes: knots per record over all directions
     unsigned* bnd;  // impulse-accumulation mean, mixed form: [2 passes][2 parts][C] per-channel bounds (float bits)
     int* cumcfg;    // impulse-accumulation mean: anchor span (words) and CTAs per span, set by the factor kernel
@@ -119,15 +119,17 @@ struct memd_plan {
     cudaGraphExec_t exec;
     int64_t graph_launches;
     cudaEvent_t e0, e1;
-    // mixed form, tensor-core projection: tf32 split of the signal and of the
+    // FP64 and mixed forms, tensor-core projection: tf32 split of the signal and of the
     // directions ([rows][Cp], zero-padded channels) and their TMA descriptors
-    int tc;          // k_project_tc replaces k_project_mx
+    int tc;          // k_project_tc replaces k_project_mx / k_project_extrema
     int Cp;          // channels rounded up to 32
     int tc_nt;       // directions per tile (MMA N)
     float* xbig;
     float* xsmall;
     float* dbig;
     float* dsmall;
+    float* xmx;      // FP64 form: largest |x| per 128-sample tile and channel (scaled)
+    float* dfl;      // FP64 form: the directions rounded to float
     memd::TcMaps maps;
     // substitution work queue (persistent sweeps pull segments by ticket)
     int squeue;       // 1: queue, 0: one warp per possible segment
@@ -393,11 +395,17 @@ static cudaError_t set_attrs(memd_plan* p)
     if constexpr (P == MEMD_PREC_MIXED) {
         e = cudaFuncSetAttribute(k_project_mx, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p->proj_smem);
         if (e == cudaSuccess && p->tc)
-            e = cudaFuncSetAttribute(k_project_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            e = cudaFuncSetAttribute(k_project_tc<XT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)tc_smem_bytes(p->tc_nt));
-    } else
+    } else {
         e = cudaFuncSetAttribute(k_project_extrema<R, XT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)p->proj_smem);
+        if constexpr (P == MEMD_PREC_F64) {
+            if (e == cudaSuccess && p->tc)
+                e = cudaFuncSetAttribute(k_project_tc<XT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)tc_smem_bytes(p->tc_nt));
+        }
+    }
     return e;
 }
 
@@ -411,52 +419,62 @@ static void enqueue_sift(memd_plan* p, cudaStream_t s, memd_trace_entry* trace, 
     const Geom& g = p->g;
     const bool stop = p->cfg.stop_mode == MEMD_STOP_CRITERION;
     const int trace_rows = stop && trace ? (int)(p->cfg.num_imfs * (p->cfg.max_iter + 1)) : 0;
-    if constexpr (P == MEMD_PREC_F64) {
-        if (p->cum && p->nchunks > 1) {
-            // several passes: the knots of all directions first, which set the
-            // mean's anchor spacing, so that it does not depend on the passes
-            cudaMemsetAsync(p->tot, 0, sizeof(unsigned long long) * (size_t)std::max(1, p->ep.n), s);
-            for (int ch = 0; ch < p->nchunks; ++ch) {
-                const int k0 = ch * p->Kc, kc = std::min(p->Kc, g.K - k0);
-                lc.begin(MEMD_STAGE_PROJECT);
-                k_project_extrema<R, XT><<<dim3((unsigned)((g.L + kProjTN - 1) / kProjTN),
-                                                (unsigned)((kc + kProjTK - 1) / kProjTK)), 256, p->proj_smem, s>>>(
-                    (const XT*)p->X, (const R*)p->dir, p->bits, g, k0, kc, p->ep);
+    // projection and extrema bitmasks of one direction pass; split: the signal's
+    // tf32 split first (once per sift)
+    auto project = [&](int k0, int kc, bool split) {
+        dim3 pg((unsigned)((g.L + kProjTN - 1) / kProjTN), (unsigned)((kc + kProjTK - 1) / kProjTK));
+        lc.begin(MEMD_STAGE_PROJECT);
+        if constexpr (P != MEMD_PREC_F32) {
+            if (p->tc) {
+                if (split) {
+                    if constexpr (P == MEMD_PREC_MIXED) {
+                        const size_t n = (size_t)g.L * p->Cp;
+                        k_split_tf32<<<(unsigned)std::min<size_t>((n + 255) / 256, 4096), 256, 0, s>>>(
+                            p->X, 1, p->xbig, p->xsmall, g.L, g.C, p->Cp);
+                    } else {
+                        k_split_tf32_f64<<<dim3((unsigned)((g.L + kTcRows - 1) / kTcRows), (unsigned)(p->Cp / 32)), 256, 0,
+                                           s>>>((const double*)p->X, p->xexp, p->xbig, p->xsmall, p->xmx, g.L, g.C, p->Cp,
+                                                p->ep);
+                    }
+                    lc.end(MEMD_STAGE_PROJECT);
+                    lc.begin(MEMD_STAGE_PROJECT);
+                }
+                dim3 tg((unsigned)((g.L + kTcRows - 1) / kTcRows), (unsigned)((kc + p->tc_nt - 1) / p->tc_nt));
+                k_project_tc<XT><<<tg, kTcThreads, tc_smem_bytes(p->tc_nt), s>>>(
+                    p->maps, (const XT*)p->X, P == MEMD_PREC_MIXED ? (const float*)p->dir : p->dfl, p->bits, g, k0, kc,
+                    p->Cp, p->tc_nt, p->st, p->ep, P == MEMD_PREC_MIXED ? nullptr : (const double*)p->dir, p->xmx,
+                    p->xexp);
                 lc.end(MEMD_STAGE_PROJECT);
-                lc.begin(MEMD_STAGE_COMPACT);
-                k_count_knots<<<dim3((unsigned)((g.W + 4095) / 4096), (unsigned)(2 * kc)), 256, 0, s>>>(p->bits, p->tot,
-                                                                                                       g, p->ep);
-                lc.end(MEMD_STAGE_COMPACT);
+                return;
             }
+        }
+        if constexpr (P == MEMD_PREC_MIXED)
+            k_project_mx<<<pg, 256, p->proj_smem, s>>>((const float2*)p->X, (const float*)p->dir,
+                                                       (const float*)p->dir + (size_t)g.K * g.C, p->bits, g, k0, kc,
+                                                       p->st, p->ep);
+        else
+            k_project_extrema<R, XT><<<pg, 256, p->proj_smem, s>>>((const XT*)p->X, (const R*)p->dir, p->bits, g, k0, kc,
+                                                                   p->ep);
+        lc.end(MEMD_STAGE_PROJECT);
+    };
+    const bool recount = P == MEMD_PREC_F64 && p->cum && p->nchunks > 1;
+    if (recount) {
+        // several passes: the knots of all directions first, which set the
+        // mean's anchor spacing, so that it does not depend on the passes
+        cudaMemsetAsync(p->tot, 0, sizeof(unsigned long long) * (size_t)std::max(1, p->ep.n), s);
+        for (int ch = 0; ch < p->nchunks; ++ch) {
+            const int k0 = ch * p->Kc, kc = std::min(p->Kc, g.K - k0);
+            project(k0, kc, ch == 0);
+            lc.begin(MEMD_STAGE_COMPACT);
+            k_count_knots<<<dim3((unsigned)((g.W + 4095) / 4096), (unsigned)(2 * kc)), 256, 0, s>>>(p->bits, p->tot, g,
+                                                                                                   p->ep);
+            lc.end(MEMD_STAGE_COMPACT);
         }
     }
     for (int ch = 0; ch < p->nchunks; ++ch) {
         const int k0 = ch * p->Kc;
         const int kc = std::min(p->Kc, g.K - k0);
-        dim3 pg((unsigned)((g.L + kProjTN - 1) / kProjTN), (unsigned)((kc + kProjTK - 1) / kProjTK));
-        lc.begin(MEMD_STAGE_PROJECT);
-        if constexpr (P == MEMD_PREC_MIXED) {
-            if (p->tc) {
-                if (ch == 0) {  // tf32 split of the signal's first differences, once per sift
-                    const size_t n = (size_t)g.L * p->Cp;
-                    k_split_tf32<<<(unsigned)std::min<size_t>((n + 255) / 256, 4096), 256, 0, s>>>(
-                        p->X, 1, p->xbig, p->xsmall, g.L, g.C, p->Cp);
-                    lc.end(MEMD_STAGE_PROJECT);
-                    lc.begin(MEMD_STAGE_PROJECT);
-                }
-                dim3 tg((unsigned)((g.L + kTcRows - 1) / kTcRows), (unsigned)((kc + p->tc_nt - 1) / p->tc_nt));
-                k_project_tc<<<tg, kTcThreads, tc_smem_bytes(p->tc_nt), s>>>(
-                    p->maps, (const float2*)p->X, (const float*)p->dir, p->bits, g, k0, kc, p->Cp, p->tc_nt, p->st,
-                    p->ep);
-            } else {
-                k_project_mx<<<pg, 256, p->proj_smem, s>>>((const float2*)p->X, (const float*)p->dir,
-                                                           (const float*)p->dir + (size_t)g.K * g.C, p->bits, g, k0, kc,
-                                                           p->st, p->ep);
-            }
-        } else
-            k_project_extrema<R, XT><<<pg, 256, p->proj_smem, s>>>((const XT*)p->X, (const R*)p->dir, p->bits, g, k0, kc,
-                                                                   p->ep);
-        lc.end(MEMD_STAGE_PROJECT);
+        project(k0, kc, ch == 0 && !recount);
         if (g.mirror) {
             const unsigned mb = (unsigned)((32L * kc + 127) / 128);
             lc.begin(MEMD_STAGE_PROJECT);
@@ -760,9 +778,17 @@ static void split_directions(memd_plan* p, cudaStream_t s, Launches& lc)
 {
     if (!p->tc) return;
     const size_t n = (size_t)p->g.K * p->Cp;
+    const void* d = p->dir;
+    if (p->prec == MEMD_PREC_F64) {
+        const int kc = p->g.K * p->g.C;
+        lc.begin(MEMD_STAGE_OTHER);
+        k_float_directions<<<(unsigned)std::min((kc + 255) / 256, 1024), 256, 0, s>>>((const double*)p->dir, p->dfl, kc);
+        lc.end(MEMD_STAGE_OTHER);
+        d = p->dfl;
+    }
     lc.begin(MEMD_STAGE_OTHER);
-    k_split_tf32<<<(unsigned)std::min<size_t>((n + 255) / 256, 1024), 256, 0, s>>>(p->dir, 0, p->dbig, p->dsmall,
-                                                                                   p->g.K, p->g.C, p->Cp);
+    k_split_tf32<<<(unsigned)std::min<size_t>((n + 255) / 256, 1024), 256, 0, s>>>(d, 0, p->dbig, p->dsmall, p->g.K,
+                                                                                   p->g.C, p->Cp);
     lc.end(MEMD_STAGE_OTHER);
 }
 
@@ -798,8 +824,8 @@ static void enqueue_inputs(memd_plan* p, const typename Prec<P>::T* d_y, const t
     cudaMemcpyAsync(p->dir, d_dir, sizeof(T) * (size_t)g.K * g.C, cudaMemcpyDeviceToDevice, s);
     if constexpr (P == MEMD_PREC_MIXED) {  // float directions: the low words are zero
         cudaMemsetAsync((float*)p->dir + (size_t)g.K * g.C, 0, sizeof(float) * (size_t)g.K * g.C, s);
-        split_directions(p, s, lc);
     }
+    split_directions(p, s, lc);
 }
 
 template <int P>
@@ -954,9 +980,9 @@ static memd_status batched_inputs(memd_plan* p, int n, const int64_t* lengths, c
     cudaMemcpyAsync(p->dir, d_dir, sizeof(T) * (size_t)g.K * C, cudaMemcpyDeviceToDevice, s);
     if constexpr (P == MEMD_PREC_MIXED) {
         cudaMemsetAsync((float*)p->dir + (size_t)g.K * C, 0, sizeof(float) * (size_t)g.K * C, s);
-        Launches lc;
-        split_directions(p, s, lc);
     }
+    Launches lc;
+    split_directions(p, s, lc);
     // the copies and clears above must have been accepted before the graph
     // runs on the buffers they fill
     e = cudaGetLastError();
@@ -1413,8 +1439,8 @@ static memd_status create_plan(const memd_config* cfg, const memd_tuning* tun, m
     const int Lh = p->batched ? std::max(p->Lrec, kEpochAlign) : (p->g.mirror ? 2 * L : L);
     ALLOC(p->rtab, rb * (size_t)(Lh + 1));
     if (p->cum) ALLOC(p->rtab3, (f64 ? 16 : 8) * (size_t)(Lh + 1));
+    if (f64) ALLOC(p->xexp, sizeof(unsigned) * (size_t)std::max<int64_t>(1, c.max_epochs) * C);
     if (p->cum && f64) {
-        ALLOC(p->xexp, sizeof(unsigned) * (size_t)std::max<int64_t>(1, c.max_epochs) * C);
         if (p->nchunks > 1) ALLOC(p->tot, sizeof(unsigned long long) * (size_t)std::max<int64_t>(1, c.max_epochs));
     } else if (p->cum) {
         ALLOC(p->bnd, sizeof(unsigned) * 4 * (size_t)C);
@@ -1435,9 +1461,13 @@ static memd_status create_plan(const memd_config* cfg, const memd_tuning* tun, m
         ALLOC(p->ep_yoff, sizeof(long long) * me);
         ALLOC(p->ep.cnt, sizeof(int) * 2 * (size_t)K * me);
     }
-    // mixed form: the tensor-core projection's tf32 splits
+    // FP64 and mixed forms: the tensor-core projection's tf32 splits
     p->Cp = (C + kTcKB - 1) / kTcKB * kTcKB;
-    p->tc = c.precision == MEMD_PREC_MIXED && c.projection == 0;
+    // FP64: from 5e6 direction-channel-samples on (8 x 2,000 x 64: 10 us a sift on
+    // the FP64 pipe, 20 split + product; 19 x 7,501 x 50: 31 against 26; 32 x
+    // 30,504 x 64: 132 against 41), or where the tile width is given
+    p->tc = c.projection == 0 && (c.precision == MEMD_PREC_MIXED ||
+                                  (f64 && (tu.proj_tile_n || (double)K * C * L >= 5e6)));
     if (p->tc) {
         // directions per tile: 64 by default (more, narrower tiles keep more
         // CTAs in flight; the kernel is latency-bound, not tensor-bound)
@@ -1446,6 +1476,10 @@ static memd_status create_plan(const memd_config* cfg, const memd_tuning* tun, m
         ALLOC(p->xsmall, sizeof(float) * (size_t)L * p->Cp);
         ALLOC(p->dbig, sizeof(float) * (size_t)K * p->Cp);
         ALLOC(p->dsmall, sizeof(float) * (size_t)K * p->Cp);
+        if (f64) {
+            ALLOC(p->xmx, sizeof(float) * (size_t)((L + kTcRows - 1) / kTcRows) * p->Cp);
+            ALLOC(p->dfl, sizeof(float) * (size_t)K * C);
+        }
     }
     p->squeue = tu.solve_queue == 1;
     p->cum_ctas = tu.mean_ctas ? tu.mean_ctas : 2048;

@@ -1,4 +1,5 @@
-// memd_tc.cuh -- projection + extrema bitmasks on the tensor cores (mixed form).
+// memd_tc.cuh -- projection + extrema bitmasks on the tensor cores (mixed and
+// FP64 forms).
 //
 // The reference projects with cublasSgemm (memReducedEpochs_dev.cu:1182-1184)
 // and then flags strict local extrema of every projected direction
@@ -40,6 +41,18 @@
 // sample-to-sample change rather than its size: smooth late-IMF signals, whose
 // neighbouring projections agree to many digits, stay decidable on the tensor
 // cores.
+//
+// FP64 form.  The extrema are those of the FP64 projections summed over the
+// channels in order with fma (k_project_extrema), bit for bit: the bound also
+// covers their rounding, 2 (C + 1) 2^-53 sum_c |d_c| max|x_c| over the tile,
+// the truncation of the differences (2^-23 S) and the directions' rounding to
+// float (2^-24 S), and a sign within it is decided again from those
+// projections themselves.  The differences are scaled by a power of two per
+// record (the exponent of its largest input sample), so that the float range
+// does not limit the signal's; whatever still leaves it is decided in FP64.
+// Rows equal to a neighbour in every channel need no decision.
+// 32 x 30,504, 64 directions: 132 us a sift with k_project_extrema (bound by
+// the FP64 pipe), 7 us split + 30 .. 37 us here.
 //
 // Every wait on an mbarrier is bounded (iterations and clock); a wait that
 // runs out sets MEMD_FLAG_DEVICE_TIMEOUT in the run state, waits (bounded)
@@ -118,6 +131,76 @@ __global__ void k_split_tf32(const void* __restrict__ src, int diff, float* __re
     }
 }
 
+// v 2^-ex as a float, truncated, by integer instructions (conversions run on
+// the FP64 pipe); 0 below float's normal range, infinite above it
+__device__ __forceinline__ float scaled_float(double v, int ex)
+{
+    const unsigned h = (unsigned)__double2hiint(v), l = (unsigned)__double2loint(v);
+    const int be = (int)((h >> 20) & 0x7ffu);
+    const int e = be - 1023 - ex + 127;
+    const unsigned m = ((h << 3) | (l >> 29)) & 0x7fffffu;
+    unsigned r = ((unsigned)e << 23) | m;
+    if (be == 0 || e <= 0) r = 0u;
+    else if (be == 0x7ff || e >= 255) r = 0x7f800000u;
+    return __uint_as_float(r | (h & 0x80000000u));
+}
+// exponent of the record's scale: of its largest input sample, over the channels
+__device__ __forceinline__ int record_scale(const unsigned* __restrict__ xexp, int rec, int C)
+{
+    unsigned m = 0u;
+    for (int c = (int)(threadIdx.x & 31); c < C; c += 32) m = max(m, xexp[(size_t)rec * C + c]);
+    m = __reduce_max_sync(kFull, m);
+    return m ? (int)m - 1022 : 0;
+}
+
+// FP64 form: the same split of the scaled first differences, and the largest
+// |x| of every 128-sample tile (with the rows before and after it) and channel,
+// xmx[tile][Cp].  CTA: one tile x 32 channels, warp w = rows 16 w .. 16 w + 15.
+__global__ void __launch_bounds__(256)
+k_split_tf32_f64(const double* __restrict__ X, const unsigned* __restrict__ xexp, float* __restrict__ big,
+                 float* __restrict__ small, float* __restrict__ xmx, int rows, int C, int Cp, Epochs ep)
+{
+    __shared__ float wmx[8][32];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int n0 = blockIdx.x * 128, c = blockIdx.y * 32 + lane;
+    const int ex = record_scale(xexp, ep.n > 0 ? ep.wep[n0 >> 5] : 0, C);
+    const bool cin = c < C;
+    constexpr int RW = 16;
+    const int r0 = n0 + warp * RW;
+    double x[RW + 2];  // rows r0 - 1 .. r0 + RW
+#pragma unroll
+    for (int k = 0; k < RW + 2; ++k) {
+        const int r = r0 - 1 + k;
+        x[k] = cin && r >= 0 && r < rows ? X[(size_t)r * C + c] : 0.0;
+    }
+    float m = 0.f;
+#pragma unroll
+    for (int k = 0; k < RW + 2; ++k) m = fmaxf(m, fabsf(scaled_float(x[k], ex)));
+#pragma unroll
+    for (int k = 0; k < RW; ++k) {
+        const int r = r0 + k;
+        if (r < rows) {
+            const float v = cin && r > 0 ? scaled_float(__dsub_rn(x[k + 1], x[k]), ex) : 0.f;
+            const float b = tf32_rna(v);
+            big[(size_t)r * Cp + c] = b;
+            small[(size_t)r * Cp + c] = tf32_rna(__fsub_rn(v, b));
+        }
+    }
+    wmx[warp][lane] = m;
+    __syncthreads();
+    if (warp == 0) {
+#pragma unroll
+        for (int w = 1; w < 8; ++w) m = fmaxf(m, wmx[w][lane]);
+        xmx[(size_t)blockIdx.x * Cp + c] = m * 1.000001f;  // the truncation undone
+    }
+}
+
+// FP64 directions rounded to float
+__global__ void k_float_directions(const double* __restrict__ d, float* __restrict__ f, int n)
+{
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) f[i] = (float)d[i];
+}
+
 struct TcMaps {
     CUtensorMap xb, xs, db, ds;
 };
@@ -167,13 +250,33 @@ __device__ __noinline__ int warp_df_diff_sign(const float2* __restrict__ x1, con
     return __shfl_sync(kFull, dd_sign(acc), 0);
 }
 
+// the FP64 form's projection of one sample (k_project_extrema's sum)
+__device__ __forceinline__ double proj_f64(const double* __restrict__ x, const double* __restrict__ d, int C)
+{
+    double a = 0.0;
+    for (int c = 0; c < C; ++c) a = __fma_rn(x[c], d[c], a);
+    return a;
+}
+// are two rows the same in every channel (bits)?
+__device__ __forceinline__ bool same_rows(const double* __restrict__ a, const double* __restrict__ b, int C)
+{
+    for (int c = 0; c < C; ++c)
+        if (__double_as_longlong(a[c]) != __double_as_longlong(b[c])) return false;
+    return true;
+}
+
 // Grid: (ceil(L / 128), ceil(Kc / nt)); nt = directions per tile (a multiple
 // of 16 in [16, 256]; narrower tiles give more CTAs, each loading the same
 // signal tile).
+template <typename XT>
 __global__ void __launch_bounds__(kTcThreads)
-k_project_tc(const __grid_constant__ TcMaps maps, const float2* __restrict__ X, const float* __restrict__ dh_all,
-             uint32_t* __restrict__ bits, Geom g, int k0, int Kc, int Cp, int nt, RunState* st, Epochs ep)
+k_project_tc(const __grid_constant__ TcMaps maps, const XT* __restrict__ X, const float* __restrict__ dh_all,
+             uint32_t* __restrict__ bits, Geom g, int k0, int Kc, int Cp, int nt, RunState* st, Epochs ep,
+             const double* __restrict__ d_all, const float* __restrict__ xmx, const unsigned* __restrict__ xexp)
 {
+    // XT: float2 (mixed form) or double (FP64 form: d_all the FP64 directions,
+    // dh_all their rounding to float, xmx and xexp from the split)
+    constexpr bool F64 = std::is_same<XT, double>::value;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     // operand tiles at a 1024-byte boundary (the 128-byte swizzle repeats
     // every 8 rows of 128 bytes)
@@ -234,6 +337,8 @@ k_project_tc(const __grid_constant__ TcMaps maps, const float2* __restrict__ X, 
         tma_load_2d(Bs, &maps.ds, &bars[0], 0, k0 + kt0);
     }
 
+    const int ex = F64 && warp == 0 ? record_scale(xexp, ep.n > 0 ? ep.wep[n0 >> 5] : 0, C) : 0;
+    const float eps = (float)(4 * C + 8) * 2.384185791e-7f + (F64 ? 1.9e-7f : 5.9604645e-8f);  // FP64: 2^-23 + 2^-24, rounded up
     int fail = 0, kb = 0;  // fail: 1 = a copy, 2 = the products did not complete in time
     for (; kb < nkb; ++kb) {
         if (tid == 0 && kb > 0) {
@@ -246,7 +351,13 @@ k_project_tc(const __grid_constant__ TcMaps maps, const float2* __restrict__ X, 
         // the halo row's differences of this block (while the copies land)
         if (tid < 32) {
             const int c = kb * kTcKB + tid;
-            xd[tid] = (has_halo && c < C) ? xdiff(X[(size_t)nh * C + c], X[(size_t)(nh - 1) * C + c]).hi : 0.f;
+            float v = 0.f;
+            if (has_halo && c < C) {
+                const XT a = X[(size_t)nh * C + c], b = X[(size_t)(nh - 1) * C + c];
+                if constexpr (F64) v = scaled_float(__dsub_rn(a, b), ex);
+                else v = xdiff(a, b).hi;
+            }
+            xd[tid] = v;
         }
         const bool got = mbar_wait_bounded(&bars[0], (uint32_t)(kb & 1), kTcWaitClocks);
         if (__syncthreads_or(!got)) {  // the same decision in every thread
@@ -282,7 +393,13 @@ k_project_tc(const __grid_constant__ TcMaps maps, const float2* __restrict__ X, 
         __syncthreads();
         if (warp == 0) {
             const float m = fmaxf(fmaxf(cmx[lane], cmx[32 + lane]), fmaxf(cmx[64 + lane], cmx[96 + lane]));
-            mx[lane] = fmaxf(m, fabsf(xd[lane])) * 1.0009765625f;
+            float b = fmaxf(m, fabsf(xd[lane])) * 1.0009765625f;
+            if constexpr (F64) {
+                // the bound itself: the differences' part and the FP64 projections'
+                const float e64 = (float)(2 * (C + 1)) * 1.11022303e-16f;
+                b = __fmaf_ru(eps, b, __fmul_ru(e64, xmx[(size_t)blockIdx.x * Cp + kb * kTcKB + lane]));
+            }
+            mx[lane] = b;
         }
         __syncthreads();
         // this block's part of the halo row and of the bound sum, per
@@ -342,9 +459,10 @@ k_project_tc(const __grid_constant__ TcMaps maps, const float2* __restrict__ X, 
     }
     // the bound on |D_tc - D| per direction, with the margin for its own rounding
     {
-        const float eps = (float)(4 * C + 8) * 2.384185791e-7f + 5.9604645e-8f;  // (4C + 8) 2^-22 + 2^-24
-        for (int kk = tid; kk < nk; kk += kTcThreads)
-            thr[kk] = 1.01f * __fmul_ru(eps, thr[kk]);
+        for (int kk = tid; kk < nk; kk += kTcThreads) {
+            if constexpr (F64) thr[kk] = __fmaf_ru(1.01f, thr[kk], 7.9e-31f);  // 2^-100: what underflow can hide
+            else thr[kk] = 1.01f * __fmul_ru(eps, thr[kk]);
+        }
     }
     // pass 1: every warp publishes its lane 0 (its first sample) for the warp before
     const uint32_t tl = taddr + ((uint32_t)(warp * 32) << 16);
@@ -366,6 +484,7 @@ k_project_tc(const __grid_constant__ TcMaps maps, const float2* __restrict__ X, 
     sample_rule(g, ep, n, inrange, endpt, interior);
     const int w = (n0 >> 5) + warp;
     int refined = 0;
+    [[maybe_unused]] int flat = -1;  // FP64: the lane's row equals a neighbour (-1: not looked at)
     for (int j0 = 0; j0 < nt; j0 += 32) {
         float v[32];
         __syncwarp();
@@ -382,14 +501,34 @@ k_project_tc(const __grid_constant__ TcMaps maps, const float2* __restrict__ X, 
             if (d0 < 0.f && d1 > 0.f) mnm |= 1u << j;
             if (interior && kk < nk) {
                 const float t = thr[kk];
-                if (fabsf(d0) <= t || fabsf(d1) <= t) nearm |= 1u << j;
+                // (FP64: a NaN is near, too)
+                if (F64 ? !(fabsf(d0) > t && fabsf(d1) > t) : (fabsf(d0) <= t || fabsf(d1) <= t)) nearm |= 1u << j;
             }
         }
         refined += __popc(nearm);
         // signs within the bound: decided again in double-float, one
         // (direction, lane) at a time by the whole warp (lanes over channels)
         uint32_t anyj = __reduce_or_sync(kFull, nearm);
-        while (anyj) {
+        if constexpr (F64) {
+            if (anyj && flat < 0)  // once per tile
+                flat = interior && (same_rows(X + (size_t)n * C, X + (size_t)(n - 1) * C, C) ||
+                                             same_rows(X + (size_t)(n + 1) * C, X + (size_t)n * C, C));
+            if (flat > 0 && nearm) mxm = mnm = nearm = 0u;  // equal neighbours: no strict extremum in any direction
+            anyj = __reduce_or_sync(kFull, nearm);
+            while (anyj) {
+                const int j = __ffs(anyj) - 1;
+                anyj &= anyj - 1u;
+                if ((nearm >> j) & 1u) {
+                    const double* dk = d_all + (size_t)(k0 + kt0 + j0 + j) * C;
+                    const double* xn = X + (size_t)n * C;
+                    const double a = proj_f64(xn - C, dk, C), b = proj_f64(xn, dk, C), e = proj_f64(xn + C, dk, C);
+                    const uint32_t bit = 1u << j;
+                    mxm = (b > a && b > e) ? (mxm | bit) : (mxm & ~bit);
+                    mnm = (b < a && b < e) ? (mnm | bit) : (mnm & ~bit);
+                }
+                __syncwarp();
+            }
+        } else while (anyj) {
             const int j = __ffs(anyj) - 1;
             anyj &= anyj - 1u;
             const int kk = j0 + j;
@@ -398,7 +537,7 @@ k_project_tc(const __grid_constant__ TcMaps maps, const float2* __restrict__ X, 
             while (need) {
                 const int l = __ffs(need) - 1;
                 need &= need - 1u;
-                const float2* xl = X + (size_t)(n0 + warp * 32 + l) * C;
+                const XT* xl = X + (size_t)(n0 + warp * 32 + l) * C;
                 const int s0 = warp_df_diff_sign(xl, xl - C, dh, C, lane);
                 const int s1 = warp_df_diff_sign(xl + C, xl, dh, C, lane);
                 if (lane == l) {
