@@ -78,7 +78,8 @@ struct memd_plan {
     void* dbuf;  // forward-eliminated right-hand sides [2][Kc][cap][C]
     void* fac;
     void* rtab;
-    void* rtab3;  // impulse-accumulation mean: 1/(3h) as double-float / in FP64
+    void* rtab3;  // impulse-accumulation mean: 1/(3h) and h/3, double-float (two tables) / FP64 (pairs)
+    int ntab;     // entries of the reciprocal tables
     unsigned* xexp;            // FP64: largest exponent [records][C] of the run's input
     unsigned long long* tot;   // the same, several passes: knots per record over all directions
     unsigned* bnd;  // impulse-accumulation mean, mixed form: [2 passes][2 parts][C] per-channel bounds (float bits)
@@ -324,9 +325,10 @@ static void launch_eval(memd_plan* p, cudaStream_t s, int k0, int kc, int first,
     if (p->cumG == G_) {                                                                                           \
         dim3 grid((unsigned)((g.W + kCumMaxWords - 1) / kCumMaxWords * kCumMaxWords),                             \
                   (unsigned)((g.C + G_ - 1) / G_));                                                                \
-        k_mean_cum<G_><<<grid, 256, sizeof(unsigned long long) * (32 * kCumMaxWords + 3) * G_, s>>>(               \
+        k_mean_cum<G_><<<grid, 256, sizeof(unsigned long long) * 32 * kCumMaxWords * G_, s>>>(               \
             (const float2*)p->X, (float2*)p->Xb, (dd*)p->acc, p->bits, p->wpref, p->knots, p->cnt,               \
-                                            (const dd*)p->rtab, (const dd*)p->rtab3, (const dd*)p->sv,           \
+                                            (const dd*)p->rtab, (const dd*)p->rtab3,                             \
+                                            (const dd*)p->rtab3 + p->ntab, (const dd*)p->sv,                      \
                                             (const dd*)p->yend, cur, other, p->cumcfg, p->cumsh, g, k0, kc, first,\
                                             last, p->st, p->ep);                                                   \
         return;                                                                                                    \
@@ -385,7 +387,7 @@ static cudaError_t set_attrs(memd_plan* p)
     if constexpr (P == MEMD_PREC_MIXED) {
         const int cb[3] = {32, 16, 8};
         for (int i = 0; i < 3 && e == cudaSuccess; ++i) {
-            const int bytes = (int)sizeof(unsigned long long) * (32 * kCumMaxWords + 3) * cb[i];
+            const int bytes = (int)sizeof(unsigned long long) * 32 * kCumMaxWords * cb[i];
             if (cb[i] == 32) e = cudaFuncSetAttribute(k_mean_cum<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
             if (cb[i] == 16) e = cudaFuncSetAttribute(k_mean_cum<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
             if (cb[i] == 8) e = cudaFuncSetAttribute(k_mean_cum<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
@@ -1438,14 +1440,15 @@ static memd_status create_plan(const memd_config* cfg, const memd_tuning* tun, m
     // longest knot gap: a record (epoch) length; mirrored knots reach 2L - 2
     const int Lh = p->batched ? std::max(p->Lrec, kEpochAlign) : (p->g.mirror ? 2 * L : L);
     ALLOC(p->rtab, rb * (size_t)(Lh + 1));
-    if (p->cum) ALLOC(p->rtab3, (f64 ? 16 : 8) * (size_t)(Lh + 1));
+    p->ntab = Lh + 1;
+    if (p->cum) ALLOC(p->rtab3, 16 * (size_t)(Lh + 1));
     if (f64) ALLOC(p->xexp, sizeof(unsigned) * (size_t)std::max<int64_t>(1, c.max_epochs) * C);
     if (p->cum && f64) {
         if (p->nchunks > 1) ALLOC(p->tot, sizeof(unsigned long long) * (size_t)std::max<int64_t>(1, c.max_epochs));
     } else if (p->cum) {
         ALLOC(p->bnd, sizeof(unsigned) * 4 * (size_t)C);
         ALLOC(p->cumcfg, sizeof(int) * 4);
-        ALLOC(p->cumsh.kq, sizeof(unsigned long long) * 35 * (size_t)p->g.W * C);
+        ALLOC(p->cumsh.kq, sizeof(unsigned long long) * 32 * (size_t)p->g.W * C);
         ALLOC(p->cumsh.anc, sizeof(unsigned long long) * 4 * (size_t)p->g.W * C);
         ALLOC(p->cumsh.arrive, sizeof(int) * (size_t)p->g.W * ((C + 7) / 8));
     }
@@ -1542,7 +1545,7 @@ static memd_status create_plan(const memd_config* cfg, const memd_tuning* tun, m
     if (e == cudaSuccess) e = cudaMemset(p->csh.hacc, 0, sizeof(unsigned long long) * 2 * (size_t)p->Kc);
     if (e == cudaSuccess) e = cudaMemset(p->csh.arrive, 0, sizeof(int) * 2 * (size_t)p->Kc);
     if (e == cudaSuccess && p->cum && !f64) {
-        e = cudaMemset(p->cumsh.kq, 0, sizeof(unsigned long long) * 35 * (size_t)p->g.W * C);
+        e = cudaMemset(p->cumsh.kq, 0, sizeof(unsigned long long) * 32 * (size_t)p->g.W * C);
         if (e == cudaSuccess) e = cudaMemset(p->cumsh.anc, 0, sizeof(unsigned long long) * 4 * (size_t)p->g.W * C);
         if (e == cudaSuccess) e = cudaMemset(p->cumsh.arrive, 0, sizeof(int) * (size_t)p->g.W * ((C + 7) / 8));
         if (e == cudaSuccess) e = cudaMemset(p->cumcfg, 0, sizeof(int) * 4);

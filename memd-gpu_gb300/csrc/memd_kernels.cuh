@@ -1350,16 +1350,14 @@ k_eval_w(XT* __restrict__ X, R* __restrict__ acc_buf, const uint32_t* __restrict
 // A natural cubic spline with knots x_j is, for n >= x_0,
 //     S(n) = P_0(n) + sum_j dd_j (n - x_j)_+^3,   dd_j = d_j - d_{j-1}
 // (the pieces agree in value, slope and curvature at every interior knot;
-// only the cubic coefficient d jumps).  The fourth forward difference of
-// (n - x)_+^3 is 1, 4, 1 at n = x-3, x-2, x-1 and zero elsewhere, so the sum
-// over all envelopes M(n) = sum_e S_e(n) obeys
-//     Delta^4 M(n) = I(n) = sum over interior knots of dd_j * {1,4,1}.
+// only the cubic coefficient d jumps), so the sum over all envelopes M(n) =
+// sum_e S_e(n) is one cubic between any two neighbouring samples whose
+// third-order coefficient changes, at a sample, by the sum of the jumps there.
 // Per span of 32 m samples (m = 1 .. 4 words, longer where the knots are
-// sparse) the kernel anchors M at the middle sample n_a (value and the first
-// three forward differences of the pieces active there, plus the impulses that
-// knots at n_a+1, n_a+2 place before n_a), then rebuilds M(n) by running the
-// difference recurrence forwards and backwards over the span.  Work per span:
-// O(knots + envelopes) instead of O(envelopes x samples).
+// sparse) the kernel anchors M at the middle sample n_a (the sums of the
+// Taylor coefficients of the pieces active there), then rebuilds M(n) by
+// carrying the cubic's coefficients forwards and backwards over the span.
+// Work per span: O(knots + envelopes) instead of O(envelopes x samples).
 //
 // The jumps q_j - q_{j-1} (q_j: d_j quantised), the anchor sums and the
 // recurrence are integers in units of q = 2^(e - 62), 2^e > 2 Kc B_c, with B_c
@@ -1376,37 +1374,92 @@ k_eval_w(XT* __restrict__ X, R* __restrict__ acc_buf, const uint32_t* __restrict
 //
 // CTA: one span (or one of the P parts of a span's directions) x G channels,
 // 8 warps, four CTAs per SM (64 registers; the accumulators of a span of at
-// most 128 samples take 33.5 KB); lane = (subgroup, channel), the (direction,
+// most 128 samples take 32.8 KB); lane = (subgroup, channel), the (direction,
 // envelope) pairs are dealt round-robin to the 8 * 32/G subgroups, which add
-// each knot's jump into a per-row array in shared memory (one 64-bit integer
-// atomic per knot).  The recurrence runs as four block-wide exact prefix sums
-// plus the cubic that matches the anchor state, so all warps share it.
+// each knot's jump into a per-row array in shared memory.  The samples on each
+// side of the anchor are dealt to all warps, each walking from the anchor to
+// its block first.
+// Bound by instruction issue (63% of the slots at 4 CTAs per SM, the rest load
+// latency).  Sums over a decomposition of 32 x 30,504, 128 directions, 80
+// sifts: 18.96 ms with mantissa shifts for the conversions, 64-bit shared
+// atomics and block-wide prefix sums that needed the knots of three samples
+// past the span; 15.42 ms with limbs, 32-bit atomics with a carry and the walk;
+// 14.89 ms with the anchor's products summed before they are rounded.
 // ---------------------------------------------------------------------------
 // The double-float v times 2^sh as a 64-bit two's-complement integer (|v 2^sh|
-// < 2^62), rounded to nearest (ties up) from the 48-bit combined mantissa, by
-// integer instructions only: the float-to-int64 conversion instructions run on
-// the FP64 pipe, 1/64 of the FP32 rate on this GPU.  Rounding to nearest keeps
-// the conversions unbiased: a truncation's one-sided error accumulates over
-// the sifts of a decomposition.
-__device__ __forceinline__ unsigned long long qfix(dd v, int sh)
+// < 2^62), rounded to nearest, in three limbs a 2^44 + b 2^22 + c that are kept
+// as float bit patterns: adding 1.5 2^23 to a float of magnitude <= 2^22 rounds
+// it to an integer, which the low bits of the sum then hold.  The conversion
+// instructions to 64-bit integers run on the FP64 pipe, 1/64 of the FP32 rate;
+// shifting the mantissas by their exponents took 33 instructions, this takes
+// 11, and differences of two values need no more than differences of the
+// patterns.  Rounding to nearest keeps the conversions unbiased: a truncation's
+// one-sided error accumulates over the sifts of a decomposition.
+struct Limbs {
+    unsigned a, b, c;
+};
+constexpr float kMagic = 12582912.0f;
+constexpr unsigned kMagicBits = 0x4b400000u;
+// s44 = 2^(sh - 44), s22 = 2^(sh - 22)
+__device__ __forceinline__ Limbs to_limbs(dd v, float s44, float s22)
 {
-    const unsigned uh = __float_as_uint(v.hi), ul = __float_as_uint(v.lo);
-    const int eh = (int)((uh >> 23) & 0xffu), el = (int)((ul >> 23) & 0xffu);
-    if (eh == 0) return 0ull;  // zero (or subnormal): below any quantum in use
-    int mh = (int)((uh & 0x7fffffu) | 0x800000u);
-    int ml = (el == 0) ? 0 : (int)((ul & 0x7fffffu) | 0x800000u);
-    if (uh >> 31) mh = -mh;
-    if (ul >> 31) ml = -ml;
-    // lo in units of 2^(eh - 174): ml 2^(el - eh + 24); |lo| <= ulp(hi) gives el <= eh - 23
-    const int dl = eh - el - 24;
-    const int mlo = (dl < 0) ? ml * 2 : (dl == 0 ? ml : (dl < 31 ? ((ml + (1 << (dl - 1))) >> dl) : 0));
-    const long long comb = (long long)mh * (1ll << 24) + (long long)mlo;  // |comb| < 2^48
-    const int s = eh - 174 + sh;                                           // value 2^sh = comb 2^s
-    long long r;
-    if (s >= 0) r = (long long)((unsigned long long)comb << min(s, 63));
-    else if (s > -63) r = (comb + (1ll << (-s - 1))) >> (-s);
-    else r = 0;
-    return (unsigned long long)r;
+    const float ma = __fmaf_rn(v.hi, s44, kMagic);
+    const float ra = __fmaf_rn(v.hi, s44, -__fsub_rn(ma, kMagic));  // exact, |ra| <= 1/2
+    const float mb = __fmaf_rn(ra, 4194304.0f, kMagic);
+    const float rb = __fmaf_rn(ra, 4194304.0f, -__fsub_rn(mb, kMagic));
+    const float ml = __fmaf_rn(v.lo, s22, kMagic);  // |lo| <= ulp(hi) / 2: below 2^16
+    const float rl = __fmaf_rn(v.lo, s22, -__fsub_rn(ml, kMagic));
+    const float mc = __fmaf_rn(__fadd_rn(rb, rl), 4194304.0f, kMagic);
+    return Limbs{__float_as_uint(ma), __float_as_uint(mb) + __float_as_uint(ml), __float_as_uint(mc)};
+}
+// x - y
+__device__ __forceinline__ unsigned long long limbs_diff(Limbs x, Limbs y)
+{
+    const long long m = (long long)(int)(x.b - y.b) * 4194304ll + (long long)(int)(x.c - y.c);
+    return (unsigned long long)m + ((unsigned long long)((x.a - y.a) << 12) << 32);
+}
+__device__ __forceinline__ unsigned long long limbs_value(Limbs x)
+{
+    return limbs_diff(x, Limbs{kMagicBits, 2u * kMagicBits, kMagicBits});
+}
+// v added to the 64-bit accumulator kept as two words, lo[i] and hi[i]: the
+// carry out of the native 32-bit addition goes with the high word (a 64-bit
+// addition in shared memory is a compare-and-swap loop)
+__device__ __forceinline__ void add_words(unsigned* lo, unsigned* hi, int i, unsigned long long v)
+{
+    const unsigned l = (unsigned)v;
+    const unsigned old = atomicAdd(&lo[i], l);
+    atomicAdd(&hi[i], (unsigned)(v >> 32) + (old + l < l ? 1u : 0u));
+}
+
+// sum of double-floats without renormalising: the high words by an error-free
+// addition, its error and the low words in l
+struct Acc {
+    float h, l;
+};
+__device__ __forceinline__ void acc_add(Acc& s, float hi, float lo)
+{
+    const float t = __fadd_rn(s.h, hi);
+    const float bb = __fsub_rn(t, s.h);
+    s.l = __fadd_rn(s.l, __fadd_rn(__fadd_rn(__fsub_rn(s.h, __fsub_rn(t, bb)), __fsub_rn(hi, bb)), lo));
+    s.h = t;
+}
+// s += a t, t a plain float
+__device__ __forceinline__ void acc_mulf(Acc& s, dd a, float t)
+{
+    const float p = __fmul_rn(a.hi, t);
+    acc_add(s, p, __fmaf_rn(a.lo, t, __fmaf_rn(a.hi, t, -p)));
+}
+__device__ __forceinline__ dd acc_dd(Acc s) { return dd_renorm(s.h, s.l); }
+// a b - c d
+__device__ __forceinline__ dd dd_diff_of_products(dd a, dd b, dd c, dd d)
+{
+    const float p = __fmul_rn(a.hi, b.hi), q = __fmul_rn(c.hi, d.hi);
+    const float e = __fmaf_rn(a.lo, b.hi, __fmaf_rn(a.hi, b.lo, __fmaf_rn(a.hi, b.hi, -p)));
+    const float f = __fmaf_rn(c.lo, d.hi, __fmaf_rn(c.hi, d.lo, __fmaf_rn(c.hi, d.hi, -q)));
+    Acc s{p, e};
+    acc_add(s, -q, -f);
+    return acc_dd(s);
 }
 
 // the non-negative integer a (< 2^63) times 2^-sh as a float, truncated to
@@ -1457,7 +1510,7 @@ constexpr int kCumMaxParts = 4;  // most CTAs sharing one span
 // Global accumulators of the spans split over several CTAs (zero between
 // launches: the CTA that finishes a span clears them).
 struct CumShared {
-    unsigned long long* kq;   // [W][35][C]: span si uses rows si*(32m+3) .. (si+1)*(32m+3)-1
+    unsigned long long* kq;   // [W][32][C]: span si uses rows si*32m .. (si+1)*32m-1
     unsigned long long* anc;  // [W][4][C]
     int* arrive;              // [groups][W]
 };
@@ -1467,8 +1520,8 @@ __global__ void __launch_bounds__(256, 4)
 k_mean_cum(const float2* __restrict__ X, float2* __restrict__ Xout, dd* __restrict__ acc_buf,
            const uint32_t* __restrict__ bits,
            const int* __restrict__ wpref, const int* __restrict__ knots, const int* __restrict__ cnt,
-           const dd* __restrict__ rtab, const dd* __restrict__ rtab3, const dd* __restrict__ sv,
-           const dd* __restrict__ yend, const unsigned* __restrict__ bnd, unsigned* __restrict__ bnd_clear,
+           const dd* __restrict__ rtab, const dd* __restrict__ rtab3, const dd* __restrict__ h3tab,
+           const dd* __restrict__ sv, const dd* __restrict__ yend, const unsigned* __restrict__ bnd, unsigned* __restrict__ bnd_clear,
            const int* __restrict__ cumcfg, CumShared sh_g, Geom g, int k0, int Kc, int first_chunk, int last_chunk,
            RunState* st, Epochs ep)
 {
@@ -1476,23 +1529,22 @@ k_mean_cum(const float2* __restrict__ X, float2* __restrict__ Xout, dd* __restri
     constexpr int NWS = 8 * SUB;
     constexpr int NE = 256;  // (direction, envelope) pairs described per round
     constexpr int KB = 4;    // knots per batch of loads
-    extern __shared__ __align__(16) unsigned long long kq[];  // [32 * kCumMaxWords + 3][G]: jump of d at row x - p0
+    extern __shared__ __align__(16) unsigned klo[];  // [32 * kCumMaxWords][G]: jump of d at row x - p0, low words
+    unsigned* const khi = klo + 32 * kCumMaxWords * G;  // high words
     // The pairs' descriptions are dead once the pairs are done; the anchor
-    // sums and the scan state live only after that, so the two share one
-    // buffer (less shared memory per CTA leaves more of the SM's L1)
+    // sums live only after that, so the two share one buffer (less shared
+    // memory per CTA leaves more of the SM's L1)
     union Shared {
         struct {
             int I[NE], J[NE], N[NE], X[NE], H[NE];
         } e;
         struct {
-            unsigned long long anc[4 * G];
-            unsigned long long part[NWS * G];  // per row group: totals of a scan pass
-            unsigned long long pst[6 * G];     // particular solution at n_a; look-ahead jumps
+            unsigned alo[4 * G], ahi[4 * G];
         } f;
     };
     __shared__ __align__(16) Shared su;
     int *eI = su.e.I, *eJ = su.e.J, *eN = su.e.N, *eX = su.e.X, *eH = su.e.H;
-    unsigned long long *anc = su.f.anc, *part = su.f.part, *pst = su.f.pst;
+    unsigned *alo = su.f.alo, *ahi = su.f.ahi;
     __shared__ int sQ, sLast;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int cc = lane % G, sub = lane / G;
@@ -1517,7 +1569,10 @@ k_mean_cum(const float2* __restrict__ X, float2* __restrict__ Xout, dd* __restri
     const int c = blockIdx.y * G + cc;
     const bool cok = c < C;
     const int cl = min(c, C - 1);  // loads of lanes past the last channel stay in bounds
-    for (int i = threadIdx.x; i < (nl + 3) * G; i += blockDim.x) kq[i] = 0ull;
+    for (int i = threadIdx.x; i < nl * G; i += blockDim.x) {
+        klo[i] = 0u;
+        khi[i] = 0u;
+    }
     // quantum: |sum over the chunk's envelopes| <= 2 Kc B < 2^ex
     const float B = __uint_as_float(bnd[cl]) + __uint_as_float(bnd[C + cl]);
     const bool bad = !(B < INFINITY);
@@ -1525,18 +1580,18 @@ k_mean_cum(const float2* __restrict__ X, float2* __restrict__ Xout, dd* __restri
     frexpf(__fmul_rn(B, (float)(2 * Kc)) * 1.0009765625f, &ex);
     ex = max(ex, -60);
     const int sh = 62 - ex;  // value = units * 2^-sh
-    const dd third = dd(1.0 / 3.0);
+    const float s44 = __int_as_float((sh - 44 + 127) << 23), s22 = __int_as_float((sh - 22 + 127) << 23);  // 2^(sh - 44), 2^(sh - 22)
     const int wa = w + (ra >> 5), ba = ra & 31;
     const int wend = min(w + mw, g.W);
     // this CTA's share of the (direction, envelope) pairs
     const int e_lo = prt * 2 * Kc / P, e_hi = (prt + 1) * 2 * Kc / P;  // 2 Kc <= 2048, P <= 4
 
-    dd aA(0.0f, 0.0f), aB(0.0f, 0.0f), aC(0.0f, 0.0f), aD(0.0f, 0.0f);  // anchor coefficients, summed in a fixed order
+    Acc aA{0.0f, 0.0f}, aB{0.0f, 0.0f}, aC{0.0f, 0.0f}, aD{0.0f, 0.0f};  // anchor coefficients, summed in a fixed order
     for (int base = e_lo; base < e_hi; base += NE) {
         __syncthreads();
         // (1) per (direction, envelope): anchor piece i (x_i <= n_a < x_{i+1}),
         //     first interior knot j past p0 and the number n of interior knots
-        //     in (p0, p0 + nl + 2]; n = -1 marks a direction that does not count
+        //     in (p0, p0 + nl); n = -1 marks a direction that does not count
         {
             const int ei = base + (int)threadIdx.x;
             int n = -1, i = 0, j = 0, xi = 0, hh = 1;
@@ -1555,8 +1610,7 @@ k_mean_cum(const float2* __restrict__ X, float2* __restrict__ Xout, dd* __restri
                     const uint32_t le = (ba == 31) ? bwa : (bwa & ((2u << ba) - 1u));
                     i = min(wp[wa] + __popc(le) - 1, ke - 2);
                     j = max(kb + 1, wp[w] + (int)(bw & 1u));
-                    int nw = wp[wend] - wp[w] - (int)(bw & 1u);  // knots in (p0, p0 + 32 m)
-                    if (wend < g.W && nl == 32 * mw) nw += __popc(bb[wend] & 7u);
+                    const int nw = wp[wend] - wp[w] - (int)(bw & 1u);  // knots in (p0, p0 + 32 m)
                     n = max(0, min(j + nw - 1, ke - 2) - j + 1);
                     const int* kn = knots + slot * g.cap;
                     xi = kn[i];
@@ -1593,22 +1647,24 @@ k_mean_cum(const float2* __restrict__ X, float2* __restrict__ Xout, dd* __restri
                 const dd s0 = sv[rb + (size_t)i * C], s1 = sv[rb + (size_t)(i + 1) * C];
                 const dd d = (s1 - s0) * rtab3[h];
                 const dd s02(2.0f * s0.hi, 2.0f * s0.lo);  // exact
-                const dd b = (y1 - y0) * rtab[h] - dd_mulf(s02 + s1, (float)h) * third;
-                const float u = (float)(na - xi);
-                const dd d3 = dd_mulf(d, 3.0f);
-                aA = aA + (dd_mulf(dd_mulf(dd_mulf(d, u) + s0, u) + b, u) + y0);
-                aB = aB + (dd_mulf(dd_mulf(d3, u) + s02, u) + b);
-                aC = aC + (dd_mulf(d3, u) + s0);
-                aD = aD + d;
+                const dd b = dd_diff_of_products(y1 - y0, rtab[h], s02 + s1, h3tab[h]);
+                const float u = (float)(na - xi), u3 = (float)(3 * (na - xi));
+                acc_mulf(aA, dd_mulf(dd_mulf(d, u) + s0, u) + b, u);
+                acc_add(aA, y0.hi, y0.lo);
+                acc_mulf(aB, dd_mulf(d, u3) + s02, u);
+                acc_add(aB, b.hi, b.lo);
+                acc_mulf(aC, d, u3);
+                acc_add(aC, s0.hi, s0.lo);
+                acc_add(aD, d.hi, d.lo);
             }
-            // (3) jumps q_j - q_{j-1} at row x_j - p0 (in 1 .. nl + 2), q_j the
+            // (3) jumps q_j - q_{j-1} at row x_j - p0 (in 1 .. nl - 1), q_j the
             //     quantised d_j = (s_{j+1} - s_j) / (3 h_j); full batches of KB
             //     knots (loads first, no predication), then the remainder
             const int j0 = eJ[le];
             if (n > 0) {
                 int xj = kn[j0];
                 dd sj = sv[rb + (size_t)j0 * C];
-                unsigned long long qprev = qfix((sj - sv[rb + (size_t)(j0 - 1) * C]) * rtab3[xj - kn[j0 - 1]], sh);
+                Limbs qprev = to_limbs((sj - sv[rb + (size_t)(j0 - 1) * C]) * rtab3[xj - kn[j0 - 1]], s44, s22);
                 int t0 = 0;
                 for (; t0 + KB <= n; t0 += KB) {
                     int xn[KB];
@@ -1630,8 +1686,9 @@ k_mean_cum(const float2* __restrict__ X, float2* __restrict__ Xout, dd* __restri
                     }
 #pragma unroll
                     for (int k = 0; k < KB; ++k) {
-                        const unsigned long long qcur = qfix((sn[k] - sj) * r3[k], sh);
-                        if (MEMD_CHECK(xj - p0 >= 0 && xj - p0 < nl + 3)) atomicAdd(&kq[(xj - p0) * G + cc], qcur - qprev);
+                        const Limbs qcur = to_limbs((sn[k] - sj) * r3[k], s44, s22);
+                        if (MEMD_CHECK(xj - p0 >= 0 && xj - p0 < nl))
+                            add_words(klo, khi, (xj - p0) * G + cc, limbs_diff(qcur, qprev));
                         qprev = qcur;
                         xj = xn[k];
                         sj = sn[k];
@@ -1640,8 +1697,9 @@ k_mean_cum(const float2* __restrict__ X, float2* __restrict__ Xout, dd* __restri
                 for (; t0 < n; ++t0) {
                     const int xn1 = kn[j0 + t0 + 1];
                     const dd sn1 = sv[rb + (size_t)(j0 + t0 + 1) * C];
-                    const unsigned long long qcur = qfix((sn1 - sj) * rtab3[xn1 - xj], sh);
-                    if (MEMD_CHECK(xj - p0 >= 0 && xj - p0 < nl + 3)) atomicAdd(&kq[(xj - p0) * G + cc], qcur - qprev);
+                    const Limbs qcur = to_limbs((sn1 - sj) * rtab3[xn1 - xj], s44, s22);
+                    if (MEMD_CHECK(xj - p0 >= 0 && xj - p0 < nl))
+                        add_words(klo, khi, (xj - p0) * G + cc, limbs_diff(qcur, qprev));
                     qprev = qcur;
                     xj = xn1;
                     sj = sn1;
@@ -1649,28 +1707,34 @@ k_mean_cum(const float2* __restrict__ X, float2* __restrict__ Xout, dd* __restri
             }
         }
     }
-    __syncthreads();  // the descriptions are dead: anc takes their place
-    for (int i = threadIdx.x; i < 4 * G; i += blockDim.x) anc[i] = 0ull;
+    __syncthreads();  // the descriptions are dead: the anchor sums take their place
+    for (int i = threadIdx.x; i < 4 * G; i += blockDim.x) {
+        alo[i] = 0u;
+        ahi[i] = 0u;
+    }
     __syncthreads();
-    atomicAdd(&anc[0 * G + cc], qfix(aA, sh));
-    atomicAdd(&anc[1 * G + cc], qfix(aB, sh));
-    atomicAdd(&anc[2 * G + cc], qfix(aC, sh));
-    atomicAdd(&anc[3 * G + cc], qfix(aD, sh));
+    add_words(alo, ahi, 0 * G + cc, limbs_value(to_limbs(acc_dd(aA), s44, s22)));
+    add_words(alo, ahi, 1 * G + cc, limbs_value(to_limbs(acc_dd(aB), s44, s22)));
+    add_words(alo, ahi, 2 * G + cc, limbs_value(to_limbs(acc_dd(aC), s44, s22)));
+    add_words(alo, ahi, 3 * G + cc, limbs_value(to_limbs(acc_dd(aD), s44, s22)));
     __syncthreads();
+    auto word = [](const unsigned* lo, const unsigned* hi, int i) -> unsigned long long {
+        return ((unsigned long long)hi[i] << 32) | lo[i];
+    };
     if (P > 1) {
         // a span shared by P CTAs: add this CTA's rows to the span's global
         // accumulators; the last CTA to arrive finishes the span and clears them
-        const int rows = 32 * mw + 3;
+        const int rows = 32 * mw;
         unsigned long long* gk = sh_g.kq + (size_t)si * rows * C + (size_t)blockIdx.y * G;
         unsigned long long* ga = sh_g.anc + (size_t)si * 4 * C + (size_t)blockIdx.y * G;
-        for (int i = threadIdx.x; i < (nl + 3) * G; i += blockDim.x) {
+        for (int i = threadIdx.x; i < nl * G; i += blockDim.x) {
             const int r = i / G, ch = i - r * G;
-            const unsigned long long v = kq[i];
+            const unsigned long long v = word(klo, khi, i);
             if (v != 0ull && blockIdx.y * G + ch < C) atomicAdd(&gk[(size_t)r * C + ch], v);
         }
         for (int i = threadIdx.x; i < 4 * G; i += blockDim.x) {
             const int r = i / G, ch = i - r * G;
-            if (blockIdx.y * G + ch < C) atomicAdd(&ga[(size_t)r * C + ch], anc[i]);
+            if (blockIdx.y * G + ch < C) atomicAdd(&ga[(size_t)r * C + ch], word(alo, ahi, i));
         }
         __threadfence();
         __syncthreads();
@@ -1678,14 +1742,15 @@ k_mean_cum(const float2* __restrict__ X, float2* __restrict__ Xout, dd* __restri
         __syncthreads();
         if (!sLast) return;  // uniform over the CTA
         __threadfence();
-        for (int i = threadIdx.x; i < (nl + 3) * G; i += blockDim.x) {
+        for (int i = threadIdx.x; i < nl * G; i += blockDim.x) {
             const int r = i / G, ch = i - r * G;
             unsigned long long v = 0ull;
             if (blockIdx.y * G + ch < C) {
                 v = __ldcg(&gk[(size_t)r * C + ch]);
                 gk[(size_t)r * C + ch] = 0ull;
             }
-            kq[i] = v;
+            klo[i] = (unsigned)v;
+            khi[i] = (unsigned)(v >> 32);
         }
         for (int i = threadIdx.x; i < 4 * G; i += blockDim.x) {
             const int r = i / G, ch = i - r * G;
@@ -1694,7 +1759,8 @@ k_mean_cum(const float2* __restrict__ X, float2* __restrict__ Xout, dd* __restri
                 v = __ldcg(&ga[(size_t)r * C + ch]);
                 ga[(size_t)r * C + ch] = 0ull;
             }
-            anc[i] = v;
+            alo[i] = (unsigned)v;
+            ahi[i] = (unsigned)(v >> 32);
         }
         if (threadIdx.x == 0) sh_g.arrive[(size_t)blockIdx.y * g.W + si] = 0;
     }
@@ -1704,84 +1770,62 @@ k_mean_cum(const float2* __restrict__ X, float2* __restrict__ Xout, dd* __restri
         q = warp_sum(q);
         if (lane == 0) sQ = q;
     }
-    // (4) M over the span, in parallel: row group rg = warp * SUB + sub owns
-    //     rows [r0, r1).  The particular solution P (zero state at row 0) is
-    //     four exclusive prefix sums of the impulses I(r) = kq[r+1] + 4 kq[r+2]
-    //     + kq[r+3]; M = P + H with H the cubic (Delta^4 H = 0) whose
-    //     differences at n_a are the anchor state minus P's.
-    const int rg = warp * SUB + sub;
-    const int RB = (nl + NWS - 1) / NWS;
-    const int r0 = min(nl, rg * RB), r1 = min(nl, r0 + RB);
-    unsigned long long e0 = 0, e1 = 0, e2 = 0;  // rows r1 .. r1 + 2, read before they are overwritten
-    __syncthreads();
-    if (r0 < r1) {
-        e0 = kq[r1 * G + cc];
-        e1 = kq[(r1 + 1) * G + cc];
-        e2 = kq[(r1 + 2) * G + cc];
-    }
-    if (rg == 0) {
-        pst[3 * G + cc] = kq[(ra + 1) * G + cc];  // jump at n_a + 1
-        pst[4 * G + cc] = kq[(ra + 2) * G + cc];  // jump at n_a + 2
-    }
     __syncthreads();
     const int Q = sQ;
     if (last_chunk && Q == 0 && blockIdx.y == 0 && threadIdx.x == 0) atomicOr(&st->flags, 1);
-    for (int r = r0; r < r1; ++r) {  // in place: I(r) reads rows > r only
-        const unsigned long long a1 = (r + 1 < r1) ? kq[(r + 1) * G + cc] : (r + 1 == r1 ? e0 : (r + 1 == r1 + 1 ? e1 : e2));
-        const unsigned long long a2 = (r + 2 < r1) ? kq[(r + 2) * G + cc] : (r + 2 == r1 ? e0 : (r + 2 == r1 + 1 ? e1 : e2));
-        const unsigned long long a3 = (r + 3 < r1) ? kq[(r + 3) * G + cc] : (r + 3 == r1 ? e0 : (r + 3 == r1 + 1 ? e1 : e2));
-        kq[r * G + cc] = a1 + (a2 << 2) + a3;
-    }
-    for (int pass = 0; pass < 4; ++pass) {
-        unsigned long long run = 0;
-        for (int r = r0; r < r1; ++r) {
-            const unsigned long long t = kq[r * G + cc];
-            kq[r * G + cc] = run;
-            run += t;
+    if (!cok) return;
+    // (4) M over the span: the samples on either side of the anchor in blocks,
+    //     one per subgroup: forwards from the anchor, or backwards, the cubic's
+    //     coefficients carried from sample to sample (at first without output,
+    //     up to the block) and d changed at every knot
+    constexpr int per = NWS / 2;  // blocks per side
+    const int rg = warp * SUB + sub;
+    const bool back = rg >= per;
+    const int rows = (16 * mw + per - 1) / per, blk = back ? rg - per : rg;
+    const int lo = back ? max(0, ra - (blk + 1) * rows) : ra + blk * rows;  // rows [lo, hi)
+    const int hi = back ? ra - blk * rows : min(nl, lo + rows);
+    if (lo >= hi) return;
+    unsigned long long vA = word(alo, ahi, cc), vB = word(alo, ahi, G + cc), vC = word(alo, ahi, 2 * G + cc),
+                       vD = word(alo, ahi, 3 * G + cc);
+    auto step = [&](int r) {  // from row r - 1 to row r, or (back) from row r to row r - 1
+        const unsigned long long k = word(klo, khi, r * G + cc);
+        if (back) {
+            vD -= k;
+            vA += vC - vB - vD;
+            vB += 3ull * vD - 2ull * vC;
+            vC -= 3ull * vD;
+        } else {
+            vA += vB + vC + vD;
+            vB += 2ull * vC + 3ull * vD;
+            vC += 3ull * vD;
+            vD += k;
         }
-        part[rg * G + cc] = run;
-        __syncthreads();
-        unsigned long long off = 0;
-        for (int q = 0; q < rg; ++q) off += part[q * G + cc];
-        for (int r = r0; r < r1; ++r) kq[r * G + cc] += off;
-        if (pass < 3 && ra >= r0 && ra < r1) pst[pass * G + cc] = kq[ra * G + cc];  // P's d3, d2, d1 at n_a
-        __syncthreads();
-    }
-    if (!cok || r0 >= r1) return;
-    const unsigned long long sA = anc[cc], sB = anc[G + cc], sC = anc[2 * G + cc], sD = anc[3 * G + cc];
-    const unsigned long long k1 = pst[3 * G + cc], k2 = pst[4 * G + cc];
-    // state at n_a: differences of the anchor polynomials plus the part of the
-    // jumps at n_a + 1 and n_a + 2 that falls before n_a (Delta^4 of (n - x)_+^3
-    // is 1, 4, 1 at x - 3, x - 2, x - 1), minus P's state there
-    const unsigned long long h0 = sA - kq[ra * G + cc];
-    const unsigned long long h1 = sB + sC + sD - pst[2 * G + cc];
-    const unsigned long long h2 = 2ull * sC + 6ull * sD + k1 - pst[1 * G + cc];
-    const unsigned long long h3 = 6ull * sD + 5ull * k1 + k2 - pst[cc];
+    };
+    const int dir = back ? -1 : 1, first = back ? hi - 1 : lo;  // rows are finished from the anchor outwards
+    if (back)
+        for (int r = ra; r > first; --r) step(r);
+    else
+        for (int r = ra + 1; r <= first; ++r) step(r);
     const dd qd = dd((float)Q, 0.0f);
     constexpr int XB = 4;  // rows per batch of X loads
-    for (int rb0 = r0; rb0 < r1; rb0 += XB) {
+    const int nrow = hi - lo;
+    for (int b0 = 0; b0 < nrow; b0 += XB) {
         float2 xs[XB];
         dd ac[XB];
 #pragma unroll
         for (int k = 0; k < XB; ++k) {
-            if (rb0 + k < r1) {
-                const size_t off = (size_t)(p0 + rb0 + k) * C + c;
+            if (b0 + k < nrow) {
+                const size_t off = (size_t)(p0 + first + dir * (b0 + k)) * C + c;
                 if (last_chunk) xs[k] = X[off];
                 if (!first_chunk) ac[k] = acc_buf[off];
             }
         }
 #pragma unroll
         for (int k = 0; k < XB; ++k) {
-            const int r = rb0 + k;
-            if (r < r1) {
-                // H(n_a + t) = h0 + t h1 + C(t,2) h2 + C(t,3) h3 (Newton's form, any integer t)
-                // |t| <= 128: the binomials are exact in 32-bit integers
-                const int t = r - ra;
-                const unsigned long long c2 = (unsigned long long)(long long)(t * (t - 1) / 2);
-                const unsigned long long c3 = (unsigned long long)(long long)(t * (t - 1) * (t - 2) / 6);
-                const unsigned long long val =
-                    kq[r * G + cc] + h0 + (unsigned long long)(long long)t * h1 + c2 * h2 + c3 * h3;
-                dd tot = fix2dd(val, sh);
+            if (b0 + k < nrow) {
+                const int r = first + dir * (b0 + k);
+                if (b0 + k > 0) step(back ? r + 1 : r);
+                dd tot = fix2dd(vA, sh);
                 if (bad) tot = dd(__int_as_float(0x7fc00000), 0.0f);
                 const size_t off = (size_t)(p0 + r) * C + c;
                 if (!first_chunk) tot = tot + ac[k];
@@ -2691,13 +2735,16 @@ __global__ void k_check_coords(const int32_t* __restrict__ x, int L, int* __rest
 __global__ void k_fill_reciprocals(double* __restrict__ r64, float* __restrict__ r32, dd* __restrict__ rdd,
                                    dd* __restrict__ r3dd, double2* __restrict__ r3_64, int n)
 {
-    // r3dd (optional): 1/(3h) as a double-float; r3_64 (optional): 1/(3h) and h/3 in FP64
+    // r3dd (optional): 1/(3h) as a double-float, then, from r3dd[n] on, h/3; r3_64 (optional): 1/(3h) and h/3 in FP64
     for (int h = blockIdx.x * blockDim.x + threadIdx.x; h < n; h += gridDim.x * blockDim.x) {
         const double r = h > 0 ? __ddiv_rn(1.0, (double)h) : 0.0;
         r64[h] = r;
         r32[h] = h > 0 ? __fdiv_rn(1.0f, (float)h) : 0.0f;
         rdd[h] = dd(r);
-        if (r3dd) r3dd[h] = h > 0 ? dd(__ddiv_rn(1.0, 3.0 * (double)h)) : dd(0.0f, 0.0f);
+        if (r3dd) {
+            r3dd[h] = h > 0 ? dd(__ddiv_rn(1.0, 3.0 * (double)h)) : dd(0.0f, 0.0f);
+            r3dd[n + h] = dd(__ddiv_rn((double)h, 3.0));
+        }
         if (r3_64) r3_64[h] = make_double2(h > 0 ? __ddiv_rn(1.0, 3.0 * (double)h) : 0.0, __dmul_rn((double)h, 1.0 / 3.0));
     }
 }

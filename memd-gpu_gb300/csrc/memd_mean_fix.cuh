@@ -34,7 +34,7 @@ namespace memd {
 // 4.7e-17 / 7.4e-17; twice the span, 2x .. 4x the error.
 // Measured (FP64 form, all sifts of a decomposition, against the direct
 // evaluation of every envelope at every sample, 82% busy on the FP64 pipe): 32
-// x 30,504, 64 directions, 80 sifts: 117.6 -> 21.9 ms of the mean (29.6 with T
+// x 30,504, 64 directions, 80 sifts: 117.6 -> 21.2 ms of the mean (29.6 with T
 // <= 2 h, integer conversions on the FP64 pipe, one CTA per 64 samples and the
 // samples behind an anchor all by one warp); error of the IMFs against a
 // separate FP64 evaluation 8.2e-16 -> 4.0e-16.
@@ -130,10 +130,15 @@ k_mean_fix(const double* __restrict__ X, double* __restrict__ Xout, ulonglong2* 
     constexpr int SUB = 32 / G;
     constexpr int NWS = 8 * SUB;
     constexpr int NE = 256;  // pairs described per round
-    extern __shared__ __align__(16) unsigned long long kq_hi[];  // [kFixRows][G] jumps at row x - p0, high words
-    unsigned long long* kq_lo = kq_hi + kFixRows * G;            // low words
-    unsigned long long* an_hi = kq_lo + kFixRows * G;            // [kFixAnchors][4][G] Taylor coefficients at the anchors
-    unsigned long long* an_lo = an_hi + kFixAnchors * 4 * G;
+    // sums, as four 32-bit words each (hi's low and high word, lo's low and high
+    // word, NS apart): rows 0 .. kFixRows - 1 the jumps at row x - p0, then
+    // [kFixAnchors][4] Taylor coefficients at the anchors; [..][G]
+    constexpr int NS = (kFixRows + 4 * kFixAnchors) * G, AN = kFixRows * G;
+    extern __shared__ __align__(16) unsigned sums[];
+    auto add = [&](int i, unsigned long long hi, unsigned long long lo) {
+        add_words(sums, sums + NS, i, hi);
+        add_words(sums + 2 * NS, sums + 3 * NS, i, lo);
+    };
     __shared__ int eJ[NE], eE[NE];  // first piece of the span (-1: the pair does not count); last piece of the record
     __shared__ int sQ, sT;
     __shared__ unsigned sBad;  // channels of the span to evaluate directly
@@ -192,13 +197,9 @@ k_mean_fix(const double* __restrict__ X, double* __restrict__ Xout, ulonglong2* 
     const int c = blockIdx.y * G + cc;
     const bool cok = c < C;
     const int cl = min(c, C - 1);  // loads of lanes past the last channel stay in bounds
-    for (int i = threadIdx.x; i < nl * G; i += blockDim.x) {
-        kq_hi[i] = 0ull;
-        kq_lo[i] = 0ull;
-    }
-    for (int i = threadIdx.x; i < nA * 4 * G; i += blockDim.x) {
-        an_hi[i] = 0ull;
-        an_lo[i] = 0ull;
+    for (int j = 0; j < 4; ++j) {
+        for (int i = threadIdx.x; i < nl * G; i += blockDim.x) sums[j * NS + i] = 0u;
+        for (int i = threadIdx.x; i < nA * 4 * G; i += blockDim.x) sums[j * NS + AN + i] = 0u;
     }
     const unsigned xe = xexp[(size_t)rec * C + cl];
     const int sh = fix_shift(xe);
@@ -264,8 +265,7 @@ k_mean_fix(const double* __restrict__ X, double* __restrict__ Xout, ulonglong2* 
                 FixSum qc;
                 ok &= to_fix(d, sh, lim - 3 * lt, qc);
                 if (jump && MEMD_CHECK(xj - p0 > 0 && xj - p0 < nl)) {
-                    atomicAdd(&kq_hi[(xj - p0) * G + cc], qc.hi - qp.hi);
-                    atomicAdd(&kq_lo[(xj - p0) * G + cc], qc.lo - qp.lo);
+                    add((xj - p0) * G + cc, qc.hi - qp.hi, qc.lo - qp.lo);
                 }
                 qp = qc;
                 while (a < nA && (na < xn || j == je)) {
@@ -277,19 +277,14 @@ k_mean_fix(const double* __restrict__ X, double* __restrict__ Xout, ulonglong2* 
                     const double e = __fma_rn(d, u, s0);
                     const double cB = __fma_rn(__fma_rn(d, u3, twice(s0)), u, b);
                     FixSum f;
-                    unsigned long long* ah = an_hi + (size_t)(a * 4) * G + cc;
-                    unsigned long long* al = an_lo + (size_t)(a * 4) * G + cc;
+                    const int at = AN + a * 4 * G + cc;
                     ok &= to_fix(__fma_rn(__fma_rn(e, u, b), u, y0), sh, lim, f);
-                    atomicAdd(ah, f.hi);
-                    atomicAdd(al, f.lo);
+                    add(at, f.hi, f.lo);
                     ok &= to_fix(cB, sh, lim - lt, f);
-                    atomicAdd(ah + G, f.hi);
-                    atomicAdd(al + G, f.lo);
+                    add(at + G, f.hi, f.lo);
                     ok &= to_fix(__fma_rn(d, u3, s0), sh, lim - 2 * lt, f);
-                    atomicAdd(ah + 2 * G, f.hi);
-                    atomicAdd(al + 2 * G, f.lo);
-                    atomicAdd(ah + 3 * G, qc.hi);
-                    atomicAdd(al + 3 * G, qc.lo);
+                    add(at + 2 * G, f.hi, f.lo);
+                    add(at + 3 * G, qc.hi, qc.lo);
                     ++a;
                     na = p0 + a * T + min(T >> 1, nl - 1 - a * T);
                 }
@@ -311,26 +306,25 @@ k_mean_fix(const double* __restrict__ X, double* __restrict__ Xout, ulonglong2* 
         const auto cl_ = cg_::this_cluster();
         cl_.sync();
         constexpr int NV = (kFixRows + 4) * G / 256 + 1;
-        const unsigned long long* oh = cl_.map_shared_rank(kq_hi, 1 - half);
-        const unsigned long long* ol = oh + (kq_lo - kq_hi);
+        const unsigned* os = cl_.map_shared_rank(sums, 1 - half);
         const unsigned obad = *cl_.map_shared_rank(&sBad, 1 - half);
-        unsigned long long vh[NV], vl[NV];
         const int nk = nl * G, nv = nk + 4 * G;  // rows, then the anchor (nA = 1)
+        for (int word = 0; word < 4; word += 2) {
+            unsigned long long v[NV];
 #pragma unroll
-        for (int j = 0; j < NV; ++j) {
-            const int i = (int)threadIdx.x + 256 * j;
-            const int at = i < nk ? i : (int)(an_hi - kq_hi) + i - nk, al = i < nk ? i : (int)(an_lo - kq_lo) + i - nk;
-            vh[j] = i < nv ? oh[at] : 0ull;
-            vl[j] = i < nv ? ol[al] : 0ull;
-        }
-        cl_.sync();
+            for (int j = 0; j < NV; ++j) {
+                const int i = (int)threadIdx.x + 256 * j, at = (i < nk ? i : AN + i - nk) + word * NS;
+                v[j] = i < nv ? ((unsigned long long)os[at + NS] << 32) | os[at] : 0ull;
+            }
+            cl_.sync();
 #pragma unroll
-        for (int j = 0; j < NV; ++j) {
-            const int i = (int)threadIdx.x + 256 * j;
-            const int at = i < nk ? i : (int)(an_hi - kq_hi) + i - nk, al = i < nk ? i : (int)(an_lo - kq_lo) + i - nk;
-            if (i < nv) {
-                kq_hi[at] += vh[j];
-                kq_lo[al] += vl[j];
+            for (int j = 0; j < NV; ++j) {
+                const int i = (int)threadIdx.x + 256 * j, at = (i < nk ? i : AN + i - nk) + word * NS;
+                if (i < nv) {
+                    v[j] += ((unsigned long long)sums[at + NS] << 32) | sums[at];
+                    sums[at] = (unsigned)v[j];
+                    sums[at + NS] = (unsigned)(v[j] >> 32);
+                }
             }
         }
         if (threadIdx.x == 0) sBad |= obad;
@@ -380,7 +374,9 @@ k_mean_fix(const double* __restrict__ X, double* __restrict__ Xout, ulonglong2* 
             acc_buf[off] = o;
         }
     };
-    auto wide = [](unsigned long long hi, unsigned long long lo) -> __int128 {
+    auto wide = [&](int i) -> __int128 {
+        const unsigned long long hi = ((unsigned long long)sums[NS + i] << 32) | sums[i];
+        const unsigned long long lo = ((unsigned long long)sums[3 * NS + i] << 32) | sums[2 * NS + i];
         return ((__int128)(long long)hi << 52) + (__int128)(long long)lo;
     };
     // (3) the samples on either side of an anchor, in blocks of at most RB rows
@@ -405,18 +401,16 @@ k_mean_fix(const double* __restrict__ X, double* __restrict__ Xout, ulonglong2* 
 #pragma unroll
         for (int k = 0; k < RB; ++k) xs[k] = last_chunk && lo + k < hi ? X[(size_t)(p0 + lo + k) * C + c] : 0.0;
         if (!bad) {
-            const unsigned long long* ah = an_hi + (size_t)(a * 4) * G + cc;
-            const unsigned long long* al = an_lo + (size_t)(a * 4) * G + cc;
-            __int128 vA = wide(ah[0], al[0]), vB = wide(ah[G], al[G]), vC = wide(ah[2 * G], al[2 * G]),
-                     vD = wide(ah[3 * G], al[3 * G]);
+            const int at = AN + a * 4 * G + cc;
+            __int128 vA = wide(at), vB = wide(at + G), vC = wide(at + 2 * G), vD = wide(at + 3 * G);
             auto forth = [&](int r) {  // from row r - 1 to row r
                 vA += vB + vC + vD;
                 vB += 2 * vC + 3 * vD;
                 vC += 3 * vD;
-                vD += wide(kq_hi[r * G + cc], kq_lo[r * G + cc]);
+                vD += wide(r * G + cc);
             };
             auto aback = [&](int r) {  // from row r to row r - 1
-                vD -= wide(kq_hi[r * G + cc], kq_lo[r * G + cc]);
+                vD -= wide(r * G + cc);
                 vA += vC - vB - vD;
                 vB += 3 * vD - 2 * vC;
                 vC -= 3 * vD;
