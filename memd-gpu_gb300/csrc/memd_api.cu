@@ -277,7 +277,7 @@ static bool eval_dispatch(int G, int SPL, int W, F f)
         MEMD_CASE(4, 4, 8) MEMD_CASE(8, 8, 8) MEMD_CASE(16, 16, 8)
     } else {
         MEMD_CASE(4, 16, 8) MEMD_CASE(8, 16, 8) MEMD_CASE(16, 16, 8)
-        MEMD_CASE(4, 4, 8) MEMD_CASE(8, 8, 8) MEMD_CASE(4, 4, 16) MEMD_CASE(8, 8, 16) MEMD_CASE(16, 16, 16)
+        MEMD_CASE(4, 4, 8) MEMD_CASE(8, 8, 8)
     }
 #undef MEMD_CASE
     return false;
@@ -1373,10 +1373,11 @@ static memd_status create_plan(const memd_config* cfg, const memd_tuning* tun, m
         p->ewZ = 1;
         if ((L + 32 / p->ewG * spl - 1) / (32 / p->ewG * spl) * groups < 600) {  // about four CTAs of 8 warps per SM
             p->ewSPL = p->ewG;
+            // as many CTAs a tile (4, 2 or 1) as stay resident at once, three
+            // per SM: past that, the extra partial sums only cost
             if (!f32) {
                 const long tiles = (L + 31) / 32 * groups;
-                p->ewZ = tiles < 152 ? 4 : (tiles < 304 ? 2 : 1);
-                p->ewW = p->ewZ == 4 ? 8 : 16;
+                p->ewZ = tiles <= 114 ? 4 : (tiles <= 228 ? 2 : 1);
             }
         }
     }
