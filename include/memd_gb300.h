@@ -113,9 +113,8 @@ typedef struct {
     int32_t solve_window;  /* tridiagonal halo in knots (0 = default; <0 = exact) */
     int32_t max_epochs;    /* batched runs: epochs per call (0 = single record) */
     int32_t mean_eval;     /* mean envelope: 0 = automatic (impulse accumulation
-                              for the FP64 and mixed forms in fixed mode with
-                              the reference boundary, otherwise direct
-                              evaluation),
+                              for the FP64 and mixed forms in fixed mode,
+                              otherwise direct evaluation),
                               1 = direct evaluation of every envelope,
                               2 = impulse accumulation (mixed form, fixed mode,
                               reference boundary only) */

@@ -305,12 +305,12 @@ static void launch_eval(memd_plan* p, cudaStream_t s, int k0, int kc, int first,
 #define MEMD_CASE(G_)                                                                                              \
     if (p->cumG == G_) {                                                                                           \
         lc.dynamicSmemBytes = fix_smem_bytes(G_);                                                                  \
-        cudaLaunchKernelEx(&lc, k_mean_fix<G_>, (const double*)p->X, (double*)p->Xb, (ulonglong2*)p->acc,          \
+        cudaLaunchKernelEx(&lc, g.mirror ? k_mean_fix<G_, true> : k_mean_fix<G_, false>, (const double*)p->X, (double*)p->Xb, (ulonglong2*)p->acc,          \
                            (const uint32_t*)p->bits, (const int*)p->wpref, (const int*)p->knots,                   \
                            (const int*)p->cnt, (const double*)p->rtab, (const double2*)p->rtab3,                   \
                            (const double*)p->sv, (const double*)p->yend, (const unsigned*)p->xexp,                 \
                            (const unsigned long long*)(p->nchunks > 1 ? p->tot : nullptr), g, k0, kc, first, last, \
-                           p->st, p->ep);                                                                          \
+                           p->st, p->ep, (const int*)p->mir);                                                      \
         return;                                                                                                    \
     }
             MEMD_CASE(32) MEMD_CASE(16) MEMD_CASE(8)
@@ -325,12 +325,12 @@ static void launch_eval(memd_plan* p, cudaStream_t s, int k0, int kc, int first,
     if (p->cumG == G_) {                                                                                           \
         dim3 grid((unsigned)((g.W + kCumMaxWords - 1) / kCumMaxWords * kCumMaxWords),                             \
                   (unsigned)((g.C + G_ - 1) / G_));                                                                \
-        k_mean_cum<G_><<<grid, 256, sizeof(unsigned long long) * 32 * kCumMaxWords * G_, s>>>(               \
+        (g.mirror ? k_mean_cum<G_, true> : k_mean_cum<G_, false>)<<<grid, 256, sizeof(unsigned long long) * 32 * kCumMaxWords * G_, s>>>(               \
             (const float2*)p->X, (float2*)p->Xb, (dd*)p->acc, p->bits, p->wpref, p->knots, p->cnt,               \
                                             (const dd*)p->rtab, (const dd*)p->rtab3,                             \
                                             (const dd*)p->rtab3 + p->ntab, (const dd*)p->sv,                      \
                                             (const dd*)p->yend, cur, other, p->cumcfg, p->cumsh, g, k0, kc, first,\
-                                            last, p->st, p->ep);                                                   \
+                                            last, p->st, p->ep, p->mir);                                           \
         return;                                                                                                    \
     }
                 MEMD_CASE(32) MEMD_CASE(16) MEMD_CASE(8)
@@ -371,8 +371,6 @@ static cudaError_t set_attrs(memd_plan* p)
     using R = typename Prec<P>::R;
     using XT = typename Prec<P>::X;
     cudaError_t e = cudaSuccess;
-    if constexpr (P == MEMD_PREC_F64)
-        e = cudaFuncSetAttribute(k_mean_fix<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fix_smem_bytes(32));
     eval_dispatch<P>(p->ewG, p->ewSPL, p->ewW, [&](auto G_, auto S_, auto W_) {
         constexpr int G = decltype(G_)::value, SPL = decltype(S_)::value, W = decltype(W_)::value;
         using Sh = EvalWShape<G, SPL, R, W>;
@@ -383,16 +381,6 @@ static cudaError_t set_attrs(memd_plan* p)
             e = cudaFuncSetAttribute(k_eval_w<G, SPL, XT, R, false, W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)Sh::smem_bytes(false));
     });
-    if (e != cudaSuccess) return e;
-    if constexpr (P == MEMD_PREC_MIXED) {
-        const int cb[3] = {32, 16, 8};
-        for (int i = 0; i < 3 && e == cudaSuccess; ++i) {
-            const int bytes = (int)sizeof(unsigned long long) * 32 * kCumMaxWords * cb[i];
-            if (cb[i] == 32) e = cudaFuncSetAttribute(k_mean_cum<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-            if (cb[i] == 16) e = cudaFuncSetAttribute(k_mean_cum<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-            if (cb[i] == 8) e = cudaFuncSetAttribute(k_mean_cum<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-        }
-    }
     if (e != cudaSuccess) return e;
     if constexpr (P == MEMD_PREC_MIXED) {
         e = cudaFuncSetAttribute(k_project_mx, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p->proj_smem);
@@ -525,26 +513,29 @@ static void enqueue_sift(memd_plan* p, cudaStream_t s, memd_trace_entry* trace, 
         }
         lc.begin(MEMD_STAGE_SOLVE);
         bool xm = false;
-#define MEMD_FWD(XM_, EPB_, NAK_)                                                                               \
-    k_solve_fwd<R, XT, XM_, EPB_, NAK_><<<p->squeue ? persistent_grid(k_solve_fwd<R, XT, XM_, EPB_, NAK_>,     \
+#define MEMD_FWD(XM_, EPB_, NAK_, MIR_)                                                                               \
+    k_solve_fwd<R, XT, XM_, EPB_, NAK_, MIR_><<<p->squeue ? persistent_grid(k_solve_fwd<R, XT, XM_, EPB_, NAK_, MIR_>,     \
                                                                       kSolveThreads, p->sms, nb) : nb,          \
                                           kSolveThreads, 0, s>>>(                                              \
         (const R*)p->yv, p->cnt, (const Fac<R>*)p->fac, (R*)p->dbuf, g, k0, kc, p->S, p->Ss, p->H, p->ngroups, \
         bcur, XM_ ? (const XT*)p->X : nullptr, p->knots, XM_ ? (const R*)p->yend : nullptr, p->ep,               \
-        p->inplace ? (R*)p->hz : nullptr, p->hsegs, q)
+        p->inplace ? (R*)p->hz : nullptr, p->hsegs, q, p->mir)
         if constexpr (P != MEMD_PREC_F32) {
             if (p->cum) {  // knot values from the working signal (the impulse-accumulation path)
                 xm = true;
                 if (p->ep.n > 0) {  // batched runs: record ends found by position
-                    if (g.nak) MEMD_FWD(true, true, true);
-                    else MEMD_FWD(true, true, false);
-                } else if (g.nak) MEMD_FWD(true, false, true);
-                else MEMD_FWD(true, false, false);
+                    if (g.nak) MEMD_FWD(true, true, true, false);
+                    else MEMD_FWD(true, true, false, false);
+                } else if (g.mirror) {
+                    if (g.nak) MEMD_FWD(true, false, true, true);
+                    else MEMD_FWD(true, false, false, true);
+                } else if (g.nak) MEMD_FWD(true, false, true, false);
+                else MEMD_FWD(true, false, false, false);
             }
         }
         if (!xm) {
-            if (g.nak) MEMD_FWD(false, false, true);
-            else MEMD_FWD(false, false, false);
+            if (g.nak) MEMD_FWD(false, false, true, false);
+            else MEMD_FWD(false, false, false, false);
         }
 #undef MEMD_FWD
         lc.end(MEMD_STAGE_SOLVE);
@@ -1327,8 +1318,7 @@ static memd_status create_plan(const memd_config* cfg, const memd_tuning* tun, m
         // automatic: as many directions per pass as the free memory allows,
         // with separate right-hand-side and solution arrays while all of them
         // fit (the faster layout), solving in place when that fits more
-        const bool cum_cfg = c.precision != MEMD_PREC_F32 && c.stop_mode == MEMD_STOP_FIXED &&
-                             c.boundary == MEMD_BOUNDARY_REFERENCE && c.mean_eval != 1;
+        const bool cum_cfg = c.precision != MEMD_PREC_F32 && c.stop_mode == MEMD_STOP_FIXED && c.mean_eval != 1;
         const int want = std::min(K, kc_limit);
         const int fit_sep = directions_that_fit(c, p->g, p->real_bytes, p->xbytes, p->tbytes, cum_cfg, false);
         if (fit_sep >= want || !inplace_ok) {
@@ -1339,8 +1329,7 @@ static memd_status create_plan(const memd_config* cfg, const memd_tuning* tun, m
             want_inplace = fit_inp > fit_sep;
         }
     } else if (c.dir_chunk <= 0) {  // layout fixed by the tuning: the directions that fit with it
-        const bool cum_cfg = c.precision != MEMD_PREC_F32 && c.stop_mode == MEMD_STOP_FIXED &&
-                             c.boundary == MEMD_BOUNDARY_REFERENCE && c.mean_eval != 1;
+        const bool cum_cfg = c.precision != MEMD_PREC_F32 && c.stop_mode == MEMD_STOP_FIXED && c.mean_eval != 1;
         const int fit = directions_that_fit(c, p->g, p->real_bytes, p->xbytes, p->tbytes, cum_cfg, want_inplace);
         p->Kc = std::max(1, std::min({K, fit, kc_limit}));
     }
@@ -1396,8 +1385,7 @@ static memd_status create_plan(const memd_config* cfg, const memd_tuning* tun, m
         return set_error(MEMD_ERR_UNSUPPORTED,
                          "plan: impulse-accumulation mean needs the mixed form in fixed mode with the reference boundary");
     }
-    p->cum = (cum_ok || (f64 && c.stop_mode == MEMD_STOP_FIXED && c.boundary == MEMD_BOUNDARY_REFERENCE)) &&
-             c.mean_eval != 1;
+    p->cum = c.precision != MEMD_PREC_F32 && c.stop_mode == MEMD_STOP_FIXED && c.mean_eval != 1;
     p->cumG = C >= 32 ? 32 : (C > 8 ? 16 : 8);
     const size_t rb = (size_t)p->real_bytes;
     if (c.precision == MEMD_PREC_MIXED)

@@ -240,6 +240,13 @@ __device__ __forceinline__ bool dir_qualifies(const Geom& g, const Epochs& ep, c
 constexpr int kMirWords = 16;
 enum { kMirLsym = 0, kMirRsym = 1, kMirNl = 2, kMirNr = 4, kMirLsrc = 6, kMirRsrc = 10 };
 
+// The sample whose value knot i (of E, at position p) of an envelope takes
+// (mirror boundary; mi: the direction's record).
+__device__ __forceinline__ int mirror_source(const int* __restrict__ mi, int env, int i, int E, int p)
+{
+    return i < mi[kMirNl + env] ? 2 * mi[kMirLsym] - p : (i >= E - mi[kMirNr + env] ? 2 * mi[kMirRsym] - p : p);
+}
+
 // Bounds-checked build (-DMEMD_CHECKED): MEMD_CHECK(cond) is false when an
 // index check fails, which also records the failure in g_memd_check (read and
 // cleared by the host after each run, reported as MEMD_FLAG_CHECK_FAILED); the

@@ -748,12 +748,14 @@ k_solve_queue(const int* __restrict__ cnt, Geom g, int k0, int Kc, int S, int Ss
     }
 }
 
-template <typename real, typename XT, bool XM, bool EPB, bool NAK>
+// MIR (with XM): mirror boundary, one record
+template <typename real, typename XT, bool XM, bool EPB, bool NAK, bool MIR = false>
 __global__ void __launch_bounds__(kSolveThreads)
 k_solve_fwd(const real* __restrict__ yv, const int* __restrict__ cnt, const Fac<real>* __restrict__ fac,
             real* __restrict__ dbuf, Geom g, int k0, int Kc, int S, int Ss, int H, int ngroups,
             unsigned* __restrict__ bnd, const XT* __restrict__ X, const int* __restrict__ knots,
-            const real* __restrict__ yend, Epochs ep, real* __restrict__ hz, int hsegs, SolveQueue q)
+            const real* __restrict__ yend, Epochs ep, real* __restrict__ hz, int hsegs, SolveQueue q,
+            const int* __restrict__ mir)
 {
     // hz != nullptr (the backward sweep solves in place in dbuf): the first H
     // rows of every segment also go to hz[slot][segment][H][C], the halo the
@@ -779,11 +781,17 @@ k_solve_fwd(const real* __restrict__ yv, const int* __restrict__ cnt, const Fac<
     const int* kn = knots + slot * g.cap;
     const int nrec = EPB ? ep.n : 1;
     const real* ye = XM ? yend + slot * nrec * 2 * (size_t)C + cl : nullptr;
+    // mirror boundary (one record): the direction's mirrored knots
+    [[maybe_unused]] const int* mi = MIR ? mir + (size_t)(k0 + it.kk) * kMirWords : nullptr;
     // (XM) knot r at sample n: its record and whether it is the record's
-    // first (1) or last (2) knot
+    // first (1) or last (2) knot; mirrored: e = the sample its value is from
     auto endfl = [&](int r, int n, int& e) -> int {
         if constexpr (!EPB) {
             e = 0;
+            if constexpr (MIR) {
+                e = mirror_source(mi, it.env, r, E, n);
+                return 3;
+            }
             return r == 0 ? 1 : (r == E - 1 ? 2 : 0);
         } else {
             e = ep.wep[n >> 5];
@@ -792,6 +800,7 @@ k_solve_fwd(const real* __restrict__ yv, const int* __restrict__ cnt, const Fac<
         }
     };
     auto yx = [&](int n, int fl, int e) -> real {
+        if constexpr (MIR) return xval<real>(X[(size_t)e * C + cl]);
         if (fl) return ye[(size_t)e * 2 * C + (fl == 2 ? C : 0)];
         return xval<real>(X[(size_t)n * C + cl]);
     };
@@ -915,7 +924,9 @@ k_solve_fwd(const real* __restrict__ yv, const int* __restrict__ cnt, const Fac<
     for (int base = is; base < i1; base += B) {
         const bool full = base >= i0 && base + B <= i1 && base + B < E;
         if constexpr (XM && !EPB) {
-            if (full && base + B < E - 1) batch(std::true_type{}, std::true_type{}, base);
+            // (mirrored: at most two knots per end)
+            if (full && base + B < E - 1 && !(MIR && (base < 1 || base + B >= E - 2)))
+                batch(std::true_type{}, std::true_type{}, base);
             else if (full) batch(std::true_type{}, std::false_type{}, base);
             else batch(std::false_type{}, std::false_type{}, base);
         } else {
@@ -1181,16 +1192,26 @@ k_eval_w(XT* __restrict__ X, R* __restrict__ acc_buf, const uint32_t* __restrict
         if (lane == 0) sQ = q;
     }
     const int s_first = sgrp * SPL;
-    for (int j = 0; j < SPL; ++j) accs[(s_first + j) * G + cc] = R(0.0f);
     const R third = R(1.0 / 3.0);
     const R* yc = yv + c;
     const R* sc = sv + c;
     bool overflow = false;
 
-    // CTAs per tile (FP32: one, its sum over the directions keeps its order)
+    // CTAs per tile (FP32: one, its sum over the directions keeps its order).
+    // FP64: the directions in NZ slices whatever the CTAs per tile, so that the
+    // sum's order, and with it a record's result, does not depend on the launch
+    // (a record alone or in a batch)
     constexpr bool ONE = std::is_same<R, float>::value;
+    namespace cg_ = cooperative_groups;
     const int Z = ONE ? 1 : (int)gridDim.z, zr = ONE ? 0 : (int)blockIdx.z;
-    for (int kk = zr * WARPS + warp; kk < Kc; kk += WARPS * Z) {
+    const int NZ = std::is_same<R, double>::value ? 4 : Z;
+    constexpr int EPT = (T * G + 32 * WARPS - 1) / (32 * WARPS);  // tile elements per thread
+    R tots[EPT];
+#pragma unroll
+    for (int q = 0; q < EPT; ++q) tots[q] = R(0.0f);
+    for (int z0 = 0; z0 < NZ; z0 += Z) {
+    for (int j = 0; j < SPL; ++j) accs[(s_first + j) * G + cc] = R(0.0f);
+    for (int kk = (z0 + zr) * WARPS + warp; kk < Kc; kk += WARPS * NZ) {
         const int k = k0 + kk;
         if (!dir_qualifies(g, ep, cnt, k, rec)) continue;
         if (cnt[k] > g.cap || cnt[g.K + k] > g.cap) continue;
@@ -1309,45 +1330,57 @@ k_eval_w(XT* __restrict__ X, R* __restrict__ acc_buf, const uint32_t* __restrict
             }
         }
     }
-    if (overflow) atomicOr(&st->flags, 2);
     // the tile's CTAs (a cluster along z) have their partial sums ready; each
-    // adds them up, in the order of the warps over all of them, for a share of
-    // the tile
-    namespace cg_ = cooperative_groups;
+    // adds them up, in the order of the warps over all of them, for its share
+    // of the tile
     if (!ONE && Z > 1) cg_::this_cluster().sync();
     else __syncthreads();
+#pragma unroll
+    for (int q = 0; q < EPT; ++q) {
+        const int idx = threadIdx.x + q * 32 * WARPS;
+        if (idx >= T * G || (Z > 1 && (idx >> 5) % Z != zr)) continue;
+        R tot = tots[q];
+        if (z0 == 0 && !first_chunk) {
+            const int t = idx / G, cch = cg * G + (idx - t * G);
+            if (t < nl && cch < C) tot = acc_buf[(size_t)(n0 + t) * C + cch];
+        }
+        for (int z = 0; z < Z; ++z) {
+            const unsigned char* base = !ONE && Z > 1 ? cg_::this_cluster().map_shared_rank(smem_raw, z) : smem_raw;
+#pragma unroll
+            for (int w = 0; w < WARPS; ++w) tot = add_(tot, reinterpret_cast<const R*>(base + (size_t)w * PW)[idx]);
+        }
+        tots[q] = tot;
+    }
+    // the next slice reuses the sums, and no CTA ends while others read them
+    if (!ONE && Z > 1) cg_::this_cluster().sync();
+    else if (z0 + Z < NZ) __syncthreads();
+    }  // slices
+    if (overflow) atomicOr(&st->flags, 2);
     const int Q = sQ;
     if (!M && last_chunk && Q == 0 && (blockIdx.x == 0 || ep.n > 0) && blockIdx.y == 0 && threadIdx.x == 0)
         atomicOr(&st->flags, 1);
-    for (int idx = threadIdx.x + zr * (int)blockDim.x; idx < T * G; idx += (int)blockDim.x * Z) {
+#pragma unroll
+    for (int q = 0; q < EPT; ++q) {
+        const int idx = threadIdx.x + q * 32 * WARPS;
+        if (idx >= T * G || (Z > 1 && (idx >> 5) % Z != zr)) continue;
         const int t = idx / G, ch = idx - t * G;
         const int cch = cg * G + ch;
         if (t >= nl || cch >= C) continue;
         const size_t off = (size_t)(n0 + t) * C + cch;
-        R tot = first_chunk ? R(0.0f) : acc_buf[off];
-        if constexpr (ONE) {
-#pragma unroll
-            for (int w = 0; w < WARPS; ++w) tot = add_(tot, reinterpret_cast<const R*>(smem_raw + (size_t)w * PW)[idx]);
-        } else for (int z = 0; z < Z; ++z) {
-            const unsigned char* base = Z > 1 ? cg_::this_cluster().map_shared_rank(smem_raw, z) : smem_raw;
-#pragma unroll
-            for (int w = 0; w < WARPS; ++w) tot = add_(tot, reinterpret_cast<const R*>(base + (size_t)w * PW)[idx]);
-        }
         if (last_chunk) {
-            const R mval = div_(mul_(tot, R(0.5f)), R(Q));
+            const R mval = div_(mul_(tots[q], R(0.5f)), R(Q));
             if (M) M[off] = mval;
             else X[off] = xsub(X[off], mval);
         } else {
-            acc_buf[off] = tot;
+            acc_buf[off] = tots[q];
         }
     }
-    if (!ONE && Z > 1) cg_::this_cluster().sync();  // the others may still be reading this CTA's sums
 }
 
 // ---------------------------------------------------------------------------
 // Mean envelope by impulse accumulation (mixed form, fixed mode).
 //
-// A natural cubic spline with knots x_j is, for n >= x_0,
+// A cubic spline with knots x_j is, for n >= x_0,
 //     S(n) = P_0(n) + sum_j dd_j (n - x_j)_+^3,   dd_j = d_j - d_{j-1}
 // (the pieces agree in value, slope and curvature at every interior knot;
 // only the cubic coefficient d jumps), so the sum over all envelopes M(n) =
@@ -1515,7 +1548,7 @@ struct CumShared {
     int* arrive;              // [groups][W]
 };
 
-template <int G>
+template <int G, bool MIR>
 __global__ void __launch_bounds__(256, 4)
 k_mean_cum(const float2* __restrict__ X, float2* __restrict__ Xout, dd* __restrict__ acc_buf,
            const uint32_t* __restrict__ bits,
@@ -1523,8 +1556,11 @@ k_mean_cum(const float2* __restrict__ X, float2* __restrict__ Xout, dd* __restri
            const dd* __restrict__ rtab, const dd* __restrict__ rtab3, const dd* __restrict__ h3tab,
            const dd* __restrict__ sv, const dd* __restrict__ yend, const unsigned* __restrict__ bnd, unsigned* __restrict__ bnd_clear,
            const int* __restrict__ cumcfg, CumShared sh_g, Geom g, int k0, int Kc, int first_chunk, int last_chunk,
-           RunState* st, Epochs ep)
+           RunState* st, Epochs ep, const int* __restrict__ mir)
 {
+    // MIR (mirror boundary, one record): the knot list is [left mirrored |
+    // interior | right mirrored]; mirrored knots past the ends, and those that fall between an
+    // end and its first extremum, are knots like the others
     constexpr int SUB = 32 / G;
     constexpr int NWS = 8 * SUB;
     constexpr int NE = 256;  // (direction, envelope) pairs described per round
@@ -1608,11 +1644,20 @@ k_mean_cum(const float2* __restrict__ X, float2* __restrict__ Xout, dd* __restri
                     const uint32_t bw = bb[w];
                     const uint32_t bwa = bb[wa];
                     const uint32_t le = (ba == 31) ? bwa : (bwa & ((2u << ba) - 1u));
-                    i = min(wp[wa] + __popc(le) - 1, ke - 2);
-                    j = max(kb + 1, wp[w] + (int)(bw & 1u));
-                    const int nw = wp[wend] - wp[w] - (int)(bw & 1u);  // knots in (p0, p0 + 32 m)
-                    n = max(0, min(j + nw - 1, ke - 2) - j + 1);
                     const int* kn = knots + slot * g.cap;
+                    const int before = wp[w] + (int)(bw & 1u);  // knots at or before p0
+                    const int nw = wp[wend] - before;           // knots in (p0, p0 + 32 m)
+                    if constexpr (MIR) {
+                        int lp0, lp1, rp0, rp1;
+                        mirror_positions(mir + (size_t)k * kMirWords, kn, env, ke, lp0, lp1, rp0, rp1);
+                        i = min(max(mirror_before(na + 1, lp0, lp1, rp0, rp1) + wp[wa] + __popc(le) - 1, 0), ke - 2);
+                        j = max(1, mirror_before(p0 + 1, lp0, lp1, rp0, rp1) + before);
+                        n = max(0, min(mirror_before(p0 + nl, lp0, lp1, rp0, rp1) + before + nw, ke - 1) - j);
+                    } else {
+                        i = min(wp[wa] + __popc(le) - 1, ke - 2);
+                        j = max(kb + 1, before);
+                        n = max(0, min(j + nw - 1, ke - 2) - j + 1);
+                    }
                     xi = kn[i];
                     hh = kn[i + 1] - xi;
                 }
@@ -1642,8 +1687,16 @@ k_mean_cum(const float2* __restrict__ X, float2* __restrict__ Xout, dd* __restri
                 // knot values: X at interior knots, the record's clamped end knots from yend
                 const dd* ye = yend + (slot * (ep.n > 0 ? ep.n : 1) + rec) * 2 * (size_t)C + cl;
                 const int rbeg = ep.n > 0 ? ep.off[rec] : 0;
-                const dd y0 = (xi == rbeg) ? ye[0] : xval<dd>(X[(size_t)xi * C + cl]);
-                const dd y1 = (xi + h == rend - 1) ? ye[C] : xval<dd>(X[(size_t)(xi + h) * C + cl]);
+                dd y0, y1;
+                if constexpr (MIR) {
+                    const int* mi = mir + (size_t)(k0 + kk) * kMirWords;
+                    const int E = cnt[env * g.K + k0 + kk];
+                    y0 = xval<dd>(X[(size_t)mirror_source(mi, env, i, E, xi) * C + cl]);
+                    y1 = xval<dd>(X[(size_t)mirror_source(mi, env, i + 1, E, xi + h) * C + cl]);
+                } else {
+                    y0 = (xi == rbeg) ? ye[0] : xval<dd>(X[(size_t)xi * C + cl]);
+                    y1 = (xi + h == rend - 1) ? ye[C] : xval<dd>(X[(size_t)(xi + h) * C + cl]);
+                }
                 const dd s0 = sv[rb + (size_t)i * C], s1 = sv[rb + (size_t)(i + 1) * C];
                 const dd d = (s1 - s0) * rtab3[h];
                 const dd s02(2.0f * s0.hi, 2.0f * s0.lo);  // exact

@@ -1,5 +1,5 @@
 // memd_mean_fix.cuh -- mean envelope of the FP64 form by impulse accumulation
-// in wide fixed point (fixed number of sifts, reference boundary).
+// in wide fixed point (fixed number of sifts).
 #pragma once
 
 #include "memd_kernels.cuh"
@@ -118,15 +118,18 @@ __device__ __forceinline__ double twice(double v)
 // cluster share a 64-sample span: each takes half the pairs, then, with the
 // other's sums from distributed shared memory, half the rows.
 // Bound by the FP64 pipe at dense knots, by load latency at sparse ones.
-template <int G>
+template <int G, bool MIR>
 __global__ void __launch_bounds__(256, 3)
 k_mean_fix(const double* __restrict__ X, double* __restrict__ Xout, ulonglong2* __restrict__ acc_buf,
            const uint32_t* __restrict__ bits, const int* __restrict__ wpref, const int* __restrict__ knots,
            const int* __restrict__ cnt, const double* __restrict__ rtab, const double2* __restrict__ rtab3,
            const double* __restrict__ sv, const double* __restrict__ yend, const unsigned* __restrict__ xexp,
            const unsigned long long* __restrict__ tot, Geom g, int k0, int Kc, int first_chunk, int last_chunk,
-           RunState* st, Epochs ep)
+           RunState* st, Epochs ep, const int* __restrict__ mir)
 {
+    // MIR (mirror boundary, one record): the knot list is [left mirrored |
+    // interior | right mirrored]
+
     constexpr int SUB = 32 / G;
     constexpr int NWS = 8 * SUB;
     constexpr int NE = 256;  // pairs described per round
@@ -167,6 +170,10 @@ k_mean_fix(const double* __restrict__ X, double* __restrict__ Xout, ulonglong2* 
             const int b = ep.n > 0 ? ep.cnt[((size_t)g.K + k) * ep.n + rec] : cnt[g.K + k];
             q += (a > 3 && b > 3) ? 1 : 0;
             et += (unsigned long long)(a + b);
+            if constexpr (MIR) {  // interior knots, as the count of several passes
+                const int* mi = mir + (size_t)k * kMirWords;
+                et -= (unsigned long long)(mi[kMirNl] + mi[kMirNr] + mi[kMirNl + 1] + mi[kMirNr + 1]);
+            }
         }
         q = warp_sum(q);
         et = warp_sum(et);
@@ -224,7 +231,13 @@ k_mean_fix(const double* __restrict__ X, double* __restrict__ Xout, ulonglong2* 
                     const int* wp = wpref + slot * (g.W + 1);
                     const int kb = ep.n > 0 ? wp[ep.w0[rec]] : 0;
                     je = (ep.n > 0 ? wp[ep.w0[rec + 1]] : (env ? En : Ex)) - 2;
-                    const int at = wp[w] + (int)(bits[slot * g.W + w] & 1u);  // knots at or before p0
+                    int at = wp[w] + (int)(bits[slot * g.W + w] & 1u);  // knots at or before p0
+                    if constexpr (MIR) {
+                        int lp0, lp1, rp0, rp1;
+                        mirror_positions(mir + (size_t)k * kMirWords, knots + slot * g.cap, env, je + 2, lp0, lp1, rp0,
+                                         rp1);
+                        at += mirror_before(p0 + 1, lp0, lp1, rp0, rp1);
+                    }
                     j = min(max(at - 1, kb), je);
                 }
             }
@@ -270,8 +283,15 @@ k_mean_fix(const double* __restrict__ X, double* __restrict__ Xout, ulonglong2* 
                 qp = qc;
                 while (a < nA && (na < xn || j == je)) {
                     // S(na + t) = A + B t + C t^2 + d t^3 on this piece
-                    const double y0 = (xj == roff) ? ye[0] : X[(size_t)xj * C + cl];
-                    const double y1 = (xn == rlast) ? ye[C] : X[(size_t)xn * C + cl];
+                    double y0, y1;
+                    if constexpr (MIR) {
+                        const int* mi = mir + (size_t)(k0 + kk) * kMirWords;
+                        y0 = X[(size_t)mirror_source(mi, env, j, je + 2, xj) * C + cl];
+                        y1 = X[(size_t)mirror_source(mi, env, j + 1, je + 2, xn) * C + cl];
+                    } else {
+                        y0 = (xj == roff) ? ye[0] : X[(size_t)xj * C + cl];
+                        y1 = (xn == rlast) ? ye[C] : X[(size_t)xn * C + cl];
+                    }
                     const double u = from_int<double>(na - xj), u3 = from_int<double>(3 * (na - xj));
                     const double b = __fma_rn(-r3.y, __fma_rn(2.0, s0, s1), __dmul_rn(__dsub_rn(y1, y0), rtab[h]));
                     const double e = __fma_rn(d, u, s0);
@@ -446,13 +466,22 @@ k_mean_fix(const double* __restrict__ X, double* __restrict__ Xout, ulonglong2* 
                         const int kb = ep.n > 0 ? wp[ep.w0[rec]] : 0;
                         const int wn = n >> 5;
                         const int before = wp[wn] + __popc(bits[slot * g.W + wn] & ((1u << (n & 31)) - 1u));
-                        const int i = max(before - 1, kb);
                         const int* kn = knots + slot * g.cap;
+                        int i = max(before - 1, kb);
+                        const int* mi = mir + (size_t)k * kMirWords;
+                        const int E = cnt[env * g.K + k];
+                        if constexpr (MIR) {
+                            int lp0, lp1, rp0, rp1;
+                            mirror_positions(mi, kn, env, E, lp0, lp1, rp0, rp1);
+                            i = min(max(mirror_before(n, lp0, lp1, rp0, rp1) + before - 1, 0), E - 2);
+                        }
                         const double* sp = sv + slot * (size_t)g.cap * C + c;
                         const double* ye = yend + (slot * (ep.n > 0 ? ep.n : 1) + rec) * 2 * (size_t)C + c;
                         const int xi = kn[i], xn = kn[i + 1];
-                        const double y0 = (xi == roff) ? ye[0] : X[(size_t)xi * C + c];
-                        const double y1 = (xn == rlast) ? ye[C] : X[(size_t)xn * C + c];
+                        const double y0 = MIR ? X[(size_t)mirror_source(mi, env, i, E, xi) * C + c]
+                                                   : (xi == roff ? ye[0] : X[(size_t)xi * C + c]);
+                        const double y1 = MIR ? X[(size_t)mirror_source(mi, env, i + 1, E, xn) * C + c]
+                                                   : (xn == rlast ? ye[C] : X[(size_t)xn * C + c]);
                         const double s0 = sp[(size_t)i * C], s1 = sp[(size_t)(i + 1) * C];
                         const double t = (double)(n - xi);
                         const double h3 = __dmul_rn((double)(xn - xi), 1.0 / 3.0);

@@ -69,3 +69,26 @@ def test_values_outside_the_fixed_point_range_are_evaluated_directly(value, chun
     # 1e-310: the values are subnormal, multiples of 2^-1074
     tol = 64 * max(2.0 ** -53 * np.abs(np.where(np.isfinite(y), y, 0.0)).max(), 2.0 ** -1074)
     assert (np.abs(np.where(np.isfinite(b), a - b, 0.0)) <= tol).all()
+
+
+# records whose mirrored knots reach the ends from one or two extrema, spans of 32 to 128 samples
+@pytest.mark.parametrize("chunk", [0, 5])
+@pytest.mark.parametrize("C,L,K,period", [(1, 40, 4, 6), (3, 65, 8, 9), (8, 500, 12, 30), (17, 1000, 9, 60),
+                                          (32, 4099, 20, 14), (5, 3001, 16, 300)])
+def test_impulse_means_with_mirrored_ends_match_direct_evaluation(C, L, K, period, chunk):
+    y, d = signal(C, L, period, 11), oracle.directions(C, K)
+    kw = dict(boundary=mg.BOUNDARY_MIRROR, dir_chunk=chunk)
+    a, sa = one_sift(y, d, **kw)
+    b, sb = one_sift(y, d, mean_eval=1, **kw)
+    assert sa.flags == sb.flags and np.array_equal(np.isnan(a), np.isnan(b))
+    assert np.nanmax(np.abs(a - b), initial=0.0) <= 64 * 2.0 ** -53 * np.abs(y).max()
+    outs = []
+    for mean_eval in (0, 1):  # mixed form: double-float means, float32 outputs of the same input
+        plan = mg.Plan(C, L, K, 2, 1, mg.PREC_MIXED, mean_eval=mean_eval, **kw)
+        o = torch.empty((2, C, L), dtype=torch.float32, device="cuda")
+        plan.run(torch.as_tensor(y, dtype=torch.float32).cuda(), torch.as_tensor(d, dtype=torch.float32).cuda(), o)
+        plan.close()
+        outs.append(o.cpu().numpy().astype(np.float64))
+    assert np.array_equal(np.isnan(outs[0]), np.isnan(outs[1]))
+    # both round a mean good to ~1e-13 to float32: one ulp of the largest value apart at most
+    assert np.nanmax(np.abs(outs[0] - outs[1]), initial=0.0) <= 2.0 ** -22 * np.abs(y).max()
