@@ -67,14 +67,13 @@ struct memd_plan {
     int bpass;                  // (sift, chunk) passes enqueued so far in the decomposition being built
     size_t proj_smem;
     void* X;
-    void* Xb;  // impulse-accumulation mean: the other working-signal buffer (the mean kernel reads X, writes Xb)
+    void* Xb;  // fixed mode: the other working-signal buffer (the mean kernel reads X, writes Xb)
     void* run;
     void* dir;   // FP64/FP32: K x C; mixed: high words then low words
     void* acc;
     void* imf;
-    void* yv;
     void* sv;
-    void* yend;  // impulse-accumulation mean: clamped end-knot values [2][Kc][records][2][C] (no yv gather)
+    void* yend;  // clamped end-knot values [2][Kc][records][2][C] (the other knots' are read from the signal)
     void* dbuf;  // forward-eliminated right-hand sides [2][Kc][cap][C]
     void* fac;
     void* rtab;
@@ -197,8 +196,7 @@ static bool make_tile_map(CUtensorMap* m, void* base, uint64_t cols, uint64_t ro
 // buffers once.  Fewer passes re-run the projection, compaction and mean over
 // the record fewer times (512 batched epochs of 32 x 1024..8192 samples, 64
 // directions: three passes 1.80 s, one pass 1.31 s).
-static int directions_that_fit(const memd_config& c, const Geom& g, int rb, int xbytes, int tbytes, bool cum,
-                               bool inplace)
+static int directions_that_fit(const memd_config& c, const Geom& g, int rb, int xbytes, int tbytes, bool inplace)
 {
     size_t fr = 0, tot = 0;
     if (cudaMemGetInfo(&fr, &tot) != cudaSuccess || fr == 0) {
@@ -208,9 +206,8 @@ static int directions_that_fit(const memd_config& c, const Geom& g, int rb, int 
     const double C = g.C, L = g.L, cap = g.cap, W = g.W;
     const bool stop = c.stop_mode == MEMD_STOP_CRITERION;
     // eliminated right-hand sides and solutions (one array in place, with a
-    // quarter for the halo copies at most), knot values unless the mean reads
-    // the signal
-    const double arrays = (inplace ? 1.25 : 2.0) + (cum ? 0.0 : 1.0);
+    // quarter for the halo copies at most)
+    const double arrays = inplace ? 1.25 : 2.0;
     const double per_dir = 2.0 * cap * (4.0 + 4.0 * rb + (double)rb * C * arrays) + 8.0 * (2.0 * W + 1.0) +
                            (stop ? (double)rb * std::ceil(C / 4.0) * L : 0.0);
     const double fixed = C * L * (3.0 * xbytes + (double)tbytes * (double)c.num_imfs + 2.0 * rb) + 8.0 * 39.0 * W * C +
@@ -355,9 +352,9 @@ static void launch_eval(memd_plan* p, cudaStream_t s, int k0, int kc, int first,
             at[0].val.clusterDim.z = (unsigned)p->ewZ;
             lc.attrs = at;
             lc.numAttrs = p->ewZ > 1 ? 1 : 0;
-            cudaLaunchKernelEx(&lc, kern, (XT*)p->X, (R*)p->acc, (const uint32_t*)p->bits, (const int*)p->wpref,
+            cudaLaunchKernelEx(&lc, kern, (const XT*)p->X, (XT*)p->Xb, (R*)p->acc, (const uint32_t*)p->bits, (const int*)p->wpref,
                                (const int*)p->knots, (const int*)p->cnt, (const R*)p->rtab, (const R*)p->sv,
-                               (const R*)p->yv, g, k0, kc, first, last, p->st, stopm ? (R*)p->M : (R*)nullptr,
+                               (const R*)p->yend, g, k0, kc, first, last, p->st, stopm ? (R*)p->M : (R*)nullptr,
                                stopm ? (R*)p->part : (R*)nullptr, (const int*)p->mir, p->ep);
         };
         if (stopm) go(k_eval_w<G, SPL, XT, R, true, W>);
@@ -485,8 +482,8 @@ static void enqueue_sift(memd_plan* p, cudaStream_t s, memd_trace_entry* trace, 
         }
         lc.begin(MEMD_STAGE_COMPACT);
         k_compact<R, XT><<<dim3((unsigned)nch, (unsigned)(2 * kc)), 512, 0, s>>>(
-            p->bits, p->wpref, p->knots, p->cnt, (R*)p->yv, (const XT*)p->X, trace, g, k0, kc, p->st, trace_rows,
-            p->cum ? (R*)p->yend : nullptr, p->ep, p->mir, p->csh, nch);
+            p->bits, p->wpref, p->knots, p->cnt, (const XT*)p->X, trace, g, k0, kc, p->st, trace_rows,
+            (R*)p->yend, p->ep, p->mir, p->csh, nch);
         lc.end(MEMD_STAGE_COMPACT);
         const long nsegf = (g.cap + p->Sf - 1) / p->Sf;
         const long nf = 2L * kc * nsegf;
@@ -512,31 +509,21 @@ static void enqueue_sift(memd_plan* p, cudaStream_t s, memd_trace_entry* trace, 
             lc.end(MEMD_STAGE_SOLVE);
         }
         lc.begin(MEMD_STAGE_SOLVE);
-        bool xm = false;
-#define MEMD_FWD(XM_, EPB_, NAK_, MIR_)                                                                               \
-    k_solve_fwd<R, XT, XM_, EPB_, NAK_, MIR_><<<p->squeue ? persistent_grid(k_solve_fwd<R, XT, XM_, EPB_, NAK_, MIR_>,     \
-                                                                      kSolveThreads, p->sms, nb) : nb,          \
-                                          kSolveThreads, 0, s>>>(                                              \
-        (const R*)p->yv, p->cnt, (const Fac<R>*)p->fac, (R*)p->dbuf, g, k0, kc, p->S, p->Ss, p->H, p->ngroups, \
-        bcur, XM_ ? (const XT*)p->X : nullptr, p->knots, XM_ ? (const R*)p->yend : nullptr, p->ep,               \
-        p->inplace ? (R*)p->hz : nullptr, p->hsegs, q, p->mir)
-        if constexpr (P != MEMD_PREC_F32) {
-            if (p->cum) {  // knot values from the working signal (the impulse-accumulation path)
-                xm = true;
-                if (p->ep.n > 0) {  // batched runs: record ends found by position
-                    if (g.nak) MEMD_FWD(true, true, true, false);
-                    else MEMD_FWD(true, true, false, false);
-                } else if (g.mirror) {
-                    if (g.nak) MEMD_FWD(true, false, true, true);
-                    else MEMD_FWD(true, false, false, true);
-                } else if (g.nak) MEMD_FWD(true, false, true, false);
-                else MEMD_FWD(true, false, false, false);
-            }
-        }
-        if (!xm) {
-            if (g.nak) MEMD_FWD(false, false, true, false);
-            else MEMD_FWD(false, false, false, false);
-        }
+#define MEMD_FWD(EPB_, NAK_, MIR_)                                                                              \
+    k_solve_fwd<R, XT, EPB_, NAK_, MIR_><<<p->squeue ? persistent_grid(k_solve_fwd<R, XT, EPB_, NAK_, MIR_>,   \
+                                                                       kSolveThreads, p->sms, nb) : nb,         \
+                                           kSolveThreads, 0, s>>>(                                             \
+        p->cnt, (const Fac<R>*)p->fac, (R*)p->dbuf, g, k0, kc, p->S, p->Ss, p->H, p->ngroups, bcur,            \
+        (const XT*)p->X, p->knots, (const R*)p->yend, p->ep, p->inplace ? (R*)p->hz : nullptr, p->hsegs, q,     \
+        p->mir)
+        if (p->ep.n > 0) {  // batched runs: record ends found by position
+            if (g.nak) MEMD_FWD(true, true, false);
+            else MEMD_FWD(true, false, false);
+        } else if (g.mirror) {
+            if (g.nak) MEMD_FWD(false, true, true);
+            else MEMD_FWD(false, false, true);
+        } else if (g.nak) MEMD_FWD(false, true, false);
+        else MEMD_FWD(false, false, false);
 #undef MEMD_FWD
         lc.end(MEMD_STAGE_SOLVE);
         lc.begin(MEMD_STAGE_SOLVE);
@@ -571,7 +558,7 @@ static void enqueue_sift(memd_plan* p, cudaStream_t s, memd_trace_entry* trace, 
         launch_eval<P>(p, s, k0, kc, ch == 0, ch == p->nchunks - 1);
         lc.end(MEMD_STAGE_EVAL);
         ++p->bpass;
-        if (p->cum && ch == p->nchunks - 1) std::swap(p->X, p->Xb);  // the next pass reads the updated signal
+        if (p->Xb && ch == p->nchunks - 1) std::swap(p->X, p->Xb);  // the next pass reads the updated signal
         if (stop) {
             const bool last = ch == p->nchunks - 1;
             RecStop* rs = p->batched ? (RecStop*)p->recstop : nullptr;
@@ -1318,19 +1305,17 @@ static memd_status create_plan(const memd_config* cfg, const memd_tuning* tun, m
         // automatic: as many directions per pass as the free memory allows,
         // with separate right-hand-side and solution arrays while all of them
         // fit (the faster layout), solving in place when that fits more
-        const bool cum_cfg = c.precision != MEMD_PREC_F32 && c.stop_mode == MEMD_STOP_FIXED && c.mean_eval != 1;
         const int want = std::min(K, kc_limit);
-        const int fit_sep = directions_that_fit(c, p->g, p->real_bytes, p->xbytes, p->tbytes, cum_cfg, false);
+        const int fit_sep = directions_that_fit(c, p->g, p->real_bytes, p->xbytes, p->tbytes, false);
         if (fit_sep >= want || !inplace_ok) {
             p->Kc = std::max(1, std::min(want, fit_sep));
         } else {
-            const int fit_inp = directions_that_fit(c, p->g, p->real_bytes, p->xbytes, p->tbytes, cum_cfg, true);
+            const int fit_inp = directions_that_fit(c, p->g, p->real_bytes, p->xbytes, p->tbytes, true);
             p->Kc = std::max(1, std::min(want, std::max(fit_sep, fit_inp)));
             want_inplace = fit_inp > fit_sep;
         }
     } else if (c.dir_chunk <= 0) {  // layout fixed by the tuning: the directions that fit with it
-        const bool cum_cfg = c.precision != MEMD_PREC_F32 && c.stop_mode == MEMD_STOP_FIXED && c.mean_eval != 1;
-        const int fit = directions_that_fit(c, p->g, p->real_bytes, p->xbytes, p->tbytes, cum_cfg, want_inplace);
+        const int fit = directions_that_fit(c, p->g, p->real_bytes, p->xbytes, p->tbytes, want_inplace);
         p->Kc = std::max(1, std::min({K, fit, kc_limit}));
     }
     p->Kc = std::min(p->Kc, 1024);
@@ -1400,7 +1385,7 @@ static memd_status create_plan(const memd_config* cfg, const memd_tuning* tun, m
         if (st == MEMD_OK) st = dev_alloc(p, (void**)&(ptr), (bytes)); \
     } while (0)
     ALLOC(p->X, (size_t)p->xbytes * CL);
-    if (p->cum) ALLOC(p->Xb, (size_t)p->xbytes * CL);
+    if (c.stop_mode == MEMD_STOP_FIXED) ALLOC(p->Xb, (size_t)p->xbytes * CL);
     ALLOC(p->run, (size_t)p->xbytes * CL);
     ALLOC(p->dir, 8 * (size_t)K * C);
     if (p->nchunks > 1) ALLOC(p->acc, (p->cum && f64 ? 16 : rb) * CL);  // FP64: the exact 128-bit sum
@@ -1415,8 +1400,7 @@ static memd_status create_plan(const memd_config* cfg, const memd_tuning* tun, m
     ALLOC(p->csh.hacc, sizeof(unsigned long long) * 2 * Kc);
     ALLOC(p->csh.arrive, sizeof(int) * 2 * Kc);
     ALLOC(p->fac, rb * 4 * 2 * Kc * p->g.cap);
-    if (!p->cum) ALLOC(p->yv, rb * 2 * Kc * p->g.cap * C);
-    else ALLOC(p->yend, rb * 2 * Kc * (size_t)std::max<int64_t>(1, c.max_epochs) * 2 * C);  // [2][Kc][epochs][2][C]
+    ALLOC(p->yend, rb * 2 * Kc * (size_t)std::max<int64_t>(1, c.max_epochs) * 2 * C);  // [2][Kc][epochs][2][C]
     ALLOC(p->sv, rb * 2 * Kc * p->g.cap * C);
     p->inplace = want_inplace;
     p->hsegs = p->H > 0 ? (int)solve_segments_max(p->g.cap, p->S, p->Ss, p->H) : 0;

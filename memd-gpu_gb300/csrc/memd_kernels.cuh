@@ -30,7 +30,8 @@
 //   wpref[env][kk][w]               knots before word w (w <= W)
 //   knots[env][kk][i]               knot sample indices, i < E <= cap
 //   fac[env][kk][i]                 Fac<real> per knot row
-//   yv[env][kk][i][c]               knot values (end knots clamped)
+//   yend[env][kk][record][2][c]     clamped end-knot values (the others are read
+//                                   from X at the knots)
 //   sv[env][kk][i][c]               spline solution per knot and channel
 // env 0 = maxima (upper envelope), 1 = minima (lower envelope); kk indexes the
 // directions of the current chunk, counts cnt[env][k] use the global k.
@@ -130,8 +131,7 @@ k_project_extrema(const XT* __restrict__ X, const real* __restrict__ dir,
 // Knot lists.  The bitmask of each (envelope, direction) is cut into chunks of
 // kCompactChunk words; CTA (chunk, slot) of 512 threads writes the knots of its
 // chunk (each thread an ordered run of words, a block scan of the popcounts,
-// the offset of the chunk from k_compact_count's per-chunk totals) and gathers
-// their values; the last CTA of a slot to arrive (an atomic counter, no
+// the offset of the chunk from k_compact_count's per-chunk totals); the last CTA of a slot to arrive (an atomic counter, no
 // waiting) writes the count, the trace entry, the mirrored knots and the
 // end-point clamp.  A record of up to kCompactChunk words is one chunk and
 // needs no count pass.
@@ -167,20 +167,20 @@ k_compact_count(const uint32_t* __restrict__ bits, int* __restrict__ ctot, Geom 
 template <typename real, typename XT>
 __global__ void __launch_bounds__(512)
 k_compact(const uint32_t* __restrict__ bits, int* __restrict__ wpref, int* __restrict__ knots,
-          int* __restrict__ cnt, real* __restrict__ yv, const XT* __restrict__ X,
+          int* __restrict__ cnt, const XT* __restrict__ X,
           memd_trace_entry* __restrict__ trace, Geom g, int k0, int Kc, RunState* st, int trace_rows,
           real* __restrict__ yend, Epochs ep, const int* __restrict__ mir, CompactShared cs, int nch)
 {
-    // yend != nullptr: the knot values are not gathered; only the two end
-    // knots' values (clamped) are written, to yend[env][kk][2][C], and the
+    // The knot values are not gathered: only the two end knots' values (clamped)
+    // of each record are written, to yend[env][kk][record][2][C], and the
     // consumers read the interior knot values from X.
     // trace_rows > 0: trace is the base of a [trace_rows][K][2] array and the
     // row of this pass is st->trace_row (stop mode); otherwise trace points at
     // this pass's [K][2] block.
     // g.mirror: the knot list is [left mirrored | interior extrema | right
     // mirrored] (mir from k_mirror); wpref and the bitmask count the interior
-    // extrema only, the knot values come from the mirrored knots' source
-    // samples, and the reference's end-point clamp does not apply.
+    // extrema only, the consumers read the mirrored knots' values at their
+    // source samples, and the reference's end-point clamp does not apply.
     const int chunk = blockIdx.x;
     const int slot_i = blockIdx.y;
     const int env = slot_i / Kc, kk = slot_i - env * Kc;
@@ -244,15 +244,6 @@ k_compact(const uint32_t* __restrict__ bits, int* __restrict__ wpref, int* __res
     h = warp_sum<unsigned long long>(h);
     if (lane == 0) hsum[wid] = h;
     __syncthreads();
-    // values of this chunk's interior knots, every channel (contiguous per knot)
-    if (!yend) {
-        real* y = yv + slot * (size_t)g.cap * C;
-        const int i0 = nlm + off, i1 = min(g.cap, nlm + off + total_s);
-        for (int idx = threadIdx.x; idx < (i1 - i0) * C; idx += blockDim.x) {
-            const int i = i0 + idx / C, c = idx % C;
-            y[(size_t)i * C + c] = xval<real>(X[(size_t)kn[i] * C + c]);
-        }
-    }
     unsigned long long hchunk = 0;
     if (threadIdx.x == 0)
         for (int i = 0; i < (int)(blockDim.x >> 5); ++i) hchunk += hsum[i];
@@ -310,31 +301,18 @@ k_compact(const uint32_t* __restrict__ bits, int* __restrict__ wpref, int* __res
             tr[(size_t)(k0 + kk) * 2 + env] = e;
         }
         total_s = E;
-        off_s = Eint;
     }
     __syncthreads();
-    const int E = total_s, Eint = off_s;
+    const int E = total_s;
     if (E > g.cap || E < 2) return;
     const int nrec = ep.n > 0 ? ep.n : 1;
     if (ep.n > 0) {
         for (int e = threadIdx.x; e < ep.n; e += blockDim.x)
             ep.cnt[((size_t)env * g.K + k0 + kk) * ep.n + e] = __ldcg(&wp[ep.w0[e + 1]]) - __ldcg(&wp[ep.w0[e]]);
     }
-    if (mi) {
-        // the mirrored knots' values from their source samples
-        if (!yend) {
-            real* y = yv + slot * (size_t)g.cap * C;
-            for (int idx = threadIdx.x; idx < (nlm + nrm) * C; idx += blockDim.x) {
-                const int j = idx / C, c = idx % C;
-                const int i = j < nlm ? j : nlm + Eint + (j - nlm);
-                const int src = j < nlm ? mi[kMirLsrc + 2 * env + j] : mi[kMirRsrc + 2 * env + (j - nlm)];
-                y[(size_t)i * C + c] = xval<real>(X[(size_t)src * C + c]);
-            }
-        }
-        return;
-    }
+    if (mi) return;
     // The end-point clamp of the two end knots of each record (REF:447-486
-    // max, 545-584 min); the raw end values were gathered with the chunks.
+    // max, 545-584 min).
     for (int idx = threadIdx.x; idx < nrec * C; idx += blockDim.x) {
         const int e = idx / C, c = idx - e * C;
         const int kb = ep.n > 0 ? __ldcg(&wp[ep.w0[e]]) : 0;
@@ -358,15 +336,9 @@ k_compact(const uint32_t* __restrict__ bits, int* __restrict__ wpref, int* __res
             t = fmad_(slope, real(xE - xb), bb);
             if (env == 0 ? (t > vE) : (t < vE)) vE = t;
         }
-        if (yend) {
-            real* ye = yend + ((slot * nrec) + e) * 2 * (size_t)C;
-            ye[c] = v0;
-            ye[C + c] = vE;
-        } else {
-            real* y = yv + slot * (size_t)g.cap * C;
-            y[(size_t)kb * C + c] = v0;
-            y[(size_t)(ke - 1) * C + c] = vE;
-        }
+        real* ye = yend + ((slot * nrec) + e) * 2 * (size_t)C;
+        ye[c] = v0;
+        ye[C + c] = vE;
     }
 }
 
@@ -748,10 +720,9 @@ k_solve_queue(const int* __restrict__ cnt, Geom g, int k0, int Kc, int S, int Ss
     }
 }
 
-// MIR (with XM): mirror boundary, one record
-template <typename real, typename XT, bool XM, bool EPB, bool NAK, bool MIR = false>
+template <typename real, typename XT, bool EPB, bool NAK, bool MIR>
 __global__ void __launch_bounds__(kSolveThreads)
-k_solve_fwd(const real* __restrict__ yv, const int* __restrict__ cnt, const Fac<real>* __restrict__ fac,
+k_solve_fwd(const int* __restrict__ cnt, const Fac<real>* __restrict__ fac,
             real* __restrict__ dbuf, Geom g, int k0, int Kc, int S, int Ss, int H, int ngroups,
             unsigned* __restrict__ bnd, const XT* __restrict__ X, const int* __restrict__ knots,
             const real* __restrict__ yend, Epochs ep, real* __restrict__ hz, int hsegs, SolveQueue q,
@@ -761,9 +732,10 @@ k_solve_fwd(const real* __restrict__ yv, const int* __restrict__ cnt, const Fac<
     // rows of every segment also go to hz[slot][segment][H][C], the halo the
     // backward sweep of the segment before reads while this one's rows are
     // being overwritten by their solutions
-    // XM: knot values read from the working signal, y_i = X[x_i] (interior
-    // knots) and yend (the clamped end knots of each record), instead of yv;
-    // EPB (with XM): batched epochs, a record's end knots found by position.
+    // Knot values: the working signal, y_i = X[x_i], at interior knots and yend
+    // (the clamped end knots of each record).  EPB: batched epochs, a record's
+    // end knots found by position.  MIR: mirror boundary (one record), values
+    // at the mirrored knots' source samples.
     // Rows of a record's end knots are the identity rows of the
     // factorisation (lm == 0): their right-hand side is 0.
     constexpr int B = kSolveBatch;
@@ -777,13 +749,11 @@ k_solve_fwd(const real* __restrict__ yv, const int* __restrict__ cnt, const Fac<
     const int cl = min(it.c, C - 1);
     const size_t slot = (size_t)it.env * Kc + it.kk;
     const Fac<real>* f = fac + slot * g.cap;
-    const real* y = XM ? nullptr : yv + slot * (size_t)g.cap * C + cl;
     const int* kn = knots + slot * g.cap;
     const int nrec = EPB ? ep.n : 1;
-    const real* ye = XM ? yend + slot * nrec * 2 * (size_t)C + cl : nullptr;
-    // mirror boundary (one record): the direction's mirrored knots
+    const real* ye = yend + slot * nrec * 2 * (size_t)C + cl;
     [[maybe_unused]] const int* mi = MIR ? mir + (size_t)(k0 + it.kk) * kMirWords : nullptr;
-    // (XM) knot r at sample n: its record and whether it is the record's
+    // knot r at sample n: its record and whether it is the record's
     // first (1) or last (2) knot; mirrored: e = the sample its value is from
     auto endfl = [&](int r, int n, int& e) -> int {
         if constexpr (!EPB) {
@@ -805,14 +775,10 @@ k_solve_fwd(const real* __restrict__ yv, const int* __restrict__ cnt, const Fac<
         return xval<real>(X[(size_t)n * C + cl]);
     };
     auto yrow = [&](int r) -> real {
-        if constexpr (!XM) {
-            return y[(size_t)r * C];
-        } else {
-            const int n = kn[r];
-            int e;
-            const int fl = endfl(r, n, e);
-            return yx(n, fl, e);
-        }
+        const int n = kn[r];
+        int e;
+        const int fl = endfl(r, n, e);
+        return yx(n, fl, e);
     };
     real* o = dbuf + slot * (size_t)g.cap * C + cl;
     const int is = (H < 0) ? 0 : max(0, i0 - H);
@@ -846,7 +812,7 @@ k_solve_fwd(const real* __restrict__ yv, const int* __restrict__ cnt, const Fac<
                 fih = fr.ih;
             }
             flm = fr.lm;
-            if (XM && base + 1 + lane < E) {
+            if (base + 1 + lane < E) {
                 fx = kn[base + 1 + lane];
                 if (EPB) ffl = endfl(base + 1 + lane, fx, fe);
             }
@@ -855,11 +821,11 @@ k_solve_fwd(const real* __restrict__ yv, const int* __restrict__ cnt, const Fac<
         // batched (EPB): a full batch none of whose knots ends a record (one
         // vote over the lanes' end flags) reads every value from the signal
         bool inner_rt = false;
-        if constexpr (FULL && EPB && XM) inner_rt = !__any_sync(0xffffffffu, ffl != 0);
+        if constexpr (FULL && EPB) inner_rt = !__any_sync(0xffffffffu, ffl != 0);
         if (inner_rt) {
 #pragma unroll
             for (int k = 0; k < B; ++k) yb[k] = xval<real>(X[(size_t)__shfl_sync(0xffffffffu, fx, k) * C + cl]);
-        } else if constexpr (XM) {
+        } else {
 #pragma unroll
             for (int k = 0; k < B; ++k) {
                 const int n = __shfl_sync(0xffffffffu, fx, k);
@@ -876,10 +842,6 @@ k_solve_fwd(const real* __restrict__ yv, const int* __restrict__ cnt, const Fac<
                 }
                 yb[k] = (FULL || (k < nb && base + 1 + k < E)) ? yx(n, fl, e) : real(0);
             }
-        } else {
-#pragma unroll
-            for (int k = 0; k < B; ++k)
-                yb[k] = (FULL || (k < nb && base + 1 + k < E)) ? y[(size_t)(base + 1 + k) * C] : real(0);
         }
 #pragma unroll
         for (int k = 0; k < B; ++k) {
@@ -923,7 +885,7 @@ k_solve_fwd(const real* __restrict__ yv, const int* __restrict__ cnt, const Fac<
     };
     for (int base = is; base < i1; base += B) {
         const bool full = base >= i0 && base + B <= i1 && base + B < E;
-        if constexpr (XM && !EPB) {
+        if constexpr (!EPB) {
             // (mirrored: at most two knots per end)
             if (full && base + B < E - 1 && !(MIR && (base < 1 || base + B >= E - 2)))
                 batch(std::true_type{}, std::true_type{}, base);
@@ -1136,6 +1098,14 @@ __device__ __forceinline__ void mirror_positions(const int* __restrict__ mi, con
 // (8 channels x 2,000 samples, 64 directions, stop mode: 64-sample tiles of 8
 // warps took 104 us a pass in double-float, 20 .. 31 us so; FP64 343 us with a
 // block per tile that took one direction at a time, 53 .. 75 us so.)
+// A lane's sample costs the cubic, the sum in shared memory and one bit of the
+// knots' word (after a knot, the next interval's coefficients); the offset in
+// the interval counts up in floating point (exact).  Bound by issue and the
+// latency of that sum, so by the warps resident: five CTAs per SM in FP32 (48
+// registers), three in the others.  The lane's sums in registers instead (80
+// registers and more, the loop unrolled) took 17.6 ms for the 80 sifts of 32 x
+// 30,504, 64 directions in FP32, 11.5 so; 14.7 with the interval looked up and
+// the offset converted at every sample.
 // ---------------------------------------------------------------------------
 template <int G, int SPL, typename R, int WARPS>
 struct EvalWShape {
@@ -1143,22 +1113,25 @@ struct EvalWShape {
     static constexpr int T = NS * SPL;
     static constexpr int MI = T / 2 + 4;
     static constexpr int NW = T / 32;
-    // per warp: accumulator tile, (stop mode) spread tile, knots, bit words
+    // per warp: its sums of the tile, (stop mode) spread tile, knots and the rows
+    // of their values, bit words
     __host__ __device__ static constexpr size_t per_warp(bool stopm)
     {
-        return (size_t)(stopm ? 2 : 1) * sizeof(R) * T * G + sizeof(int) * (MI + 1) + sizeof(uint32_t) * (NW + 1);
+        return (size_t)(stopm ? 2 : 1) * sizeof(R) * T * G + 2 * sizeof(int) * (MI + 1) + sizeof(uint32_t) * (NW + 1);
     }
     static constexpr size_t smem_bytes(bool stopm) { return WARPS * ((per_warp(stopm) + 15) / 16 * 16); }
 };
 
 template <int G, int SPL, typename XT, typename R, bool STOPM, int WARPS>
-__global__ void __launch_bounds__(32 * WARPS)
-k_eval_w(XT* __restrict__ X, R* __restrict__ acc_buf, const uint32_t* __restrict__ bits,
+__global__ void __launch_bounds__(32 * WARPS, sizeof(R) == 4 ? 5 : 3)
+k_eval_w(const XT* __restrict__ X, XT* __restrict__ Xout, R* __restrict__ acc_buf, const uint32_t* __restrict__ bits,
          const int* __restrict__ wpref, const int* __restrict__ knots, const int* __restrict__ cnt,
-         const R* __restrict__ rtab, const R* __restrict__ sv, const R* __restrict__ yv, Geom g,
+         const R* __restrict__ rtab, const R* __restrict__ sv, const R* __restrict__ yend, Geom g,
          int k0, int Kc, int first_chunk, int last_chunk, RunState* st, R* __restrict__ M,
          R* __restrict__ part, const int* __restrict__ mir, Epochs ep)
 {
+    // Fixed mode: the last pass writes the updated signal to Xout (the tiles'
+    // knots outside them are read from X).  Stop mode: it writes the mean to M.
     // g.mirror: intervals count the mirrored knots too (mirror_before).
     // ep.n > 0 (batched): a tile (T | 512) lies in one record; pieces, the
     // qualified directions and Q are the record's own.
@@ -1175,16 +1148,19 @@ k_eval_w(XT* __restrict__ X, R* __restrict__ acc_buf, const uint32_t* __restrict
     const int c = cg * G + cc;
     const bool cok = c < g.C;
     const int rec = ep.n > 0 ? ep.wep[n0 >> 5] : 0;
-    const int rend = ep.n > 0 ? ep.off[rec] + ep.len[rec] : g.L;
+    const int roff = ep.n > 0 ? ep.off[rec] : 0;
+    const int rend = ep.n > 0 ? roff + ep.len[rec] : g.L;
     if (n0 >= rend) return;  // gap between epochs; uniform over the CTA
     const int nl = min(T, rend - n0);
     const int C = g.C;
+    const int cl = min(c, C - 1);  // loads of lanes past the last channel stay in bounds
     const int w0 = n0 >> 5;
     unsigned char* wb = smem_raw + (size_t)warp * PW;
-    R* accs = reinterpret_cast<R*>(wb);                        // [T][G]
-    R* us = accs + (STOPM ? T * G : 0);                        // [T][G] (stop mode)
-    int* kx = reinterpret_cast<int*>(accs + (STOPM ? 2 : 1) * T * G);
-    uint32_t* wd = reinterpret_cast<uint32_t*>(kx + MI + 1);
+    R* accs = reinterpret_cast<R*>(wb);                        // [T][G], the warp's sums of a slice
+    R* us = accs + (STOPM ? T * G : 0);                        // [T][G] (stop mode): the spread U - L
+    int* kx = reinterpret_cast<int*>(accs + (STOPM ? 2 : 1) * T * G);  // knots
+    int* ks = kx + MI + 1;                                     // the rows of their values
+    uint32_t* wd = reinterpret_cast<uint32_t*>(ks + MI + 1);   // bit words
     if (warp == 0) {
         int q = 0;
         for (int k = lane; k < g.K; k += 32) q += dir_qualifies(g, ep, cnt, k, rec) ? 1 : 0;
@@ -1192,9 +1168,10 @@ k_eval_w(XT* __restrict__ X, R* __restrict__ acc_buf, const uint32_t* __restrict
         if (lane == 0) sQ = q;
     }
     const int s_first = sgrp * SPL;
+    const int nv = nl - s_first;  // samples of this lane: j < nv
     const R third = R(1.0 / 3.0);
-    const R* yc = yv + c;
-    const R* sc = sv + c;
+    const XT* Xc = X + cl;
+    const R* sc = sv + cl;
     bool overflow = false;
 
     // CTAs per tile (FP32: one, its sum over the directions keeps its order).
@@ -1245,86 +1222,114 @@ k_eval_w(XT* __restrict__ X, R* __restrict__ acc_buf, const uint32_t* __restrict
                 m = MI - 1;
             }
             const int* kn = knots + slot * g.cap;
-            const size_t base = (slot * (size_t)g.cap + ia) * C;  // knot ia, channel 0
+            const R* sb = sc + (slot * (size_t)g.cap + ia) * C;  // knot ia
+            const R* ye = yend + (slot * (ep.n > 0 ? ep.n : 1) + rec) * 2 * (size_t)C + cl;
             __syncwarp();
-            for (int j = lane; j <= m; j += 32) kx[j] = kn[ia + j];
+            // a knot's value: the signal's row there (a mirrored knot: at its source
+            // sample), or one of the record's clamped end values (-1, -2)
+            for (int j = lane; j <= m; j += 32) {
+                const int x = kn[ia + j];
+                kx[j] = x;
+                ks[j] = g.mirror ? mirror_source(mir + (size_t)k * kMirWords, env, ia + j, Ee, x)
+                                 : (x == roff ? -1 : (x == rend - 1 ? -2 : x));
+            }
             if (lane < NW) wd[lane] = myw;
             __syncwarp();
-            int cntb = 0;
+            auto yk = [&](int j) -> R {
+                const int q = ks[j];
+                if (q < 0) return ye[q == -1 ? 0 : C];
+                return xval<R>(Xc[(size_t)q * C]);
+            };
+            int before = 0;  // the tile's knots before the lane's first sample
 #pragma unroll
             for (int q = 0; q < NW; ++q) {
                 const uint32_t w = wd[q];
-                if (32 * q + 32 <= s_first) cntb += __popc(w);
-                else if (32 * q < s_first) cntb += __popc(w & ((1u << (s_first - 32 * q)) - 1u));
+                if (32 * q + 32 <= s_first) before += __popc(w);
+                else if (32 * q < s_first) before += __popc(w & ((1u << (s_first - 32 * q)) - 1u));
             }
-            int cur = -2, x0 = 0;  // -2: no interval loaded yet (li >= 0 never equals cur + 1)
-            R ca = R(0.0f), cb = R(0.0f), c2 = R(0.0f), cd = R(0.0f);
-            R ynx = R(0.0f), snx = R(0.0f);  // values at knot cur + 1
+            // bit j: a knot at the lane's sample j, after which the interval is the next
+            uint32_t kw = wd[s_first >> 5] >> (s_first & 31);
+            int iv = cl0 + before - 1;
+            bool lag = iv < kb;  // before the first knot the first interval already applies
+            if (g.mirror) {
+                const int f = n0 + s_first;
+                iv = mirror_before(f, lp0, lp1, rp0, rp1) + cl0 + before - 1;
+                lag = iv < 0;
+                const unsigned d0 = (unsigned)(lp0 - f), d1 = (unsigned)(lp1 - f), d2 = (unsigned)(rp0 - f),
+                               d3 = (unsigned)(rp1 - f);
+                kw |= (d0 < 32u ? 1u << d0 : 0u) | (d1 < 32u ? 1u << d1 : 0u) | (d2 < 32u ? 1u << d2 : 0u) |
+                      (d3 < 32u ? 1u << d3 : 0u);
+            }
+            int li = min(max(iv + (lag ? 1 : 0) - ia, 0), m - 1);
+            R ca, cb, c2, cd, y0 = R(0.0f), s0 = R(0.0f), ynx = R(0.0f), snx = R(0.0f);
+            int x0 = 0;
+            auto coefficients = [&]() {  // of interval li, from its two knots
+                x0 = kx[li];
+                const int h = kx[li + 1] - x0;
+                const R ih = rtab[h];
+                const R slope = mul_(sub_(ynx, y0), ih);
+                ca = y0;
+                cb = fmad_(-mul_(from_int<R>(h), third), fmad_(R(2), s0, snx), slope);
+                c2 = s0;
+                cd = mul_(sub_(snx, s0), mul_(ih, third));
+            };
+            if (nv > 0) {
+                y0 = yk(li);
+                s0 = sb[(size_t)li * C];
+                ynx = yk(li + 1);
+                snx = sb[(size_t)(li + 1) * C];
+            }
+            coefficients();
+            [[maybe_unused]] float tf = (float)(n0 + s_first - x0);
+            const int je = min(SPL, nv);
 #pragma unroll 2
-            for (int j = 0; j < SPL; ++j) {
-                const int t = s_first + j;
-                if (t < nl && cok) {
-                    int iv = max(cl0 + cntb - 1, kb);
-                    if (g.mirror)
-                        iv = min(max(mirror_before(n0 + t, lp0, lp1, rp0, rp1) + cl0 + cntb - 1, 0), Ee - 2);
-                    const int li = min(iv - ia, m - 1);
-                    if (li != cur) {
-                        R y0, s0;
-                        if (li == cur + 1) {
-                            y0 = ynx;
-                            s0 = snx;
-                        } else {
-                            y0 = yc[base + (size_t)li * C];
-                            s0 = sc[base + (size_t)li * C];
-                        }
-                        ynx = yc[base + (size_t)(li + 1) * C];
-                        snx = sc[base + (size_t)(li + 1) * C];
-                        cur = li;
-                        x0 = kx[li];
-                        const int h = kx[li + 1] - x0;
-                        const R ih = rtab[h];
-                        const R slope = mul_(sub_(ynx, y0), ih);
-                        ca = y0;
-                        cb = fmad_(-mul_(from_int<R>(h), third), fmad_(R(2), s0, snx), slope);
-                        c2 = s0;
-                        cd = mul_(sub_(snx, s0), mul_(ih, third));
-                    }
-                    R v;
-                    if constexpr (std::is_same<R, double>::value) {
-                        const double tt = from_int<double>(n0 + t - x0);
-                        v = fmad_(fmad_(fmad_(cd, tt, c2), tt, cb), tt, ca);
+            for (int j = 0; j < je; ++j) {
+                R v;
+                if constexpr (std::is_same<R, double>::value) {
+                    const double tt = from_int<double>(n0 + s_first + j - x0);
+                    v = fmad_(fmad_(fmad_(cd, tt, c2), tt, cb), tt, ca);
+                } else {
+                    v = fmat_(fmat_(fmat_(cd, tf, c2), tf, cb), tf, ca);
+                    tf += 1.0f;  // exact
+                }
+                const int idx = (s_first + j) * G + cc;
+                if constexpr (STOPM) {
+                    if (env == 0) {
+                        us[idx] = v;
                     } else {
-                        const float tt = (float)(n0 + t - x0);
-                        v = fmat_(fmat_(fmat_(cd, tt, c2), tt, cb), tt, ca);
+                        const R uu = us[idx];
+                        accs[idx] = add_(accs[idx], add_(uu, v));
+                        us[idx] = sub_(uu, v);
                     }
-                    const int idx = t * G + cc;
-                    if constexpr (STOPM) {
-                        if (env == 0) {
-                            us[idx] = v;
-                        } else {
-                            const R uu = us[idx];
-                            accs[idx] = add_(accs[idx], add_(uu, v));
-                            us[idx] = sub_(uu, v);
-                        }
-                    } else {
-                        accs[idx] = add_(accs[idx], v);
+                } else {
+                    accs[idx] = add_(accs[idx], v);
+                }
+                if (kw & 1u) {  // a knot here: the next sample is in the next interval
+                    if (lag) lag = false;
+                    else if (li < m - 1) {
+                        ++li;
+                        y0 = ynx;
+                        s0 = snx;
+                        ynx = yk(li + 1);
+                        snx = sb[(size_t)(li + 1) * C];
+                        coefficients();
+                        if constexpr (!std::is_same<R, double>::value) tf = (float)(n0 + s_first + j + 1 - x0);
                     }
                 }
-                cntb += (int)((wd[t >> 5] >> (t & 31)) & 1u);
+                kw >>= 1;
             }
             if constexpr (STOPM) {
                 if (env == 1) {
                     __syncwarp();
                     for (int j = 0; j < SPL; ++j) {
-                        const int t = s_first + j;
                         R d2 = R(0.0f);
-                        if (cok && t < nl) {
-                            const R uu = us[t * G + cc];
+                        if (cok && j < nv) {
+                            const R uu = us[(s_first + j) * G + cc];
                             d2 = mul_(uu, uu);
                         }
 #pragma unroll
                         for (int o = 1; o < G; o <<= 1) d2 = add_(d2, shfl_xor_(d2, o));
-                        if (cc == 0 && t < nl) part[((size_t)cg * Kc + kk) * g.L + n0 + t] = d2;
+                        if (cc == 0 && j < nv) part[((size_t)cg * Kc + kk) * g.L + n0 + s_first + j] = d2;
                     }
                 }
             }
@@ -1370,7 +1375,7 @@ k_eval_w(XT* __restrict__ X, R* __restrict__ acc_buf, const uint32_t* __restrict
         if (last_chunk) {
             const R mval = div_(mul_(tots[q], R(0.5f)), R(Q));
             if (M) M[off] = mval;
-            else X[off] = xsub(X[off], mval);
+            else Xout[off] = xsub(X[off], mval);
         } else {
             acc_buf[off] = tots[q];
         }
