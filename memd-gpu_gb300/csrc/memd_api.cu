@@ -271,10 +271,11 @@ static bool eval_dispatch(int G, int SPL, int W, F f)
     }
     if constexpr (P == MEMD_PREC_F32) {
         MEMD_CASE(4, 32, 8) MEMD_CASE(8, 32, 8) MEMD_CASE(16, 32, 8) MEMD_CASE(32, 32, 8)
-        MEMD_CASE(4, 4, 8) MEMD_CASE(8, 8, 8) MEMD_CASE(16, 16, 8)
+        MEMD_CASE(4, 16, 8) MEMD_CASE(4, 8, 8) MEMD_CASE(4, 4, 8) MEMD_CASE(8, 16, 8) MEMD_CASE(8, 8, 8)
+        MEMD_CASE(16, 16, 8)
     } else {
         MEMD_CASE(4, 16, 8) MEMD_CASE(8, 16, 8) MEMD_CASE(16, 16, 8)
-        MEMD_CASE(4, 4, 8) MEMD_CASE(8, 8, 8)
+        MEMD_CASE(4, 8, 8) MEMD_CASE(4, 4, 8) MEMD_CASE(8, 8, 8)
     }
 #undef MEMD_CASE
     return false;
@@ -1333,26 +1334,25 @@ static memd_status create_plan(const memd_config* cfg, const memd_tuning* tun, m
                                                    "threads (fewer directions per chunk or longer segments)");
         }
     }
-    // evaluation tile: G channel lanes x SPL samples per lane, in 8 warps; while
-    // tiles of that size leave the GPU idle, 32-sample tiles (SPL = G) and, but
-    // for FP32 (whose sum over the directions keeps its order), a tile's
-    // directions dealt to several CTAs
+    // evaluation tile: G channel lanes x SPL samples per lane, in 8 warps, as
+    // long as still gives three CTAs per SM (a tile costs its directions'
+    // descriptions whatever its length: 2 x 147,478 x 45, FP32, 576 tiles of 256
+    // samples 144 us a sift, 4609 of 32 samples 186), 32 samples at least; and,
+    // but for FP32 (whose sum over the directions keeps its order), a tile's
+    // directions dealt to as many CTAs (4, 2 or 1) as stay resident at once and
+    // have a direction for each of their warps
     {
         const bool f32 = c.precision == MEMD_PREC_F32;
-        const int gmax = f32 ? 32 : 16, spl = f32 ? 32 : 16;
-        p->ewG = std::min(gmax, std::max(4, next_pow2(C)));
+        p->ewG = std::min(f32 ? 32 : 16, std::max(4, next_pow2(C)));
         const long groups = (C + p->ewG - 1) / p->ewG;
-        p->ewSPL = spl;
+        auto tiles = [&](int spl) { return (L + 32 / p->ewG * spl - 1) / (32 / p->ewG * spl) * groups; };
+        p->ewSPL = f32 ? 32 : 16;
         p->ewW = 8;
+        while (p->ewSPL > p->ewG && tiles(p->ewSPL) < 456) p->ewSPL /= 2;
         p->ewZ = 1;
-        if ((L + 32 / p->ewG * spl - 1) / (32 / p->ewG * spl) * groups < 600) {  // about four CTAs of 8 warps per SM
-            p->ewSPL = p->ewG;
-            // as many CTAs a tile (4, 2 or 1) as stay resident at once, three
-            // per SM: past that, the extra partial sums only cost
-            if (!f32) {
-                const long tiles = (L + 31) / 32 * groups;
-                p->ewZ = tiles <= 114 ? 4 : (tiles <= 228 ? 2 : 1);
-            }
+        if (!f32 && p->ewSPL == p->ewG) {
+            const long t = tiles(p->ewSPL);
+            p->ewZ = t <= 114 && p->Kc >= 32 ? 4 : (t <= 228 && p->Kc >= 16 ? 2 : 1);
         }
     }
     p->egroups = (C + p->ewG - 1) / p->ewG;

@@ -1091,7 +1091,8 @@ __device__ __forceinline__ void mirror_positions(const int* __restrict__ mi, con
 // E_min > 3): each warp's directions in order, then the warps' partial sums in
 // warp order; the last chunk applies X -= (sum/2)/Q (REF:832-864).
 // X is float (FP32 path), float2 (double-float, mixed path) or double.
-// The tile is 32 samples (SPL = G) until the launch fills the GPU, and the
+// The tile is as long as still gives three CTAs per SM (32 samples at least),
+// and the
 // FP64 and double-float forms deal a tile's directions to a cluster of two or
 // four CTAs then: a small record is bound by one warp's walk over its
 // directions, and in FP64 by the FP64 pipe of the few SMs that have a tile.
@@ -1175,13 +1176,14 @@ k_eval_w(const XT* __restrict__ X, XT* __restrict__ Xout, R* __restrict__ acc_bu
     bool overflow = false;
 
     // CTAs per tile (FP32: one, its sum over the directions keeps its order).
-    // FP64: the directions in NZ slices whatever the CTAs per tile, so that the
+    // FP64: the directions in NZ slices (Z divides 4, and is 1 where Kc has fewer
+    // than eight a slice for it) whatever the CTAs per tile, so that the
     // sum's order, and with it a record's result, does not depend on the launch
     // (a record alone or in a batch)
     constexpr bool ONE = std::is_same<R, float>::value;
     namespace cg_ = cooperative_groups;
     const int Z = ONE ? 1 : (int)gridDim.z, zr = ONE ? 0 : (int)blockIdx.z;
-    const int NZ = std::is_same<R, double>::value ? 4 : Z;
+    const int NZ = std::is_same<R, double>::value ? min(4, (Kc + WARPS - 1) / WARPS) : Z;
     constexpr int EPT = (T * G + 32 * WARPS - 1) / (32 * WARPS);  // tile elements per thread
     R tots[EPT];
 #pragma unroll
