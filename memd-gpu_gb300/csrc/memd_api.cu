@@ -550,8 +550,7 @@ static void enqueue_sift(memd_plan* p, cudaStream_t s, memd_trace_entry* trace, 
         if (nak_ends) {
             const long nt = 2L * kc * p->ep.n * g.C;
             lc.begin(MEMD_STAGE_SOLVE);
-            k_nak_ends<R><<<(unsigned)((nt + 127) / 128), 128, 0, s>>>(p->knots, p->cnt, p->wpref,
-                                                                        (const Fac<R>*)p->fac, (R*)p->sv, g, k0, kc,
+            k_nak_ends<R><<<(unsigned)((nt + 127) / 128), 128, 0, s>>>(p->knots, p->cnt, p->wpref, (R*)p->sv, g, k0, kc,
                                                                         p->ep, bcur);
             lc.end(MEMD_STAGE_SOLVE);
         }

@@ -59,6 +59,22 @@ __device__ __forceinline__ dd operator/(dd a, dd b)
     const float q2 = __fdiv_rn(r.hi, b.hi);
     return dd_renorm(q1, q2);
 }
+// a b - c d - e f: the products' leading words subtracted error-free, one
+// renormalisation
+__device__ __forceinline__ dd dd_three_products(dd a, dd b, dd c, dd d, dd e, dd f)
+{
+    const float p = __fmul_rn(a.hi, b.hi), q = __fmul_rn(c.hi, d.hi), r = __fmul_rn(e.hi, f.hi);
+    const float pe = __fmaf_rn(a.lo, b.hi, __fmaf_rn(a.hi, b.lo, __fmaf_rn(a.hi, b.hi, -p)));
+    const float qe = __fmaf_rn(c.lo, d.hi, __fmaf_rn(c.hi, d.lo, __fmaf_rn(c.hi, d.hi, -q)));
+    const float re = __fmaf_rn(e.lo, f.hi, __fmaf_rn(e.hi, f.lo, __fmaf_rn(e.hi, f.hi, -r)));
+    const float s = __fsub_rn(p, q);
+    const float sb = __fsub_rn(p, s);  // the part of q taken off, as rounded
+    const float se = __fadd_rn(__fsub_rn(p, __fadd_rn(s, sb)), __fsub_rn(sb, q));
+    const float t = __fsub_rn(s, r);
+    const float tb = __fsub_rn(s, t);
+    const float te = __fadd_rn(__fsub_rn(s, __fadd_rn(t, tb)), __fsub_rn(tb, r));
+    return dd_renorm(t, __fadd_rn(__fadd_rn(se, te), __fsub_rn(__fsub_rn(pe, qe), re)));
+}
 __device__ __forceinline__ bool operator>(dd a, dd b) { return a.hi > b.hi || (a.hi == b.hi && a.lo > b.lo); }
 __device__ __forceinline__ bool operator<(dd a, dd b) { return b > a; }
 __device__ __forceinline__ dd dd_sqrt(dd a)
@@ -137,13 +153,12 @@ template <> __device__ __forceinline__ float2 xfrom<float2>(float2 v) { return v
 // Channel-independent factorisation of the natural-spline system of one
 // (direction, envelope), per knot row i (Thomas elimination without pivoting):
 //   g_i = d_i - l_i * cp_{i-1};  m = 1/g_i;  lm = l_i/g_i;  cp = u_i/g_i;
-//   ih = 1 / (x_{i+1} - x_i)  (0 for the last row); for the double-float
-//   form 3 / (x_{i+1} - x_i), the factor 3 of the right-hand side
-//   3 (slope_i - slope_{i-1}) folded in.
-// FP64: the right-hand side's factors folded into the row instead,
+//   ih = 1 / (x_{i+1} - x_i)  (0 for the last row).
+// FP64 and double-float: the right-hand side's factors folded into the row
+// instead,
 //   m 3 (slope_i - slope_{i-1}) = a (y_{i+1} - y_i) - b (y_i - y_{i-1}),
-// so that a row of the forward sweep is four FP64 operations (a = b = 0 in
-// the identity rows of record ends).
+// so that a row of the forward sweep is a difference and three products (a =
+// b = 0 in the identity rows of record ends).
 template <typename real>
 struct alignas(4 * sizeof(real)) Fac {
     real m, lm, cp, ih;
@@ -152,13 +167,12 @@ template <>
 struct alignas(32) Fac<double> {
     double a, b, lm, cp;
 };
-template <typename real>
-constexpr bool kFacIh3 = false;
 template <>
-constexpr bool kFacIh3<dd> = true;
-__device__ __forceinline__ double fac_ih(double r) { return r; }
-__device__ __forceinline__ float fac_ih(float r) { return r; }
-__device__ __forceinline__ dd fac_ih(dd r) { return dd_mulf(r, 3.0f); }
+struct alignas(32) Fac<dd> {
+    dd a, b, lm, cp;
+};
+template <typename real>
+constexpr bool kFacAB = !std::is_same<real, float>::value;
 
 // Geometry of one record (or the widest epoch of a batch).
 struct Geom {

@@ -414,8 +414,8 @@ k_factor(const int* __restrict__ knots, const int* __restrict__ cnt, const real*
     real cp = real(0);
     int xl = js > 0 ? x[js - 1] : 0;
     int xi = x[js];
-    [[maybe_unused]] real rl = real(0);  // FP64: 1 / (spacing to the left) of the next row
-    if constexpr (std::is_same<real, double>::value) rl = js > 0 ? rtab[xi - xl] : real(0);
+    [[maybe_unused]] real rl = real(0);  // 1 / (spacing to the left) of the next row
+    if constexpr (kFacAB<real>) rl = js > 0 ? rtab[xi - xl] : real(0);
     constexpr int FB = 8;  // knot positions loaded per batch (independent loads)
     // FULL (compile-time): all FB rows are owned (>= i0, < i1) and have a right
     // neighbour, so no row needs a guard
@@ -489,16 +489,16 @@ k_factor(const int* __restrict__ knots, const int* __restrict__ cnt, const real*
                 const real gp = fmad_(-l, cp, from_int<real>(di[k]));
                 const real m = recip_(gp);
                 cp = mul_(from_int<real>(ui[k]), m);
-                if constexpr (std::is_same<real, double>::value) {
+                if constexpr (kFacAB<real>) {
                     if (FULL || i >= i0) {
-                        Fac<double> o;
-                        double m3 = di[k] == 1 ? 0.0 : __dmul_rn(3.0, m);  // 1: an identity row
+                        Fac<real> o;
+                        real m3 = di[k] == 1 ? real(0) : mul_(real(3), m);  // 1: an identity row
                         if constexpr (NAK) {
-                            if (wd[k] > 0) m3 = __dmul_rn(m3, __ddiv_rn(from_int<double>(wn[k]), from_int<double>(wd[k])));
+                            if (wd[k] > 0) m3 = mul_(m3, div_(from_int<real>(wn[k]), from_int<real>(wd[k])));
                         }
-                        o.a = __dmul_rn(m3, rt[k]);
-                        o.b = __dmul_rn(m3, rl);
-                        o.lm = __dmul_rn(l, m);
+                        o.a = mul_(m3, rt[k]);
+                        o.b = mul_(m3, rl);
+                        o.lm = mul_(l, m);
                         o.cp = cp;
                         f[i] = o;
                     }
@@ -511,7 +511,7 @@ k_factor(const int* __restrict__ knots, const int* __restrict__ cnt, const real*
                     }
                     o.lm = mul_(l, m);
                     o.cp = cp;
-                    o.ih = (FULL || i < E - 1) ? fac_ih(rt[k]) : real(0);
+                    o.ih = (FULL || i < E - 1) ? rt[k] : real(0);
                     f[i] = o;
                 }
             }
@@ -783,12 +783,12 @@ k_solve_fwd(const int* __restrict__ cnt, const Fac<real>* __restrict__ fac,
     real* o = dbuf + slot * (size_t)g.cap * C + cl;
     const int is = (H < 0) ? 0 : max(0, i0 - H);
     real yi = yrow(is);
-    // FP64: the knot values' difference to the left instead of its slope
-    constexpr bool F64 = std::is_same<real, double>::value;
+    // a / b rows: the knot values' difference to the left instead of its slope
+    constexpr bool AB = kFacAB<real>, F64 = std::is_same<real, double>::value;
     real slope_prev = real(0);
     if (is > 0) {
         slope_prev = sub_(yi, yrow(is - 1));
-        if constexpr (!F64) slope_prev = mul_(slope_prev, f[is - 1].ih);
+        if constexpr (!AB) slope_prev = mul_(slope_prev, f[is - 1].ih);
     }
     real dprev = real(0);
     float ymax = 0.0f;
@@ -804,7 +804,7 @@ k_solve_fwd(const int* __restrict__ cnt, const Fac<real>* __restrict__ fac,
         int fx = 0, ffl = 0, fe = 0;
         if (lane < nb) {
             const Fac<real> fr = MEMD_CHECK(base + lane < g.cap) ? f[base + lane] : Fac<real>{};
-            if constexpr (F64) {
+            if constexpr (AB) {
                 fm = fr.a;
                 fih = fr.b;
             } else {
@@ -849,14 +849,20 @@ k_solve_fwd(const int* __restrict__ cnt, const Fac<real>* __restrict__ fac,
             if (FULL || k < nb) {
                 const int i = base + k;
                 const real ynext = yb[k];
-                if constexpr (F64) {
-                    // d_i = (a dy_i - b dy_{i-1}) - lm d_{i-1}: one operation on the
-                    // serial chain; identity rows (a = 0) are 0
+                if constexpr (AB) {
+                    // d_i = (a dy_i - b dy_{i-1}) - lm d_{i-1}: in FP64 one operation on
+                    // the serial chain; identity rows (a = 0) are 0
                     const real dy = (FULL || i < E - 1) ? sub_(ynext, yi) : real(0);
-                    const real rhs = is_zero(m) ? real(0) : fmad_(m, dy, -mul_(ih, slope_prev));
-                    const real dcur = fmad_(-lm, dprev, rhs);
+                    real dcur;
+                    if constexpr (F64) {
+                        const real rhs = is_zero(m) ? real(0) : fmad_(m, dy, -mul_(ih, slope_prev));
+                        dcur = fmad_(-lm, dprev, rhs);
+                    } else {
+                        dcur = is_zero(m) ? real(0) : dd_three_products(m, dy, ih, slope_prev, lm, dprev);
+                    }
                     if (FULL || i >= i0) {
                         if (cok && MEMD_CHECK(i >= 0 && i < g.cap)) o[(size_t)i * C] = dcur;
+                        if constexpr (!F64) ymax = fmaxf(ymax, magf(yi));
                     }
                     slope_prev = dy;
                     yi = ynext;
@@ -867,10 +873,7 @@ k_solve_fwd(const int* __restrict__ cnt, const Fac<real>* __restrict__ fac,
                 if (FULL || i < E - 1) slope = mul_(sub_(ynext, yi), ih);
                 // identity rows (record ends) have lm = 0 and m = 1; a not-a-knot
                 // row 1 also has lm = 0, so NAK tells them apart by m
-                if (NAK ? !is_one(m) : !is_zero(lm)) {
-                    if constexpr (kFacIh3<real>) r = sub_(slope, slope_prev);  // slopes carry the factor 3
-                    else r = mul_(real(3), sub_(slope, slope_prev));
-                }
+                if (NAK ? !is_one(m) : !is_zero(lm)) r = mul_(real(3), sub_(slope, slope_prev));
                 const real dcur = fmad_(-lm, dprev, mul_(m, r));
                 // rows before i0 only warm the recurrence up
                 if (FULL || i >= i0) {
@@ -926,7 +929,7 @@ k_solve_bwd(const int* __restrict__ cnt, const Fac<real>* __restrict__ fac, cons
     // warp that owns row E-3 (its window always reaches row E-1, and row E-2
     // does not depend on s_{E-1}), which also writes row E-1.
     constexpr int B = kSolveBatch;
-    constexpr bool F64 = std::is_same<real, double>::value;  // no bounds (bnd is null)
+    constexpr bool BND = std::is_same<real, dd>::value;  // only the mixed form's mean reads the bounds
     SolveItem it;
     bool first = true;
     while (solve_next(it, first, 1, q, cnt, g, k0, Kc, S, Ss, H, ngroups)) {
@@ -953,11 +956,17 @@ k_solve_bwd(const int* __restrict__ cnt, const Fac<real>* __restrict__ fac, cons
     auto batch = [&](auto full, int top) {
         constexpr bool FULL = decltype(full)::value;
         const int nb = FULL ? B : min(B, top - i0 + 1);
-        real fcp = real(0), fih = real(0);
+        real fcp = real(0);
+        [[maybe_unused]] float fh2 = 0.0f;  // h^2 / 4 of the row's right piece
         if (lane < nb) {
-            const Fac<real> fr = MEMD_CHECK(top - lane >= 0 && top - lane < g.cap) ? f[top - lane] : Fac<real>{};
-            fcp = fr.cp;
-            if constexpr (!F64) fih = fr.ih;
+            const int r = top - lane;
+            if (MEMD_CHECK(r >= 0 && r < g.cap)) fcp = f[r].cp;
+            if constexpr (BND) {
+                if (bnd && r < E - 1) {
+                    const float h = (float)(kn[r + 1] - kn[r]);
+                    fh2 = 0.25f * h * h;
+                }
+            }
         }
         real db[B];
 #pragma unroll
@@ -968,7 +977,7 @@ k_solve_bwd(const int* __restrict__ cnt, const Fac<real>* __restrict__ fac, cons
 #pragma unroll
         for (int k = 0; k < B; ++k) {
             const real cp = shfl_idx_(fcp, k);
-            [[maybe_unused]] const real ihr = F64 ? real(0) : shfl_idx_(fih, k);
+            [[maybe_unused]] const float h2 = BND ? __shfl_sync(kFull, fh2, k) : 0.0f;
             if (FULL || k < nb) {
                 const int i = top - k;
                 real sol = fmad_(-cp, snext, db[k]);
@@ -978,19 +987,14 @@ k_solve_bwd(const int* __restrict__ cnt, const Fac<real>* __restrict__ fac, cons
                 }
                 if (FULL || i < i1) {
                     if (cok && !(NAK && nak && i == E - 1) && MEMD_CHECK(i >= 0 && i < g.cap)) o[(size_t)i * C] = sol;
-                    if (!F64 && bnd && (FULL || i < E - 1)) {
-                        // h^2 = 1 / ih^2 (9 / ih^2 when ih holds 3/h); the approximate
-                        // division's error is inside the 1.01 margin applied at the end
-                        const float ih = magf(ihr);
-                        spart = fmaxf(spart, __fdividef((kFacIh3<real> ? 2.25f : 0.25f) * (magf(sol) + magf(snext)), ih * ih));
-                    }
+                    if constexpr (BND) spart = fmaxf(spart, h2 * (magf(sol) + magf(snext)));  // h2 = 0 in the last row
                     if constexpr (NAK) {
                         if (nak && i == E - 3) {
                             const int hb = kn[E - 1] - kn[E - 2];
                             const real sl =
                                 add_(snext, div_(mul_(sub_(snext, sol), real(hb)), real(kn[E - 2] - kn[E - 3])));
                             if (cok) o[(size_t)(E - 1) * C] = sl;
-                            if (!F64 && bnd) spart = fmaxf(spart, 0.25f * (magf(snext) + magf(sl)) * (float)hb * (float)hb);
+                            if (BND && bnd) spart = fmaxf(spart, 0.25f * (magf(snext) + magf(sl)) * (float)hb * (float)hb);
                         }
                     }
                 }
@@ -1003,7 +1007,7 @@ k_solve_bwd(const int* __restrict__ cnt, const Fac<real>* __restrict__ fac, cons
         if (!NAK && top - B + 1 >= i0 && top < i1 && top < E - 1) batch(std::true_type{}, top);
         else batch(std::false_type{}, top);
     }
-    if (!F64 && bnd && cok) atomicMax(&bnd[C + it.c], __float_as_uint(spart * 1.01f));
+    if (BND && bnd && cok) atomicMax(&bnd[C + it.c], __float_as_uint(spart * 1.01f));
     }  // items
 }
 
@@ -1022,7 +1026,7 @@ k_solve_bwd(const int* __restrict__ cnt, const Fac<real>* __restrict__ fac, cons
 template <typename real>
 __global__ void __launch_bounds__(128)
 k_nak_ends(const int* __restrict__ knots, const int* __restrict__ cnt, const int* __restrict__ wpref,
-           const Fac<real>* __restrict__ fac, real* __restrict__ sv, Geom g, int k0, int Kc, Epochs ep,
+           real* __restrict__ sv, Geom g, int k0, int Kc, Epochs ep,
            unsigned* __restrict__ bnd)
 {
     const long gid = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1039,7 +1043,6 @@ k_nak_ends(const int* __restrict__ knots, const int* __restrict__ cnt, const int
     if (en - b < 4) return;
     const int* kn = knots + (size_t)slot * g.cap;
     real* s = sv + (size_t)slot * g.cap * C + c;
-    [[maybe_unused]] const Fac<real>* f = fac + (size_t)slot * g.cap;
     const real s1 = s[(size_t)(b + 1) * C], s2 = s[(size_t)(b + 2) * C];
     const real s0 = add_(s1, div_(mul_(sub_(s1, s2), real(kn[b + 1] - kn[b])), real(kn[b + 2] - kn[b + 1])));
     const real sa = s[(size_t)(en - 3) * C], sb = s[(size_t)(en - 2) * C];
@@ -1047,11 +1050,10 @@ k_nak_ends(const int* __restrict__ knots, const int* __restrict__ cnt, const int
     const real sl = add_(sb, div_(mul_(sub_(sb, sa), real(hb)), real(kn[en - 2] - kn[en - 3])));
     s[(size_t)b * C] = s0;
     s[(size_t)(en - 1) * C] = sl;
-    if constexpr (!std::is_same<real, double>::value) {
+    if constexpr (std::is_same<real, dd>::value) {
         if (bnd) {
-            const float ih = magf(f[b].ih);
-            float v = __fdividef((kFacIh3<real> ? 2.25f : 0.25f) * (magf(s0) + magf(s1)), ih * ih);
-            v = fmaxf(v, 0.25f * (magf(sb) + magf(sl)) * (float)hb * (float)hb);
+            const float ha = (float)(kn[b + 1] - kn[b]);
+            const float v = fmaxf(0.25f * (magf(s0) + magf(s1)) * ha * ha, 0.25f * (magf(sb) + magf(sl)) * (float)hb * (float)hb);
             atomicMax(&bnd[C + c], __float_as_uint(v * 1.01f));
         }
     }
