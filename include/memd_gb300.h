@@ -187,7 +187,7 @@ typedef struct memd_plan memd_plan;
  * truncation is below the arithmetic's precision), the rest are grid
  * shapes and work distribution. */
 typedef struct {
-    int32_t solve_segment;      /* longest substitution segment in knots, a power of two in [32, 1024] (256) */
+    int32_t solve_segment;      /* longest substitution segment in knots, a power of two in [32, 1024] (512, FP32 256) */
     int32_t solve_min_segment;  /* shortest substitution segment, a power of two in [16, solve_segment] (64) */
     int32_t factor_segment;     /* factorisation rows per thread, 4 .. 256 (16) */
     int32_t solve_queue;        /* substitution work: 1 = device work queue pulled by a persistent grid,

@@ -60,7 +60,8 @@ struct memd_plan {
     int xbytes;      // working-signal storage
     int tbytes;      // caller's element type
     int Kc, nchunks;
-    int S, H, Sf, Hf, Ss;  // solve segments (long / short systems) and halo; factor segments and halo
+    memd::Segs sg;  // solve segments and halo
+    int Sf, Hf;     // factor segments and halo
     int GS, ngroups;
     int ewG, ewSPL, ewW, ewZ;   // evaluation tile: channel lanes, samples per lane, warps, CTAs per tile
     int cum, cumG;              // impulse-accumulation mean (FP64 and mixed forms, fixed mode), channels per lane group
@@ -498,7 +499,7 @@ static void enqueue_sift(memd_plan* p, cudaStream_t s, memd_trace_entry* trace, 
                                                                         (Fac<R>*)p->fac, g, k0, kc, p->Sf, p->Hf,
                                                                         p->cumcfg, p->ep, p->cum_ctas);
         lc.end(MEMD_STAGE_FACTOR);
-        const long nseg = solve_segments_max(g.cap, p->S, p->Ss, p->H);
+        const long nseg = solve_segments_max(g.cap, p->sg);
         const long ns = 2L * kc * nseg * p->ngroups * 32;
         const unsigned nb = (unsigned)((ns + kSolveThreads - 1) / kSolveThreads);
         unsigned* bcur = p->bnd ? p->bnd + (size_t)(p->bpass & 1) * 2 * g.C : nullptr;
@@ -506,7 +507,7 @@ static void enqueue_sift(memd_plan* p, cudaStream_t s, memd_trace_entry* trace, 
         if (p->squeue) {
             q = p->sq;
             lc.begin(MEMD_STAGE_SOLVE);
-            k_solve_queue<<<1, 1024, 0, s>>>(p->cnt, g, k0, kc, p->S, p->Ss, p->H, p->ngroups, q);
+            k_solve_queue<<<1, 1024, 0, s>>>(p->cnt, g, k0, kc, p->sg, p->ngroups, q);
             lc.end(MEMD_STAGE_SOLVE);
         }
         lc.begin(MEMD_STAGE_SOLVE);
@@ -514,7 +515,7 @@ static void enqueue_sift(memd_plan* p, cudaStream_t s, memd_trace_entry* trace, 
     k_solve_fwd<R, XT, EPB_, NAK_, MIR_><<<p->squeue ? persistent_grid(k_solve_fwd<R, XT, EPB_, NAK_, MIR_>,   \
                                                                        kSolveThreads, p->sms, nb) : nb,         \
                                            kSolveThreads, 0, s>>>(                                             \
-        p->cnt, (const Fac<R>*)p->fac, (R*)p->dbuf, g, k0, kc, p->S, p->Ss, p->H, p->ngroups, bcur,            \
+        p->cnt, (const Fac<R>*)p->fac, (R*)p->dbuf, g, k0, kc, p->sg, p->ngroups, bcur,                        \
         (const XT*)p->X, p->knots, (const R*)p->yend, p->ep, p->inplace ? (R*)p->hz : nullptr, p->hsegs, q,     \
         p->mir)
         if (p->ep.n > 0) {  // batched runs: record ends found by position
@@ -535,17 +536,17 @@ static void enqueue_sift(memd_plan* p, cudaStream_t s, memd_trace_entry* trace, 
             k_solve_bwd<R, true, false>
                 <<<p->squeue ? persistent_grid(k_solve_bwd<R, true, false>, kSolveThreads, p->sms, nb) : nb,
                    kSolveThreads, 0, s>>>(p->cnt, (const Fac<R>*)p->fac, (const R*)p->dbuf, (R*)p->sv, g, k0, kc,
-                                          p->S, p->Ss, p->H, p->ngroups, bcur, p->knots, nullptr, 0, q);
+                                          p->sg, p->ngroups, bcur, p->knots, nullptr, 0, q);
         else if (p->inplace)
             k_solve_bwd<R, false, true>
                 <<<p->squeue ? persistent_grid(k_solve_bwd<R, false, true>, kSolveThreads, p->sms, nb) : nb,
-                   kSolveThreads, 0, s>>>(p->cnt, (const Fac<R>*)p->fac, nullptr, (R*)p->sv, g, k0, kc, p->S,
-                                          p->Ss, p->H, p->ngroups, bcur, p->knots, (const R*)p->hz, p->hsegs, q);
+                   kSolveThreads, 0, s>>>(p->cnt, (const Fac<R>*)p->fac, nullptr, (R*)p->sv, g, k0, kc,
+                                          p->sg, p->ngroups, bcur, p->knots, (const R*)p->hz, p->hsegs, q);
         else
             k_solve_bwd<R, false, false>
                 <<<p->squeue ? persistent_grid(k_solve_bwd<R, false, false>, kSolveThreads, p->sms, nb) : nb,
                    kSolveThreads, 0, s>>>(p->cnt, (const Fac<R>*)p->fac, (const R*)p->dbuf, (R*)p->sv, g, k0, kc,
-                                          p->S, p->Ss, p->H, p->ngroups, bcur, p->knots, nullptr, 0, q);
+                                          p->sg, p->ngroups, bcur, p->knots, nullptr, 0, q);
         lc.end(MEMD_STAGE_SOLVE);
         if (nak_ends) {
             const long nt = 2L * kc * p->ep.n * g.C;
@@ -1165,8 +1166,8 @@ memd_status memd_plan_get_tuning(const memd_plan* p, memd_tuning* t)
     using namespace memd;
     if (!p || !t) return set_error(MEMD_ERR_INVALID, "get_tuning: null argument");
     memset(t, 0, sizeof(*t));
-    t->solve_segment = p->S;
-    t->solve_min_segment = p->Ss;
+    t->solve_segment = p->sg.S;
+    t->solve_min_segment = p->sg.Ss;
     t->factor_segment = p->Sf;
     t->solve_queue = p->squeue ? 1 : 2;
     t->mean_ctas = p->cum_ctas;
@@ -1266,9 +1267,9 @@ static memd_status create_plan(const memd_config* cfg, const memd_tuning* tun, m
     p->g.nak = c.spline_end == MEMD_SPLINE_NOT_A_KNOT;
     p->g.mirror = c.boundary == MEMD_BOUNDARY_MIRROR;
     if (c.solve_window < 0) {
-        p->S = p->g.cap;
-        p->Ss = p->g.cap;
-        p->H = -1;
+        p->sg.S = p->g.cap;
+        p->sg.Ss = p->g.cap;
+        p->sg.H = -1;
         p->Sf = p->g.cap;
         p->Hf = -1;
     } else {
@@ -1284,9 +1285,9 @@ static memd_status create_plan(const memd_config* cfg, const memd_tuning* tun, m
         // rows, divisions and integer conversions on the FP64 pipe -> 16 + 24
         // rows, without them: 98.7 -> 51.9 us at IMF 1, 70.1 -> 25.5 us at IMF 8)
         const bool wide = f64 || c.precision == MEMD_PREC_MIXED;
-        p->S = tu.solve_segment ? tu.solve_segment : 256;
-        p->Ss = tu.solve_min_segment ? tu.solve_min_segment : std::min(64, p->S);
-        p->H = c.solve_window > 0 ? (int)c.solve_window : (f64 ? 48 : (wide ? 32 : 24));
+        p->sg.S = tu.solve_segment ? tu.solve_segment : (wide ? 512 : 256);
+        p->sg.Ss = tu.solve_min_segment ? tu.solve_min_segment : std::min(64, p->sg.S);
+        p->sg.H = c.solve_window > 0 ? (int)c.solve_window : (f64 ? 48 : (wide ? 32 : 24));
         // short factorisation segments (the pivot recurrence is latency-bound)
         p->Sf = tu.factor_segment ? tu.factor_segment : 16;
         p->Hf = f64 ? 24 : (wide ? 16 : 20);
@@ -1298,7 +1299,7 @@ static memd_status create_plan(const memd_config* cfg, const memd_tuning* tun, m
     // Not for one record with not-a-knot ends, whose backward sweep writes the
     // last row from another segment's warp (batched runs set their ends after
     // the sweep).
-    const bool inplace_ok = (p->H < 0 || p->Ss >= p->H) && !(p->g.nak && !p->batched);
+    const bool inplace_ok = (p->sg.H < 0 || p->sg.Ss >= p->sg.H) && !(p->g.nak && !p->batched);
     p->Kc = (c.dir_chunk > 0) ? std::min<int>((int)c.dir_chunk, K) : K;
     bool want_inplace = tu.solve_layout == 1 && inplace_ok;
     if (c.dir_chunk <= 0 && tu.solve_layout == 0) {
@@ -1323,10 +1324,13 @@ static memd_status create_plan(const memd_config* cfg, const memd_tuning* tun, m
     p->nchunks = (K + p->Kc - 1) / p->Kc;
     p->GS = 32;  // solve: one warp per (envelope, direction, segment, 32 channels)
     p->ngroups = (C + 31) / 32;
+    // (FP32 keeps one rule for every launch: where a window starts may show in
+    // its last bits)
+    p->sg.slots = c.precision == MEMD_PREC_F32 ? 256 : std::max(256, 2 * p->Kc * p->ngroups);
     {
         // the factorisation and substitution kernels index their threads in 32 bits
         const double nfac = 2.0 * p->Kc * (double)((p->g.cap + p->Sf - 1) / p->Sf);
-        const double nsol = 2.0 * p->Kc * (double)solve_segments_max(p->g.cap, p->S, p->Ss, p->H) * p->ngroups * 32.0;
+        const double nsol = 2.0 * p->Kc * (double)solve_segments_max(p->g.cap, p->sg) * p->ngroups * 32.0;
         if (nfac >= 2147483648.0 || nsol >= 2147483648.0) {
             delete p;
             return set_error(MEMD_ERR_UNSUPPORTED, "plan: a factorisation or substitution launch would exceed 2^31 "
@@ -1402,10 +1406,10 @@ static memd_status create_plan(const memd_config* cfg, const memd_tuning* tun, m
     ALLOC(p->yend, rb * 2 * Kc * (size_t)std::max<int64_t>(1, c.max_epochs) * 2 * C);  // [2][Kc][epochs][2][C]
     ALLOC(p->sv, rb * 2 * Kc * p->g.cap * C);
     p->inplace = want_inplace;
-    p->hsegs = p->H > 0 ? (int)solve_segments_max(p->g.cap, p->S, p->Ss, p->H) : 0;
+    p->hsegs = p->sg.H > 0 ? (int)solve_segments_max(p->g.cap, p->sg) : 0;
     if (p->inplace) {
         p->dbuf = p->sv;
-        if (p->H > 0) ALLOC(p->hz, rb * 2 * Kc * (size_t)p->hsegs * p->H * C);
+        if (p->sg.H > 0) ALLOC(p->hz, rb * 2 * Kc * (size_t)p->hsegs * p->sg.H * C);
     } else {
         ALLOC(p->dbuf, rb * 2 * Kc * p->g.cap * C);
     }

@@ -544,9 +544,9 @@ k_factor(const int* __restrict__ knots, const int* __restrict__ cnt, const real*
 // power H; the rows a thread reads from the next segment are that segment's
 // own converged values, so the result does not depend on the segmentation.
 // H < 0 selects the exact single-window solve.  Segments hold the longest
-// power of two in [Ss, S] knots that leaves the system more than 16 segments
-// (more, shorter segments keep the GPU busy when the knot sets are short;
-// longer ones spend less on halos).  The segment index is the
+// power of two in [Ss, S] knots that still gives the launch enough warps (more,
+// shorter segments keep the GPU busy when the knot sets are short; longer ones
+// spend less on halos).  The segment index is the
 // slowest grid index, so whole CTAs past the active segments exit at once.
 // bnd != nullptr: raise bnd[c] (forward: max |y| over the segment's knots) and
 // bnd[C + c] (backward: max h^2 (|s_i| + |s_{i+1}|) / 4 over its pieces), float
@@ -560,29 +560,46 @@ struct SolveItem {
     bool ok;
 };
 
-// Segment length of a system of E knots: the longest power of two in [Ss, S]
-// that still gives it more than 16 segments (H < 0: one window over all).
-__device__ __forceinline__ int solve_seg_len(int E, int cap, int S, int Ss, int H)
+// Segment lengths of the substitution.
+struct Segs {
+    int S, Ss;  // longest, shortest (powers of two)
+    int H;      // halo (< 0: one window over all)
+    int slots;  // systems x channel groups of a launch, 256 at least
+};
+
+// The fewest knots a system must exceed for segments of t: enough that a launch
+// of such systems has 4096 warps, about what is resident at once (six CTAs of
+// four per SM), and at t = 512 four times that (with 4352, one wave and a
+// rest, 32 x 30,504 x 128 was slower than with 256).
+__host__ __device__ inline long seg_limit(int t, const Segs& sg)
 {
-    if (H < 0) return cap;
-    for (int t = S; t > Ss; t >>= 1)
-        if (E > 16 * t) return t;
-    return Ss;
+    return (t > 256 ? 4l : 1l) * 4096l * t / sg.slots;
+}
+
+// Segment length of a system of E knots: the longest power of two in [Ss, S]
+// whose limit it exceeds (H < 0: one window over all).
+__device__ __forceinline__ int solve_seg_len(int E, int cap, const Segs& sg)
+{
+    if (sg.H < 0) return cap;
+    for (int t = sg.S; t > sg.Ss; t >>= 1)
+        if (E > seg_limit(t, sg)) return t;
+    return sg.Ss;
 }
 
 // The most segments solve_seg_len gives a system of at most cap knots (the
-// static grid's segment rows): systems of E in (16 t, hi] knots take segments
-// of t, hi the smaller bound left by the longer segments, the rest take Ss.
-__host__ __device__ inline long solve_segments_max(int cap, int S, int Ss, int H)
+// static grid's segment rows): systems of more than t's limit, at most the
+// limit of the longer segments, take segments of t, the rest take Ss.
+__host__ __device__ inline long solve_segments_max(int cap, const Segs& sg)
 {
-    if (H < 0) return 1;
+    if (sg.H < 0) return 1;
     long m = 0;
-    int hi = cap;
-    for (int t = S; t > Ss; t >>= 1) {
-        if (hi > 16 * t) m = m > (hi + t - 1) / t ? m : (hi + t - 1) / t;
-        hi = hi < 16 * t ? hi : 16 * t;
+    long hi = cap;
+    for (int t = sg.S; t > sg.Ss; t >>= 1) {
+        const long lim = seg_limit(t, sg);
+        if (hi > lim) m = m > (hi + t - 1) / t ? m : (hi + t - 1) / t;
+        hi = hi < lim ? hi : lim;
     }
-    const long r = (hi + Ss - 1) / Ss;
+    const long r = (hi + sg.Ss - 1) / sg.Ss;
     return m > r ? m : r;
 }
 
@@ -598,7 +615,7 @@ struct SolveQueue {
 };
 
 __device__ __forceinline__ SolveItem solve_item_of(int env, int kk, int seg, int cgi, const int* cnt, const Geom& g,
-                                                   int k0, int S, int Ss, int H)
+                                                   int k0, Segs sg)
 {
     SolveItem it;
     it.seg = seg;
@@ -608,7 +625,7 @@ __device__ __forceinline__ SolveItem solve_item_of(int env, int kk, int seg, int
     it.ok = false;
     it.E = cnt[env * g.K + k0 + kk];
     if (it.E > g.cap || it.E < 2) return it;
-    const int Se = solve_seg_len(it.E, g.cap, S, Ss, H);
+    const int Se = solve_seg_len(it.E, g.cap, sg);
     it.i0 = seg * Se;
     if (it.i0 >= it.E) return it;
     it.i1 = min(it.E, it.i0 + Se);
@@ -618,7 +635,7 @@ __device__ __forceinline__ SolveItem solve_item_of(int env, int kk, int seg, int
 
 // static mapping: warp w of the launch = item w (segments up to the capacity;
 // those past a system's knots exit)
-__device__ __forceinline__ SolveItem solve_item(const int* cnt, const Geom& g, int k0, int Kc, int S, int Ss, int H,
+__device__ __forceinline__ SolveItem solve_item(const int* cnt, const Geom& g, int k0, int Kc, Segs sg,
                                                 int ngroups)
 {
     // 32-bit index arithmetic: the plan keeps the launch below 2^31 threads
@@ -629,13 +646,13 @@ __device__ __forceinline__ SolveItem solve_item(const int* cnt, const Geom& g, i
     const unsigned segu = item / nsl;
     const int slot = (int)(item - segu * nsl);
     const int seg = (int)segu;
-    return solve_item_of(slot / Kc, slot % Kc, seg, cgi, cnt, g, k0, S, Ss, H);
+    return solve_item_of(slot / Kc, slot % Kc, seg, cgi, cnt, g, k0, sg);
 }
 
 // queue mapping: item = segment index over all slots x channel group; the
 // slot by binary search in the prefix
 __device__ __forceinline__ SolveItem solve_item_queued(int item, const SolveQueue& q, const int* cnt, const Geom& g,
-                                                       int k0, int Kc, int S, int Ss, int H, int ngroups)
+                                                       int k0, int Kc, Segs sg, int ngroups)
 {
     const int cgi = item % ngroups;
     const int si = item / ngroups;
@@ -645,32 +662,32 @@ __device__ __forceinline__ SolveItem solve_item_queued(int item, const SolveQueu
         if (__ldg(&q.pref[mid]) <= si) lo = mid;
         else hi = mid;
     }
-    return solve_item_of(lo / Kc, lo % Kc, si - __ldg(&q.pref[lo]), cgi, cnt, g, k0, S, Ss, H);
+    return solve_item_of(lo / Kc, lo % Kc, si - __ldg(&q.pref[lo]), cgi, cnt, g, k0, sg);
 }
 
 // The next item of this warp: the static mapping (one item, q.pref == nullptr)
 // or the queue's next ticket; false when there is none.
 __device__ __forceinline__ bool solve_next(SolveItem& it, bool& first, int which, const SolveQueue& q, const int* cnt,
-                                           const Geom& g, int k0, int Kc, int S, int Ss, int H, int ngroups)
+                                           const Geom& g, int k0, int Kc, Segs sg, int ngroups)
 {
     if (!q.pref) {
         if (!first) return false;
         first = false;
-        it = solve_item(cnt, g, k0, Kc, S, Ss, H, ngroups);
+        it = solve_item(cnt, g, k0, Kc, sg, ngroups);
         return true;
     }
     int item = 0;
     if ((threadIdx.x & 31) == 0) item = atomicAdd(&q.ticket[which], 1);
     item = __shfl_sync(kFull, item, 0);
     if (item >= __ldcg(q.total)) return false;
-    it = solve_item_queued(item, q, cnt, g, k0, Kc, S, Ss, H, ngroups);
+    it = solve_item_queued(item, q, cnt, g, k0, Kc, sg, ngroups);
     return true;
 }
 
 // One CTA of 1024 threads: segments per slot, their exclusive prefix, the item
 // count, and both tickets reset for the pass.
 __global__ void __launch_bounds__(1024)
-k_solve_queue(const int* __restrict__ cnt, Geom g, int k0, int Kc, int S, int Ss, int H, int ngroups, SolveQueue q)
+k_solve_queue(const int* __restrict__ cnt, Geom g, int k0, int Kc, Segs sg, int ngroups, SolveQueue q)
 {
     __shared__ int wsum[32];
     __shared__ int carry;
@@ -683,7 +700,7 @@ k_solve_queue(const int* __restrict__ cnt, Geom g, int k0, int Kc, int S, int Ss
             const int env = slot / Kc, kk = slot - env * Kc;
             const int E = cnt[env * g.K + k0 + kk];
             if (E <= g.cap && E >= 2) {
-                const int Se = solve_seg_len(E, g.cap, S, Ss, H);
+                const int Se = solve_seg_len(E, g.cap, sg);
                 nseg = (E + Se - 1) / Se;
             }
         }
@@ -723,7 +740,7 @@ k_solve_queue(const int* __restrict__ cnt, Geom g, int k0, int Kc, int S, int Ss
 template <typename real, typename XT, bool EPB, bool NAK, bool MIR>
 __global__ void __launch_bounds__(kSolveThreads)
 k_solve_fwd(const int* __restrict__ cnt, const Fac<real>* __restrict__ fac,
-            real* __restrict__ dbuf, Geom g, int k0, int Kc, int S, int Ss, int H, int ngroups,
+            real* __restrict__ dbuf, Geom g, int k0, int Kc, Segs sg, int ngroups,
             unsigned* __restrict__ bnd, const XT* __restrict__ X, const int* __restrict__ knots,
             const real* __restrict__ yend, Epochs ep, real* __restrict__ hz, int hsegs, SolveQueue q,
             const int* __restrict__ mir)
@@ -739,9 +756,10 @@ k_solve_fwd(const int* __restrict__ cnt, const Fac<real>* __restrict__ fac,
     // Rows of a record's end knots are the identity rows of the
     // factorisation (lm == 0): their right-hand side is 0.
     constexpr int B = kSolveBatch;
+    const int H = sg.H;
     SolveItem it;
     bool first = true;
-    while (solve_next(it, first, 0, q, cnt, g, k0, Kc, S, Ss, H, ngroups)) {
+    while (solve_next(it, first, 0, q, cnt, g, k0, Kc, sg, ngroups)) {
     if (!it.ok) continue;  // uniform over the warp
     const int lane = threadIdx.x & 31;
     const int C = g.C, E = it.E, i0 = it.i0, i1 = it.i1;
@@ -914,7 +932,7 @@ k_solve_fwd(const int* __restrict__ cnt, const Fac<real>* __restrict__ fac,
 template <typename real, bool NAK, bool INPL>
 __global__ void __launch_bounds__(kSolveThreads)
 k_solve_bwd(const int* __restrict__ cnt, const Fac<real>* __restrict__ fac, const real* __restrict__ dbuf,
-            real* __restrict__ sv, Geom g, int k0, int Kc, int S, int Ss, int H, int ngroups,
+            real* __restrict__ sv, Geom g, int k0, int Kc, Segs sg, int ngroups,
             unsigned* __restrict__ bnd, const int* __restrict__ knots, const real* __restrict__ hz, int hsegs,
             SolveQueue q)
 {
@@ -930,9 +948,10 @@ k_solve_bwd(const int* __restrict__ cnt, const Fac<real>* __restrict__ fac, cons
     // does not depend on s_{E-1}), which also writes row E-1.
     constexpr int B = kSolveBatch;
     constexpr bool BND = std::is_same<real, dd>::value;  // only the mixed form's mean reads the bounds
+    const int H = sg.H;
     SolveItem it;
     bool first = true;
-    while (solve_next(it, first, 1, q, cnt, g, k0, Kc, S, Ss, H, ngroups)) {
+    while (solve_next(it, first, 1, q, cnt, g, k0, Kc, sg, ngroups)) {
     if (!it.ok) continue;  // uniform over the warp
     const int lane = threadIdx.x & 31;
     const int C = g.C, E = it.E, i0 = it.i0, i1 = it.i1;
