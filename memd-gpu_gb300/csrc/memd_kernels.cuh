@@ -1445,7 +1445,11 @@ k_eval_w(const XT* __restrict__ X, XT* __restrict__ Xout, R* __restrict__ acc_bu
 // sifts: 18.96 ms with mantissa shifts for the conversions, 64-bit shared
 // atomics and block-wide prefix sums that needed the knots of three samples
 // past the span; 15.42 ms with limbs, 32-bit atomics with a carry and the walk;
-// 14.89 ms with the anchor's products summed before they are rounded.
+// 14.89 ms with the anchor's products summed before they are rounded; 14.2 ms
+// with the pieces' rows and reciprocals fetched one per lane ahead of the
+// anchor and handed out by shuffles (they were two loads a knot, the second
+// waiting for the first).  Fetching the next pair's rows ahead, to L2, L1 or in
+// registers, gave nothing more.
 // ---------------------------------------------------------------------------
 // The double-float v times 2^sh as a 64-bit two's-complement integer (|v 2^sh|
 // < 2^62), rounded to nearest, in three limbs a 2^44 + b 2^22 + c that are kept
@@ -1468,7 +1472,7 @@ __device__ __forceinline__ Limbs to_limbs(dd v, float s44, float s22)
     const float ra = __fmaf_rn(v.hi, s44, -__fsub_rn(ma, kMagic));  // exact, |ra| <= 1/2
     const float mb = __fmaf_rn(ra, 4194304.0f, kMagic);
     const float rb = __fmaf_rn(ra, 4194304.0f, -__fsub_rn(mb, kMagic));
-    const float ml = __fmaf_rn(v.lo, s22, kMagic);  // |lo| <= ulp(hi) / 2: below 2^16
+    const float ml = __fmaf_rn(v.lo, s22, kMagic);  // |lo|: at most an ulp of hi, below 2^18
     const float rl = __fmaf_rn(v.lo, s22, -__fsub_rn(ml, kMagic));
     const float mc = __fmaf_rn(__fadd_rn(rb, rl), 4194304.0f, kMagic);
     return Limbs{__float_as_uint(ma), __float_as_uint(mb) + __float_as_uint(ml), __float_as_uint(mc)};
@@ -1512,15 +1516,17 @@ __device__ __forceinline__ void acc_mulf(Acc& s, dd a, float t)
     acc_add(s, p, __fmaf_rn(a.lo, t, __fmaf_rn(a.hi, t, -p)));
 }
 __device__ __forceinline__ dd acc_dd(Acc s) { return dd_renorm(s.h, s.l); }
-// a b - c d
-__device__ __forceinline__ dd dd_diff_of_products(dd a, dd b, dd c, dd d)
+// Products without renormalisation (their value is the same), for sums and
+// conversions: the low word may reach an ulp of the high word.
+__device__ __forceinline__ dd raw_mul(dd a, dd b)
 {
-    const float p = __fmul_rn(a.hi, b.hi), q = __fmul_rn(c.hi, d.hi);
-    const float e = __fmaf_rn(a.lo, b.hi, __fmaf_rn(a.hi, b.lo, __fmaf_rn(a.hi, b.hi, -p)));
-    const float f = __fmaf_rn(c.lo, d.hi, __fmaf_rn(c.hi, d.lo, __fmaf_rn(c.hi, d.hi, -q)));
-    Acc s{p, e};
-    acc_add(s, -q, -f);
-    return acc_dd(s);
+    const float p = __fmul_rn(a.hi, b.hi);
+    return dd(p, __fmaf_rn(a.hi, b.lo, __fmaf_rn(a.lo, b.hi, __fmaf_rn(a.hi, b.hi, -p))));
+}
+__device__ __forceinline__ dd raw_mulf(dd a, float t)
+{
+    const float p = __fmul_rn(a.hi, t);
+    return dd(p, __fmaf_rn(a.lo, t, __fmaf_rn(a.hi, t, -p)));
 }
 
 // the non-negative integer a (< 2^63) times 2^-sh as a float, truncated to
@@ -1612,6 +1618,7 @@ k_mean_cum(const float2* __restrict__ X, float2* __restrict__ Xout, dd* __restri
     __shared__ int sQ, sLast;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int cc = lane % G, sub = lane / G;
+    const unsigned submask = (G == 32 ? 0xffffffffu : (1u << (G & 31)) - 1u) << (sub * G);
     const int C = g.C;
     const int mw = min(max(cumcfg[0], 1), kCumMaxWords), P = min(max(cumcfg[1], 1), kCumMaxParts);
     // CTA b works on part b % P of span b / P (launched: W rounded up to a
@@ -1708,6 +1715,22 @@ k_mean_cum(const float2* __restrict__ X, float2* __restrict__ Xout, dd* __restri
             const size_t slot = (size_t)env * Kc + kk;
             const int* kn = knots + slot * g.cap;
             const size_t rb = slot * (size_t)g.cap * C + cl;
+            // The pieces j - 1 .. j + n - 1 around the interior knots, one per
+            // lane: first sample's row and 1 / (3 h), handed out by shuffles in (3)
+            const int j0 = eJ[le];
+            int xrow = 0;
+            dd xr3(0.0f, 0.0f);
+            auto load_pieces = [&](int q0) {
+                const int q = min(q0 + cc, n);
+                const int x = kn[j0 - 1 + q];
+                xrow = x - p0;
+                xr3 = rtab3[kn[j0 + q] - x];
+            };
+            auto piece_row = [&](int q) { return __shfl_sync(submask, xrow, q, G); };
+            auto piece_r3 = [&](int q) {
+                return dd(__shfl_sync(submask, xr3.hi, q, G), __shfl_sync(submask, xr3.lo, q, G));
+            };
+            if (n > 0) load_pieces(0);
             // (2) anchor: Taylor coefficients of the piece at n_a
             {
                 const int i = eI[le];
@@ -1726,64 +1749,50 @@ k_mean_cum(const float2* __restrict__ X, float2* __restrict__ Xout, dd* __restri
                     y1 = (xi + h == rend - 1) ? ye[C] : xval<dd>(X[(size_t)(xi + h) * C + cl]);
                 }
                 const dd s0 = sv[rb + (size_t)i * C], s1 = sv[rb + (size_t)(i + 1) * C];
-                const dd d = (s1 - s0) * rtab3[h];
-                const dd s02(2.0f * s0.hi, 2.0f * s0.lo);  // exact
-                const dd b = dd_diff_of_products(y1 - y0, rtab[h], s02 + s1, h3tab[h]);
                 const float u = (float)(na - xi), u3 = (float)(3 * (na - xi));
+                const dd s02(2.0f * s0.hi, 2.0f * s0.lo);  // exact
+                const dd d = (s1 - s0) * rtab3[h];
+                const dd b = raw_mul(y1 - y0, rtab[h]) + (-raw_mul(s02 + s1, h3tab[h]));
+                const dd c2 = s0 + raw_mulf(d, u3);  // half the second derivative at n_a
                 acc_mulf(aA, dd_mulf(dd_mulf(d, u) + s0, u) + b, u);
                 acc_add(aA, y0.hi, y0.lo);
-                acc_mulf(aB, dd_mulf(d, u3) + s02, u);
+                acc_mulf(aB, c2 + s0, u);
                 acc_add(aB, b.hi, b.lo);
-                acc_mulf(aC, d, u3);
-                acc_add(aC, s0.hi, s0.lo);
+                acc_add(aC, c2.hi, c2.lo);
                 acc_add(aD, d.hi, d.lo);
             }
             // (3) jumps q_j - q_{j-1} at row x_j - p0 (in 1 .. nl - 1), q_j the
             //     quantised d_j = (s_{j+1} - s_j) / (3 h_j); full batches of KB
             //     knots (loads first, no predication), then the remainder
-            const int j0 = eJ[le];
             if (n > 0) {
-                int xj = kn[j0];
-                dd sj = sv[rb + (size_t)j0 * C];
-                Limbs qprev = to_limbs((sj - sv[rb + (size_t)(j0 - 1) * C]) * rtab3[xj - kn[j0 - 1]], s44, s22);
-                int t0 = 0;
-                for (; t0 + KB <= n; t0 += KB) {
-                    int xn[KB];
-                    dd sn[KB], r3[KB];
-                    const int* knp = kn + j0 + t0 + 1;
-                    const dd* svp = sv + rb + (size_t)(j0 + t0 + 1) * C;
+                const dd* svp = sv + rb + (size_t)(j0 - 1) * C;  // piece q starts at row q
+                dd sj = svp[C];
+                Limbs qprev = to_limbs(raw_mul(sj - svp[0], piece_r3(0)), s44, s22);
+                for (int c0 = 0; c0 <= n; c0 += G) {
+                    if (c0 > 0) load_pieces(c0);
+                    const int qe = min(n, c0 + G - 1);
+                    int q = max(1, c0);
+                    for (; q + KB - 1 <= qe; q += KB) {
+                        dd sn[KB];
 #pragma unroll
-                    for (int k = 0; k < KB; ++k) {
-                        xn[k] = knp[k];
-                        sn[k] = svp[(size_t)k * C];
-                    }
-                    {
-                        int xa = xj;
+                        for (int k = 0; k < KB; ++k) sn[k] = svp[(size_t)(q + 1 + k) * C];
 #pragma unroll
                         for (int k = 0; k < KB; ++k) {
-                            r3[k] = rtab3[xn[k] - xa];
-                            xa = xn[k];
+                            const Limbs qcur = to_limbs(raw_mul(sn[k] - sj, piece_r3(q + k)), s44, s22);
+                            const int row = piece_row(q + k);
+                            if (MEMD_CHECK(row >= 0 && row < nl)) add_words(klo, khi, row * G + cc, limbs_diff(qcur, qprev));
+                            qprev = qcur;
+                            sj = sn[k];
                         }
                     }
-#pragma unroll
-                    for (int k = 0; k < KB; ++k) {
-                        const Limbs qcur = to_limbs((sn[k] - sj) * r3[k], s44, s22);
-                        if (MEMD_CHECK(xj - p0 >= 0 && xj - p0 < nl))
-                            add_words(klo, khi, (xj - p0) * G + cc, limbs_diff(qcur, qprev));
+                    for (; q <= qe; ++q) {
+                        const dd sn1 = svp[(size_t)(q + 1) * C];
+                        const Limbs qcur = to_limbs(raw_mul(sn1 - sj, piece_r3(q)), s44, s22);
+                        const int row = piece_row(q);
+                        if (MEMD_CHECK(row >= 0 && row < nl)) add_words(klo, khi, row * G + cc, limbs_diff(qcur, qprev));
                         qprev = qcur;
-                        xj = xn[k];
-                        sj = sn[k];
+                        sj = sn1;
                     }
-                }
-                for (; t0 < n; ++t0) {
-                    const int xn1 = kn[j0 + t0 + 1];
-                    const dd sn1 = sv[rb + (size_t)(j0 + t0 + 1) * C];
-                    const Limbs qcur = to_limbs((sn1 - sj) * rtab3[xn1 - xj], s44, s22);
-                    if (MEMD_CHECK(xj - p0 >= 0 && xj - p0 < nl))
-                        add_words(klo, khi, (xj - p0) * G + cc, limbs_diff(qcur, qprev));
-                    qprev = qcur;
-                    xj = xn1;
-                    sj = sn1;
                 }
             }
         }

@@ -92,3 +92,19 @@ def test_impulse_means_with_mirrored_ends_match_direct_evaluation(C, L, K, perio
     assert np.array_equal(np.isnan(outs[0]), np.isnan(outs[1]))
     # both round a mean good to ~1e-13 to float32: one ulp of the largest value apart at most
     assert np.nanmax(np.abs(outs[0] - outs[1]), initial=0.0) <= 2.0 ** -22 * np.abs(y).max()
+
+
+# spans of 128 samples (few knots on average) of which some hold more knots than a pair has lanes; 8, 16, 32 lanes
+@pytest.mark.parametrize("C,L,K", [(3, 16384, 9), (12, 16385, 17), (33, 16415, 6)])
+def test_mixed_mean_of_spans_with_more_knots_than_lanes(C, L, K):
+    y, d = signal(C, L, 400, 13), oracle.directions(C, K)
+    y[:, 6000:6500] += 0.3 * np.random.default_rng(5).normal(size=(C, 500))
+    outs = []
+    for mean_eval in (0, 1):
+        plan = mg.Plan(C, L, K, 2, 1, mg.PREC_MIXED, mean_eval=mean_eval)
+        o = torch.empty((2, C, L), dtype=torch.float32, device="cuda")
+        plan.run(torch.as_tensor(y, dtype=torch.float32).cuda(), torch.as_tensor(d, dtype=torch.float32).cuda(), o)
+        plan.close()
+        outs.append(o.cpu().numpy().astype(np.float64))
+    # both round a mean good to ~1e-13 to float32: one ulp of the largest value apart at most
+    assert np.abs(outs[0] - outs[1]).max() <= 2.0 ** -22 * np.abs(y).max()
