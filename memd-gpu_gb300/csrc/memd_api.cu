@@ -487,21 +487,22 @@ static void enqueue_sift(memd_plan* p, cudaStream_t s, memd_trace_entry* trace, 
             p->bits, p->wpref, p->knots, p->cnt, (const XT*)p->X, trace, g, k0, kc, p->st, trace_rows,
             (R*)p->yend, p->ep, p->mir, p->csh, nch);
         lc.end(MEMD_STAGE_COMPACT);
+        constexpr int T = solve_threads<R>();
         const long nsegf = (g.cap + p->Sf - 1) / p->Sf;
         const long nf = 2L * kc * nsegf;
         lc.begin(MEMD_STAGE_FACTOR);
         if (g.nak)
-            k_factor<R, true><<<(unsigned)((nf + 127) / 128), 128, 0, s>>>(p->knots, p->cnt, (const R*)p->rtab,
+            k_factor<R, true><<<(unsigned)((nf + T - 1) / T), T, 0, s>>>(p->knots, p->cnt, (const R*)p->rtab,
                                                                        (Fac<R>*)p->fac, g, k0, kc, p->Sf, p->Hf,
                                                                        p->cumcfg, p->ep, p->cum_ctas);
         else
-            k_factor<R, false><<<(unsigned)((nf + 127) / 128), 128, 0, s>>>(p->knots, p->cnt, (const R*)p->rtab,
+            k_factor<R, false><<<(unsigned)((nf + T - 1) / T), T, 0, s>>>(p->knots, p->cnt, (const R*)p->rtab,
                                                                         (Fac<R>*)p->fac, g, k0, kc, p->Sf, p->Hf,
                                                                         p->cumcfg, p->ep, p->cum_ctas);
         lc.end(MEMD_STAGE_FACTOR);
         const long nseg = solve_segments_max(g.cap, p->sg);
         const long ns = 2L * kc * nseg * p->ngroups * 32;
-        const unsigned nb = (unsigned)((ns + kSolveThreads - 1) / kSolveThreads);
+        const unsigned nb = (unsigned)((ns + T - 1) / T);
         unsigned* bcur = p->bnd ? p->bnd + (size_t)(p->bpass & 1) * 2 * g.C : nullptr;
         SolveQueue q{};  // null prefix: the static mapping
         if (p->squeue) {
@@ -513,8 +514,8 @@ static void enqueue_sift(memd_plan* p, cudaStream_t s, memd_trace_entry* trace, 
         lc.begin(MEMD_STAGE_SOLVE);
 #define MEMD_FWD(EPB_, NAK_, MIR_)                                                                              \
     k_solve_fwd<R, XT, EPB_, NAK_, MIR_><<<p->squeue ? persistent_grid(k_solve_fwd<R, XT, EPB_, NAK_, MIR_>,   \
-                                                                       kSolveThreads, p->sms, nb) : nb,         \
-                                           kSolveThreads, 0, s>>>(                                             \
+                                                                       T, p->sms, nb) : nb,         \
+                                           T, 0, s>>>(                                             \
         p->cnt, (const Fac<R>*)p->fac, (R*)p->dbuf, g, k0, kc, p->sg, p->ngroups, bcur,                        \
         (const XT*)p->X, p->knots, (const R*)p->yend, p->ep, p->inplace ? (R*)p->hz : nullptr, p->hsegs, q,     \
         p->mir)
@@ -534,18 +535,18 @@ static void enqueue_sift(memd_plan* p, cudaStream_t s, memd_trace_entry* trace, 
         const bool nak_ends = g.nak && p->ep.n > 0;
         if (g.nak && !nak_ends)  // one record: never in place (its sweep writes the last row from another warp)
             k_solve_bwd<R, true, false>
-                <<<p->squeue ? persistent_grid(k_solve_bwd<R, true, false>, kSolveThreads, p->sms, nb) : nb,
-                   kSolveThreads, 0, s>>>(p->cnt, (const Fac<R>*)p->fac, (const R*)p->dbuf, (R*)p->sv, g, k0, kc,
+                <<<p->squeue ? persistent_grid(k_solve_bwd<R, true, false>, T, p->sms, nb) : nb,
+                   T, 0, s>>>(p->cnt, (const Fac<R>*)p->fac, (const R*)p->dbuf, (R*)p->sv, g, k0, kc,
                                           p->sg, p->ngroups, bcur, p->knots, nullptr, 0, q);
         else if (p->inplace)
             k_solve_bwd<R, false, true>
-                <<<p->squeue ? persistent_grid(k_solve_bwd<R, false, true>, kSolveThreads, p->sms, nb) : nb,
-                   kSolveThreads, 0, s>>>(p->cnt, (const Fac<R>*)p->fac, nullptr, (R*)p->sv, g, k0, kc,
+                <<<p->squeue ? persistent_grid(k_solve_bwd<R, false, true>, T, p->sms, nb) : nb,
+                   T, 0, s>>>(p->cnt, (const Fac<R>*)p->fac, nullptr, (R*)p->sv, g, k0, kc,
                                           p->sg, p->ngroups, bcur, p->knots, (const R*)p->hz, p->hsegs, q);
         else
             k_solve_bwd<R, false, false>
-                <<<p->squeue ? persistent_grid(k_solve_bwd<R, false, false>, kSolveThreads, p->sms, nb) : nb,
-                   kSolveThreads, 0, s>>>(p->cnt, (const Fac<R>*)p->fac, (const R*)p->dbuf, (R*)p->sv, g, k0, kc,
+                <<<p->squeue ? persistent_grid(k_solve_bwd<R, false, false>, T, p->sms, nb) : nb,
+                   T, 0, s>>>(p->cnt, (const Fac<R>*)p->fac, (const R*)p->dbuf, (R*)p->sv, g, k0, kc,
                                           p->sg, p->ngroups, bcur, p->knots, nullptr, 0, q);
         lc.end(MEMD_STAGE_SOLVE);
         if (nak_ends) {

@@ -23,14 +23,16 @@ from collections import OrderedDict
 # kernel name prefix -> sift stage (the stage names of the plan's profile)
 STAGES = (
     ("k_split_tf32", "project"),
+    ("k_float_directions", "project"),
     ("k_project", "project"),
     ("k_compact", "compact"),
     ("k_mirror", "compact"),
     ("k_factor", "factor"),
     ("k_solve", "solve"),
-    ("k_mean_cum", "eval"),
+    ("k_nak_ends", "solve"),
+    ("k_mean", "eval"),
+    ("k_count_knots", "eval"),
     ("k_eval", "eval"),
-    ("k_amp", "stop"),
     ("k_stop", "stop"),
     ("k_decide", "stop"),
     ("k_apply", "stop"),
@@ -42,6 +44,8 @@ def short_name(full: str) -> str:
     s = full
     if s.startswith("void "):
         s = s[5:]
+    if s.startswith("memd::"):
+        s = s[6:]
     depth = 0
     for i, ch in enumerate(s):
         if ch == "<":
