@@ -61,7 +61,7 @@ struct memd_plan {
     int tbytes;      // caller's element type
     int Kc, nchunks;
     memd::Segs sg;  // solve segments and halo
-    int Sf, Hf;     // factor segments and halo
+    int Sf, Sl, Hf; // factor segments (shorter ones for at most 2 Sl knots) and halo
     int GS, ngroups;
     int ewG, ewSPL, ewW, ewZ;   // evaluation tile: channel lanes, samples per lane, warps, CTAs per tile
     int cum, cumG;              // impulse-accumulation mean (FP64 and mixed forms, fixed mode), channels per lane group
@@ -488,16 +488,16 @@ static void enqueue_sift(memd_plan* p, cudaStream_t s, memd_trace_entry* trace, 
             (R*)p->yend, p->ep, p->mir, p->csh, nch);
         lc.end(MEMD_STAGE_COMPACT);
         constexpr int T = solve_threads<R>();
-        const long nsegf = (g.cap + p->Sf - 1) / p->Sf;
+        const long nsegf = fac_segments_max(g.cap, p->Sf, p->Sl);
         const long nf = 2L * kc * nsegf;
         lc.begin(MEMD_STAGE_FACTOR);
         if (g.nak)
             k_factor<R, true><<<(unsigned)((nf + T - 1) / T), T, 0, s>>>(p->knots, p->cnt, (const R*)p->rtab,
-                                                                       (Fac<R>*)p->fac, g, k0, kc, p->Sf, p->Hf,
+                                                                       (Fac<R>*)p->fac, g, k0, kc, p->Sf, p->Sl, p->Hf,
                                                                        p->cumcfg, p->ep, p->cum_ctas);
         else
             k_factor<R, false><<<(unsigned)((nf + T - 1) / T), T, 0, s>>>(p->knots, p->cnt, (const R*)p->rtab,
-                                                                        (Fac<R>*)p->fac, g, k0, kc, p->Sf, p->Hf,
+                                                                        (Fac<R>*)p->fac, g, k0, kc, p->Sf, p->Sl, p->Hf,
                                                                         p->cumcfg, p->ep, p->cum_ctas);
         lc.end(MEMD_STAGE_FACTOR);
         const long nseg = solve_segments_max(g.cap, p->sg);
@@ -1284,7 +1284,8 @@ static memd_status create_plan(const memd_config* cfg, const memd_tuning* tun, m
         // latency-bound, ~600 ns a row in FP64, once the knots are sparse
         // (k_factor<double>, 32 x 30,504, 64 directions, segments of 64 + 40
         // rows, divisions and integer conversions on the FP64 pipe -> 16 + 24
-        // rows, without them: 98.7 -> 51.9 us at IMF 1, 70.1 -> 25.5 us at IMF 8)
+        // rows, without them: 98.7 -> 51.9 us at IMF 1, 70.1 -> 25.5 us at IMF
+        // 8); shorter ones where the knots are few (fac_seg_len)
         const bool wide = f64 || c.precision == MEMD_PREC_MIXED;
         p->sg.S = tu.solve_segment ? tu.solve_segment : (wide ? 512 : 256);
         p->sg.Ss = tu.solve_min_segment ? tu.solve_min_segment : std::min(64, p->sg.S);
@@ -1321,6 +1322,9 @@ static memd_status create_plan(const memd_config* cfg, const memd_tuning* tun, m
         p->Kc = std::max(1, std::min({K, fit, kc_limit}));
     }
     p->Kc = std::min(p->Kc, 1024);
+    // (in FP32 the segments' length shows in the last bits: it stays)
+    if (c.solve_window >= 0 && !tu.factor_segment && c.precision != MEMD_PREC_F32)
+        p->Sl = kFacShortRows / (2 * p->Kc);
     *kc_used = p->Kc;
     p->nchunks = (K + p->Kc - 1) / p->Kc;
     p->GS = 32;  // solve: one warp per (envelope, direction, segment, 32 channels)
@@ -1330,7 +1334,7 @@ static memd_status create_plan(const memd_config* cfg, const memd_tuning* tun, m
     p->sg.slots = c.precision == MEMD_PREC_F32 ? 256 : std::max(256, 2 * p->Kc * p->ngroups);
     {
         // the factorisation and substitution kernels index their threads in 32 bits
-        const double nfac = 2.0 * p->Kc * (double)((p->g.cap + p->Sf - 1) / p->Sf);
+        const double nfac = 2.0 * p->Kc * (double)fac_segments_max(p->g.cap, p->Sf, p->Sl);
         const double nsol = 2.0 * p->Kc * (double)solve_segments_max(p->g.cap, p->sg) * p->ngroups * 32.0;
         if (nfac >= 2147483648.0 || nsol >= 2147483648.0) {
             delete p;

@@ -344,16 +344,46 @@ k_compact(const uint32_t* __restrict__ bits, int* __restrict__ wpref, int* __res
 
 // ---------------------------------------------------------------------------
 // Channel-independent factorisation.  One thread per (envelope, direction,
-// segment of Sf rows); the pivot recurrence starts Hf rows early (exact when
+// segment of fac_seg_len rows); the pivot recurrence starts Hf rows early (exact when
 // the window reaches row 0, whose pivot is 1 with cp = 0; otherwise the
 // start error decays by a factor u l / (2 (l + u) - l cp)^2 <= 1/12 per row,
 // cp <= 1/2, l and u the row's neighbouring spacings; identity and
 // not-a-knot end rows restart it).  rtab[h] = 1/h.
 // ---------------------------------------------------------------------------
+// Rows per thread for a system of E knots: Sf, half of it for at most 2 Sl
+// knots, a quarter for at most Sl (Sl = 0: always Sf).  A thread's rows come
+// one after another and so do its warm-up rows, so few knots leave the GPU idle
+// on a few long chains: shorter segments repeat more warm-up and end sooner.
+// FP64, a warp alone on its SM: ~105 clocks an operation, 7 a warm-up row and
+// 11 an own row, 344 for 24 + 16 rows and 212 for 24 + 4; but at 16 clocks of
+// the SM's pipe each, 2 Kc E rows in segments of 4 cost 2.5 times the pipe time
+// of 16, and the two meet at 2 Kc E = 150,000 .. 300,000.  Measured with the
+// limit at 0 / 75,000 / 150,000 / 300,000 / 600,000: 4 x 1,000 3.64 / 3.26 / 3.26
+// / 3.26 / 3.27 ms; 19 x 7,501 not-a-knot 15.25 / 14.57 / 14.40 / 14.40 / 14.41;
+// 8 x 2,000 stop 7.82 / 7.41 / 7.37 / 7.37 / 7.38; 32 x 30,504 x 64 43.89 / 43.55
+// / 43.49 / 43.57 / 43.90; mixed 16 x 12,003 mirrored 8.29 / 8.14 / 8.07 / 8.04 /
+// 8.08 (double-float has fewer warm-up rows and no shared pipe, and gains less).
+constexpr int kFacShortRows = 150000;
+__host__ __device__ inline int fac_seg_len(int E, int Sf, int Sl)
+{
+    return E > 2 * Sl ? Sf : E > Sl ? Sf / 2 : Sf / 4;
+}
+// the most segments of a system of at most cap knots
+__host__ __device__ inline int fac_segments_max(int cap, int Sf, int Sl)
+{
+    int m = 0;
+    for (int q = 4, hi = cap; q >= 1; q >>= 1) {  // Sf, Sf / 2, Sf / 4 rows
+        const int t = Sf * q / 4, lim = q == 4 ? 2 * Sl : q == 2 ? Sl : 0;
+        if (hi > lim) m = m > (hi + t - 1) / t ? m : (hi + t - 1) / t;
+        hi = hi < lim ? hi : lim;
+    }
+    return m;
+}
+
 template <typename real, bool NAK>
 __global__ void __launch_bounds__(128)
 k_factor(const int* __restrict__ knots, const int* __restrict__ cnt, const real* __restrict__ rtab,
-         Fac<real>* __restrict__ fac, Geom g, int k0, int Kc, int Sf, int Hf, int* __restrict__ cumcfg,
+         Fac<real>* __restrict__ fac, Geom g, int k0, int Kc, int Sf, int Sl, int Hf, int* __restrict__ cumcfg,
          Epochs ep, int cum_ctas)
 {
     // cumcfg != nullptr (impulse-accumulation mean): block 0 picks the mean
@@ -397,16 +427,16 @@ k_factor(const int* __restrict__ knots, const int* __restrict__ cnt, const real*
     const unsigned gid = blockIdx.x * blockDim.x + threadIdx.x;
     const unsigned nsys = 2u * (unsigned)Kc;
     const unsigned segu = gid / nsys;
-    if (segu >= (unsigned)((g.cap + Sf - 1) / Sf)) return;
     const int seg = (int)segu;
     const int sys = (int)(gid - segu * nsys);
     const int env = sys >= Kc ? 1 : 0;
     const int kk = sys - env * Kc;
     const int E = cnt[env * g.K + k0 + kk];
     if (E > g.cap) return;
-    const int i0 = seg * Sf;
-    if (i0 >= E) return;
-    const int i1 = min(E, i0 + Sf);
+    const int Se = fac_seg_len(E, Sf, Sl);
+    if (segu >= (unsigned)((E + Se - 1) / Se)) return;
+    const int i0 = seg * Se;
+    const int i1 = min(E, i0 + Se);
     const size_t slot = (size_t)env * Kc + kk;
     const int* x = knots + slot * g.cap;
     Fac<real>* f = fac + slot * g.cap;

@@ -108,3 +108,14 @@ def test_mixed_mean_of_spans_with_more_knots_than_lanes(C, L, K):
         outs.append(o.cpu().numpy().astype(np.float64))
     # both round a mean good to ~1e-13 to float32: one ulp of the largest value apart at most
     assert np.abs(outs[0] - outs[1]).max() <= 2.0 ** -22 * np.abs(y).max()
+
+
+# factorisation segments of 4, 8 and 16 rows (the knots of 2 x 64 systems: about L / 3.6 each), odd remainders
+@pytest.mark.parametrize("spline", [mg.SPLINE_NATURAL, mg.SPLINE_NOT_A_KNOT])
+@pytest.mark.parametrize("C,L,K", [(2, 37, 3), (2, 2003, 64), (3, 6001, 64), (2, 12007, 64), (5, 1000, 9)])
+def test_factorisation_segments_leave_the_pivots_alone(C, L, K, spline):
+    y, d = signal(C, L, 3.6, 17), oracle.directions(C, K)
+    a, sa = one_sift(y, d, spline_end=spline)
+    b, sb = one_sift(y, d, spline_end=spline, tuning=dict(factor_segment=16))
+    # 24 warm-up rows bring the start error (at most 1/2, 12 times less a row) to 4e-27, which rounding removes
+    assert sa.flags == sb.flags and np.array_equal(a, b, equal_nan=True)
