@@ -487,21 +487,22 @@ static void enqueue_sift(memd_plan* p, cudaStream_t s, memd_trace_entry* trace, 
             p->bits, p->wpref, p->knots, p->cnt, (const XT*)p->X, trace, g, k0, kc, p->st, trace_rows,
             (R*)p->yend, p->ep, p->mir, p->csh, nch);
         lc.end(MEMD_STAGE_COMPACT);
-        constexpr int T = solve_threads<R>();
         const long nsegf = fac_segments_max(g.cap, p->Sf, p->Sl);
         const long nf = 2L * kc * nsegf;
+        const int TF = solve_threads<R>(nf / 32);
         lc.begin(MEMD_STAGE_FACTOR);
         if (g.nak)
-            k_factor<R, true><<<(unsigned)((nf + T - 1) / T), T, 0, s>>>(p->knots, p->cnt, (const R*)p->rtab,
+            k_factor<R, true><<<(unsigned)((nf + TF - 1) / TF), TF, 0, s>>>(p->knots, p->cnt, (const R*)p->rtab,
                                                                        (Fac<R>*)p->fac, g, k0, kc, p->Sf, p->Sl, p->Hf,
                                                                        p->cumcfg, p->ep, p->cum_ctas);
         else
-            k_factor<R, false><<<(unsigned)((nf + T - 1) / T), T, 0, s>>>(p->knots, p->cnt, (const R*)p->rtab,
+            k_factor<R, false><<<(unsigned)((nf + TF - 1) / TF), TF, 0, s>>>(p->knots, p->cnt, (const R*)p->rtab,
                                                                         (Fac<R>*)p->fac, g, k0, kc, p->Sf, p->Sl, p->Hf,
                                                                         p->cumcfg, p->ep, p->cum_ctas);
         lc.end(MEMD_STAGE_FACTOR);
         const long nseg = solve_segments_max(g.cap, p->sg);
         const long ns = 2L * kc * nseg * p->ngroups * 32;
+        const int T = solve_threads<R>(ns / 32);
         const unsigned nb = (unsigned)((ns + T - 1) / T);
         unsigned* bcur = p->bnd ? p->bnd + (size_t)(p->bpass & 1) * 2 * g.C : nullptr;
         SolveQueue q{};  // null prefix: the static mapping

@@ -583,16 +583,18 @@ k_factor(const int* __restrict__ knots, const int* __restrict__ cnt, const real*
 // bits; their sum bounds |S(n)| (the linear interpolant plus h^2/8 max|S''|).
 // ---------------------------------------------------------------------------
 constexpr int kSolveThreads = 128;
-// Threads per CTA of the factorisation and the sweeps.  FP64: one warp, so that
-// the warps that have rows spread over the SMs evenly (an FP64 operation of any
-// of an SM's warps takes the SM's one pipe 16 clocks): 8 x 2,000 stop 8.03 ->
-// 7.82 ms, 19 x 7,501 not-a-knot 15.40 -> 15.22, 32 x 30,504 44.6 -> 44.0.  FP32
-// and double-float: one warp costs the wide and long records 0.4 .. 0.7% (CTAs
-// past the knots) and gains nothing elsewhere.
+// Threads per CTA of a launch of `warps` warps of the factorisation or a sweep.
+// FP64: one warp, so that the warps that have rows spread over the SMs evenly
+// (an FP64 operation of any of an SM's warps takes the SM's one pipe 16 clocks):
+// 8 x 2,000 stop 8.03 -> 7.82 ms, 19 x 7,501 not-a-knot 15.40 -> 15.22, 32 x
+// 30,504 44.6 -> 44.0, 12 epochs 79.6 -> 78.6 (12,000 warps a sweep).  Not for
+// the largest launches, whose CTAs past the knots count: 512 epochs (295,000
+// warps) 2,554 -> 2,573 ms.  FP32 and double-float: one warp costs the wide and
+// long records 0.4 .. 0.7% and gains nothing elsewhere.
 template <typename real>
-constexpr int solve_threads()
+inline int solve_threads(long warps)
 {
-    return std::is_same<real, double>::value ? 32 : kSolveThreads;
+    return std::is_same<real, double>::value && warps <= 65536 ? 32 : kSolveThreads;
 }
 constexpr int kSolveBatch = 8;
 
