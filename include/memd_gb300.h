@@ -189,7 +189,7 @@ typedef struct memd_plan memd_plan;
 typedef struct {
     int32_t solve_segment;      /* longest substitution segment in knots, a power of two in [32, 1024] (512, FP32 256) */
     int32_t solve_min_segment;  /* shortest substitution segment, a power of two in [16, solve_segment] (64) */
-    int32_t factor_segment;     /* factorisation rows per thread, 4 .. 256 (16) */
+    int32_t factor_segment;     /* factorisation rows per thread, 4 .. 256 (16; 8 or 4 for few knots) */
     int32_t solve_queue;        /* substitution work: 1 = device work queue pulled by a persistent grid,
                                    2 or 0 = one warp per possible segment (the default) */
     int32_t mean_ctas;          /* impulse-accumulation mean: CTAs the split of spans over CTAs aims for,

@@ -82,11 +82,10 @@ def store(key: str, choice: dict, meta: dict, path: str | None = None) -> None:
 
 def search_space(precision: int, cum: bool) -> dict:
     """Values tried per knob (0 = the default)."""
-    f64 = int(precision) == 0
     space = {
         "solve_segment": [0, 128, 256],
         "solve_min_segment": [0, 32, 128],
-        "factor_segment": [0, 32, 128] if f64 else [0, 8, 32],
+        "factor_segment": [0, 8, 32],
         "solve_queue": [0, 1],
     }
     if cum:
