@@ -80,7 +80,7 @@ struct memd_plan {
     void* rtab;
     void* rtab3;  // impulse-accumulation mean: 1/(3h) and h/3, double-float (two tables) / FP64 (pairs)
     int ntab;     // entries of the reciprocal tables
-    unsigned* xexp;            // FP64: largest exponent [records][C] of the run's input
+    unsigned* xexp;            // FP64 form, tensor-core projection: largest exponent [records][C] of the run's input
     unsigned long long* tot;   // the same, several passes: knots per record over all directions
     unsigned* bnd;  // impulse-accumulation mean, mixed form: [2 passes][2 parts][C] per-channel bounds (float bits)
     int* cumcfg;    // impulse-accumulation mean: anchor span (words) and CTAs per span, set by the factor kernel
@@ -307,7 +307,7 @@ static void launch_eval(memd_plan* p, cudaStream_t s, int k0, int kc, int first,
         cudaLaunchKernelEx(&lc, g.mirror ? k_mean_fix<G_, true> : k_mean_fix<G_, false>, (const double*)p->X, (double*)p->Xb, (ulonglong2*)p->acc,          \
                            (const uint32_t*)p->bits, (const int*)p->wpref, (const int*)p->knots,                   \
                            (const int*)p->cnt, (const double*)p->rtab, (const double2*)p->rtab3,                   \
-                           (const double*)p->sv, (const double*)p->yend, (const unsigned*)p->xexp,                 \
+                           (const double*)p->sv, (const double*)p->yend,                                           \
                            (const unsigned long long*)(p->nchunks > 1 ? p->tot : nullptr), g, k0, kc, first, last, \
                            p->st, p->ep, (const int*)p->mir);                                                      \
         return;                                                                                                    \
@@ -1424,7 +1424,6 @@ static memd_status create_plan(const memd_config* cfg, const memd_tuning* tun, m
     ALLOC(p->rtab, rb * (size_t)(Lh + 1));
     p->ntab = Lh + 1;
     if (p->cum) ALLOC(p->rtab3, 16 * (size_t)(Lh + 1));
-    if (f64) ALLOC(p->xexp, sizeof(unsigned) * (size_t)std::max<int64_t>(1, c.max_epochs) * C);
     if (p->cum && f64) {
         if (p->nchunks > 1) ALLOC(p->tot, sizeof(unsigned long long) * (size_t)std::max<int64_t>(1, c.max_epochs));
     } else if (p->cum) {
@@ -1462,6 +1461,7 @@ static memd_status create_plan(const memd_config* cfg, const memd_tuning* tun, m
         ALLOC(p->dbig, sizeof(float) * (size_t)K * p->Cp);
         ALLOC(p->dsmall, sizeof(float) * (size_t)K * p->Cp);
         if (f64) {
+            ALLOC(p->xexp, sizeof(unsigned) * (size_t)std::max<int64_t>(1, c.max_epochs) * C);
             ALLOC(p->xmx, sizeof(float) * (size_t)((L + kTcRows - 1) / kTcRows) * p->Cp);
             ALLOC(p->dfl, sizeof(float) * (size_t)K * C);
         }

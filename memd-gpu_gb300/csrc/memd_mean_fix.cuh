@@ -13,15 +13,22 @@ namespace memd {
 // what happens at the knots: between an anchor sample and its neighbours the
 // sum of all envelopes is one cubic, whose third-order coefficient jumps by
 // d_j - d_{j-1} at every knot x_j.  FP64 operations are left at the knots
-// (two) and at the anchors (thirteen) only; every sum is an integer sum.
+// (two) and at the anchors (ten) only; every sum is an integer sum.
 //
-// Fixed point: values are integers in units of 2^-sh, 2^-sh = 2^(ex - 85) with
-// 2^ex > max|x| over the record's channel (k_to_sample_major, k_batched_in),
-// held as two words, v = hi 2^52 + lo with 0 <= lo < 2^52.  An FP64 value keeps all its
-// bits down to 2^-33 of the channel's largest sample and 2^-85 of it below
-// that; sums over at most 2048 (direction, envelope) pairs stay inside both
-// words, and the exact sums make the result independent of the order, of the
-// direction chunks and of the batch a record is in.
+// Fixed point: values are integers in units of 2^-sh, held as two words, v =
+// hi 2^52 + lo with 0 <= lo < 2^52.  The unit is the span's own: 2^-sh =
+// 2^(ex - 85) with 2^ex > max|x| over the channel's samples in the span, so a
+// quiet stretch keeps its accuracy however loud the rest of the channel is (a
+// third-order coefficient is rounded to the unit and then multiplied by up to
+// (T/2)^3 = 2^15: with a unit of the whole channel, a stretch 2^-26 as loud as
+// the channel's largest sample lost a few bits at T = 64).  Where a coefficient
+// does not fit (knots or overshoot from outside the span, 2^12 and more times
+// its samples), the unit is raised by exactly what the span's largest needs and
+// the pairs are gone through once more for those channels.  Sums over at most
+// 2048 (direction, envelope) pairs stay inside both words, and the exact sums
+// make the result independent of the order, of the batch a record is in and of
+// the direction passes (of several passes that need units raised differently,
+// the sums are brought to the coarsest, within its rounding).
 //
 // Anchors: every T samples, T the power of two in [8, 64] with T <= 3 h (h:
 // the record's mean knot spacing over all directions; 8 at the densest
@@ -37,26 +44,29 @@ namespace memd {
 // x 30,504, 64 directions, 80 sifts: 117.6 -> 21.2 ms of the mean (29.6 with T
 // <= 2 h, integer conversions on the FP64 pipe, one CTA per 64 samples and the
 // samples behind an anchor all by one warp); error of the IMFs against a
-// separate FP64 evaluation 8.2e-16 -> 4.0e-16.
+// separate FP64 evaluation 8.2e-16 -> 4.0e-16.  The unit per span (its samples
+// read once more, the coefficients' exponents followed) costs 1.2% of the run:
+// 43.5 -> 44.05 ms.
 //
-// A span whose values leave the fixed-point range (non-finite values, or
-// splines that overshoot the signal thousands of times), and a channel so
-// small that its third-order coefficients would be subnormal, is evaluated
-// directly, pair by pair in direction order, with k_eval_w's arithmetic.
+// A span with non-finite values, and one so small that its third-order
+// coefficients would be subnormal, is evaluated directly, pair by pair in
+// direction order, with k_eval_w's arithmetic.
 struct FixSum {
     unsigned long long hi, lo;
 };
 constexpr unsigned long long kFixLo = (1ull << 52) - 1ull;
 constexpr int kFixBits = 85;   // units per 2^ex: 2^85
-constexpr unsigned kFixMinExp = 128;  // smallest biased exponent of a channel's maximum (0: an all-zero channel)
+constexpr int kFixMin = 128 << 20;  // smallest high word of a span's largest value (0: all zero)
+constexpr int kFixInf = 0x7ff << 20;
+constexpr int kFixUnitExp = 32;  // smallest exponent a unit is chosen for: 2^-1075, where no subnormal is too large
 constexpr int kFixRows = 64;   // longest span
 constexpr int kFixAnchors = 4; // anchors of a span: 32 / 8
 
-// v 2^sh rounded to nearest; false when |v 2^sh| could reach 2^lim (or v is
-// not finite).  Integer instructions only: FP64 <-> integer conversions run on
-// the FP64 pipe.
-__device__ __forceinline__ bool to_fix(double v, int sh, int lim, FixSum& r)
+// v 2^sh rounded to nearest; raises mx to |v|'s high word.  Integer
+// instructions only: FP64 <-> integer conversions run on the FP64 pipe.
+__device__ __forceinline__ FixSum to_fix(double v, int sh, int& mx)
 {
+    FixSum r;
     const long long b = __double_as_longlong(v);
     const int be = (int)((unsigned long long)b >> 52) & 0x7ff;
     long long m = (b & (long long)kFixLo) | (be ? (1ll << 52) : 0ll);
@@ -71,8 +81,12 @@ __device__ __forceinline__ bool to_fix(double v, int sh, int lim, FixSum& r)
         r.hi = (unsigned long long)(n >> 52);
         r.lo = (unsigned long long)n & kFixLo;
     }
-    return be != 0x7ff && (s <= lim - 53 || m == 0);
+    mx = max(mx, __double2hiint(v) & 0x7fffffff);
+    return r;
 }
+// how far the unit 2^-sh must be raised so that every value with a high word
+// of at most mx stays below 2^lim units
+__device__ __forceinline__ int fix_excess(int mx, int sh, int lim) { return (mx >> 20) - 1075 + sh - (lim - 53); }
 
 // the 128-bit two's-complement integer n times 2^-sh, rounded to nearest even
 __device__ __forceinline__ double from_fix(__int128 n, int sh)
@@ -95,14 +109,30 @@ __device__ __forceinline__ double from_fix(__int128 n, int sh)
     return neg ? -v : v;
 }
 
-// accumulator of several direction passes: the exact sum, or (kFixTag in the
-// top bits, which a sum below 2^116 cannot have) the FP64 sum of a span that
-// was evaluated directly
-constexpr unsigned long long kFixTag = 0x5a5ull << 52;
-__device__ __forceinline__ bool fix_tagged(ulonglong2 v) { return (v.y & (0xfffull << 52)) == kFixTag; }
+// accumulator of several direction passes: the exact sum (below 2^115) in 116
+// bits and, in the top 12, how far its unit is raised, or kFixDirect and the
+// FP64 sum of a span that was evaluated directly
+constexpr int kFixDirect = 0xfff;
+__device__ __forceinline__ ulonglong2 fix_pack(__int128 v, int raise)
+{
+    return make_ulonglong2((unsigned long long)v,
+                           ((unsigned long long)((unsigned __int128)v >> 64) & kFixLo) | ((unsigned long long)raise << 52));
+}
+__device__ __forceinline__ int fix_raise(ulonglong2 o) { return (int)(o.y >> 52); }
+__device__ __forceinline__ __int128 fix_sum(ulonglong2 o)
+{
+    const long long hi = (long long)(o.y << 12) >> 12;
+    return ((__int128)hi << 64) | (__int128)o.x;
+}
+// v in a unit raised by n >= 0 more, rounded to nearest
+__device__ __forceinline__ __int128 fix_coarser(__int128 v, int n)
+{
+    if (n == 0) return v;
+    return n > 120 ? (__int128)0 : (v + ((__int128)1 << (n - 1))) >> n;
+}
 
-// 2^ex > max|x|: ex from the largest biased exponent of the channel's samples
-__device__ __forceinline__ int fix_shift(unsigned be) { return kFixBits - ((int)be - 1022); }
+// 2^ex > max|x|: ex from the high word of the largest sample
+__device__ __forceinline__ int fix_shift(int mx) { return kFixBits - (max(mx >> 20, kFixUnitExp) - 1022); }
 
 // 2 v (exact); by an integer addition to the exponent for a normal value
 __device__ __forceinline__ double twice(double v)
@@ -123,8 +153,7 @@ __global__ void __launch_bounds__(256, 3)
 k_mean_fix(const double* __restrict__ X, double* __restrict__ Xout, ulonglong2* __restrict__ acc_buf,
            const uint32_t* __restrict__ bits, const int* __restrict__ wpref, const int* __restrict__ knots,
            const int* __restrict__ cnt, const double* __restrict__ rtab, const double2* __restrict__ rtab3,
-           const double* __restrict__ sv, const double* __restrict__ yend, const unsigned* __restrict__ xexp,
-           const unsigned long long* __restrict__ tot, Geom g, int k0, int Kc, int first_chunk, int last_chunk,
+           const double* __restrict__ sv, const double* __restrict__ yend, const unsigned long long* __restrict__ tot, Geom g, int k0, int Kc, int first_chunk, int last_chunk,
            RunState* st, Epochs ep, const int* __restrict__ mir)
 {
     // MIR (mirror boundary, one record): the knot list is [left mirrored |
@@ -145,6 +174,7 @@ k_mean_fix(const double* __restrict__ X, double* __restrict__ Xout, ulonglong2* 
     __shared__ int eJ[NE], eE[NE];  // first piece of the span (-1: the pair does not count); last piece of the record
     __shared__ int sQ, sT;
     __shared__ unsigned sBad;  // channels of the span to evaluate directly
+    __shared__ int sMax[G], sRaise[G];  // high word of the channels' largest sample; how far their units are raised
     __shared__ unsigned long long sEt;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int cc = lane % G, sub = lane / G;
@@ -159,6 +189,7 @@ k_mean_fix(const double* __restrict__ X, double* __restrict__ Xout, ulonglong2* 
         sBad = 0u;
         sEt = 0ull;
     }
+    if (threadIdx.x < G) sMax[threadIdx.x] = sRaise[threadIdx.x] = 0;
     __syncthreads();
     {
         // qualified directions, and the knots of all of them (spans of several
@@ -204,19 +235,36 @@ k_mean_fix(const double* __restrict__ X, double* __restrict__ Xout, ulonglong2* 
     const int c = blockIdx.y * G + cc;
     const bool cok = c < C;
     const int cl = min(c, C - 1);  // loads of lanes past the last channel stay in bounds
+    double xr[kFixRows * G / 256];  // the span's samples of this thread's channel (blockDim.x is a multiple of G)
+#pragma unroll
+    for (int k = 0; k < kFixRows * G / 256; ++k) {
+        const int r = (int)threadIdx.x / G + k * (256 / G);
+        xr[k] = r < nl ? X[(size_t)(p0 + r) * C + cl] : 0.0;
+    }
     for (int j = 0; j < 4; ++j) {
         for (int i = threadIdx.x; i < nl * G; i += blockDim.x) sums[j * NS + i] = 0u;
         for (int i = threadIdx.x; i < nA * 4 * G; i += blockDim.x) sums[j * NS + AN + i] = 0u;
     }
-    const unsigned xe = xexp[(size_t)rec * C + cl];
-    const int sh = fix_shift(xe);
+    {
+        int m = 0;
+#pragma unroll
+        for (int k = 0; k < kFixRows * G / 256; ++k) {
+            const int h = (__double2hiint(xr[k]) & 0x7fffffff) | (__double2loint(xr[k]) ? 1 : 0);
+            m = max(m, h < kFixInf ? h : 0);
+        }
+        if (m) atomicMax(&sMax[cc], m);
+    }
     // the sum of the 2K envelopes stays below 2^115: A, B T/2, C (T/2)^2 and
     // d (T/2)^3 of each below 2^lim
     const int lim = 108 - (32 - __clz(2 * g.K - 1));
     const int lt = 30 - __clz(T);  // log2(T / 2)
-    bool ok = xe == 0u || xe >= kFixMinExp;
     const int rlast = rend - 1;
+    int raise = 0, sh = 0;                // how far the channel's unit is raised; 2^-sh, the unit
+    bool again = false;
+    unsigned obad = 0u;                   // the other half's sBad
+    int mA = 0, mB = 0, mC = 0, mD = 0;   // high words of the largest of the anchors' coefficients and of d
 
+    for (;;) {
     for (int base = e_lo; base < e_hi; base += NE) {
         __syncthreads();
         {
@@ -247,6 +295,7 @@ k_mean_fix(const double* __restrict__ X, double* __restrict__ Xout, ulonglong2* 
             }
         }
         __syncthreads();
+        sh = fix_shift(sMax[cc]) - raise;
         const int nround = min(NE, e_hi - base);
         for (int le = warp * SUB + sub; le < nround; le += NWS) {
             int j = eJ[le];
@@ -275,8 +324,7 @@ k_mean_fix(const double* __restrict__ X, double* __restrict__ Xout, ulonglong2* 
                 const int h = xn - xj;
                 const double2 r3 = rtab3[h];  // 1 / (3 h), h / 3
                 const double d = __dmul_rn(__dsub_rn(s1, s0), r3.x);
-                FixSum qc;
-                ok &= to_fix(d, sh, lim - 3 * lt, qc);
+                const FixSum qc = to_fix(d, sh, mD);
                 if (jump && MEMD_CHECK(xj - p0 > 0 && xj - p0 < nl)) {
                     add((xj - p0) * G + cc, qc.hi - qp.hi, qc.lo - qp.lo);
                 }
@@ -296,14 +344,13 @@ k_mean_fix(const double* __restrict__ X, double* __restrict__ Xout, ulonglong2* 
                     const double b = __fma_rn(-r3.y, __fma_rn(2.0, s0, s1), __dmul_rn(__dsub_rn(y1, y0), rtab[h]));
                     const double e = __fma_rn(d, u, s0);
                     const double cB = __fma_rn(__fma_rn(d, u3, twice(s0)), u, b);
-                    FixSum f;
                     const int at = AN + a * 4 * G + cc;
-                    ok &= to_fix(__fma_rn(__fma_rn(e, u, b), u, y0), sh, lim, f);
-                    add(at, f.hi, f.lo);
-                    ok &= to_fix(cB, sh, lim - lt, f);
-                    add(at + G, f.hi, f.lo);
-                    ok &= to_fix(__fma_rn(d, u3, s0), sh, lim - 2 * lt, f);
-                    add(at + 2 * G, f.hi, f.lo);
+                    const FixSum fA = to_fix(__fma_rn(__fma_rn(e, u, b), u, y0), sh, mA);
+                    const FixSum fB = to_fix(cB, sh, mB);
+                    const FixSum fC = to_fix(__fma_rn(d, u3, s0), sh, mC);
+                    add(at, fA.hi, fA.lo);
+                    add(at + G, fB.hi, fB.lo);
+                    add(at + 2 * G, fC.hi, fC.lo);
                     add(at + 3 * G, qc.hi, qc.lo);
                     ++a;
                     na = p0 + a * T + min(T >> 1, nl - 1 - a * T);
@@ -318,16 +365,37 @@ k_mean_fix(const double* __restrict__ X, double* __restrict__ Xout, ulonglong2* 
             }
         }
     }
-    if (!ok) atomicOr(&sBad, 1u << cc);
+    if (again) break;
+    const int over = max(max(fix_excess(mA, sh, lim), fix_excess(mB, sh, lim - lt)),
+                         max(fix_excess(mC, sh, lim - 2 * lt), fix_excess(mD, sh, lim - 3 * lt)));
+    const int large = max(sMax[cc], mA);
+    if (max(max(mA, mB), max(mC, mD)) >= kFixInf || (large > 0 && large < kFixMin)) atomicOr(&sBad, 1u << cc);
+    else if (over > 0) atomicMax(&sRaise[cc], over);
     __syncthreads();
+    raise = sRaise[cc];
+    if (pair) {  // the same decisions in both halves
+        namespace cg_ = cooperative_groups;
+        const auto cl_ = cg_::this_cluster();
+        cl_.sync();
+        obad = *cl_.map_shared_rank(&sBad, 1 - half);
+        raise = max(raise, cl_.map_shared_rank(sRaise, 1 - half)[cc]);
+    }
+    if (((sBad | obad) >> cc) & 1u) raise = 0;
+    again = __syncthreads_or(raise > 0);
+    if (!again) break;
+    for (int j = 0; j < 4; ++j) {
+        for (int i = threadIdx.x; i < nl * G; i += blockDim.x) sums[j * NS + i] = 0u;
+        for (int i = threadIdx.x; i < nA * 4 * G; i += blockDim.x) sums[j * NS + AN + i] = 0u;
+    }
+    }  // once more
+    if (again) __syncthreads();
     if (pair) {
         // the other half's sums: read them all, and only then change this CTA's
         namespace cg_ = cooperative_groups;
         const auto cl_ = cg_::this_cluster();
-        cl_.sync();
+        if (again) cl_.sync();
         constexpr int NV = (kFixRows + 4) * G / 256 + 1;
         const unsigned* os = cl_.map_shared_rank(sums, 1 - half);
-        const unsigned obad = *cl_.map_shared_rank(&sBad, 1 - half);
         const int nk = nl * G, nv = nk + 4 * G;  // rows, then the anchor (nA = 1)
         for (int word = 0; word < 4; word += 2) {
             unsigned long long v[NV];
@@ -347,33 +415,36 @@ k_mean_fix(const double* __restrict__ X, double* __restrict__ Xout, ulonglong2* 
                 }
             }
         }
-        if (threadIdx.x == 0) sBad |= obad;
         __syncthreads();
     }
     const int Q = sQ;
     if (last_chunk && Q == 0 && blockIdx.y == 0 && threadIdx.x == 0) atomicOr(&st->flags, 1);
     if (!cok) return;
     const double qd = (double)Q, rq = Q > 0 ? __ddiv_rn(1.0, qd) : __longlong_as_double(0x7ff8000000000000ll);
-    const bool bad = (sBad >> cc) & 1u;
+    const bool bad = ((sBad | obad) >> cc) & 1u;
     // M's sum at row r is done: X -= M / 2 / Q, or on to the next pass; x: X there
     auto emit = [&](int r, __int128 v, double vd, double x) {
         const size_t off = (size_t)(p0 + r) * C + c;
         bool isd = bad;
+        int up = raise, shv = sh;
         if (!first_chunk) {
             const ulonglong2 o = acc_buf[off];
-            if (fix_tagged(o) || isd) {
-                const double od = fix_tagged(o) ? __longlong_as_double((long long)o.x)
-                                                : from_fix((__int128)(((unsigned __int128)o.y << 64) | o.x), sh);
+            const int ro = fix_raise(o);
+            if (ro == kFixDirect || isd) {
+                const double od = ro == kFixDirect ? __longlong_as_double((long long)o.x)
+                                                   : from_fix(fix_sum(o), sh + raise - ro);
                 vd = __dadd_rn(od, isd ? vd : from_fix(v, sh));
                 isd = true;
             } else {
-                v += (__int128)(((unsigned __int128)o.y << 64) | o.x);
+                up = max(ro, raise);
+                v = fix_coarser(v, up - raise) + fix_coarser(fix_sum(o), up - ro);
+                shv = sh + raise - up;
             }
         }
         if (last_chunk) {
             // (sum / 2) / Q rounded as a division: quotient by the reciprocal,
             // one correction by the remainder
-            const double val = __dmul_rn(isd ? vd : from_fix(v, sh), 0.5);
+            const double val = __dmul_rn(isd ? vd : from_fix(v, shv), 0.5);
             double m;
             if (isd) {
                 m = __ddiv_rn(val, qd);
@@ -383,15 +454,8 @@ k_mean_fix(const double* __restrict__ X, double* __restrict__ Xout, ulonglong2* 
             }
             Xout[off] = __dsub_rn(x, m);
         } else {
-            ulonglong2 o;
-            if (isd) {
-                o.x = (unsigned long long)__double_as_longlong(vd);
-                o.y = kFixTag;
-            } else {
-                o.x = (unsigned long long)v;
-                o.y = (unsigned long long)((unsigned __int128)v >> 64);
-            }
-            acc_buf[off] = o;
+            acc_buf[off] = isd ? make_ulonglong2((unsigned long long)__double_as_longlong(vd), (unsigned long long)kFixDirect << 52)
+                               : fix_pack(v, up);
         }
     };
     auto wide = [&](int i) -> __int128 {
