@@ -1488,11 +1488,14 @@ k_eval_w(const XT* __restrict__ X, XT* __restrict__ Xout, R* __restrict__ acc_bu
 // sifts: 18.96 ms with mantissa shifts for the conversions, 64-bit shared
 // atomics and block-wide prefix sums that needed the knots of three samples
 // past the span; 15.42 ms with limbs, 32-bit atomics with a carry and the walk;
-// 14.89 ms with the anchor's products summed before they are rounded; 14.2 ms
-// with the pieces' rows and reciprocals fetched one per lane ahead of the
+// 14.89 ms with the anchor's products left as they are before they are summed;
+// 14.2 ms with the pieces' rows and reciprocals fetched one per lane ahead of the
 // anchor and handed out by shuffles (they were two loads a knot, the second
 // waiting for the first).  Fetching the next pair's rows ahead, to L2, L1 or in
-// registers, gave nothing more.
+// registers, gave nothing more.  The anchors' sums are renormalised at each
+// addition: with a low word that is never brought back to half an ulp of the
+// high word the rounding of 16 to 64 terms was 1.8 to 2.9 times as large for
+// 0.2 ms less.
 // ---------------------------------------------------------------------------
 // The double-float v times 2^sh as a 64-bit two's-complement integer (|v 2^sh|
 // < 2^62), rounded to nearest, in three limbs a 2^44 + b 2^22 + c that are kept
@@ -1540,25 +1543,6 @@ __device__ __forceinline__ void add_words(unsigned* lo, unsigned* hi, int i, uns
     atomicAdd(&hi[i], (unsigned)(v >> 32) + (old + l < l ? 1u : 0u));
 }
 
-// sum of double-floats without renormalising: the high words by an error-free
-// addition, its error and the low words in l
-struct Acc {
-    float h, l;
-};
-__device__ __forceinline__ void acc_add(Acc& s, float hi, float lo)
-{
-    const float t = __fadd_rn(s.h, hi);
-    const float bb = __fsub_rn(t, s.h);
-    s.l = __fadd_rn(s.l, __fadd_rn(__fadd_rn(__fsub_rn(s.h, __fsub_rn(t, bb)), __fsub_rn(hi, bb)), lo));
-    s.h = t;
-}
-// s += a t, t a plain float
-__device__ __forceinline__ void acc_mulf(Acc& s, dd a, float t)
-{
-    const float p = __fmul_rn(a.hi, t);
-    acc_add(s, p, __fmaf_rn(a.lo, t, __fmaf_rn(a.hi, t, -p)));
-}
-__device__ __forceinline__ dd acc_dd(Acc s) { return dd_renorm(s.h, s.l); }
 // Products without renormalisation (their value is the same), for sums and
 // conversions: the low word may reach an ulp of the high word.
 __device__ __forceinline__ dd raw_mul(dd a, dd b)
@@ -1700,7 +1684,8 @@ k_mean_cum(const float2* __restrict__ X, float2* __restrict__ Xout, dd* __restri
     // this CTA's share of the (direction, envelope) pairs
     const int e_lo = prt * 2 * Kc / P, e_hi = (prt + 1) * 2 * Kc / P;  // 2 Kc <= 2048, P <= 4
 
-    Acc aA{0.0f, 0.0f}, aB{0.0f, 0.0f}, aC{0.0f, 0.0f}, aD{0.0f, 0.0f};  // anchor coefficients, summed in a fixed order
+    // anchor coefficients, summed in a fixed order
+    dd aA(0.0f, 0.0f), aB(0.0f, 0.0f), aC(0.0f, 0.0f), aD(0.0f, 0.0f);
     for (int base = e_lo; base < e_hi; base += NE) {
         __syncthreads();
         // (1) per (direction, envelope): anchor piece i (x_i <= n_a < x_{i+1}),
@@ -1797,12 +1782,10 @@ k_mean_cum(const float2* __restrict__ X, float2* __restrict__ Xout, dd* __restri
                 const dd d = (s1 - s0) * rtab3[h];
                 const dd b = raw_mul(y1 - y0, rtab[h]) + (-raw_mul(s02 + s1, h3tab[h]));
                 const dd c2 = s0 + raw_mulf(d, u3);  // half the second derivative at n_a
-                acc_mulf(aA, dd_mulf(dd_mulf(d, u) + s0, u) + b, u);
-                acc_add(aA, y0.hi, y0.lo);
-                acc_mulf(aB, c2 + s0, u);
-                acc_add(aB, b.hi, b.lo);
-                acc_add(aC, c2.hi, c2.lo);
-                acc_add(aD, d.hi, d.lo);
+                aA = aA + (raw_mulf(dd_mulf(dd_mulf(d, u) + s0, u) + b, u) + y0);
+                aB = aB + (raw_mulf(c2 + s0, u) + b);
+                aC = aC + c2;
+                aD = aD + d;
             }
             // (3) jumps q_j - q_{j-1} at row x_j - p0 (in 1 .. nl - 1), q_j the
             //     quantised d_j = (s_{j+1} - s_j) / (3 h_j); full batches of KB
@@ -1846,10 +1829,10 @@ k_mean_cum(const float2* __restrict__ X, float2* __restrict__ Xout, dd* __restri
         ahi[i] = 0u;
     }
     __syncthreads();
-    add_words(alo, ahi, 0 * G + cc, limbs_value(to_limbs(acc_dd(aA), s44, s22)));
-    add_words(alo, ahi, 1 * G + cc, limbs_value(to_limbs(acc_dd(aB), s44, s22)));
-    add_words(alo, ahi, 2 * G + cc, limbs_value(to_limbs(acc_dd(aC), s44, s22)));
-    add_words(alo, ahi, 3 * G + cc, limbs_value(to_limbs(acc_dd(aD), s44, s22)));
+    add_words(alo, ahi, 0 * G + cc, limbs_value(to_limbs(aA, s44, s22)));
+    add_words(alo, ahi, 1 * G + cc, limbs_value(to_limbs(aB, s44, s22)));
+    add_words(alo, ahi, 2 * G + cc, limbs_value(to_limbs(aC, s44, s22)));
+    add_words(alo, ahi, 3 * G + cc, limbs_value(to_limbs(aD, s44, s22)));
     __syncthreads();
     auto word = [](const unsigned* lo, const unsigned* hi, int i) -> unsigned long long {
         return ((unsigned long long)hi[i] << 32) | lo[i];
