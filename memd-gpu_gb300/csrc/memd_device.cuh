@@ -265,6 +265,7 @@ __device__ __forceinline__ int mirror_source(const int* __restrict__ mi, int env
 // index check fails, which also records the failure in g_memd_check (read and
 // cleared by the host after each run, reported as MEMD_FLAG_CHECK_FAILED); the
 // guarded access is then skipped instead of touching memory out of bounds.
+// Quotients formed without the division instruction are compared with it.
 // In the normal build the checks compile away.
 #ifdef MEMD_CHECKED
 __device__ int g_memd_check;
@@ -366,24 +367,33 @@ __device__ __forceinline__ dd sqrt_(dd a) { return dd_sqrt(a); }
 __device__ __forceinline__ double fmat_(double a, float t, double c) { return __fma_rn(a, (double)t, c); }
 __device__ __forceinline__ float fmat_(float a, float t, float c) { return __fmaf_rn(a, t, c); }
 __device__ __forceinline__ dd fmat_(dd a, float t, dd c) { return dd_mulf(a, t) + c; }
-// 1/a: IEEE division for float (the FP32 form keeps the reference's
-// arithmetic); for double within 0.501 ulp; for a double-float, the correctly rounded float
-// reciprocal refined by one Newton step with an fma residual (~47 bits, a
-// quarter of the instructions of the double-float division)
+// 1/a: correctly rounded for double and float; for a double-float, the correctly
+// rounded float reciprocal refined by one Newton step with an fma residual (~47
+// bits, a quarter of the instructions of the double-float division)
 __device__ __forceinline__ double recip_(double a)
 {
     // a in float's normal range (pivots of integer spacings): the float
     // reciprocal x of a's leading 24 bits, moved between the formats by integer
-    // instructions, and one third-order step x + x (e + e^2), e = 1 - a x
-    // (|e| < 2^-21: e^3 is below the last place by 2^-10).  Three FP64
-    // operations on the pivots' serial chain, on a pipe that takes 64 cycles a
-    // warp instruction.
+    // instructions, and one cubically convergent hyperpower step (Altman 1960) x
+    // + x (e + e^2), e = 1 - a x (|e| < 2^-21: e^3 is below the last place by
+    // 2^-10).  Three FP64 operations on the pivots' serial chain, on a pipe that
+    // takes 64 cycles a warp instruction.
     const unsigned h = (unsigned)__double2hiint(a), l = (unsigned)__double2loint(a);
     const float x0 = __frcp_rn(__uint_as_float((h & 0x80000000u) | ((((h & 0x7fffffffu) - ((1023u - 127u) << 20)) << 3) | (l >> 29))));
     const unsigned b = __float_as_uint(x0);
     const double x = __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + ((1023u - 127u) << 20))), (int)(b << 29));
     const double e = __fma_rn(-a, x, 1.0);
-    return __fma_rn(x, __fma_rn(e, e, e), x);
+    const double y = __fma_rn(x, __fma_rn(e, e, e), x);
+    // The last place, in integers: y's mantissa Y is the nearest to 2^105 / A (A
+    // a's mantissa; 2^104 / A for a power of two) when 2 |2^105 - A Y| <= A, and
+    // the difference is small enough to be had from the low 64 bits of A Y.
+    constexpr unsigned long long kMant = (1ull << 52) - 1ull;
+    const unsigned long long A = ((unsigned long long)__double_as_longlong(a) & kMant) | (1ull << 52);
+    const long long yb = __double_as_longlong(y);
+    const long long r2 = (long long)(0ull - A * (((unsigned long long)yb & kMant) | (1ull << 52))) * 2;
+    const double q = __longlong_as_double(yb + (r2 > (long long)A ? 1 : 0) - (r2 < -(long long)A ? 1 : 0));
+    (void)MEMD_CHECK(q == __ddiv_rn(1.0, a));
+    return q;
 }
 __device__ __forceinline__ float recip_(float a) { return __fdiv_rn(1.0f, a); }
 __device__ __forceinline__ dd recip_(dd a)

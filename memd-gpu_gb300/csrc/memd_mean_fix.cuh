@@ -442,8 +442,10 @@ k_mean_fix(const double* __restrict__ X, double* __restrict__ Xout, ulonglong2* 
             }
         }
         if (last_chunk) {
-            // (sum / 2) / Q rounded as a division: quotient by the reciprocal,
-            // one correction by the remainder
+            // (sum / 2) / Q rounded as a division: quotient by the correctly
+            // rounded reciprocal, one correction by the remainder (Markstein 1990;
+            // the remainder is exact, the units of a sum that is not evaluated
+            // directly being far above the subnormals)
             const double val = __dmul_rn(isd ? vd : from_fix(v, shv), 0.5);
             double m;
             if (isd) {
@@ -451,6 +453,7 @@ k_mean_fix(const double* __restrict__ X, double* __restrict__ Xout, ulonglong2* 
             } else {
                 const double q0 = __dmul_rn(val, rq);
                 m = __fma_rn(__fma_rn(-q0, qd, val), rq, q0);
+                (void)MEMD_CHECK(m == __ddiv_rn(val, qd) || Q == 0);
             }
             Xout[off] = __dsub_rn(x, m);
         } else {
