@@ -345,7 +345,7 @@ static void launch_eval(memd_plan* p, cudaStream_t s, int k0, int kc, int first,
             cudaLaunchConfig_t lc{};
             lc.gridDim = dim3(grid.x, grid.y, (unsigned)p->ewZ);
             lc.blockDim = dim3(32 * W);
-            lc.dynamicSmemBytes = Sh::smem_bytes(stopm);
+            lc.dynamicSmemBytes = Sh::smem_bytes(stopm, p->ewZ);
             lc.stream = s;
             cudaLaunchAttribute at[1];
             at[0].id = cudaLaunchAttributeClusterDimension;
@@ -375,10 +375,10 @@ static cudaError_t set_attrs(memd_plan* p)
         using Sh = EvalWShape<G, SPL, R, W>;
         if (e == cudaSuccess)
             e = cudaFuncSetAttribute(k_eval_w<G, SPL, XT, R, true, W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)Sh::smem_bytes(true));
+                                     (int)Sh::smem_bytes(true, p->ewZ));
         if (e == cudaSuccess)
             e = cudaFuncSetAttribute(k_eval_w<G, SPL, XT, R, false, W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)Sh::smem_bytes(false));
+                                     (int)Sh::smem_bytes(false, p->ewZ));
     });
     if (e != cudaSuccess) return e;
     if constexpr (P == MEMD_PREC_MIXED) {
@@ -1356,7 +1356,7 @@ static memd_status create_plan(const memd_config* cfg, const memd_tuning* tun, m
         const long groups = (C + p->ewG - 1) / p->ewG;
         auto tiles = [&](int spl) { return (L + 32 / p->ewG * spl - 1) / (32 / p->ewG * spl) * groups; };
         p->ewSPL = f32 ? 32 : 16;
-        p->ewW = 8;
+        p->ewW = kEvalWarps;
         while (p->ewSPL > p->ewG && tiles(p->ewSPL) < 456) p->ewSPL /= 2;
         p->ewZ = 1;
         if (!f32 && p->ewSPL == p->ewG) {
@@ -1397,7 +1397,10 @@ static memd_status create_plan(const memd_config* cfg, const memd_tuning* tun, m
     if (c.stop_mode == MEMD_STOP_FIXED) ALLOC(p->Xb, (size_t)p->xbytes * CL);
     ALLOC(p->run, (size_t)p->xbytes * CL);
     ALLOC(p->dir, 8 * (size_t)K * C);
-    if (p->nchunks > 1) ALLOC(p->acc, (p->cum && f64 ? 16 : rb) * CL);  // FP64: the exact 128-bit sum
+    // several passes: FP64 impulse mean, the exact 128-bit sum; FP64 and mixed direct evaluation, the total and the sum of
+    // a group that a pass ends in
+    if (p->nchunks > 1)
+        ALLOC(p->acc, (p->cum ? (f64 ? 16 : rb) : rb * (c.precision != MEMD_PREC_F32 && p->Kc % kEvalWarps ? 2 : 1)) * CL);
     ALLOC(p->imf, (size_t)p->tbytes * CL * (size_t)c.num_imfs);
     ALLOC(p->bits, sizeof(uint32_t) * 2 * Kc * p->g.W);
     ALLOC(p->wpref, sizeof(int) * 2 * Kc * (p->g.W + 1));

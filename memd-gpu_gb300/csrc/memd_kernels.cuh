@@ -1152,8 +1152,13 @@ __device__ __forceinline__ void mirror_positions(const int* __restrict__ mi, con
 //   a = y_i, b = (y_{i+1}-y_i)/h - h(2 s_i + s_{i+1})/3, c = s_i,
 //   d = (s_{i+1} - s_i)/(3h)
 // when the interval changes.  The sum over qualified directions (E_max > 3 &&
-// E_min > 3): each warp's directions in order, then the warps' partial sums in
-// warp order; the last chunk applies X -= (sum/2)/Q (REF:832-864).
+// E_min > 3), FP32: each warp's directions in order, then the warps' partial
+// sums in warp order.  FP64 and double-float: in order within groups of WARPS
+// directions, counted over all passes, and the groups' sums in order, so that
+// neither the passes nor the CTAs per tile (a record alone or in a batch) show
+// in the result; a warp leaves its direction's values in shared memory, a CTA
+// adds up a group at a time.  The last chunk applies X -= (sum/2)/Q
+// (REF:832-864).
 // X is float (FP32 path), float2 (double-float, mixed path) or double.
 // The tile is as long as still gives three CTAs per SM (32 samples at least),
 // and the
@@ -1172,19 +1177,25 @@ __device__ __forceinline__ void mirror_positions(const int* __restrict__ mi, con
 // 30,504, 64 directions in FP32, 11.5 so; 14.7 with the interval looked up and
 // the offset converted at every sample.
 // ---------------------------------------------------------------------------
+constexpr int kEvalWarps = 8;  // warps of a CTA
+
 template <int G, int SPL, typename R, int WARPS>
 struct EvalWShape {
     static constexpr int NS = 32 / G;
     static constexpr int T = NS * SPL;
     static constexpr int MI = T / 2 + 4;
     static constexpr int NW = T / 32;
-    // per warp: its sums of the tile, (stop mode) spread tile, knots and the rows
+    // per warp: its sums (FP32) or its direction's values of the tile, (stop mode) spread tile, knots and the rows
     // of their values, bit words
     __host__ __device__ static constexpr size_t per_warp(bool stopm)
     {
         return (size_t)(stopm ? 2 : 1) * sizeof(R) * T * G + 2 * sizeof(int) * (MI + 1) + sizeof(uint32_t) * (NW + 1);
     }
-    static constexpr size_t smem_bytes(bool stopm) { return WARPS * ((per_warp(stopm) + 15) / 16 * 16); }
+    // several CTAs per tile: and the groups' sums of a round and the one before
+    static constexpr size_t smem_bytes(bool stopm, int Z)
+    {
+        return WARPS * ((per_warp(stopm) + 15) / 16 * 16) + (Z > 1 ? 2 * sizeof(R) * T * G : 0);
+    }
 };
 
 template <int G, int SPL, typename XT, typename R, bool STOPM, int WARPS>
@@ -1221,7 +1232,7 @@ k_eval_w(const XT* __restrict__ X, XT* __restrict__ Xout, R* __restrict__ acc_bu
     const int cl = min(c, C - 1);  // loads of lanes past the last channel stay in bounds
     const int w0 = n0 >> 5;
     unsigned char* wb = smem_raw + (size_t)warp * PW;
-    R* accs = reinterpret_cast<R*>(wb);                        // [T][G], the warp's sums of a slice
+    R* accs = reinterpret_cast<R*>(wb);                        // [T][G], the warp's sums or its direction's values
     R* us = accs + (STOPM ? T * G : 0);                        // [T][G] (stop mode): the spread U - L
     int* kx = reinterpret_cast<int*>(accs + (STOPM ? 2 : 1) * T * G);  // knots
     int* ks = kx + MI + 1;                                     // the rows of their values
@@ -1239,26 +1250,48 @@ k_eval_w(const XT* __restrict__ X, XT* __restrict__ Xout, R* __restrict__ acc_bu
     const R* sc = sv + cl;
     bool overflow = false;
 
-    // CTAs per tile (FP32: one, its sum over the directions keeps its order).
-    // FP64: the directions in NZ slices (Z divides 4, and is 1 where Kc has fewer
-    // than eight a slice for it) whatever the CTAs per tile, so that the
-    // sum's order, and with it a record's result, does not depend on the launch
-    // (a record alone or in a batch)
+    // Z CTAs per tile (FP32: one) take the directions in turn, a warp each
     constexpr bool ONE = std::is_same<R, float>::value;
     namespace cg_ = cooperative_groups;
     const int Z = ONE ? 1 : (int)gridDim.z, zr = ONE ? 0 : (int)blockIdx.z;
-    const int NZ = std::is_same<R, double>::value ? min(4, (Kc + WARPS - 1) / WARPS) : Z;
     constexpr int EPT = (T * G + 32 * WARPS - 1) / (32 * WARPS);  // tile elements per thread
+    auto share = [&](int idx) {  // is element idx summed by this CTA? (idx: threadIdx.x + q 32 WARPS)
+        return idx < T * G && (Z == 1 || (idx >> 5) % Z == zr);
+    };
+    auto offset = [&](int idx, size_t& off) {  // of element idx in the record; is it there?
+        const int t = idx / G, cch = cg * G + (idx - t * G);
+        off = (size_t)(n0 + t) * C + cch;
+        return idx < T * G && t < nl && cch < C;
+    };
+    const size_t CL = (size_t)g.L * C;
     R tots[EPT];
+    auto earlier_passes = [&]() {
 #pragma unroll
-    for (int q = 0; q < EPT; ++q) tots[q] = R(0.0f);
-    for (int z0 = 0; z0 < NZ; z0 += Z) {
-    for (int j = 0; j < SPL; ++j) accs[(s_first + j) * G + cc] = R(0.0f);
-    for (int kk = (z0 + zr) * WARPS + warp; kk < Kc; kk += WARPS * NZ) {
-        const int k = k0 + kk;
-        if (!dir_qualifies(g, ep, cnt, k, rec)) continue;
-        if (cnt[k] > g.cap || cnt[g.K + k] > g.cap) continue;
-        for (int env = 0; env < 2; ++env) {
+        for (int q = 0; q < EPT; ++q) {
+            const int idx = threadIdx.x + q * 32 * WARPS;
+            size_t off;
+            tots[q] = !first_chunk && share(idx) && offset(idx, off) ? acc_buf[off] : R(0.0f);
+        }
+    };
+    if constexpr (!ONE) earlier_passes();
+    if constexpr (ONE)
+        for (int j = 0; j < SPL; ++j) accs[(s_first + j) * G + cc] = R(0.0f);
+    // groups start at multiples of WARPS of all directions: the pass begins within one and may end within one
+    const int lead = ONE ? 0 : k0 % WARPS;
+    auto group_ends = [&](int kz) { return kz < Kc && (kz + WARPS <= Kc || k0 + Kc == g.K); };  // in this pass
+    for (int base = -lead, round = 0; base < Kc; base += WARPS * Z, ++round) {
+        const int kk = base + zr * WARPS + warp, k = k0 + kk;
+        bool counts = true;
+        if constexpr (ONE) {
+            if (kk >= Kc) break;
+            if (!dir_qualifies(g, ep, cnt, k, rec)) continue;
+            if (cnt[k] > g.cap || cnt[g.K + k] > g.cap) continue;
+        } else {
+            counts = kk >= 0 && kk < Kc && dir_qualifies(g, ep, cnt, k, rec) && cnt[k] <= g.cap && cnt[g.K + k] <= g.cap;
+            if (!counts)
+                for (int j = 0; j < SPL; ++j) accs[(s_first + j) * G + cc] = R(0.0f);
+        }
+        for (int env = 0; counts && env < 2; ++env) {
             const size_t slot = (size_t)env * Kc + kk;
             const int* wp = wpref + slot * (g.W + 1);
             const uint32_t* b = bits + slot * g.W;
@@ -1364,11 +1397,11 @@ k_eval_w(const XT* __restrict__ X, XT* __restrict__ Xout, R* __restrict__ acc_bu
                         us[idx] = v;
                     } else {
                         const R uu = us[idx];
-                        accs[idx] = add_(accs[idx], add_(uu, v));
+                        accs[idx] = ONE ? add_(accs[idx], add_(uu, v)) : add_(uu, v);
                         us[idx] = sub_(uu, v);
                     }
                 } else {
-                    accs[idx] = add_(accs[idx], v);
+                    accs[idx] = ONE || env == 1 ? add_(accs[idx], v) : v;
                 }
                 if (kw & 1u) {  // a knot here: the next sample is in the next interval
                     if (lag) lag = false;
@@ -1400,32 +1433,56 @@ k_eval_w(const XT* __restrict__ X, XT* __restrict__ Xout, R* __restrict__ acc_bu
                 }
             }
         }
-    }
-    // the tile's CTAs (a cluster along z) have their partial sums ready; each
-    // adds them up, in the order of the warps over all of them, for its share
-    // of the tile
-    if (!ONE && Z > 1) cg_::this_cluster().sync();
-    else __syncthreads();
+        if constexpr (!ONE) {
+            // the CTA's group
+            R* gs = reinterpret_cast<R*>(smem_raw + WARPS * PW) + (round & 1) * T * G;
+            const int kz = base + zr * WARPS;
+            __syncthreads();
 #pragma unroll
-    for (int q = 0; q < EPT; ++q) {
-        const int idx = threadIdx.x + q * 32 * WARPS;
-        if (idx >= T * G || (Z > 1 && (idx >> 5) % Z != zr)) continue;
-        R tot = tots[q];
-        if (z0 == 0 && !first_chunk) {
-            const int t = idx / G, cch = cg * G + (idx - t * G);
-            if (t < nl && cch < C) tot = acc_buf[(size_t)(n0 + t) * C + cch];
-        }
-        for (int z = 0; z < Z; ++z) {
-            const unsigned char* base = !ONE && Z > 1 ? cg_::this_cluster().map_shared_rank(smem_raw, z) : smem_raw;
+            for (int q = 0; q < EPT; ++q) {
+                const int idx = threadIdx.x + q * 32 * WARPS;
+                if (idx >= T * G) continue;
+                R v[WARPS];
 #pragma unroll
-            for (int w = 0; w < WARPS; ++w) tot = add_(tot, reinterpret_cast<const R*>(base + (size_t)w * PW)[idx]);
+                for (int w = 0; w < WARPS; ++w) v[w] = reinterpret_cast<const R*>(smem_raw + (size_t)w * PW)[idx];
+                size_t off;
+                R sum = R(0.0f);
+                if (kz < 0 && offset(idx, off)) sum = acc_buf[CL + off];
+#pragma unroll
+                for (int w = 0; w < WARPS; ++w) sum = add_(sum, v[w]);
+                if (Z > 1) gs[idx] = sum;
+                else if (group_ends(kz)) tots[q] = add_(tots[q], sum);
+                if (!group_ends(kz) && kz < Kc && offset(idx, off)) acc_buf[CL + off] = sum;
+            }
+            // the groups of the round, in order, each CTA for its share of the tile (the
+            // next round's go to the other half: one barrier a round)
+            if (Z > 1) {
+                cg_::this_cluster().sync();
+#pragma unroll
+                for (int q = 0; q < EPT; ++q) {
+                    const int idx = threadIdx.x + q * 32 * WARPS;
+                    if (!share(idx)) continue;
+                    for (int z = 0; z < Z; ++z)
+                        if (group_ends(base + z * WARPS)) tots[q] = add_(tots[q], cg_::this_cluster().map_shared_rank(gs, z)[idx]);
+                }
+            } else {
+                __syncthreads();
+            }
         }
-        tots[q] = tot;
     }
-    // the next slice reuses the sums, and no CTA ends while others read them
-    if (!ONE && Z > 1) cg_::this_cluster().sync();
-    else if (z0 + Z < NZ) __syncthreads();
-    }  // slices
+    if (Z > 1) cg_::this_cluster().sync();  // no CTA ends while others read its sums
+    if constexpr (ONE) {
+        __syncthreads();
+        earlier_passes();  // (here: the loop has no registers to spare)
+#pragma unroll
+        for (int q = 0; q < EPT; ++q) {
+            const int idx = threadIdx.x + q * 32 * WARPS;
+            if (!share(idx)) continue;
+#pragma unroll
+            for (int w = 0; w < WARPS; ++w)
+                tots[q] = add_(tots[q], reinterpret_cast<const R*>(smem_raw + (size_t)w * PW)[idx]);
+        }
+    }
     if (overflow) atomicOr(&st->flags, 2);
     const int Q = sQ;
     if (!M && last_chunk && Q == 0 && (blockIdx.x == 0 || ep.n > 0) && blockIdx.y == 0 && threadIdx.x == 0)
@@ -1433,11 +1490,9 @@ k_eval_w(const XT* __restrict__ X, XT* __restrict__ Xout, R* __restrict__ acc_bu
 #pragma unroll
     for (int q = 0; q < EPT; ++q) {
         const int idx = threadIdx.x + q * 32 * WARPS;
-        if (idx >= T * G || (Z > 1 && (idx >> 5) % Z != zr)) continue;
-        const int t = idx / G, ch = idx - t * G;
-        const int cch = cg * G + ch;
-        if (t >= nl || cch >= C) continue;
-        const size_t off = (size_t)(n0 + t) * C + cch;
+        if (!share(idx)) continue;
+        size_t off;
+        if (!offset(idx, off)) continue;
         if (last_chunk) {
             const R mval = div_(mul_(tots[q], R(0.5f)), R(Q));
             if (M) M[off] = mval;
