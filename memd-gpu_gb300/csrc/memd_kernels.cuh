@@ -1452,7 +1452,7 @@ k_eval_w(const XT* __restrict__ X, XT* __restrict__ Xout, R* __restrict__ acc_bu
                 for (int w = 0; w < WARPS; ++w) sum = add_(sum, v[w]);
                 if (Z > 1) gs[idx] = sum;
                 else if (group_ends(kz)) tots[q] = add_(tots[q], sum);
-                if (!group_ends(kz) && kz < Kc && offset(idx, off)) acc_buf[CL + off] = sum;
+                else if (offset(idx, off)) acc_buf[CL + off] = sum;
             }
             // the groups of the round, in order, each CTA for its share of the tile (the
             // next round's go to the other half: one barrier a round)
@@ -1464,6 +1464,14 @@ k_eval_w(const XT* __restrict__ X, XT* __restrict__ Xout, R* __restrict__ acc_bu
                     if (!share(idx)) continue;
                     for (int z = 0; z < Z; ++z)
                         if (group_ends(base + z * WARPS)) tots[q] = add_(tots[q], cg_::this_cluster().map_shared_rank(gs, z)[idx]);
+                }
+                if (!group_ends(kz) && kz < Kc) {  // (now that the tile's first CTA has read the pass before's)
+#pragma unroll
+                    for (int q = 0; q < EPT; ++q) {
+                        const int idx = threadIdx.x + q * 32 * WARPS;
+                        size_t off;
+                        if (offset(idx, off)) acc_buf[CL + off] = gs[idx];
+                    }
                 }
             } else {
                 __syncthreads();
