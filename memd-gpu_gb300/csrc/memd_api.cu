@@ -1323,16 +1323,16 @@ static memd_status create_plan(const memd_config* cfg, const memd_tuning* tun, m
         p->Kc = std::max(1, std::min({K, fit, kc_limit}));
     }
     p->Kc = std::min(p->Kc, 1024);
-    // (in FP32 the segments' length shows in the last bits: it stays)
+    // segment lengths go by all directions, not by a pass's, so that how many
+    // passes the memory allows does not show in a result (in FP32 the segments'
+    // length shows in the last bits: one rule for every launch)
     if (c.solve_window >= 0 && !tu.factor_segment && c.precision != MEMD_PREC_F32)
-        p->Sl = kFacShortRows / (2 * p->Kc);
+        p->Sl = kFacShortRows / (2 * K);
     *kc_used = p->Kc;
     p->nchunks = (K + p->Kc - 1) / p->Kc;
     p->GS = 32;  // solve: one warp per (envelope, direction, segment, 32 channels)
     p->ngroups = (C + 31) / 32;
-    // (FP32 keeps one rule for every launch: where a window starts may show in
-    // its last bits)
-    p->sg.slots = c.precision == MEMD_PREC_F32 ? 256 : std::max(256, 2 * p->Kc * p->ngroups);
+    p->sg.slots = c.precision == MEMD_PREC_F32 ? 256 : std::max(256, 2 * K * p->ngroups);
     {
         // the factorisation and substitution kernels index their threads in 32 bits
         const double nfac = 2.0 * p->Kc * (double)fac_segments_max(p->g.cap, p->Sf, p->Sl);

@@ -356,8 +356,8 @@ k_compact(const uint32_t* __restrict__ bits, int* __restrict__ wpref, int* __res
 // on a few long chains: shorter segments repeat more warm-up and end sooner.
 // FP64, a warp alone on its SM: ~105 clocks an operation, 7 a warm-up row and
 // 11 an own row, 344 for 24 + 16 rows and 212 for 24 + 4; but at 16 clocks of
-// the SM's pipe each, 2 Kc E rows in segments of 4 cost 2.5 times the pipe time
-// of 16, and the two meet at 2 Kc E = 150,000 .. 300,000.  Measured with the
+// the SM's pipe each, 2 K E rows in segments of 4 cost 2.5 times the pipe time
+// of 16, and the two meet at 2 K E = 150,000 .. 300,000.  Measured with the
 // limit at 0 / 75,000 / 150,000 / 300,000 / 600,000: 4 x 1,000 3.64 / 3.26 / 3.26
 // / 3.26 / 3.27 ms; 19 x 7,501 not-a-knot 15.25 / 14.57 / 14.40 / 14.40 / 14.41;
 // 8 x 2,000 stop 7.82 / 7.41 / 7.37 / 7.37 / 7.38; 32 x 30,504 x 64 43.89 / 43.55
@@ -607,7 +607,7 @@ struct SolveItem {
 struct Segs {
     int S, Ss;  // longest, shortest (powers of two)
     int H;      // halo (< 0: one window over all)
-    int slots;  // systems x channel groups of a launch, 256 at least
+    int slots;  // systems x channel groups over all directions, 256 at least
 };
 
 // The fewest knots a system must exceed for segments of t: enough that a launch
