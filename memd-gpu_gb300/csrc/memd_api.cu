@@ -1397,10 +1397,8 @@ static memd_status create_plan(const memd_config* cfg, const memd_tuning* tun, m
     if (c.stop_mode == MEMD_STOP_FIXED) ALLOC(p->Xb, (size_t)p->xbytes * CL);
     ALLOC(p->run, (size_t)p->xbytes * CL);
     ALLOC(p->dir, 8 * (size_t)K * C);
-    // several passes: FP64 impulse mean, the exact 128-bit sum; FP64 and mixed direct evaluation, the total and the sum of
-    // a group that a pass ends in
-    if (p->nchunks > 1)
-        ALLOC(p->acc, (p->cum ? (f64 ? 16 : rb) : rb * (c.precision != MEMD_PREC_F32 && p->Kc % kEvalWarps ? 2 : 1)) * CL);
+    // several passes, FP64: the exact 128-bit sum, or the total and the sum of a group that a pass ends in
+    if (p->nchunks > 1) ALLOC(p->acc, (f64 && (p->cum || p->Kc % kEvalWarps) ? 16 : rb) * CL);
     ALLOC(p->imf, (size_t)p->tbytes * CL * (size_t)c.num_imfs);
     ALLOC(p->bits, sizeof(uint32_t) * 2 * Kc * p->g.W);
     ALLOC(p->wpref, sizeof(int) * 2 * Kc * (p->g.W + 1));

@@ -1152,13 +1152,20 @@ __device__ __forceinline__ void mirror_positions(const int* __restrict__ mi, con
 //   a = y_i, b = (y_{i+1}-y_i)/h - h(2 s_i + s_{i+1})/3, c = s_i,
 //   d = (s_{i+1} - s_i)/(3h)
 // when the interval changes.  The sum over qualified directions (E_max > 3 &&
-// E_min > 3), FP32: each warp's directions in order, then the warps' partial
-// sums in warp order.  FP64 and double-float: in order within groups of WARPS
-// directions, counted over all passes, and the groups' sums in order, so that
-// neither the passes nor the CTAs per tile (a record alone or in a batch) show
-// in the result; a warp leaves its direction's values in shared memory, a CTA
-// adds up a group at a time.  The last chunk applies X -= (sum/2)/Q
-// (REF:832-864).
+// E_min > 3):
+//   FP32          each warp's directions in order, then the warps' partial sums
+//                 in warp order
+//   double-float  the same, over four slices of the pass's directions whatever
+//                 the CTAs per tile, so that a record alone and in a batch give
+//                 the same
+//   FP64          in order within groups of WARPS directions, counted over all
+//                 passes, and the groups' sums in order, so that the passes do
+//                 not show in the result either; a warp leaves its direction's
+//                 values in shared memory, a CTA adds up a group at a time
+// The last chunk applies X -= (sum/2)/Q (REF:832-864).
+// The order is more than a matter of the last place: where all envelopes agree
+// (a record's clamped end), the stop rule asks whether the mean of equal values
+// came out as that value.
 // X is float (FP32 path), float2 (double-float, mixed path) or double.
 // The tile is as long as still gives three CTAs per SM (32 samples at least),
 // and the
@@ -1185,16 +1192,16 @@ struct EvalWShape {
     static constexpr int T = NS * SPL;
     static constexpr int MI = T / 2 + 4;
     static constexpr int NW = T / 32;
-    // per warp: its sums (FP32) or its direction's values of the tile, (stop mode) spread tile, knots and the rows
+    // per warp: its sums or (FP64) its direction's values of the tile, (stop mode) spread tile, knots and the rows
     // of their values, bit words
     __host__ __device__ static constexpr size_t per_warp(bool stopm)
     {
         return (size_t)(stopm ? 2 : 1) * sizeof(R) * T * G + 2 * sizeof(int) * (MI + 1) + sizeof(uint32_t) * (NW + 1);
     }
-    // several CTAs per tile: and the groups' sums of a round and the one before
+    // FP64, several CTAs per tile: and the groups' sums of a round and the one before
     static constexpr size_t smem_bytes(bool stopm, int Z)
     {
-        return WARPS * ((per_warp(stopm) + 15) / 16 * 16) + (Z > 1 ? 2 * sizeof(R) * T * G : 0);
+        return WARPS * ((per_warp(stopm) + 15) / 16 * 16) + (std::is_same<R, double>::value && Z > 1 ? 2 * sizeof(R) * T * G : 0);
     }
 };
 
@@ -1251,7 +1258,7 @@ k_eval_w(const XT* __restrict__ X, XT* __restrict__ Xout, R* __restrict__ acc_bu
     bool overflow = false;
 
     // Z CTAs per tile (FP32: one) take the directions in turn, a warp each
-    constexpr bool ONE = std::is_same<R, float>::value;
+    constexpr bool ONE = std::is_same<R, float>::value, GRP = std::is_same<R, double>::value;
     namespace cg_ = cooperative_groups;
     const int Z = ONE ? 1 : (int)gridDim.z, zr = ONE ? 0 : (int)blockIdx.z;
     constexpr int EPT = (T * G + 32 * WARPS - 1) / (32 * WARPS);  // tile elements per thread
@@ -1273,23 +1280,26 @@ k_eval_w(const XT* __restrict__ X, XT* __restrict__ Xout, R* __restrict__ acc_bu
             tots[q] = !first_chunk && share(idx) && offset(idx, off) ? acc_buf[off] : R(0.0f);
         }
     };
-    if constexpr (!ONE) earlier_passes();
-    if constexpr (ONE)
-        for (int j = 0; j < SPL; ++j) accs[(s_first + j) * G + cc] = R(0.0f);
+    if constexpr (GRP) earlier_passes();
     // groups start at multiples of WARPS of all directions: the pass begins within one and may end within one
-    const int lead = ONE ? 0 : k0 % WARPS;
+    const int lead = GRP ? k0 % WARPS : 0;
     auto group_ends = [&](int kz) { return kz < Kc && (kz + WARPS <= Kc || k0 + Kc == g.K); };  // in this pass
-    for (int base = -lead, round = 0; base < Kc; base += WARPS * Z, ++round) {
+    // slices (double-float; Z divides 4, and is 1 where Kc has fewer than eight directions a slice for it)
+    const int NZ = GRP || ONE ? 1 : min(4, (Kc + WARPS - 1) / WARPS);
+    for (int z0 = 0; z0 < NZ; z0 += Z) {
+    if constexpr (!GRP)
+        for (int j = 0; j < SPL; ++j) accs[(s_first + j) * G + cc] = R(0.0f);
+    for (int base = GRP ? -lead : z0 * WARPS, round = 0; base < Kc; base += WARPS * (GRP ? Z : NZ), ++round) {
         const int kk = base + zr * WARPS + warp, k = k0 + kk;
         bool counts = true;
-        if constexpr (ONE) {
-            if (kk >= Kc) break;
-            if (!dir_qualifies(g, ep, cnt, k, rec)) continue;
-            if (cnt[k] > g.cap || cnt[g.K + k] > g.cap) continue;
-        } else {
+        if constexpr (GRP) {
             counts = kk >= 0 && kk < Kc && dir_qualifies(g, ep, cnt, k, rec) && cnt[k] <= g.cap && cnt[g.K + k] <= g.cap;
             if (!counts)
                 for (int j = 0; j < SPL; ++j) accs[(s_first + j) * G + cc] = R(0.0f);
+        } else {
+            if (kk >= Kc) break;
+            if (!dir_qualifies(g, ep, cnt, k, rec)) continue;
+            if (cnt[k] > g.cap || cnt[g.K + k] > g.cap) continue;
         }
         for (int env = 0; counts && env < 2; ++env) {
             const size_t slot = (size_t)env * Kc + kk;
@@ -1397,11 +1407,11 @@ k_eval_w(const XT* __restrict__ X, XT* __restrict__ Xout, R* __restrict__ acc_bu
                         us[idx] = v;
                     } else {
                         const R uu = us[idx];
-                        accs[idx] = ONE ? add_(accs[idx], add_(uu, v)) : add_(uu, v);
+                        accs[idx] = GRP ? add_(uu, v) : add_(accs[idx], add_(uu, v));
                         us[idx] = sub_(uu, v);
                     }
                 } else {
-                    accs[idx] = ONE || env == 1 ? add_(accs[idx], v) : v;
+                    accs[idx] = GRP && env == 0 ? v : add_(accs[idx], v);
                 }
                 if (kw & 1u) {  // a knot here: the next sample is in the next interval
                     if (lag) lag = false;
@@ -1433,7 +1443,7 @@ k_eval_w(const XT* __restrict__ X, XT* __restrict__ Xout, R* __restrict__ acc_bu
                 }
             }
         }
-        if constexpr (!ONE) {
+        if constexpr (GRP) {
             // the CTA's group
             R* gs = reinterpret_cast<R*>(smem_raw + WARPS * PW) + (round & 1) * T * G;
             const int kz = base + zr * WARPS;
@@ -1478,19 +1488,26 @@ k_eval_w(const XT* __restrict__ X, XT* __restrict__ Xout, R* __restrict__ acc_bu
             }
         }
     }
-    if (Z > 1) cg_::this_cluster().sync();  // no CTA ends while others read its sums
-    if constexpr (ONE) {
-        __syncthreads();
-        earlier_passes();  // (here: the loop has no registers to spare)
+    if constexpr (!GRP) {
+        // the slice's partial sums, in the order of the warps, each CTA for its share of the tile
+        if (Z > 1) cg_::this_cluster().sync();
+        else __syncthreads();
+        if (z0 == 0) earlier_passes();  // (FP32: the loop has no registers to spare)
 #pragma unroll
         for (int q = 0; q < EPT; ++q) {
             const int idx = threadIdx.x + q * 32 * WARPS;
             if (!share(idx)) continue;
+            for (int z = 0; z < Z; ++z) {
+                const unsigned char* wz = Z > 1 ? cg_::this_cluster().map_shared_rank(smem_raw, z) : smem_raw;
 #pragma unroll
-            for (int w = 0; w < WARPS; ++w)
-                tots[q] = add_(tots[q], reinterpret_cast<const R*>(smem_raw + (size_t)w * PW)[idx]);
+                for (int w = 0; w < WARPS; ++w) tots[q] = add_(tots[q], reinterpret_cast<const R*>(wz + (size_t)w * PW)[idx]);
+            }
         }
+        if (Z == 1 && z0 + Z < NZ) __syncthreads();  // the next slice reuses the sums
     }
+    // ... and no CTA ends while others read its sums
+    if (Z > 1) cg_::this_cluster().sync();
+    }  // slices
     if (overflow) atomicOr(&st->flags, 2);
     const int Q = sQ;
     if (!M && last_chunk && Q == 0 && (blockIdx.x == 0 || ep.n > 0) && blockIdx.y == 0 && threadIdx.x == 0)
