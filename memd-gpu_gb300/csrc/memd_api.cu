@@ -103,6 +103,7 @@ struct memd_plan {
     int inplace;    // the backward sweep writes the solution over dbuf (dbuf == sv)
     int egroups; // evaluation channel groups
     uint32_t* bits;
+    size_t bits_stride;  // words from one pass's bitmasks to the next's (0: one pass's, used by all)
     int* wpref;
     int* knots;
     int* cnt;
@@ -409,8 +410,8 @@ static void enqueue_sift(memd_plan* p, cudaStream_t s, memd_trace_entry* trace, 
     const bool stop = p->cfg.stop_mode == MEMD_STOP_CRITERION;
     const int trace_rows = stop && trace ? (int)(p->cfg.num_imfs * (p->cfg.max_iter + 1)) : 0;
     // projection and extrema bitmasks of one direction pass; split: the signal's
-    // tf32 split first (once per sift)
-    auto project = [&](int k0, int kc, bool split) {
+    // tf32 split first (once per sift); tally: count the doubtful signs
+    auto project = [&](int k0, int kc, bool split, bool tally) {
         dim3 pg((unsigned)((g.L + kProjTN - 1) / kProjTN), (unsigned)((kc + kProjTK - 1) / kProjTK));
         lc.begin(MEMD_STAGE_PROJECT);
         if constexpr (P != MEMD_PREC_F32) {
@@ -432,7 +433,7 @@ static void enqueue_sift(memd_plan* p, cudaStream_t s, memd_trace_entry* trace, 
                 k_project_tc<XT><<<tg, kTcThreads, tc_smem_bytes(p->tc_nt), s>>>(
                     p->maps, (const XT*)p->X, P == MEMD_PREC_MIXED ? (const float*)p->dir : p->dfl, p->bits, g, k0, kc,
                     p->Cp, p->tc_nt, p->st, p->ep, P == MEMD_PREC_MIXED ? nullptr : (const double*)p->dir, p->xmx,
-                    p->xexp);
+                    p->xexp, tally);
                 lc.end(MEMD_STAGE_PROJECT);
                 return;
             }
@@ -447,13 +448,16 @@ static void enqueue_sift(memd_plan* p, cudaStream_t s, memd_trace_entry* trace, 
         lc.end(MEMD_STAGE_PROJECT);
     };
     const bool recount = P == MEMD_PREC_F64 && p->cum && p->nchunks > 1;
+    uint32_t* const bits0 = p->bits;
     if (recount) {
         // several passes: the knots of all directions first, which set the
-        // mean's anchor spacing, so that it does not depend on the passes
+        // mean's anchor spacing, so that it does not depend on the passes (the
+        // bitmasks are kept for the passes, if there was memory for all of them)
         cudaMemsetAsync(p->tot, 0, sizeof(unsigned long long) * (size_t)std::max(1, p->ep.n), s);
         for (int ch = 0; ch < p->nchunks; ++ch) {
             const int k0 = ch * p->Kc, kc = std::min(p->Kc, g.K - k0);
-            project(k0, kc, ch == 0);
+            if (p->bits_stride) p->bits = bits0 + p->bits_stride * (size_t)ch;
+            project(k0, kc, ch == 0, p->bits_stride > 0);
             lc.begin(MEMD_STAGE_COMPACT);
             k_count_knots<<<dim3((unsigned)((g.W + 4095) / 4096), (unsigned)(2 * kc)), 256, 0, s>>>(p->bits, p->tot, g,
                                                                                                    p->ep);
@@ -463,7 +467,8 @@ static void enqueue_sift(memd_plan* p, cudaStream_t s, memd_trace_entry* trace, 
     for (int ch = 0; ch < p->nchunks; ++ch) {
         const int k0 = ch * p->Kc;
         const int kc = std::min(p->Kc, g.K - k0);
-        project(k0, kc, ch == 0 && !recount);
+        if (p->bits_stride) p->bits = bits0 + p->bits_stride * (size_t)ch;
+        else project(k0, kc, ch == 0 && !recount, true);
         if (g.mirror) {
             const unsigned mb = (unsigned)((32L * kc + 127) / 128);
             lc.begin(MEMD_STAGE_PROJECT);
@@ -577,6 +582,7 @@ static void enqueue_sift(memd_plan* p, cudaStream_t s, memd_trace_entry* trace, 
             lc.end(MEMD_STAGE_OTHER);
         }
     }
+    p->bits = bits0;
     if (stop && p->batched) {
         RecStop* rs = (RecStop*)p->recstop;
         lc.begin(MEMD_STAGE_OTHER);
@@ -1400,7 +1406,6 @@ static memd_status create_plan(const memd_config* cfg, const memd_tuning* tun, m
     // several passes, FP64: the exact 128-bit sum, or the total and the sum of a group that a pass ends in
     if (p->nchunks > 1) ALLOC(p->acc, (f64 && (p->cum || p->Kc % kEvalWarps) ? 16 : rb) * CL);
     ALLOC(p->imf, (size_t)p->tbytes * CL * (size_t)c.num_imfs);
-    ALLOC(p->bits, sizeof(uint32_t) * 2 * Kc * p->g.W);
     ALLOC(p->wpref, sizeof(int) * 2 * Kc * (p->g.W + 1));
     ALLOC(p->knots, sizeof(int) * 2 * Kc * p->g.cap);
     ALLOC(p->cnt, sizeof(int) * 2 * (size_t)K);
@@ -1476,6 +1481,16 @@ static memd_status create_plan(const memd_config* cfg, const memd_tuning* tun, m
     }
     ALLOC(p->st, sizeof(RunState));
     ALLOC(p->coord_bad, sizeof(int));
+    if (p->cum && f64 && p->nchunks > 1 && st == MEMD_OK) {
+        // the bitmasks of all directions (L / 4 bytes each), as long as they take a
+        // tenth of what is left at most; else a pass's, projected again for the pass
+        const size_t stride = 2 * Kc * p->g.W, all = sizeof(uint32_t) * stride * (size_t)p->nchunks;
+        size_t fr = 0, tot = 0;
+        if (cudaMemGetInfo(&fr, &tot) == cudaSuccess && all <= fr / 10 && dev_alloc(p, (void**)&p->bits, all) == MEMD_OK)
+            p->bits_stride = stride;
+        cudaGetLastError();
+    }
+    if (!p->bits_stride) ALLOC(p->bits, sizeof(uint32_t) * 2 * Kc * p->g.W);
 #undef ALLOC
     if (st != MEMD_OK) {
         memd_plan_destroy(p);

@@ -272,7 +272,8 @@ template <typename XT>
 __global__ void __launch_bounds__(kTcThreads)
 k_project_tc(const __grid_constant__ TcMaps maps, const XT* __restrict__ X, const float* __restrict__ dh_all,
              uint32_t* __restrict__ bits, Geom g, int k0, int Kc, int Cp, int nt, RunState* st, Epochs ep,
-             const double* __restrict__ d_all, const float* __restrict__ xmx, const unsigned* __restrict__ xexp)
+             const double* __restrict__ d_all, const float* __restrict__ xmx, const unsigned* __restrict__ xexp,
+             bool tally)
 {
     // XT: float2 (mixed form) or double (FP64 form: d_all the FP64 directions,
     // dh_all their rounding to float, xmx and xexp from the split)
@@ -565,7 +566,7 @@ k_project_tc(const __grid_constant__ TcMaps maps, const XT* __restrict__ X, cons
         }
     }
     refined = warp_sum(refined);
-    if (lane == 0 && refined) atomicAdd(&st->pad[3], refined);
+    if (lane == 0 && refined && tally) atomicAdd(&st->pad[3], refined);
     tc_fence_before();
     __syncthreads();
     if (warp == 0) {
