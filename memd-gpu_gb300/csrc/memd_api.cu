@@ -769,9 +769,8 @@ static void split_directions(memd_plan* p, cudaStream_t s, Launches& lc)
     const size_t n = (size_t)p->g.K * p->Cp;
     const void* d = p->dir;
     if (p->prec == MEMD_PREC_F64) {
-        const int kc = p->g.K * p->g.C;
         lc.begin(MEMD_STAGE_OTHER);
-        k_float_directions<<<(unsigned)std::min((kc + 255) / 256, 1024), 256, 0, s>>>((const double*)p->dir, p->dfl, kc);
+        k_float_directions<<<(unsigned)((p->g.K + 7) / 8), 256, 0, s>>>((const double*)p->dir, p->dfl, p->g.K, p->g.C);
         lc.end(MEMD_STAGE_OTHER);
         d = p->dfl;
     }

@@ -48,8 +48,9 @@
 // the truncation of the differences (2^-23 S) and the directions' rounding to
 // float (2^-24 S), and a sign within it is decided again from those
 // projections themselves.  The differences are scaled by a power of two per
-// record (the exponent of its largest input sample), so that the float range
-// does not limit the signal's; whatever still leaves it is decided in FP64.
+// record (the exponent of its largest input sample) and the directions by one
+// each, so that the float range does not limit theirs; whatever still leaves it
+// is decided in FP64.
 // Rows equal to a neighbour in every channel need no decision.
 // 32 x 30,504, 64 directions: 132 us a sift with k_project_extrema (bound by
 // the FP64 pipe), 7 us split + 30 .. 37 us here.
@@ -195,10 +196,23 @@ k_split_tf32_f64(const double* __restrict__ X, const unsigned* __restrict__ xexp
     }
 }
 
-// FP64 directions rounded to float
-__global__ void k_float_directions(const double* __restrict__ d, float* __restrict__ f, int n)
+// FP64 directions rounded to float, each scaled by a power of two so that its
+// largest finite entry is in [1, 2) (the signs of its differences stay).  One
+// warp per direction.
+__global__ void k_float_directions(const double* __restrict__ d, float* __restrict__ f, int K, int C)
 {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) f[i] = (float)d[i];
+    const int k = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    if (k >= K) return;
+    d += (size_t)k * C;
+    int be = 0;
+    for (int c = lane; c < C; c += 32) {
+        int e = -1100;
+        if (isfinite(d[c]) && d[c] != 0.0) (void)frexp(d[c], &e);
+        be = c == lane ? e : max(be, e);
+    }
+    if (lane >= C) be = -1100;
+    be = (int)(__reduce_max_sync(kFull, (unsigned)(be + 2000))) - 2000;
+    for (int c = lane; c < C; c += 32) f[(size_t)k * C + c] = (float)ldexp(d[c], 1 - be);
 }
 
 struct TcMaps {
@@ -424,7 +438,8 @@ k_project_tc(const __grid_constant__ TcMaps maps, const XT* __restrict__ X, cons
                 for (int u = 0; u < DB; ++u) {
                     const int kk = kb0 + 4 * u;
                     float h = __fmul_rn(dv[u], xdl);
-                    float sh = __fmul_ru(fabsf(dv[u]), mxl);
+                    // (FP64: 2^-100 for an entry that a float flushed, far above 2^-126 / eps)
+                    float sh = __fmul_ru(F64 ? __fadd_ru(fabsf(dv[u]), 7.9e-31f) : fabsf(dv[u]), mxl);
 #pragma unroll
                     for (int o = 16; o > 0; o >>= 1) {
                         h = __fadd_rn(h, __shfl_xor_sync(kFull, h, o));
@@ -461,7 +476,9 @@ k_project_tc(const __grid_constant__ TcMaps maps, const XT* __restrict__ X, cons
     // the bound on |D_tc - D| per direction, with the margin for its own rounding
     {
         for (int kk = tid; kk < nk; kk += kTcThreads) {
-            if constexpr (F64) thr[kk] = __fmaf_ru(1.01f, thr[kk], 7.9e-31f);  // 2^-100: what underflow can hide
+            // FP64: plus 2^-100, what underflow can hide (entries below 2, scaled differences
+            // cut at 2^-126); no sign is certain where a product's partial sums might overflow
+            if constexpr (F64) thr[kk] = thr[kk] < eps * 8.5e37f ? __fmaf_ru(1.01f, thr[kk], 7.9e-31f) : INFINITY;
             else thr[kk] = 1.01f * __fmul_ru(eps, thr[kk]);
         }
     }
