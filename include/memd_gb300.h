@@ -189,7 +189,8 @@ typedef struct memd_plan memd_plan;
 typedef struct {
     int32_t solve_segment;      /* longest substitution segment in knots, a power of two in [32, 1024] (512, FP32 256) */
     int32_t solve_min_segment;  /* shortest substitution segment, a power of two in [16, solve_segment] (64) */
-    int32_t factor_segment;     /* factorisation rows per thread, 4 .. 256 (16; 8 or 4 for few knots) */
+    int32_t factor_segment;     /* factorisation rows per thread, 4 .. 256 (FP32 16; FP64 and mixed: 16, 8 or 4 by
+                                   the knots of each pass, reported as 0) */
     int32_t solve_queue;        /* substitution work: 1 = device work queue pulled by a persistent grid,
                                    2 or 0 = one warp per possible segment (the default) */
     int32_t mean_ctas;          /* impulse-accumulation mean: CTAs the split of spans over CTAs aims for,
@@ -209,7 +210,8 @@ void memd_default_config(memd_config* cfg);
 memd_status memd_plan_create(const memd_config* cfg, memd_plan** plan);
 /* memd_plan_create with explicit launch shapes (tuning may be NULL: defaults). */
 memd_status memd_plan_create_tuned(const memd_config* cfg, const memd_tuning* tuning, memd_plan** plan);
-/* The launch shapes a plan uses (the defaults filled in). */
+/* The launch shapes a plan uses (the defaults filled in, but for what it
+ * chooses by the data, which is 0): a plan made with them is the same plan. */
 memd_status memd_plan_get_tuning(const memd_plan* plan, memd_tuning* tuning);
 memd_status memd_plan_destroy(memd_plan* plan);
 /* Device bytes held by the plan. */

@@ -1175,7 +1175,7 @@ memd_status memd_plan_get_tuning(const memd_plan* p, memd_tuning* t)
     memset(t, 0, sizeof(*t));
     t->solve_segment = p->sg.S;
     t->solve_min_segment = p->sg.Ss;
-    t->factor_segment = p->Sf;
+    t->factor_segment = p->Sl > 0 ? 0 : p->Sf;
     t->solve_queue = p->squeue ? 1 : 2;
     t->mean_ctas = p->cum_ctas;
     t->proj_tile_n = p->tc ? p->tc_nt : 0;

@@ -81,16 +81,18 @@ def store(key: str, choice: dict, meta: dict, path: str | None = None) -> None:
 
 
 def search_space(precision: int, cum: bool) -> dict:
-    """Values tried per knob (0 = the default)."""
+    """Values tried per knob (0 = the form's default: segments of 512 knots at
+    most, FP32 256; factorisation rows by the knots, FP32 16)."""
+    f32 = int(precision) == 1
     space = {
-        "solve_segment": [0, 128, 256],
+        "solve_segment": [0, 128, 512 if f32 else 256],
         "solve_min_segment": [0, 32, 128],
         "factor_segment": [0, 8, 32],
         "solve_queue": [0, 1],
     }
     if cum:
         space["mean_ctas"] = [0, 1024, 4096]
-    if int(precision) == 2:
+    if not f32:
         space["proj_tile_n"] = [0, 32, 128]
     return space
 
