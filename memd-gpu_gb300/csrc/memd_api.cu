@@ -1327,6 +1327,13 @@ static memd_status create_plan(const memd_config* cfg, const memd_tuning* tun, m
         const int fit = directions_that_fit(c, p->g, p->real_bytes, p->xbytes, p->tbytes, want_inplace);
         p->Kc = std::max(1, std::min({K, fit, kc_limit}));
     }
+    {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        p->sms = 0;
+        cudaDeviceGetAttribute(&p->sms, cudaDevAttrMultiProcessorCount, dev);
+        if (p->sms < 1) p->sms = 1;
+    }
     p->Kc = std::min(p->Kc, 1024);
     // segment lengths go by all directions, not by a pass's, so that how many
     // passes the memory allows does not show in a result (in FP32 the segments'
@@ -1362,11 +1369,12 @@ static memd_status create_plan(const memd_config* cfg, const memd_tuning* tun, m
         auto tiles = [&](int spl) { return (L + 32 / p->ewG * spl - 1) / (32 / p->ewG * spl) * groups; };
         p->ewSPL = f32 ? 32 : 16;
         p->ewW = kEvalWarps;
-        while (p->ewSPL > p->ewG && tiles(p->ewSPL) < 456) p->ewSPL /= 2;
+        const long resident = 3L * p->sms;
+        while (p->ewSPL > p->ewG && tiles(p->ewSPL) < resident) p->ewSPL /= 2;
         p->ewZ = 1;
         if (!f32 && p->ewSPL == p->ewG) {
             const long t = tiles(p->ewSPL);
-            p->ewZ = t <= 114 && p->Kc >= 32 ? 4 : (t <= 228 && p->Kc >= 16 ? 2 : 1);
+            p->ewZ = 4 * t <= resident && p->Kc >= 4 * kEvalWarps ? 4 : (2 * t <= resident && p->Kc >= 2 * kEvalWarps ? 2 : 1);
         }
     }
     p->egroups = (C + p->ewG - 1) / p->ewG;
@@ -1504,13 +1512,6 @@ static memd_status create_plan(const memd_config* cfg, const memd_tuning* tun, m
             memd_plan_destroy(p);
             return set_error(MEMD_ERR_CUDA, "plan: TMA descriptors (cuTensorMapEncodeTiled) could not be made");
         }
-    }
-    {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        p->sms = 0;
-        cudaDeviceGetAttribute(&p->sms, cudaDevAttrMultiProcessorCount, dev);
-        if (p->sms < 1) p->sms = 1;
     }
     cudaError_t e = cudaMallocHost((void**)&p->host_flag, sizeof(int));
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&p->cap, cudaStreamNonBlocking);

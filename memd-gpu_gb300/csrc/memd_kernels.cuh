@@ -613,7 +613,8 @@ struct Segs {
 // The fewest knots a system must exceed for segments of t: enough that a launch
 // of such systems has 4096 warps, about what is resident at once (six CTAs of
 // four per SM), and at t = 512 four times that (with 4352, one wave and a
-// rest, 32 x 30,504 x 128 was slower than with 256).
+// rest, 32 x 30,504 x 128 was slower than with 256).  Numbers, not the device's
+// SM count: a result's last bits stay the same on every device.
 __host__ __device__ inline long seg_limit(int t, const Segs& sg)
 {
     return (t > 256 ? 4l : 1l) * 4096l * t / sg.slots;
