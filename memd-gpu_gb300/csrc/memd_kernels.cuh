@@ -1161,8 +1161,11 @@ __device__ __forceinline__ void mirror_positions(const int* __restrict__ mi, con
 //                 the same
 //   FP64          in order within groups of WARPS directions, counted over all
 //                 passes, and the groups' sums in order, so that the passes do
-//                 not show in the result either; a warp leaves its direction's
-//                 values in shared memory, a CTA adds up a group at a time
+//                 not show in the result either: of every WARPS full groups a
+//                 warp takes one; for the rest, and for tiles of several CTAs, a
+//                 warp leaves one direction's values in shared memory and the CTA
+//                 adds up the group (a barrier a group: 32 x 30,504, 64 directions
+//                 all so, 122 ms of evaluation against 115)
 // The last chunk applies X -= (sum/2)/Q (REF:832-864).
 // The order is more than a matter of the last place: where all envelopes agree
 // (a record's clamped end), the stop rule asks whether the mean of equal values
@@ -1193,16 +1196,17 @@ struct EvalWShape {
     static constexpr int T = NS * SPL;
     static constexpr int MI = T / 2 + 4;
     static constexpr int NW = T / 32;
-    // per warp: its sums or (FP64) its direction's values of the tile, (stop mode) spread tile, knots and the rows
-    // of their values, bit words
+    // per warp: its sums of the tile, (stop mode) the spread or (FP64) the upper envelope, knots and the rows of their
+    // values, bit words
+    static constexpr bool GRP = std::is_same<R, double>::value;
     __host__ __device__ static constexpr size_t per_warp(bool stopm)
     {
-        return (size_t)(stopm ? 2 : 1) * sizeof(R) * T * G + 2 * sizeof(int) * (MI + 1) + sizeof(uint32_t) * (NW + 1);
+        return (size_t)(stopm || GRP ? 2 : 1) * sizeof(R) * T * G + 2 * sizeof(int) * (MI + 1) + sizeof(uint32_t) * (NW + 1);
     }
     // FP64, several CTAs per tile: and the groups' sums of a round and the one before
     static constexpr size_t smem_bytes(bool stopm, int Z)
     {
-        return WARPS * ((per_warp(stopm) + 15) / 16 * 16) + (std::is_same<R, double>::value && Z > 1 ? 2 * sizeof(R) * T * G : 0);
+        return WARPS * ((per_warp(stopm) + 15) / 16 * 16) + (GRP && Z > 1 ? 2 * sizeof(R) * T * G : 0);
     }
 };
 
@@ -1240,9 +1244,10 @@ k_eval_w(const XT* __restrict__ X, XT* __restrict__ Xout, R* __restrict__ acc_bu
     const int cl = min(c, C - 1);  // loads of lanes past the last channel stay in bounds
     const int w0 = n0 >> 5;
     unsigned char* wb = smem_raw + (size_t)warp * PW;
-    R* accs = reinterpret_cast<R*>(wb);                        // [T][G], the warp's sums or its direction's values
-    R* us = accs + (STOPM ? T * G : 0);                        // [T][G] (stop mode): the spread U - L
-    int* kx = reinterpret_cast<int*>(accs + (STOPM ? 2 : 1) * T * G);  // knots
+    constexpr bool ONE = std::is_same<R, float>::value, GRP = Sh::GRP;
+    R* accs = reinterpret_cast<R*>(wb);                        // [T][G], the warp's sums
+    R* us = accs + (STOPM || GRP ? T * G : 0);                 // [T][G]: U, then (stop mode) the spread U - L
+    int* kx = reinterpret_cast<int*>(accs + (STOPM || GRP ? 2 : 1) * T * G);  // knots
     int* ks = kx + MI + 1;                                     // the rows of their values
     uint32_t* wd = reinterpret_cast<uint32_t*>(ks + MI + 1);   // bit words
     if (warp == 0) {
@@ -1259,7 +1264,6 @@ k_eval_w(const XT* __restrict__ X, XT* __restrict__ Xout, R* __restrict__ acc_bu
     bool overflow = false;
 
     // Z CTAs per tile (FP32: one) take the directions in turn, a warp each
-    constexpr bool ONE = std::is_same<R, float>::value, GRP = std::is_same<R, double>::value;
     namespace cg_ = cooperative_groups;
     const int Z = ONE ? 1 : (int)gridDim.z, zr = ONE ? 0 : (int)blockIdx.z;
     constexpr int EPT = (T * G + 32 * WARPS - 1) / (32 * WARPS);  // tile elements per thread
@@ -1290,19 +1294,16 @@ k_eval_w(const XT* __restrict__ X, XT* __restrict__ Xout, R* __restrict__ acc_bu
     for (int z0 = 0; z0 < NZ; z0 += Z) {
     if constexpr (!GRP)
         for (int j = 0; j < SPL; ++j) accs[(s_first + j) * G + cc] = R(0.0f);
-    for (int base = GRP ? -lead : z0 * WARPS, round = 0; base < Kc; base += WARPS * (GRP ? Z : NZ), ++round) {
-        const int kk = base + zr * WARPS + warp, k = k0 + kk;
-        bool counts = true;
-        if constexpr (GRP) {
-            counts = kk >= 0 && kk < Kc && dir_qualifies(g, ep, cnt, k, rec) && cnt[k] <= g.cap && cnt[g.K + k] <= g.cap;
-            if (!counts)
-                for (int j = 0; j < SPL; ++j) accs[(s_first + j) * G + cc] = R(0.0f);
-        } else {
-            if (kk >= Kc) break;
-            if (!dir_qualifies(g, ep, cnt, k, rec)) continue;
-            if (cnt[k] > g.cap || cnt[g.K + k] > g.cap) continue;
-        }
-        for (int env = 0; counts && env < 2; ++env) {
+    for (int base = GRP ? -lead : z0 * WARPS, round = 0, each = 1; base < Kc; base += WARPS * (GRP ? Z * each : NZ), ++round) {
+    // FP64, one CTA per tile: a group per warp while there is one for each
+    if constexpr (GRP) each = Z == 1 && base >= 0 && base + WARPS * WARPS <= Kc ? WARPS : 1;
+    bool begun = false;
+    for (int i = 0; i < (GRP ? each : 1); ++i) {
+        const int kk = GRP && each > 1 ? base + WARPS * warp + i : base + zr * WARPS + warp, k = k0 + kk;
+        if ((GRP && kk < 0) || kk >= Kc) continue;
+        if (!dir_qualifies(g, ep, cnt, k, rec)) continue;
+        if (cnt[k] > g.cap || cnt[g.K + k] > g.cap) continue;
+        for (int env = 0; env < 2; ++env) {
             const size_t slot = (size_t)env * Kc + kk;
             const int* wp = wpref + slot * (g.W + 1);
             const uint32_t* b = bits + slot * g.W;
@@ -1403,16 +1404,17 @@ k_eval_w(const XT* __restrict__ X, XT* __restrict__ Xout, R* __restrict__ acc_bu
                     tf += 1.0f;  // exact
                 }
                 const int idx = (s_first + j) * G + cc;
-                if constexpr (STOPM) {
+                if constexpr (STOPM || GRP) {
                     if (env == 0) {
                         us[idx] = v;
                     } else {
                         const R uu = us[idx];
-                        accs[idx] = GRP ? add_(uu, v) : add_(accs[idx], add_(uu, v));
-                        us[idx] = sub_(uu, v);
+                        if (GRP && !begun) accs[idx] = add_(uu, v);
+                        else accs[idx] = add_(accs[idx], add_(uu, v));
+                        if constexpr (STOPM) us[idx] = sub_(uu, v);
                     }
                 } else {
-                    accs[idx] = GRP && env == 0 ? v : add_(accs[idx], v);
+                    accs[idx] = add_(accs[idx], v);
                 }
                 if (kw & 1u) {  // a knot here: the next sample is in the next interval
                     if (lag) lag = false;
@@ -1444,7 +1446,22 @@ k_eval_w(const XT* __restrict__ X, XT* __restrict__ Xout, R* __restrict__ acc_bu
                 }
             }
         }
-        if constexpr (GRP) {
+        begun = true;
+    }
+    if constexpr (GRP) {
+        if (!begun)
+            for (int j = 0; j < SPL; ++j) accs[(s_first + j) * G + cc] = R(0.0f);
+        if (each > 1) {  // the warps' groups, in order
+            __syncthreads();
+#pragma unroll
+            for (int q = 0; q < EPT; ++q) {
+                const int idx = threadIdx.x + q * 32 * WARPS;
+                if (idx >= T * G) continue;
+#pragma unroll
+                for (int w = 0; w < WARPS; ++w) tots[q] = add_(tots[q], reinterpret_cast<const R*>(smem_raw + (size_t)w * PW)[idx]);
+            }
+            __syncthreads();
+        } else {
             // the CTA's group
             R* gs = reinterpret_cast<R*>(smem_raw + WARPS * PW) + (round & 1) * T * G;
             const int kz = base + zr * WARPS;
@@ -1488,6 +1505,7 @@ k_eval_w(const XT* __restrict__ X, XT* __restrict__ Xout, R* __restrict__ acc_bu
                 __syncthreads();
             }
         }
+    }
     }
     if constexpr (!GRP) {
         // the slice's partial sums, in the order of the warps, each CTA for its share of the tile
