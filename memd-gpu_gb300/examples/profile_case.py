@@ -33,6 +33,8 @@ def main():
     ap.add_argument("--runs", type=int, default=1)
     ap.add_argument("--projection", default="auto", choices=["auto", "cuda-cores"],
                     help="mixed form: tensor-core (auto) or CUDA-core projection")
+    ap.add_argument("--mean-eval", type=int, default=0, choices=[0, 1],
+                    help="eeg32: 1 = direct evaluation of every envelope")
     ap.add_argument("--stages", action="store_true",
                     help="also print the per-stage times of one eager run (CUDA events per kernel)")
     a = ap.parse_args()
@@ -45,7 +47,7 @@ def main():
         C, L, K = 32, 30504, 128
         y = torch.as_tensor(mg.synth_eeg(C, L, 256.0, seed=0).astype(np.float32), dtype=tdt, device="cuda")
         d = mg.directions(C, K, dtype="f32").to(tdt)
-        plan = mg.Plan(C, L, K, 9, 10, precision=prec, projection=proj)
+        plan = mg.Plan(C, L, K, 9, 10, precision=prec, projection=proj, mean_eval=a.mean_eval)
         out = torch.empty((9, C, L), dtype=tdt, device="cuda")
         for _ in range(a.runs):
             st = plan.run(y, d, out)
