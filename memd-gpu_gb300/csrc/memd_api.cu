@@ -1173,9 +1173,10 @@ memd_status memd_plan_get_tuning(const memd_plan* p, memd_tuning* t)
     using namespace memd;
     if (!p || !t) return set_error(MEMD_ERR_INVALID, "get_tuning: null argument");
     memset(t, 0, sizeof(*t));
-    t->solve_segment = p->sg.S;
-    t->solve_min_segment = p->sg.Ss;
-    t->factor_segment = p->Sl > 0 ? 0 : p->Sf;
+    const bool whole = p->sg.H < 0;  // one window over all knots: no segments to choose
+    t->solve_segment = whole ? 0 : p->sg.S;
+    t->solve_min_segment = whole ? 0 : p->sg.Ss;
+    t->factor_segment = whole || p->Sl > 0 ? 0 : p->Sf;
     t->solve_queue = p->squeue ? 1 : 2;
     t->mean_ctas = p->cum_ctas;
     t->proj_tile_n = p->tc ? p->tc_nt : 0;

@@ -22,3 +22,13 @@ def test_a_plan_made_from_a_plans_tuning_is_the_same_plan(precision, tuning):
     assert t["factor_segment"] == fixed
     first.close()
     second.close()
+
+
+@pytest.mark.parametrize("precision", [mg.PREC_F64, mg.PREC_F32, mg.PREC_MIXED])
+def test_a_plan_without_segments_reports_none(precision):
+    first = mg.Plan(3, 9000, 8, 2, 2, precision, solve_window=-1)
+    t = first.tuning()
+    second = mg.Plan(3, 9000, 8, 2, 2, precision, solve_window=-1, tuning=t)
+    assert second.tuning() == t and t["solve_segment"] == t["solve_min_segment"] == t["factor_segment"] == 0
+    first.close()
+    second.close()
