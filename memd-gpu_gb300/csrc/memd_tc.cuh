@@ -51,9 +51,13 @@
 // record (the exponent of its largest input sample) and the directions by one
 // each, so that the float range does not limit theirs; whatever still leaves it
 // is decided in FP64.
-// Rows equal to a neighbour in every channel need no decision.
-// 32 x 30,504, 64 directions: 132 us a sift with k_project_extrema (bound by
-// the FP64 pipe), 7 us split + 30 .. 37 us here.
+// Rows equal to a neighbour in every channel need no decision.  A loud sample
+// makes every quiet one of its tile doubtful in every direction, so a decision
+// is a dot product a lane, its neighbours' taken from their lanes.
+// 32 x 30,504, 64 directions, all 80 sifts: 10.7 ms with k_project_extrema
+// (bound by the FP64 pipe), 3.1 here with the split; 15 samples 1e6 times as
+// loud 9.3, one channel 1e8 times as loud 9.4 (three dot products by one lane,
+// its loads one by one: 3.9, 19.0 and 17.4).
 //
 // Every wait on an mbarrier is bounded (iterations and clock); a wait that
 // runs out sets MEMD_FLAG_DEVICE_TIMEOUT in the run state, waits (bounded)
@@ -267,8 +271,20 @@ __device__ __noinline__ int warp_df_diff_sign(const float2* __restrict__ x1, con
 // the FP64 form's projection of one sample (k_project_extrema's sum)
 __device__ __forceinline__ double proj_f64(const double* __restrict__ x, const double* __restrict__ d, int C)
 {
+    constexpr int B = 8;  // loads per batch
     double a = 0.0;
-    for (int c = 0; c < C; ++c) a = __fma_rn(x[c], d[c], a);
+    int c = 0;
+    for (; c + B <= C; c += B) {
+        double xv[B], dv[B];
+#pragma unroll
+        for (int k = 0; k < B; ++k) {
+            xv[k] = x[c + k];
+            dv[k] = d[c + k];
+        }
+#pragma unroll
+        for (int k = 0; k < B; ++k) a = __fma_rn(xv[k], dv[k], a);
+    }
+    for (; c < C; ++c) a = __fma_rn(x[c], d[c], a);
     return a;
 }
 // are two rows the same in every channel (bits)?
@@ -533,18 +549,42 @@ k_project_tc(const __grid_constant__ TcMaps maps, const XT* __restrict__ X, cons
                                              same_rows(X + (size_t)(n + 1) * C, X + (size_t)n * C, C));
             if (flat > 0 && nearm) mxm = mnm = nearm = 0u;  // equal neighbours: no strict extremum in any direction
             anyj = __reduce_or_sync(kFull, nearm);
+            // up to 16 directions a time: a lane projects its own sample where it or a
+            // neighbour is doubtful, and takes the neighbours' from their lanes; the
+            // samples before and after the warp's are projected together beforehand,
+            // two lanes a direction
+            const int row0 = n0 + warp * 32;
+            const double* xe = X + (size_t)min(max(lane & 1 ? row0 + 32 : row0 - 1, 0), g.L - 1) * C;
+            const double* dj = d_all + (size_t)(k0 + kt0 + j0) * C;
             while (anyj) {
-                const int j = __ffs(anyj) - 1;
-                anyj &= anyj - 1u;
-                if ((nearm >> j) & 1u) {
-                    const double* dk = d_all + (size_t)(k0 + kt0 + j0 + j) * C;
-                    const double* xn = X + (size_t)n * C;
-                    const double a = proj_f64(xn - C, dk, C), b = proj_f64(xn, dk, C), e = proj_f64(xn + C, dk, C);
-                    const uint32_t bit = 1u << j;
-                    mxm = (b > a && b > e) ? (mxm | bit) : (mxm & ~bit);
-                    mnm = (b < a && b < e) ? (mnm | bit) : (mnm & ~bit);
+                int je = -1, q = 0;
+                uint32_t left = anyj;
+                for (; left && q < 16; ++q) {
+                    const int j = __ffs(left) - 1;
+                    left &= left - 1u;
+                    const uint32_t m = __ballot_sync(kFull, (nearm >> j) & 1u);
+                    if ((lane >> 1) == q && (lane & 1 ? m >> 31 : m & 1u)) je = j;
                 }
+                const double pe = je >= 0 ? proj_f64(xe, dj + (size_t)je * C, C) : 0.0;
                 __syncwarp();
+                for (int i = 0; i < q; ++i) {
+                    const int j = __ffs(anyj) - 1;
+                    anyj &= anyj - 1u;
+                    const bool near = (nearm >> j) & 1u;
+                    const uint32_t m = __ballot_sync(kFull, near);
+                    double b = 0.0;
+                    if (((m | m << 1 | m >> 1) >> lane) & 1u) b = proj_f64(X + (size_t)min(n, g.L - 1) * C, dj + (size_t)j * C, C);
+                    __syncwarp();
+                    double a = __shfl_up_sync(kFull, b, 1), e = __shfl_down_sync(kFull, b, 1);
+                    const double ea = __shfl_sync(kFull, pe, 2 * i), ee = __shfl_sync(kFull, pe, 2 * i + 1);
+                    if (lane == 0) a = ea;
+                    if (lane == 31) e = ee;
+                    if (near) {
+                        const uint32_t bit = 1u << j;
+                        mxm = (b > a && b > e) ? (mxm | bit) : (mxm & ~bit);
+                        mnm = (b < a && b < e) ? (mnm | bit) : (mnm & ~bit);
+                    }
+                }
             }
         } else while (anyj) {
             const int j = __ffs(anyj) - 1;

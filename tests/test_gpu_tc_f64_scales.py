@@ -81,3 +81,13 @@ def test_flushed_differences_times_large_entries(scale):
     y[1, 200:900] *= 2.0 ** -119
     d = np.stack([np.ones(K), rng.choice([-1.0, 1.0], K) * 2.0 ** -11 * rng.uniform(0.5, 2.0, K)], axis=1)
     same(y, d * scale)
+
+
+# a loud sample in every tile of 128: every quiet sample's sign is doubtful in every direction, at the warps' first and
+# last samples too; channel counts around the batches of eight loads, more and fewer directions than sixteen
+@pytest.mark.parametrize("C,K", [(1, 5), (7, 16), (8, 17), (33, 40), (20, 70)])
+def test_doubtful_signs_everywhere(C, K):
+    rng = np.random.default_rng([C, K])
+    y = rng.standard_normal((C, 1111))
+    y[:, 60::128] *= 1e9
+    same(y, oracle.directions(C, K))
