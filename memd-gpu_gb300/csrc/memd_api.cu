@@ -358,7 +358,7 @@ static void launch_eval(memd_plan* p, cudaStream_t s, int k0, int kc, int first,
             cudaLaunchKernelEx(&lc, kern, (const XT*)p->X, (XT*)p->Xb, (R*)p->acc, (const uint32_t*)p->bits, (const int*)p->wpref,
                                (const int*)p->knots, (const int*)p->cnt, (const R*)p->rtab, (const R*)p->sv,
                                (const R*)p->yend, g, k0, kc, first, last, p->st, stopm ? (R*)p->M : (R*)nullptr,
-                               stopm ? (R*)p->part : (R*)nullptr, (const int*)p->mir, p->ep);
+                               stopm ? (R*)p->part : (R*)nullptr, (const int*)p->mir, p->ep, 3 * p->sms);
         };
         if (stopm) go(k_eval_w<G, SPL, XT, R, true, W>);
         else go(k_eval_w<G, SPL, XT, R, false, W>);
@@ -1366,17 +1366,10 @@ static memd_status create_plan(const memd_config* cfg, const memd_tuning* tun, m
     {
         const bool f32 = c.precision == MEMD_PREC_F32;
         p->ewG = std::min(f32 ? 32 : 16, std::max(4, next_pow2(C)));
-        const long groups = (C + p->ewG - 1) / p->ewG;
-        auto tiles = [&](int spl) { return (L + 32 / p->ewG * spl - 1) / (32 / p->ewG * spl) * groups; };
-        p->ewSPL = f32 ? 32 : 16;
+        const int groups = (C + p->ewG - 1) / p->ewG, resident = 3 * p->sms;
         p->ewW = kEvalWarps;
-        const long resident = 3L * p->sms;
-        while (p->ewSPL > p->ewG && tiles(p->ewSPL) < resident) p->ewSPL /= 2;
-        p->ewZ = 1;
-        if (!f32 && p->ewSPL == p->ewG) {
-            const long t = tiles(p->ewSPL);
-            p->ewZ = 4 * t <= resident && p->Kc >= 4 * kEvalWarps ? 4 : (2 * t <= resident && p->Kc >= 2 * kEvalWarps ? 2 : 1);
-        }
+        p->ewSPL = eval_samples(f32 ? 32 : 16, p->ewG, groups, L, resident);
+        p->ewZ = f32 ? 1 : eval_ctas(16, p->ewG, groups, L, p->Kc, resident);
     }
     p->egroups = (C + p->ewG - 1) / p->ewG;
     // mean envelope: impulse accumulation for the FP64 and mixed forms in fixed

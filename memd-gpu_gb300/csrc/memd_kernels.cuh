@@ -1156,9 +1156,9 @@ __device__ __forceinline__ void mirror_positions(const int* __restrict__ mi, con
 // E_min > 3):
 //   FP32          each warp's directions in order, then the warps' partial sums
 //                 in warp order
-//   double-float  the same, over four slices of the pass's directions whatever
-//                 the CTAs per tile, so that a record alone and in a batch give
-//                 the same
+//   double-float  the same, over as many slices of the pass's directions as a
+//                 tile of the record has CTAs when it is alone, so that it gives
+//                 the same in a batch (whose tiles have no more CTAs each)
 //   FP64          in order within groups of WARPS directions, counted over all
 //                 passes, and the groups' sums in order, so that the passes do
 //                 not show in the result either: of every WARPS full groups a
@@ -1190,6 +1190,22 @@ __device__ __forceinline__ void mirror_positions(const int* __restrict__ mi, con
 // ---------------------------------------------------------------------------
 constexpr int kEvalWarps = 8;  // warps of a CTA
 
+// Samples per lane of a launch's tiles, at most spl: as many as still give
+// `resident` tiles (three CTAs per SM), G at least.
+__host__ __device__ inline int eval_samples(int spl, int G, int groups, int L, int resident)
+{
+    while (spl > G && (L + 32 / G * spl - 1) / (32 / G * spl) * groups < resident) spl /= 2;
+    return spl;
+}
+// CTAs per tile (FP64, double-float): 4, 2 or 1, as many as stay resident and
+// have a direction for each of their warps.
+__host__ __device__ inline int eval_ctas(int spl, int G, int groups, int L, int Kc, int resident)
+{
+    if (eval_samples(spl, G, groups, L, resident) > G) return 1;
+    const int t = (L + 31) / 32 * groups;  // tiles of 32 samples
+    return 4 * t <= resident && Kc >= 4 * kEvalWarps ? 4 : (2 * t <= resident && Kc >= 2 * kEvalWarps ? 2 : 1);
+}
+
 template <int G, int SPL, typename R, int WARPS>
 struct EvalWShape {
     static constexpr int NS = 32 / G;
@@ -1216,7 +1232,7 @@ k_eval_w(const XT* __restrict__ X, XT* __restrict__ Xout, R* __restrict__ acc_bu
          const int* __restrict__ wpref, const int* __restrict__ knots, const int* __restrict__ cnt,
          const R* __restrict__ rtab, const R* __restrict__ sv, const R* __restrict__ yend, Geom g,
          int k0, int Kc, int first_chunk, int last_chunk, RunState* st, R* __restrict__ M,
-         R* __restrict__ part, const int* __restrict__ mir, Epochs ep)
+         R* __restrict__ part, const int* __restrict__ mir, Epochs ep, int resident)
 {
     // Fixed mode: the last pass writes the updated signal to Xout (the tiles'
     // knots outside them are read from X).  Stop mode: it writes the mean to M.
@@ -1289,8 +1305,8 @@ k_eval_w(const XT* __restrict__ X, XT* __restrict__ Xout, R* __restrict__ acc_bu
     // groups start at multiples of WARPS of all directions: the pass begins within one and may end within one
     const int lead = GRP ? k0 % WARPS : 0;
     auto group_ends = [&](int kz) { return kz < Kc && (kz + WARPS <= Kc || k0 + Kc == g.K); };  // in this pass
-    // slices (double-float; Z divides 4, and is 1 where Kc has fewer than eight directions a slice for it)
-    const int NZ = GRP || ONE ? 1 : min(4, (Kc + WARPS - 1) / WARPS);
+    // slices (double-float): powers of two, Z at least
+    const int NZ = GRP || ONE ? 1 : max(Z, eval_ctas(16, G, (int)gridDim.y, rend - roff, Kc, resident));
     for (int z0 = 0; z0 < NZ; z0 += Z) {
     if constexpr (!GRP)
         for (int j = 0; j < SPL; ++j) accs[(s_first + j) * G + cc] = R(0.0f);

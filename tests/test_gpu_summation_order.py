@@ -40,8 +40,8 @@ def test_direct_evaluation_does_not_depend_on_the_passes(C, L, K, stop):
 
 @pytest.mark.parametrize("precision", [mg.PREC_F64, mg.PREC_MIXED])
 def test_direct_evaluation_of_a_batch_equals_its_records(precision):
-    C, K = 6, 40  # alone a record's tiles have four CTAs, in the batch one
-    lengths = [300 + 37 * e for e in range(40)]
+    C, K = 6, 40  # alone a record's tiles have four CTAs, the last two records' two and one; in the batch one
+    lengths = [300 + 37 * e for e in range(40)] + [4700, 9000]
     recs = [near_constant(C, n, 10 + e) for e, n in enumerate(lengths)]
     d = oracle.directions(C, K)
     tdt = torch.float64 if precision == mg.PREC_F64 else torch.float32
@@ -52,7 +52,7 @@ def test_direct_evaluation_of_a_batch_equals_its_records(precision):
     plan.run_batched(y, lengths, off, torch.as_tensor(d, dtype=tdt).cuda(), out)
     plan.close()
     out = out.cpu().numpy()
-    for e in (0, 7, 23, 39):
+    for e in (0, 7, 23, 39, 40, 41):
         n = lengths[e]
         got = out[2 * off[e]:2 * off[e] + 2 * C * n].reshape(2, C, n)
         assert np.array_equal(got, single(recs[e], d, 2, 2, precision, mean_eval=1)), e
